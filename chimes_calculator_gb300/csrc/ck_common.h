@@ -75,6 +75,10 @@ struct TupleRec {
     // DevParamSet::tc3 (3-body tuples) or tc4 (4-body tuples), in floats; -1
     // when absent
     int tc_off, tc_pad;
+    // fixed-point form (FP64; see FxStream): the tuple's stream in fx3 / fx4,
+    // its parts' boundaries and the power of two its coefficients are scaled by
+    int fx_off, fx_split[9];
+    double fx_amp;
     double rin[6], rout[6], lam[6], xavg[6], xdiff[6];
     // reciprocals for the factored kernels: 1/lam, 1/xdiff, and the cutoff's
     // 1/rc (cubic) or Tersoff threshold rc - f*rc and 1/(rc - threshold)
@@ -97,6 +101,32 @@ struct FactRow {
     int end;
 };
 constexpr int kFactMaxDim = 128;   // largest R^K and R^(P-K) kept in shared memory per cluster
+
+// Fixed-point coefficient streams of the FP64 form (ck_fixed.cuh).  A tuple's
+// coefficients are scaled by 2^-e, fx_amp = 2^e the smallest power of two with
+// sum |a| <= 0.9 fx_amp and max |a| <= 0.24 fx_amp, and kept at 2^kFxCoef as two
+// limbs {h, l}, a = h 2^kFxLimb + l.
+//   3-body (FxPair): per column J = (q_ik, q_jk) with coefficients, in ascending
+//   order, a header {q_ik | q_jk << 8, mask of its q_ij} and a coefficient per
+//   mask bit; fx_split[k], k = 0..8: eight parts of about equal work.
+//   4-body (FxEnt): the row entries {h, l, J | I's powers << 16, 1 at the
+//   row's last entry}, then the column entries likewise (columns and rows
+//   exchanged); fx_split[0..4] / [4..8]: four parts of the rows / columns.
+// Splits are offsets from fx_off, at record boundaries.
+struct __attribute__((aligned(8))) FxPair {
+    int x, y;
+};
+struct __attribute__((aligned(16))) FxEnt {
+    int h, l, code, last;
+};
+constexpr int kFxLimb = 28;
+constexpr int kFxCoef = 61;
+constexpr int kFxSum = 59;
+CK_HD constexpr int fx_kd(int R) {   // bits of (R - 1)^2: the dT tables' scale
+    int k = 0;
+    while ((1 << k) < (R - 1) * (R - 1)) k++;
+    return k;
+}
 
 // Tensor-core 3-body images (DevParamSet::tc3): with Rw powers per pair the
 // MMA's K is Rw padded to 8 or 16 and N = Rw^2 padded to 16; a tuple stores
@@ -200,6 +230,10 @@ struct DevParamSet {
     // table lengths, for the index checks of the checked build (CK_BOUNDS):
     // 3-/4-body coefficients, factored entries, tensor-core image floats
     long long n_c3, n_c4, n_fe3, n_fe4, n_tc3, n_tc4;
+    // fixed-point streams (FP64 form); fx3_max = longest 3-body stream
+    const FxPair* fx3; const FxEnt* fx4;
+    long long n_fx3, n_fx4;
+    int fx3_max, fx_pad;
     const FactRow* fr3; const FactEntD* fe3d; const FactEntF* fe3f;
     const FactRow* fr4; const FactEntD* fe4d; const FactEntF* fe4f;
     // per-pair-type tables [npairs] (null when some tuple's cutoffs differ by tuple)

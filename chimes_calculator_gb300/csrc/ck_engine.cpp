@@ -121,6 +121,7 @@ int Engine::load_params(const std::string& path, std::string& err) {
     rel(h.pt3); rel(h.pt4);
     rel(h.tc3);
     rel(h.tc4);
+    rel(h.fx3); rel(h.fx4);
     rel(h.t2rec); rel(h.tab2r); rel(h.tab2c);
     rel(h.t3rec); rel(h.tab3r); rel(h.tab3v);
     // this set's cluster buckets follow those of the sets loaded before it
@@ -158,7 +159,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     int stride3 = 0, stride4 = 0;
     bool fact3 = factored, fact4 = factored;
     bool pc3 = pair_cache, pc4 = pair_cache;
-    int rf3 = 0, rf4 = 0;
+    int rf3 = 0, rf4 = 0, xs3 = 0;
     bool tc3 = precision == kMixed, tc4 = precision == kMixed;
     int r4_lo = 1 << 30;   // the 4-body tensor-core kernel needs one R over the batch's sets
     bool enum_serial = false;
@@ -210,6 +211,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
         if (P.o3 > 0) {
             fact3 = fact3 && V.R3 > 0;
             rf3 = std::max(rf3, V.R3);
+            xs3 = std::max(xs3, V.fx3_max);
             pc3 = pc3 && V.pt3;
             tc3 = tc3 && V.tc3 != nullptr;
         }
@@ -255,6 +257,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     avail_pc4_ = avail_fact4_ && pc4 && !enum_serial && pc_size;
     tuning.rf3 = rf3;
     tuning.rf4 = rf4;
+    tuning.xs3 = xs3;
     V_ = BatchView();
     V_.n_sys = S;
     V_.n_in_total = in_off;
@@ -458,6 +461,10 @@ Status Engine::enqueue(std::string& err) {
             launch_pair_tables(B, d_l2_owner_.p, 3, L, q);
             launch_bucket(B, 3, q);
             launch_force3tc(B, L, q);
+        } else if (L.fact3 && L.precision == kFP64) {
+            launch_pair_tables_x(B, d_l2_owner_.p, 3, L, q);
+            launch_bucket(B, 3, q);
+            launch_force3x(B, L, q);
         } else if (L.fact3) {
             launch_pair_tables(B, d_l2_owner_.p, 3, L, q);
             launch_bucket(B, 3, q);
@@ -472,6 +479,10 @@ Status Engine::enqueue(std::string& err) {
         if (L.fact4 && L.tc4) {
             launch_bucket(B, 4, q);
             launch_force4tc(B, L, q);
+        } else if (L.fact4 && L.precision == kFP64) {
+            launch_pair_tables_x(B, d_l2_owner_.p, 4, L, q);
+            launch_bucket(B, 4, q);
+            launch_force4x(B, L, q);
         } else if (L.fact4) {
             launch_pair_tables(B, d_l2_owner_.p, 4, L, q);
             launch_bucket(B, 4, q);
@@ -533,7 +544,7 @@ Status Engine::launch(std::string& err) {
     std::vector<long long> key = {(long long)V_.n_sys, V_.n_in_total, V_.n_atoms_total, V_.n_ghost_total,
                                   V_.n_bins_total, n2_cap_, n3_cap_, n4_cap_, precision, tuning.tpc3, tuning.tpc4,
                                   tuning.stride3, tuning.stride4, tuning.blocks_per_sm, profile ? 1 : 0,
-                                  tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.ftpc3, tuning.ftpc4,
+                                  tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
                                   tuning.tc3, tuning.tc4};
     for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
@@ -716,18 +727,21 @@ Status Engine::autotune(int* chosen, std::string& err) {
     double a, b;
     Status st = run_once(a, b);   // warm-up and list sizing
     const bool do3 = tuning.stride3 > 0, do4 = tuning.stride4 > 0;
-    // candidates per body order: factored kernels (1, 2, 4 lanes per cluster)
-    // where the tables exist, then the per-coefficient kernels (1..32 lanes)
-    // (3-body factored also without its Y table).  The factored forms differ
+    // candidates per body order: factored kernels where the tables exist (FP64:
+    // 1, 2, 4 or 8 warps per 32 clusters; mixed: 1, 2, 4 lanes per cluster), then the per-coefficient kernels (1..32 lanes)
+    // (mixed 3-body factored also without its Y table).  Its factored forms differ
     // in shared memory per cluster, so each is tried at 8 and at up to 16
     // resident one-warp blocks per SM (capped by its occupancy); the per-SM
     // count is refined below.
     // (in the mixed form also the tensor-core contractions)
     struct Cand { int fact, tpc, noy, fbps, tc; };
-    auto cands = [](bool can_fact, bool with_noy, bool with_tc) {
+    const bool mixed = precision == kMixed;
+    auto cands = [mixed](bool can_fact, bool with_noy, bool with_tc) {
         std::vector<Cand> v;
         if (with_tc) v.push_back({1, 1, 0, 0, 1});
-        if (can_fact)
+        if (can_fact && !mixed)
+            for (int t : {1, 2, 4, 8}) v.push_back({1, t, 0, 0, 0});
+        if (can_fact && mixed)
             for (int t : {1, 2, 4})
                 for (int nf : {0, 1}) {
                     if (nf && !with_noy) continue;
@@ -776,8 +790,8 @@ Status Engine::autotune(int* chosen, std::string& err) {
     tuning.want_fact4 = b4.fact;
     tuning.want_tc3 = b3.tc;
     tuning.want_tc4 = b4.tc;
-    // (the tensor-core forms' occupancy is fixed by their shared memory)
-    const bool f3 = tuning.fact3 != 0 && !tuning.tc3, f4 = tuning.fact4 != 0 && !tuning.tc4;
+    // (the tensor-core and fixed-point forms always run at their full occupancy)
+    const bool f3 = mixed && tuning.fact3 != 0 && !tuning.tc3, f4 = mixed && tuning.fact4 != 0 && !tuning.tc4;
     // resident blocks per SM: 4-warp blocks for the per-coefficient kernels,
     // one-warp blocks for the factored ones (capped by their occupancy)
     const int bps[] = {1, 2, 4, 8};

@@ -1,6 +1,7 @@
-// Factored 3-body and 4-body contraction.
+// Factored 3-body and 4-body contraction of the mixed form (the FP64 form's is
+// ck_fixed.cu), and the bucketing of the clusters that both use.
 //
-// The per-coefficient form (k_forcen in ck_force.cu) spends about 2P+P FP64
+// The per-coefficient form (k_forcen in ck_force.cu) spends about 2P+P
 // operations on every coefficient term: the product of P Chebyshev values and
 // P gradient terms.  Here a cluster's pairs are split into row pairs (the
 // first K) and column pairs (the rest), and the coefficient list of each
@@ -17,8 +18,7 @@
 // bucket padded with -1 to a multiple of 32 slots, so every warp works on one
 // tuple: loop bounds and coefficient loads are uniform across the warp (the
 // loads are broadcasts).  TPC lanes share a cluster (TPC = 1, 2 or 4): one
-// lane streams both passes' entries; two lanes (FP64) take one pass each;
-// otherwise the lanes take whole records round robin.  Per-cluster tables
+// lane streams both passes' entries; more take whole records round robin.  Per-cluster tables
 // (T, dT/dr per pair, Y and X) sit in shared memory interleaved by cluster,
 // [entry][cluster].
 #include <cuda_runtime.h>
@@ -45,23 +45,10 @@ struct Split<4> {
     static constexpr int K = 3;
 };
 
-template <typename CT>
-struct EntOf;
-template <>
-struct EntOf<double> {
-    using type = FactEntD;
-};
-template <>
-struct EntOf<float> {
-    using type = FactEntF;
-};
-
-template <typename CT, int NB>
-__device__ __forceinline__ const typename EntOf<CT>::type* fact_ent(const DevParamSet& P);
-template <> __device__ __forceinline__ const FactEntD* fact_ent<double, 3>(const DevParamSet& P) { return P.fe3d; }
-template <> __device__ __forceinline__ const FactEntF* fact_ent<float, 3>(const DevParamSet& P) { return P.fe3f; }
-template <> __device__ __forceinline__ const FactEntD* fact_ent<double, 4>(const DevParamSet& P) { return P.fe4d; }
-template <> __device__ __forceinline__ const FactEntF* fact_ent<float, 4>(const DevParamSet& P) { return P.fe4f; }
+template <int NB>
+__device__ __forceinline__ const FactEntF* fact_ent(const DevParamSet& P) {
+    return NB == 3 ? P.fe3f : P.fe4f;
+}
 
 // sum over entries [e0, e1) taken by lane gl of TPC: a * V[idx]; eight
 // entries per round in two partial sums, so their loads overlap
@@ -89,24 +76,12 @@ __device__ __forceinline__ CT entry_sum(const E* __restrict__ ent, int e0, int e
 // One pass over the entries [e0, e1) of nrec consecutive records (TPC = 1):
 // z += a * V[idx] per entry; at an entry with the record-end bit (idx < 0)
 // flush(record powers, z) and start the next record.  Entries are loaded
-// eight (NOY: four) at a time regardless of where records end, so a short
-// record does not pay its own load latency.
-// The entry's multiplier is V[idx] (a table), or with NOY the product of the
-// two column pairs' values T1[q1] T2[q2] (powers in the entry's high bits).
-template <typename CT, int G, bool NOY, typename E>
-__device__ __forceinline__ CT entry_value(const E& q, const CT* V, const CT* T2, int grp) {
-    if constexpr (NOY) {
-        const int c = q.idx >> 16;
-        return V[(c & 31) * G + grp] * T2[((c >> kPowBits) & 31) * G + grp];
-    } else {
-        return V[(q.idx & 0xffff) * G + grp];
-    }
-}
-
-template <typename CT, int G, bool NOY = false, typename E, typename F>
+// eight at a time regardless of where records end, so a short record does not
+// pay its own load latency.
+template <typename CT, int G, typename E, typename F>
 __device__ __forceinline__ void flat_pass(const E* __restrict__ ent, int e0, int e1, const FactRow* rec, int nrec,
-                                          const CT* V, const CT* T2, int grp, F&& flush) {
-    constexpr int NBAT = NOY ? 4 : 8;   // the NOY form keeps fewer entries in flight (registers)
+                                          const CT* V, int grp, F&& flush) {
+    constexpr int NBAT = 8;
     CT z = CT(0);
     int r = 0;
     int pw = nrec > 0 ? rec[0].pows : 0;
@@ -118,7 +93,7 @@ __device__ __forceinline__ void flat_pass(const E* __restrict__ ent, int e0, int
             if (k + u < e1) q[u] = ent[k + u];
 #pragma unroll
         for (int u = 0; u < NBAT; u++)
-            if (k + u < e1) x[u] = entry_value<CT, G, NOY>(q[u], V, T2, grp);
+            if (k + u < e1) x[u] = V[(q[u].idx & 0xffff) * G + grp];
 #pragma unroll
         for (int u = 0; u < NBAT; u++)
             if (k + u < e1) {
@@ -489,7 +464,7 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
         }
         __syncwarp();
 
-        const auto* ent = fact_ent<CT, NB>(*P);
+        const FactEntF* ent = fact_ent<NB>(*P);
         const FactRow* rows = (NB == 3 ? P->fr3 : P->fr4) + R->f_row;
         int nrow = R->f_nrow, ncol = R->f_ncol;
         if (!ck_bound(B, R->f_ent >= 0 && R->f_ent + 2LL * R->ncoef <= (NB == 3 ? P->n_fe3 : P->n_fe4)))
@@ -629,28 +604,13 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
                 }
             }
         };
-        // (in FP32 the NOY form keeps its per-record loop: the one-stream form's
+        // (the NOY form keeps its per-record loop: the one-stream form's
         // registers cost it more resident warps than the batched loads save)
-        if constexpr (TPC == 1 && !(NOY && sizeof(CT) == 4)) {
+        if constexpr (TPC == 1 && !NOY) {
             // one lane per cluster: each pass is one stream of entries across
             // its records (loads batched across record ends)
-            if constexpr (NOY && NB == 3)
-                flat_pass<CT, G, true>(ent, R->f_ent, e_col0, rows, nrow, Tt + 1 * rs * G, Tt + 2 * rs * G, grp,
-                                       row_flush);
-            else
-                flat_pass<CT, G>(ent, R->f_ent, e_col0, rows, nrow, Y, nullptr, grp, row_flush);
-            flat_pass<CT, G>(ent, e_col0, e_col0 + R->ncoef, rows + nrow, ncol, Xv, nullptr, grp, col_flush);
-        } else if constexpr (TPC == 2 && !NOY && sizeof(CT) == 8) {
-            // two lanes per cluster (FP64): lane 0 streams the row entries, lane
-            // 1 the column entries (as many), each flushing its own records
-            // (4096-configuration batch, 4-body: 34.0 -> 31.7 ms; in FP32 the
-            // extra registers cost more than the whole runs save)
-            const bool colp = gl == 1;
-            flat_pass<CT, G>(ent, colp ? e_col0 : R->f_ent, colp ? e_col0 + R->ncoef : e_col0, colp ? rows + nrow : rows,
-                             colp ? ncol : nrow, colp ? Xv : Y, nullptr, grp, [&](int pw, CT z) {
-                                 if (colp) col_flush(pw, z);
-                                 else row_flush(pw, z);
-                             });
+            flat_pass<CT, G>(ent, R->f_ent, e_col0, rows, nrow, Y, grp, row_flush);
+            flat_pass<CT, G>(ent, e_col0, e_col0 + R->ncoef, rows + nrow, ncol, Xv, grp, col_flush);
         } else {
             // The TPC lanes of a cluster take whole records round robin
             // (adjacent records, adjacent loads), each flushing its own.  A
@@ -686,7 +646,7 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
 #pragma unroll
             for (int p = 0; p < NP; p++) Gp[p] += __shfl_xor_sync(kFull, Gp[p], off);
         }
-        if (sizeof(CT) == 4 && active && gl == 0) {   // mixed form: the epilogue in FP32
+        if (active && gl == 0) {   // the epilogue in FP32
             float drf[NP][3], rinv[NP], fcf[NP], fcdf[NP], Gf[NP];
             for (int p = 0; p < NP; p++) {
                 for (int k = 0; k < 3; k++) drf[p][k] = float(geo[(4 * p + k) * G + grp]);
@@ -698,15 +658,6 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
             double e_c, vir_c[6];
             cluster_epilogue_f32<NB>(B, id, drf, rinv, fcf, fcdf, float(S), Gf, e_c, vir_c);
             acc.add(B, s, e_c, vir_c);
-        } else if (active && gl == 0) {
-            double dr[NP][4], fc[NP], fcd[NP], Gd[NP];
-            for (int p = 0; p < NP; p++) {
-                for (int k = 0; k < 4; k++) dr[p][k] = geo[(4 * p + k) * G + grp];
-                fc[p] = fcs[p * G + grp];
-                fcd[p] = fcds[p * G + grp];
-                Gd[p] = double(Gp[p]);
-            }
-            cluster_epilogue<NB>(B, id, s, dr, fc, fcd, double(S), Gd, acc);
         }
         __syncwarp();
     }
@@ -791,12 +742,6 @@ void launch_bucket_n(const BatchView& B, cudaStream_t st) {
 
 }  // namespace
 
-size_t factored_smem_bytes(int nbody, int precision, int tpc, int rs) {
-    if (nbody == 3)
-        return precision == kMixed ? smem_bytes<3, float>(tpc, rs) : smem_bytes<3, double>(tpc, rs);
-    return precision == kMixed ? smem_bytes<4, float>(tpc, rs) : smem_bytes<4, double>(tpc, rs);
-}
-
 void launch_bucket(const BatchView& B, int nbody, cudaStream_t st) {
     if (nbody == 3) launch_bucket_n<3>(B, st);
     else launch_bucket_n<4>(B, st);
@@ -809,22 +754,18 @@ void launch_pair_tables(const BatchView& B, const int* l2_owner, int nbody, cons
     long long need = (B.n2_cap + 255) / 256;
     const unsigned grid = (unsigned)(want < need ? want : need);
     if (nbody == 3) {
-        if (L.precision == kMixed) count_launch(), k_pair_tables<3, float><<<grid, 256, 0, st>>>(B, l2_owner, rs);
-        else count_launch(), k_pair_tables<3, double><<<grid, 256, 0, st>>>(B, l2_owner, rs);
+        count_launch(), k_pair_tables<3, float><<<grid, 256, 0, st>>>(B, l2_owner, rs);
     } else {
-        if (L.precision == kMixed) count_launch(), k_pair_tables<4, float><<<grid, 256, 0, st>>>(B, l2_owner, rs);
-        else count_launch(), k_pair_tables<4, double><<<grid, 256, 0, st>>>(B, l2_owner, rs);
+        count_launch(), k_pair_tables<4, float><<<grid, 256, 0, st>>>(B, l2_owner, rs);
     }
 }
 
 void launch_force3f(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    if (L.precision == kMixed) launch_f<3, float>(B, L, st);
-    else launch_f<3, double>(B, L, st);
+    launch_f<3, float>(B, L, st);
 }
 
 void launch_force4f(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    if (L.precision == kMixed) launch_f<4, float>(B, L, st);
-    else launch_f<4, double>(B, L, st);
+    launch_f<4, float>(B, L, st);
 }
 
 }  // namespace ck

@@ -45,11 +45,12 @@ struct ForceLaunch {
     int fact3 = 0, fact4 = 0;
     int want_fact3 = 1, want_fact4 = 1;   // preference (autotuner); fact = want && tables present
     int rf3 = 0, rf4 = 0;  // powers per pair (max over the batch's sets)
-    // threads per cluster: 1, 2 or 4 (the 4-body default 4: what the autotuner
-    // picks on the FP64 workloads; untuned paths such as ck_nl_compute use it)
+    int xs3 = 0;           // longest 3-body fixed-point stream over the batch's sets (FP64 form)
+    // mixed form: threads per cluster, 1, 2 or 4; FP64 form (ck_fixed.cu):
+    // warps per 32 clusters, 1, 2, 4 or 8
     int ftpc3 = 1, ftpc4 = 4;
-    int fbps3 = 8, fbps4 = 8;      // resident one-warp blocks per SM (capped by occupancy)
-    int noy3 = 0;                  // factored 3-body without the Y table (products per entry)
+    int fbps3 = 8, fbps4 = 8;      // mixed form: resident one-warp blocks per SM (capped by occupancy)
+    int noy3 = 0;                  // mixed form: 3-body without the Y table (products per entry)
     // tensor-core 3-body contraction (mixed form only; ck_tensor.cu): tc3 = in
     // use for this launch, want_tc3 = preference (autotuner or forced)
     int tc3 = 0, want_tc3 = 0;
@@ -63,7 +64,7 @@ void launch_force2(const BatchView& B, const int* l2_owner, const ForceLaunch& L
 void launch_force3(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 
-// Factored contraction (ck_factored.cu): bucket the clusters of one body
+// Factored contraction of the mixed form (ck_factored.cu): bucket the clusters of one body
 // order by (parameter set, type tuple), then contract.  Both read their
 // counts on the device.
 void launch_bucket(const BatchView& B, int nbody, cudaStream_t st);
@@ -71,6 +72,10 @@ void launch_bucket(const BatchView& B, int nbody, cudaStream_t st);
 void launch_pair_tables(const BatchView& B, const int* l2_owner, int nbody, const ForceLaunch& L, cudaStream_t st);
 void launch_force3f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
+// The FP64 form of the factored contraction, in 64-bit fixed point (ck_fixed.cu).
+void launch_pair_tables_x(const BatchView& B, const int* l2_owner, int nbody, const ForceLaunch& L, cudaStream_t st);
+void launch_force3x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
+void launch_force4x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 // Tensor-core 3-body contraction (ck_tensor.cu): mixed form, R3 powers per
 // pair in [2, kTc3MaxR]; clusters bucketed with 128-slot padding (bk_pad3).
 bool tc3_supported(int rf3);
@@ -79,8 +84,6 @@ void launch_force3tc(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 // pair in [2, kTc4MaxR]; tiles of 32 clusters (the 4-body buckets' padding).
 bool tc4_supported(int rf4);
 void launch_force4tc(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
-// dynamic shared memory of one factored-kernel block (one warp)
-size_t factored_smem_bytes(int nbody, int precision, int tpc, int rs);
 
 // Pair-style path on a caller's neighbour list (ck_neigh.cu): list-entry
 // owners and the identity atom/slot mapping; cluster counting / filling; 1B+2B.

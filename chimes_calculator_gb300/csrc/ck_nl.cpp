@@ -76,6 +76,7 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
     L.fact4 = (eng_.factored && V.R4 > 0 && L.want_fact4) ? 1 : 0;
     L.rf3 = V.R3;
     L.rf4 = V.R4;
+    L.xs3 = V.fx3_max;
     const int nbk3 = eng_.n_buckets(3), nbk4 = eng_.n_buckets(4);
     // the cluster buckets depend on the contraction form and on the sets loaded
     const bool build = rebuild || !built_ || nall != nall_ || inum != inum_ || nent != nent_ || slot != slot_ ||
@@ -258,11 +259,13 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
             NL_TRY(d_tcount_.reserve(1));
             launch_nl_tab3(B, n3_, d_tsel_.p, d_tselr_.p, d_tcount_.p, s);
         }
+        else if (L.fact3 && L.precision == kFP64) launch_force3x(B, L, s);
         else if (L.fact3) launch_force3f(B, L, s);
         else launch_force3(B, L, s);
     }
     if (L.stride4 > 0 && n4_ > 0) {
-        if (L.fact4) launch_force4f(B, L, s);
+        if (L.fact4 && L.precision == kFP64) launch_force4x(B, L, s);
+        else if (L.fact4) launch_force4f(B, L, s);
         else launch_force4(B, L, s);
     }
     NL_TRY(cudaGetLastError());

@@ -816,6 +816,101 @@ void tc4_image(const std::vector<double>& dense, int n3, std::vector<float>& out
         }
 }
 
+// Fixed-point coefficient streams of one tuple (layout in ck_common.h): the
+// coefficients with their (row, column) indices and packed powers.
+struct FxCoef {
+    int row, col, rowp, colp;
+    double a;
+};
+void fx_limbs(double a, double amp, int& h, int& l) {
+    const long long v = std::llrint(std::ldexp(a / amp, kFxCoef));   // amp is a power of two: an exact scaling
+    const long long half = 1LL << (kFxLimb - 1);
+    h = (int)((v + half) >> kFxLimb);
+    l = (int)(v - ((long long)h << kFxLimb));
+}
+double fx_amplitude(const std::vector<FxCoef>& c) {
+    double sum = 0.0, top = 0.0;
+    for (const FxCoef& q : c) {
+        sum += std::fabs(q.a);
+        top = std::max(top, std::fabs(q.a));
+    }
+    const double need = std::max(sum / 0.9, top / 0.24);
+    if (!(need > 0.0)) return 1.0;
+    int e;
+    std::frexp(need, &e);   // need <= 2^e
+    return std::ldexp(1.0, e);
+}
+// splits of [0, total) into n parts at the record ends `ends` (ascending, the last = total), by weight
+void fx_parts(const std::vector<int>& ends, const std::vector<double>& weight, int n, int* split) {
+    double all = 0.0, w = 0.0;
+    for (double v : weight) all += v;
+    int part = 1;
+    for (size_t r = 0; r < ends.size(); r++) {
+        w += weight[r];
+        while (part < n && w >= all * part / n) split[part++] = ends[r];
+    }
+    while (part <= n) split[part++] = ends.empty() ? split[0] : ends.back();
+}
+void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxPair>& out) {
+    R.fx_amp = fx_amplitude(c);
+    R.fx_off = (int)out.size();
+    std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
+        return x.col != y.col ? x.col < y.col : x.row < y.row;
+    });
+    std::vector<int> ends;
+    std::vector<double> weight;
+    for (size_t k = 0; k < c.size();) {
+        const size_t at = out.size();
+        const int col = c[k].col;
+        int mask = 0;
+        out.push_back(FxPair{col / Rp | (col % Rp) << 8, 0});
+        while (k < c.size() && c[k].col == col) {
+            const int row = c[k].row;
+            double a = 0.0;
+            for (; k < c.size() && c[k].col == col && c[k].row == row; k++) a += c[k].a;
+            FxPair q;
+            fx_limbs(a, R.fx_amp, q.x, q.y);
+            out.push_back(q);
+            mask |= 1 << row;
+        }
+        out[at].y = mask;
+        ends.push_back((int)out.size() - R.fx_off);
+        weight.push_back(3.0 + (double)(out.size() - at - 1));
+    }
+    R.fx_split[0] = 0;
+    fx_parts(ends, weight, 8, R.fx_split);
+}
+void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
+    R.fx_amp = fx_amplitude(c);
+    R.fx_off = (int)out.size();
+    for (int side = 0; side < 2; side++) {
+        if (side == 1)
+            for (FxCoef& q : c) {
+                std::swap(q.row, q.col);
+                std::swap(q.rowp, q.colp);
+            }
+        std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
+            return x.row != y.row ? x.row < y.row : x.col < y.col;
+        });
+        std::vector<int> ends;
+        std::vector<double> weight;
+        int* split = R.fx_split + 4 * side;
+        split[0] = (int)out.size() - R.fx_off;
+        for (size_t k = 0; k < c.size(); k++) {
+            const bool last = k + 1 == c.size() || c[k + 1].row != c[k].row;
+            FxEnt q;
+            fx_limbs(c[k].a, R.fx_amp, q.h, q.l);
+            q.code = (int)((unsigned)c[k].col | (unsigned)c[k].rowp << 16);
+            q.last = last ? 1 : 0;
+            out.push_back(q);
+            if (weight.size() == ends.size()) weight.push_back(3.0);
+            weight.back() += 1.0;
+            if (last) ends.push_back((int)out.size() - R.fx_off);
+        }
+        fx_parts(ends, weight, 4, split);
+    }
+}
+
 // set_cheby_polys' Morse-map constants (chimesFF.h:553-559)
 void morse_consts(double rin, double rout, double lam, double& xavg, double& xdiff) {
     double x_min = std::exp(-1 * rin / lam);
@@ -915,7 +1010,11 @@ ParamImage pack_params(const HostParams& P) {
         long long rk = 1, rc = 1;
         for (int k = 0; k < K; k++) rk *= R_pow;
         for (int k = K; k < np; k++) rc *= R_pow;
-        const bool fact = rk <= kFactMaxDim && rc <= kFactMaxDim;
+        bool fact = rk <= kFactMaxDim && rc <= kFactMaxDim;
+        // (a coefficient that is no number has no fixed-point form: the
+        // per-coefficient kernels take such a set)
+        for (const std::vector<double>& v : Bd.coef)
+            for (double a : v) fact = fact && std::isfinite(a);
         std::vector<FactRow> fr;
         std::vector<FactEntD> fed;
         std::vector<FactEntF> fef;
@@ -925,8 +1024,10 @@ ParamImage pack_params(const HostParams& P) {
         const bool tc = nb == 3 ? fact && R_pow >= 2 && R_pow <= kTc3MaxR
                                 : fact && R_pow >= 2 && R_pow <= kTc4MaxR;
         std::vector<float> tcimg;
-        struct Shared { int coef_off, f_row, f_nrow, f_ncol, f_ent, tc_off; };
-        std::map<std::pair<int, std::vector<int>>, Shared> shared;  // (type, mapping) -> tables
+        std::vector<FxPair> fx3;
+        std::vector<FxEnt> fx4;
+        int fx3_max = 0;
+        std::map<std::pair<int, std::vector<int>>, int> shared;  // (type, mapping) -> first tuple with its tables
         for (int u = 0; u < ntup; u++) {
             TupleRec& R = tr[u];
             std::memset(&R, 0, sizeof(R));
@@ -960,10 +1061,13 @@ ParamImage pack_params(const HostParams& P) {
             auto key = std::make_pair(ti, m);
             auto it = shared.find(key);
             if (it != shared.end()) {
-                R.coef_off = it->second.coef_off;
-                R.f_row = it->second.f_row; R.f_nrow = it->second.f_nrow;
-                R.f_ncol = it->second.f_ncol; R.f_ent = it->second.f_ent;
-                R.tc_off = it->second.tc_off;
+                const TupleRec& O = tr[it->second];
+                R.coef_off = O.coef_off;
+                R.f_row = O.f_row; R.f_nrow = O.f_nrow; R.f_ncol = O.f_ncol; R.f_ent = O.f_ent;
+                R.tc_off = O.tc_off;
+                R.fx_off = O.fx_off;
+                R.fx_amp = O.fx_amp;
+                std::memcpy(R.fx_split, O.fx_split, sizeof(R.fx_split));
                 continue;
             }
             R.coef_off = (int)cd.size();
@@ -1028,7 +1132,17 @@ ParamImage pack_params(const HostParams& P) {
                 R.tc_off = (int)tcimg.size();
                 tc4_image(dense, n3, tcimg);
             }
-            shared[key] = Shared{R.coef_off, R.f_row, R.f_nrow, R.f_ncol, R.f_ent, R.tc_off};
+            if (fact && R.ncoef > 0) {
+                std::vector<FxCoef> q(R.ncoef);
+                for (int c = 0; c < R.ncoef; c++) q[c] = FxCoef{rowi[c], coli[c], rowp[c], colp[c], Bd.coef[ti][c]};
+                if (nb == 3) {
+                    fx3_stream(std::move(q), R_pow, R, fx3);
+                    fx3_max = std::max(fx3_max, R.fx_split[8]);
+                } else {
+                    fx4_stream(std::move(q), R, fx4);
+                }
+            }
+            shared[key] = u;
         }
         // per-pair-type tables when no tuple overrides a pair type's cutoffs
         std::vector<PairTab> ptab(P.npairs);
@@ -1071,6 +1185,15 @@ ParamImage pack_params(const HostParams& P) {
             H.tc4_r = R_pow;
             H.tc4 = as_off<const float>(B.add(tcimg.data(), tcimg.size()));
             H.n_tc4 = (long long)tcimg.size();
+        }
+        if (nb == 3 && !fx3.empty()) {
+            H.fx3 = as_off<const FxPair>(B.add(fx3.data(), fx3.size()));
+            H.n_fx3 = (long long)fx3.size();
+            H.fx3_max = fx3_max;
+        }
+        if (nb == 4 && !fx4.empty()) {
+            H.fx4 = as_off<const FxEnt>(B.add(fx4.data(), fx4.size()));
+            H.n_fx4 = (long long)fx4.size();
         }
         if (nb == 3) {
             H.n_c3 = (long long)cd.size();
