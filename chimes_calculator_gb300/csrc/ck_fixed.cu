@@ -19,8 +19,8 @@
 //
 // Measured (GB300, 384 configurations of 8-512 atoms, 12/10/4, 1.81 M triplets
 // and 358 k quadruplets; against the factored FP64 kernels this replaces):
-// 3-body 5.91 -> 3.50 ms, 4-body 3.12 -> 1.84 ms; 1024 atoms 12/8/4: 131 -> 86
-// and 132 -> 120 us.  The contraction no longer bounds them; the FP64 set-up of
+// 3-body 5.91 -> 3.27 ms, 4-body 3.12 -> 1.63 ms; 1024 atoms 12/8/4: 131 -> 80
+// and 132 -> 117 us.  The contraction no longer bounds them; the FP64 set-up of
 // the pairs that the cache does not hold, the FP64 epilogue and the latency
 // of both do.
 #include <cuda_runtime.h>
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
                                                      const long long* perm_n, long long perm_cap, int rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     const FxSmem<3, NW> m(smem, rs);
-    FxPair* strm = m.rest;
+    FxEnt* strm = reinterpret_cast<FxEnt*>(m.rest);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long ntiles = min(*perm_n, perm_cap) / kFxTile;
     int loaded = -1;
@@ -241,10 +241,14 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
         FxAcc g1, g2, ca, cb;
         Fx tb{0, 0}, db{0, 0};
         int qb = -1;
+        int o = len ? R->fx_split[8 * w / NW] : 0;
         const int o1 = len ? R->fx_split[8 * (w + 1) / NW] : 0;
-        for (int o = len ? R->fx_split[8 * w / NW] : 0; o < o1;) {
-            const FxPair hd = strm[o++];
-            const int b = hd.x & 0xff, c = hd.x >> 8;
+        FxEnt hd = strm[o];   // (the buffer has room for a header past the stream)
+        while (o < o1) {
+            const int b = hd.x, c = hd.y, mask = hd.z;
+            const FxEnt* q4 = strm + o + 1;
+            o += 1 + __popc(mask);
+            hd = strm[o];
             if (b != qb) {   // uniform: a new run of q_ik
                 g1.mac(db, ca.value<0>());
                 g2.mac(tb, cb.value<0>());
@@ -258,11 +262,13 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
             const Fx Y = fx_mul(tb, tc);
             FxAcc wj;
 #pragma unroll
-            for (int q = 0; q < RX; q++)
-                if (hd.y & (1 << q)) {
-                    const Fx a = fx_load(strm[o++]);
-                    wj.mac(a, X[q]);
-                    z[q].mac(a, Y);
+            for (int g = 0; g < RX / 2; g++)
+                if (mask & (1 << g)) {   // uniform
+                    const FxEnt a = *q4++;
+                    wj.mac(Fx{a.x, a.y}, X[2 * g]);
+                    wj.mac(Fx{a.z, a.w}, X[2 * g + 1]);
+                    z[2 * g].mac(Fx{a.x, a.y}, Y);
+                    z[2 * g + 1].mac(Fx{a.z, a.w}, Y);
                 }
             const Fx wv = wj.value<kFxDown>();
             ca.mac(tc, wv);
@@ -296,7 +302,7 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
 __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, int o1, const FxPair* V, const FxPair* t,
                                         const FxPair* d, int rs, double* out) {
     const FxPair *t1 = t + rs * kFxTile, *t2 = t1 + rs * kFxTile, *d1 = d + rs * kFxTile, *d2 = d1 + rs * kFxTile;
-    FxAcc S, g0, g1, g2, ra, rb, rP, rQ, rR, z;
+    FxAcc S, g0, g1, g2, ra, rb, rP, rQ, rR;
     int q0 = -1, q1 = -1;
     auto fold1 = [&]() {
         if (q1 < 0) return;
@@ -318,35 +324,26 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
         rQ = FxAcc();
         rR = FxAcc();
     };
-    constexpr int NB = 4;   // entries in flight
-    for (; o < o1; o += NB) {
-        FxEnt q[NB];
-        Fx v[NB];
+    while (o < o1) {
+        const FxEnt hd = ent[o++];
+        FxAcc z;
+        for (const int end = o + 4 * hd.x; o < end; o += 4) {
+            FxEnt q[4];
 #pragma unroll
-        for (int k = 0; k < NB; k++)
-            if (o + k < o1) q[k] = ent[o + k];
+            for (int k = 0; k < 4; k++) q[k] = ent[o + k];
 #pragma unroll
-        for (int k = 0; k < NB; k++)
-            if (o + k < o1) v[k] = fx_load(V[(q[k].code & 0xffff) * kFxTile]);
-#pragma unroll
-        for (int k = 0; k < NB; k++)
-            if (o + k < o1) {
-                z.mac(Fx{q[k].h, q[k].l}, v[k]);
-                if (q[k].last) {   // uniform: the record's last entry
-                    const int p = q[k].code >> 16;
-                    const int r0 = p & 31, r1 = (p >> kPowBits) & 31, r2 = (p >> (2 * kPowBits)) & 31;
-                    if (r0 != q0 || r1 != q1) {
-                        fold1();
-                        if (r0 != q0) fold0();
-                        q0 = r0;
-                        q1 = r1;
-                    }
-                    const Fx zv = z.value<kFxDown>();
-                    ra.mac(fx_load(t2[r2 * kFxTile]), zv);
-                    rb.mac(fx_load(d2[r2 * kFxTile]), zv);
-                    z = FxAcc();
-                }
-            }
+            for (int k = 0; k < 4; k++) z.mac(Fx{q[k].x, q[k].y}, fx_load(V[q[k].z * kFxTile]));
+        }
+        const int r0 = hd.y & 31, r1 = (hd.y >> kPowBits) & 31, r2 = (hd.y >> (2 * kPowBits)) & 31;
+        if (r0 != q0 || r1 != q1) {   // uniform
+            fold1();
+            if (r0 != q0) fold0();
+            q0 = r0;
+            q1 = r1;
+        }
+        const Fx zv = z.value<kFxDown>();
+        ra.mac(fx_load(t2[r2 * kFxTile]), zv);
+        rb.mac(fx_load(d2[r2 * kFxTile]), zv);
     }
     fold1();
     fold0();
@@ -427,7 +424,7 @@ unsigned fx_grid(const void* kern, int threads, size_t smem, long long tiles) {
 template <int RX, int NW>
 void launch_x3(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     const int rs = L.rf3;
-    const size_t smem = FxSmem<3, NW>::bytes(rs) + sizeof(FxPair) * (size_t)L.xs3;
+    const size_t smem = FxSmem<3, NW>::bytes(rs) + sizeof(FxEnt) * (size_t)(L.xs3 + 1);
     auto kern = k_forcex3<RX, NW>;
     const unsigned grid = fx_grid((const void*)kern, 32 * NW, smem, (B.perm3_cap + kFxTile - 1) / kFxTile);
     count_launch(), kern<<<grid, 32 * NW, smem, st>>>(B, B.c3, B.perm3, B.bk_start + B.nbk3, B.perm3_cap, rs);
@@ -438,7 +435,7 @@ void launch_x3_nw(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     if (L.rf3 <= 4) launch_x3<4, NW>(B, L, st);
     else if (L.rf3 <= 8) launch_x3<8, NW>(B, L, st);
     else if (L.rf3 <= 10) launch_x3<10, NW>(B, L, st);
-    else launch_x3<11, NW>(B, L, st);
+    else launch_x3<12, NW>(B, L, st);
 }
 
 template <int NW>

@@ -851,7 +851,7 @@ void fx_parts(const std::vector<int>& ends, const std::vector<double>& weight, i
     }
     while (part <= n) split[part++] = ends.empty() ? split[0] : ends.back();
 }
-void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxPair>& out) {
+void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& out) {
     R.fx_amp = fx_amplitude(c);
     R.fx_off = (int)out.size();
     std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
@@ -862,20 +862,19 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxPair>&
     for (size_t k = 0; k < c.size();) {
         const size_t at = out.size();
         const int col = c[k].col;
-        int mask = 0;
-        out.push_back(FxPair{col / Rp | (col % Rp) << 8, 0});
+        out.push_back(FxEnt{col / Rp, col % Rp, 0, 0});
         while (k < c.size() && c[k].col == col) {
-            const int row = c[k].row;
-            double a = 0.0;
-            for (; k < c.size() && c[k].col == col && c[k].row == row; k++) a += c[k].a;
-            FxPair q;
-            fx_limbs(a, R.fx_amp, q.x, q.y);
+            const int grp = c[k].row / 2;
+            double a[2] = {0.0, 0.0};
+            for (; k < c.size() && c[k].col == col && c[k].row / 2 == grp; k++) a[c[k].row % 2] += c[k].a;
+            FxEnt q;
+            fx_limbs(a[0], R.fx_amp, q.x, q.y);
+            fx_limbs(a[1], R.fx_amp, q.z, q.w);
             out.push_back(q);
-            mask |= 1 << row;
+            out[at].z |= 1 << grp;
         }
-        out[at].y = mask;
         ends.push_back((int)out.size() - R.fx_off);
-        weight.push_back(3.0 + (double)(out.size() - at - 1));
+        weight.push_back(2.0 + (double)(out.size() - at - 1));
     }
     R.fx_split[0] = 0;
     fx_parts(ends, weight, 8, R.fx_split);
@@ -896,16 +895,19 @@ void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
         std::vector<double> weight;
         int* split = R.fx_split + 4 * side;
         split[0] = (int)out.size() - R.fx_off;
-        for (size_t k = 0; k < c.size(); k++) {
-            const bool last = k + 1 == c.size() || c[k + 1].row != c[k].row;
-            FxEnt q;
-            fx_limbs(c[k].a, R.fx_amp, q.h, q.l);
-            q.code = (int)((unsigned)c[k].col | (unsigned)c[k].rowp << 16);
-            q.last = last ? 1 : 0;
-            out.push_back(q);
-            if (weight.size() == ends.size()) weight.push_back(3.0);
-            weight.back() += 1.0;
-            if (last) ends.push_back((int)out.size() - R.fx_off);
+        for (size_t k = 0; k < c.size();) {
+            const size_t at = out.size();
+            const int row = c[k].row;
+            out.push_back(FxEnt{0, c[k].rowp, 0, 0});
+            for (; k < c.size() && c[k].row == row; k++) {
+                FxEnt q{0, 0, c[k].col, 0};
+                fx_limbs(c[k].a, R.fx_amp, q.x, q.y);
+                out.push_back(q);
+            }
+            while ((out.size() - at - 1) % 4) out.push_back(FxEnt{0, 0, 0, 0});
+            out[at].x = (int)(out.size() - at - 1) / 4;
+            ends.push_back((int)out.size() - R.fx_off);
+            weight.push_back(4.0 + (double)(out.size() - at - 1));
         }
         fx_parts(ends, weight, 4, split);
     }
@@ -1024,7 +1026,7 @@ ParamImage pack_params(const HostParams& P) {
         const bool tc = nb == 3 ? fact && R_pow >= 2 && R_pow <= kTc3MaxR
                                 : fact && R_pow >= 2 && R_pow <= kTc4MaxR;
         std::vector<float> tcimg;
-        std::vector<FxPair> fx3;
+        std::vector<FxEnt> fx3;
         std::vector<FxEnt> fx4;
         int fx3_max = 0;
         std::map<std::pair<int, std::vector<int>>, int> shared;  // (type, mapping) -> first tuple with its tables
@@ -1187,7 +1189,7 @@ ParamImage pack_params(const HostParams& P) {
             H.n_tc4 = (long long)tcimg.size();
         }
         if (nb == 3 && !fx3.empty()) {
-            H.fx3 = as_off<const FxPair>(B.add(fx3.data(), fx3.size()));
+            H.fx3 = as_off<const FxEnt>(B.add(fx3.data(), fx3.size()));
             H.n_fx3 = (long long)fx3.size();
             H.fx3_max = fx3_max;
         }
