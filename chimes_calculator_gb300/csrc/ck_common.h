@@ -48,6 +48,13 @@ enum Status : int {
     kErrTimeout = -7,     // a bounded device wait expired
 };
 
+// Image shifts (i, j, k) packed 10 bits each, biased: |shift| and |difference
+// of two shifts| below 512, so shifts of up to kMaxPackShift layers.  The packed
+// shift of image k relative to image j is pack(k) - pack(j) + kShiftBias.
+constexpr int kMaxPackShift = 255;
+constexpr int kShiftBias = 512 | 512 << 10 | 512 << 20;
+CK_HD inline int pack_shift(int i, int j, int k) { return (i + 512) | (j + 512) << 10 | (k + 512) << 20; }
+
 // One 2-body pair type (chimes_2b_cutoff / morse_var, chimesFF.h:290-295).
 struct PairRec {
     double rin, rout, lam;
@@ -57,6 +64,8 @@ struct PairRec {
     // reciprocals for the 2-body kernels (as TupleRec): 1/lam, 1/xdiff, and the
     // cutoff's 1/rc (cubic) or Tersoff threshold rc - f*rc and 1/(rc - threshold)
     double inv_lam, inv_xdiff, fc_th, fc_inv;
+    // fixed-point form: the dense coefficients at fx2[coef_off ..], scaled by 1 / fx_amp
+    double fx_amp;
 };
 
 // One ordered atom-type tuple of a 3- or 4-body cluster.  Cutoffs, lambdas and
@@ -121,11 +130,12 @@ struct __attribute__((aligned(8))) FxPair {
 struct __attribute__((aligned(16))) FxEnt {
     int x, y, z, w;
 };
+constexpr int kPairFar = 1, kPairOor = 2;   // pair-entry flags: at or beyond the outer cutoff, below the inner one
 constexpr int kFxLimb = 28;
 constexpr int kFxCoef = 61;
 constexpr int kFxSum = 59;
 CK_HD constexpr int fx_kd(int R) {   // bits of (R - 1)^2: the dT tables' scale
-    int k = 0;
+    int k = 1;
     while ((1 << k) < (R - 1) * (R - 1)) k++;
     return k;
 }
@@ -233,7 +243,7 @@ struct DevParamSet {
     // 3-/4-body coefficients, factored entries, tensor-core image floats
     long long n_c3, n_c4, n_fe3, n_fe4, n_tc3, n_tc4;
     // fixed-point streams (FP64 form); fx3_max = longest 3-body stream
-    const FxEnt* fx3; const FxEnt* fx4;
+    const FxPair* fx2; const FxEnt* fx3; const FxEnt* fx4;
     long long n_fx3, n_fx4;
     int fx3_max, fx_pad;
     const FactRow* fr3; const FactEntD* fe3d; const FactEntF* fe3f;
@@ -293,6 +303,7 @@ struct BatchView {
     int* atom_self;                // [n_atoms_total] slot of the atom itself
     int* ghost_id;                 // [q] ghost id within its system, -1 = unused slot
     int* ghost_parent;             // [q] atom index (global)
+    int* ghost_sh;                 // [q] image shift, packed (pack_shift), or null
     double* ghost_fs;              // [q][3] fractional coords, input cell
     double* ghost_xn;              // [q][3] Cartesian coords, reoriented cell
     double* ghost_fn;              // [q][3] fractional coords, reoriented cell
@@ -311,6 +322,7 @@ struct BatchView {
     int* l2_ghost;                 // [n2] ghost slot of the neighbour
     double* l2_dist;               // [n2] distance in the reoriented frame
     float* l2_vec;                 // [n2][4] displacement from the list's atom (FP32), for the prefilter
+    long long* l2_key;             // [n2] neighbour's parent atom << 32 | its packed image shift, or null
     long long n2_cap;
     // 3B/4B enumeration
     int* e_cnt3; int* e_cnt4;      // [n2]
@@ -319,13 +331,21 @@ struct BatchView {
     int* c4;                       // [n4][4]
     long long n3_cap, n4_cap;
     int enum_serial;               // 1: some system has 3B and 4B terms with rc4 > rc3 (sequential enumeration)
-    // Pair-table cache of the factored kernels: the list entries (i, j) of a
+    // Pair-table cache of the mixed form: the list entries (i, j) of a
     // cluster's first atom, c3e[n3][2] = entries of ij, ik and c4e[n4][3] =
     // ij, ik, il (written by the enumeration when not null), and per entry
-    // the Chebyshev tables of body order 3 / 4 (pcd: dr[3], r, fc, fcd as
-    // doubles; pct: T[R], dT/dr[R] in the compute type)
+    // the Chebyshev tables of body order 3 / 4 (pcd: dr[3], r, fc, fcd, below
+    // rin as doubles; pct: T[R], dT/dr[R] in FP32).
     int* c3e; int* c4e;
     int use_pc3, use_pc4;
+    // Pair-entry form (FP64; all_pairs = 1): c3e[n3][3] and c4e[n4][6] hold the
+    // list entries of ALL pairs of a cluster -- jk, jl, kl from the list of
+    // their own first member's parent, -1 where that list lacks the pair -- and
+    // per entry pe = dx, dy, dz and the sum of the force scalars of every term
+    // on that pair; pcd[n2][4] = fc, fc gs / r, fc'/r, flags; pct[n2][R] (FxEnt)
+    // = T and dT limbs.
+    int all_pairs;
+    double* pe;                    // [n2][4]
     // 1: bucketing drops clusters with a pair at or beyond its tuple's outer
     // cutoff (lists built with padded cutoffs; rebucketed every evaluation)
     int bucket_cut;
@@ -334,8 +354,8 @@ struct BatchView {
     // than the margin takes no FP64 distance (null: always exact)
     const float* pos_f;
     float float_eps;
-    double* pcd3; double* pcd4;    // [n2_cap][6]
-    void* pct3; void* pct4;        // [n2_cap][2R]
+    double* pcd3; double* pcd4;
+    void* pct3; void* pct4;
     // results
     double* force;                 // [n_in_total][3]
     double* eatom;                 // [n_in_total] per-atom energy or null (pair-style path)

@@ -46,6 +46,7 @@ Engine::~Engine() {
         if (s.dev) cudaFree(s.dev);
     if (fork_) cudaEventDestroy(fork_);
     if (fork2_) cudaEventDestroy(fork2_);
+    if (pairs_) cudaEventDestroy(pairs_);
     if (join_) cudaEventDestroy(join_);
     if (stream2_) cudaStreamDestroy(stream2_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -72,6 +73,7 @@ Status Engine::init_device(std::string& err) {
     CK_TRY(cudaStreamCreateWithFlags(&stream2_, cudaStreamNonBlocking));
     CK_TRY(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
     CK_TRY(cudaEventCreateWithFlags(&fork2_, cudaEventDisableTiming));
+    CK_TRY(cudaEventCreateWithFlags(&pairs_, cudaEventDisableTiming));
     CK_TRY(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
     CK_TRY(h_flags_.reserve(8));
     CK_TRY(h_counts_.reserve(4));
@@ -121,7 +123,7 @@ int Engine::load_params(const std::string& path, std::string& err) {
     rel(h.pt3); rel(h.pt4);
     rel(h.tc3);
     rel(h.tc4);
-    rel(h.fx3); rel(h.fx4);
+    rel(h.fx2); rel(h.fx3); rel(h.fx4);
     rel(h.t2rec); rel(h.tab2r); rel(h.tab2c);
     rel(h.t3rec); rel(h.tab3r); rel(h.tab3v);
     // this set's cluster buckets follow those of the sets loaded before it
@@ -163,6 +165,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     bool tc3 = precision == kMixed, tc4 = precision == kMixed;
     int r4_lo = 1 << 30;   // the 4-body tensor-core kernel needs one R over the batch's sets
     bool enum_serial = false;
+    bool ent = precision == kFP64 && factored && pair_cache;   // FP64 pair-entry form
     double n2_est = 0.0, n3_est = 0.0, n4_est = 0.0;
     for (int s = 0; s < S; s++) {
         const SystemSpec& in = sys[s];
@@ -200,6 +203,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
         }
         d.pset = in.pset;
         if (d.has3 && d.has4 && d.c4 > d.c3) enum_serial = true;
+        ent = ent && d.n_layers <= kMaxPackShift;
         d.in_off = in_off; d.atom_off = atom_off; d.ghost_off = ghost_off; d.bin_off = bin_off;
         in_off += in.n;
         atom_off += d.n_atoms;
@@ -213,6 +217,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
             rf3 = std::max(rf3, V.R3);
             xs3 = std::max(xs3, V.fx3_max);
             pc3 = pc3 && V.pt3;
+            ent = ent && V.R3 > 0 && V.pt3;
             tc3 = tc3 && V.tc3 != nullptr;
         }
         if (P.o4 > 0) {
@@ -220,6 +225,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
             rf4 = std::max(rf4, V.R4);
             r4_lo = std::min(r4_lo, V.R4);
             pc4 = pc4 && V.pt4;
+            ent = ent && V.R4 > 0 && V.pt4;
             tc4 = tc4 && V.tc4 != nullptr;
         }
         // list-size estimates for the first capacity guess
@@ -243,7 +249,9 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     tuning.tc3 = tuning.fact3 && avail_tc3_ && tuning.want_tc3 ? 1 : 0;
     avail_tc4_ = avail_fact4_ && tc4 && r4_lo == rf4 && tc4_supported(rf4);
     tuning.tc4 = tuning.fact4 && avail_tc4_ && tuning.want_tc4 ? 1 : 0;
-    // the pair-table cache needs the enumeration that records entry indices;
+    // FP64: the pair-entry form needs tables for every body order of every set,
+    // the enumeration that records entry indices and packable image shifts.
+    // Mixed: the pair-table cache needs the enumeration that records entry indices;
     // it pays for itself while its tables stay near L2 (measured: ~10% on the
     // 3-body kernel for 25k list entries, nothing for 11M), so large batches
     // compute every pair in the cluster kernel
@@ -253,8 +261,10 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     // that stay far below the memory bandwidth.
     const bool pc_size = n2_est <= 2.0e6;
     pc_small_ = pc_size;
-    avail_pc3_ = avail_fact3_ && pc3 && !enum_serial && (pc_size || avail_tc3_);
-    avail_pc4_ = avail_fact4_ && pc4 && !enum_serial && pc_size;
+    const bool mixed = precision == kMixed;
+    avail_pc3_ = mixed && avail_fact3_ && pc3 && !enum_serial && (pc_size || avail_tc3_);
+    avail_pc4_ = mixed && avail_fact4_ && pc4 && !enum_serial && pc_size;
+    avail_ent_ = ent && !enum_serial && (rf3 > 0 || rf4 > 0);
     tuning.rf3 = rf3;
     tuning.rf4 = rf4;
     tuning.xs3 = xs3;
@@ -331,6 +341,21 @@ Status Engine::ensure_lists(std::string& err) {
     CK_TRY(d_bk_count_.reserve(nbk3_ + nbk4_ + 1));
     CK_TRY(d_bk_fill_.reserve(nbk3_ + nbk4_ + 1));
     CK_TRY(d_bk_start_.reserve(nbk3_ + nbk4_ + 2));
+    if (avail_ent_) {
+        CK_TRY(d_ghost_sh_.reserve(V_.n_ghost_total));
+        CK_TRY(d_l2_key_.reserve(n2_cap_));
+        CK_TRY(d_pe_.reserve(4 * n2_cap_));
+        if (tuning.rf3 > 0) {
+            CK_TRY(d_c3e_.reserve(3 * n3_cap_));
+            CK_TRY(d_pcd3_.reserve(4 * n2_cap_));
+            CK_TRY(d_pct3_.reserve((long long)sizeof(FxEnt) * tuning.rf3 * n2_cap_));
+        }
+        if (tuning.rf4 > 0) {
+            CK_TRY(d_c4e_.reserve(6 * n4_cap_));
+            CK_TRY(d_pcd4_.reserve(4 * n2_cap_));
+            CK_TRY(d_pct4_.reserve((long long)sizeof(FxEnt) * tuning.rf4 * n2_cap_));
+        }
+    }
     if (avail_pc3_) {
         CK_TRY(d_c3e_.reserve(2 * n3_cap_));
         CK_TRY(d_pcd3_.reserve(8 * n2_cap_));
@@ -367,8 +392,12 @@ Status Engine::ensure_lists(std::string& err) {
     B.n3_cap = n3_cap_; B.n4_cap = n4_cap_;
     B.force = d_force_.p; B.ev = d_ev_.p; B.flags = d_flags_.p; B.queue = d_queue_.p;
     B.enum_serial = enum_serial_ ? 1 : 0;
-    B.c3e = avail_pc3_ ? d_c3e_.p : nullptr;
-    B.c4e = avail_pc4_ ? d_c4e_.p : nullptr;
+    B.c3e = avail_pc3_ || (avail_ent_ && tuning.rf3 > 0) ? d_c3e_.p : nullptr;
+    B.c4e = avail_pc4_ || (avail_ent_ && tuning.rf4 > 0) ? d_c4e_.p : nullptr;
+    B.all_pairs = avail_ent_ ? 1 : 0;
+    B.ghost_sh = avail_ent_ ? d_ghost_sh_.p : nullptr;
+    B.l2_key = avail_ent_ ? d_l2_key_.p : nullptr;
+    B.pe = d_pe_.p;
     B.pcd3 = d_pcd3_.p; B.pcd4 = d_pcd4_.p;
     B.pct3 = d_pct3_.p; B.pct4 = d_pct4_.p;
     B.use_pc3 = B.use_pc4 = 0;   // set per launch from the contraction form
@@ -433,6 +462,14 @@ Status Engine::enqueue(std::string& err) {
     launch_l2(B, d_l2_owner_.p, true, st);
     ForceLaunch L = tuning;
     L.precision = precision;
+    // pair-entry form: every body order present runs in fixed point (an order
+    // that the tuning gave to the per-coefficient kernel scatters its own forces)
+    const bool ent = avail_ent_ && precision == kFP64 && ((L.stride3 > 0 && L.fact3) || (L.stride4 > 0 && L.fact4));
+    auto pairs12 = [&](cudaStream_t q) {
+        NvtxRange r("chimes: 1B+2B");
+        if (ent) launch_pairs_x(B, d_l2_owner_.p, L, q);
+        else launch_force2(B, d_l2_owner_.p, L, q);
+    };
     // Concurrent form: the second stream takes 1B+2B (it needs only the pair
     // lists) while the first enumerates the clusters, then the 4-body branch
     // while the first runs the 3-body one; both join before the copies out.
@@ -441,8 +478,8 @@ Status Engine::enqueue(std::string& err) {
     if (conc) {
         CK_TRY(cudaEventRecord(fork_, st));
         CK_TRY(cudaStreamWaitEvent(stream2_, fork_, 0));
-        NvtxRange r("chimes: 1B+2B");
-        launch_force2(B, d_l2_owner_.p, L, stream2_);
+        pairs12(stream2_);
+        CK_TRY(cudaEventRecord(pairs_, stream2_));
     }
     launch_enum(B, d_l2_owner_.p, false, st);
     exclusive_scan2(B.e_cnt3, B.e_off3, B.e_cnt4, B.e_off4, B.n2_cap, d_scan_tmp_.p, st);
@@ -462,8 +499,8 @@ Status Engine::enqueue(std::string& err) {
             launch_bucket(B, 3, q);
             launch_force3tc(B, L, q);
         } else if (L.fact3 && L.precision == kFP64) {
-            launch_pair_tables_x(B, d_l2_owner_.p, 3, L, q);
             launch_bucket(B, 3, q);
+            if (ent && conc) (void)cudaStreamWaitEvent(q, pairs_, 0);
             launch_force3x(B, L, q);
         } else if (L.fact3) {
             launch_pair_tables(B, d_l2_owner_.p, 3, L, q);
@@ -480,7 +517,6 @@ Status Engine::enqueue(std::string& err) {
             launch_bucket(B, 4, q);
             launch_force4tc(B, L, q);
         } else if (L.fact4 && L.precision == kFP64) {
-            launch_pair_tables_x(B, d_l2_owner_.p, 4, L, q);
             launch_bucket(B, 4, q);
             launch_force4x(B, L, q);
         } else if (L.fact4) {
@@ -500,15 +536,14 @@ Status Engine::enqueue(std::string& err) {
         CK_TRY(cudaEventRecord(join_, stream2_));
         body3(st);
         CK_TRY(cudaStreamWaitEvent(st, join_, 0));
+        if (ent) launch_pair_forces(B, st);
     } else {
-        {
-            NvtxRange r("chimes: 1B+2B");
-            launch_force2(B, d_l2_owner_.p, L, st);
-        }
+        pairs12(st);
         if (profile) CK_TRY(record_stage_event(ev_[2], st));
         body3(st);
         if (profile) CK_TRY(record_stage_event(ev_[3], st));
         body4(st);
+        if (ent) launch_pair_forces(B, st);
     }
     if (profile) CK_TRY(record_stage_event(ev_[4], st));
     ev_recorded_ = profile;
@@ -546,7 +581,7 @@ Status Engine::launch(std::string& err) {
                                   tuning.stride3, tuning.stride4, tuning.blocks_per_sm, profile ? 1 : 0,
                                   tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
-                                  tuning.tc3, tuning.tc4};
+                                  tuning.tc3, tuning.tc4, V_.all_pairs};
     for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
                           (const void*)V_.bin_items, (const void*)V_.l2_ghost, (const void*)V_.c3,
                           (const void*)V_.c4, (const void*)V_.force, (const void*)d_scan_tmp_.p,
@@ -554,6 +589,7 @@ Status Engine::launch(std::string& err) {
                           (const void*)V_.e_off3, (const void*)V_.psets, (const void*)V_.perm3,
                           (const void*)V_.perm4, (const void*)V_.bk_count, (const void*)V_.bk_fill,
                           (const void*)V_.bk_start, (const void*)V_.c3e, (const void*)V_.c4e,
+                          (const void*)V_.pe, (const void*)V_.l2_key, (const void*)V_.ghost_sh,
                           (const void*)V_.pcd3, (const void*)V_.pcd4, (const void*)V_.pct3, (const void*)V_.pct4})
         key.push_back((long long)(uintptr_t)p);
     if (key != graph_key_) {

@@ -115,7 +115,8 @@ public:
     bool factored = true;
     // run the 4-body branch on a second stream beside 1B+2B and 3-body (not while profiling)
     bool concurrent = true;
-    // factored kernels take the pairs of a cluster's first atom from a per-entry table cache
+    // pairs' tables once per list entry: FP64 the pair-entry form (ck_fixed.cu), mixed the
+    // pair-table cache of a cluster's first atom
     bool pair_cache = true;
     int precision = kFP64;
     bool use_graph = false;
@@ -160,7 +161,7 @@ private:
     DevBuf<DevParamSet> dsets_;
     cudaStream_t stream_ = nullptr;
     cudaStream_t stream2_ = nullptr;              // the 4-body branch
-    cudaEvent_t fork_ = nullptr, fork2_ = nullptr, join_ = nullptr;
+    cudaEvent_t fork_ = nullptr, fork2_ = nullptr, pairs_ = nullptr, join_ = nullptr;
     bool ready_ = false;
     int device_ = -1;
 
@@ -195,8 +196,11 @@ private:
     bool enum_serial_ = false;                         // staged batch needs the sequential enumeration
     bool avail_pc3_ = false, avail_pc4_ = false;       // pair-table cache usable for the staged batch
     bool pc_small_ = false;                            // list small enough for the cache to stay near L2
+    bool avail_ent_ = false;                           // FP64 pair-entry form usable for the staged batch
     DevBuf<int> d_c3e_, d_c4e_;
-    DevBuf<double> d_pcd3_, d_pcd4_;
+    DevBuf<double> d_pcd3_, d_pcd4_, d_pe_;
+    DevBuf<int> d_ghost_sh_;
+    DevBuf<long long> d_l2_key_;
     DevBuf<unsigned char> d_pct3_, d_pct4_;
     DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_;
     DevBuf<long long> d_bk_start_;

@@ -1,5 +1,6 @@
-// 3-body and 4-body contraction of the FP64 form in 64-bit fixed point
-// (arithmetic in ck_fixed.cuh, coefficient streams in ck_common.h).
+// The FP64 form of the pair stage and of the 3-body and 4-body contraction, in
+// 64-bit fixed point (arithmetic in ck_fixed.cuh, coefficient streams in
+// ck_common.h).
 //
 // For the clusters of one ordered type tuple, with X_I the products of the row
 // pairs' T (3-body: T_ij; 4-body: T_ij T_ik T_il) and Y_J those of the column
@@ -14,15 +15,19 @@
 // coefficients (one broadcast), and the warps share the cluster's tables and
 // split the coefficients (NW contiguous parts of about equal work), so that
 // few clusters still fill the GPU without lanes that read different records.
-// Everything is linear in the parts' sums; warp 0 adds them and forms the
-// forces in FP64.
+// Everything is linear in the parts' sums (exact integers); warp 0 adds them
+// and forms the force scalars.
 //
-// Measured (GB300, 384 configurations of 8-512 atoms, 12/10/4, 1.81 M triplets
-// and 358 k quadruplets; against the factored FP64 kernels this replaces):
-// 3-body 5.91 -> 3.27 ms, 4-body 3.12 -> 1.63 ms; 1024 atoms 12/8/4: 131 -> 80
-// and 132 -> 117 us.  The contraction no longer bounds them; the FP64 set-up of
-// the pairs that the cache does not hold, the FP64 epilogue and the latency
-// of both do.
+// Pair-entry form (ENT; list-build path, when every tuple uses the same cutoffs
+// for a given pair type): all pairs of a cluster are entries of some atom's
+// list (BatchView::all_pairs).  k_pairs_x computes per entry, once, the
+// geometry, the 2-body term, the cutoffs and the tables of both body orders;
+// the cluster kernels only gather them and add each pair's force scalar to its
+// entry (3 or 6 atomics and about 20 or 45 FP64 operations a cluster, where the
+// set-up and epilogue per cluster took 300 or 800); k_pair_forces then
+// turns each entry's scalar into forces and virial, once per entry and not once
+// per cluster.  Otherwise (caller's neighbour lists, per-tuple cutoffs) a
+// cluster's pairs are set up and its forces scattered in the cluster kernel.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -43,150 +48,363 @@ __device__ __forceinline__ PairTab tuple_pair_x(const TupleRec& R, int p) {
     return PairTab{R.rin[p], R.rout[p], R.xavg[p], R.xdiff[p], R.inv_lam[p], R.inv_xdiff[p], R.fc_th[p], R.fc_inv[p]};
 }
 
-// Pair-table cache of the FP64 form: for every list entry closer than the
-// body order's largest outer cutoff, the pair's geometry, cutoff and tables
-// with the pair type's constants, once per entry instead of once per cluster.
-// pcd[e][8] = dr0 dr1 dr2 r fc fc' oor gs; pct[e][2 rs] = T, then dT limbs.
-template <int NB>
-__global__ void __launch_bounds__(256) k_pair_tables_x(BatchView B, const int* l2_owner, int rs) {
-    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
-    double* pcd = NB == 3 ? B.pcd3 : B.pcd4;
-    FxPair* pct = reinterpret_cast<FxPair*>(NB == 3 ? B.pct3 : B.pct4);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n2; e += stride) {
-        const int r = l2_owner[e];
-        const SysDesc& d = B.sys[B.atom_sys[r]];
-        if (!(NB == 3 ? d.has3 : d.has4) || B.l2_dist[e] >= (NB == 3 ? d.c3 : d.c4)) continue;
-        const DevParamSet& P = B.psets[d.pset];
-        const int gi = B.atom_self[r], gj = B.l2_ghost[e];
-        double dr[3], rr;
-        pair_geom(B, d.h, gi, gj, dr, rr);
-        const int pt = P.pair_map[B.atom_type[r] * P.ntypes + B.atom_type[B.ghost_parent[gj]]];
-        const PairTab& Q = (NB == 3 ? P.pt3 : P.pt4)[pt];
-        const int Rp = NB == 3 ? P.R3 : P.R4;
-        double fc, fcd, gs;
-        FxPair* T = pct + (size_t)e * 2 * rs;
-        pair_setup_x(P, Q, rr, T, T + rs, 1, Rp, fx_kd(Rp), fc, fcd, gs, nullptr);
-        double* g = pcd + 8 * e;
-        g[0] = dr[0]; g[1] = dr[1]; g[2] = dr[2]; g[3] = rr;
-        g[4] = fc; g[5] = fcd; g[6] = rr < Q.rin ? 1.0 : 0.0; g[7] = gs;
-    }
-}
+__device__ __forceinline__ FxEnt fx_quad(const Fx& t, const Fx& d) { return FxEnt{t.h, t.l, d.h, d.l}; }
+__device__ __forceinline__ Fx quad_t(const FxEnt* q) { return fx_load(*reinterpret_cast<const FxPair*>(q)); }
 
-// Shared memory of a block (all of it dynamic: allow_max_smem's limit leaves
-// no room for static arrays), the claimed tile, then interleaved [entry][cluster]:
-//   double geo[NP * 4], fc[NP], fcd[NP], gs[NP], part[NW][NP + 1]
-//   FxPair   T[NP * rs], D[NP * rs]
-template <int NB, int NW>
-struct FxSmem {
-    static constexpr int NP = Topo<NB>::NP;
-    long long* tile;
-    double *geo, *fc, *fcd, *gs, *part;
-    FxPair *T, *D, *rest;
-    __device__ FxSmem(unsigned char* smem, int rs) {
-        tile = reinterpret_cast<long long*>(smem);
-        geo = reinterpret_cast<double*>(smem + 16);
-        fc = geo + NP * 4 * kFxTile;
-        fcd = fc + NP * kFxTile;
-        gs = fcd + NP * kFxTile;
-        part = gs + NP * kFxTile;
-        T = reinterpret_cast<FxPair*>(part + NW * (NP + 1) * kFxTile);
-        D = T + NP * rs * kFxTile;
-        rest = D + NP * rs * kFxTile;
+// Per-lane energy accumulator for one system at a time.
+struct EAcc {
+    int s = -1;
+    double v = 0.0;
+    __device__ void flush(const BatchView& B) {
+        if (s >= 0) atomicAdd(&B.ev[8 * s], v);
+        s = -1;
+        v = 0.0;
     }
-    static size_t bytes(int rs) {
-        return 16 + sizeof(double) * (size_t)(NP * 7 + NW * (NP + 1)) * kFxTile + sizeof(FxPair) * (size_t)2 * NP * rs * kFxTile;
+    __device__ void add(const BatchView& B, int sys, double e) {
+        if (sys != s) { flush(B); s = sys; }
+        v += e;
+    }
+    // warp-collective, one interaction per valid lane: lane 0 takes the warp's
+    // sum when the lanes hold one system (see EVAcc::add_warp)
+    __device__ void add_warp(const BatchView& B, int sys, double e, bool valid) {
+        const unsigned have = __ballot_sync(kFull, valid);
+        if (!have) return;
+        const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
+        if (__all_sync(kFull, !valid || sys == s0)) {
+            double x = valid ? e : 0.0;
+            for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
+            if ((threadIdx.x & 31) == 0) add(B, s0, x);
+        } else if (valid) {
+            add(B, sys, e);
+        }
+    }
+    // end of kernel: one atomic per warp when the warp holds one system
+    __device__ void flush_warp(const BatchView& B) {
+        const unsigned have = __ballot_sync(kFull, s >= 0);
+        if (!have) return;
+        const int s0 = __shfl_sync(kFull, s, __ffs(have) - 1);
+        if (__all_sync(kFull, s < 0 || s == s0)) {
+            double x = s >= 0 ? v : 0.0;
+            for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
+            if ((threadIdx.x & 31) == 0) atomicAdd(&B.ev[8 * s0], x);
+        } else {
+            flush(B);
+        }
     }
 };
 
-// Geometry, cutoffs and tables of this lane's cluster c, its pairs spread over
-// the block's warps; pairs ij, ik[, il] from the cache when there is one.
-// Returns whether the cluster is evaluated (compute_3B/4B's early-outs).
-template <int NB, int NW>
+// ---------------------------------------------------------------------------
+// Per list entry: geometry, 1-body and 2-body terms, cutoffs and tables
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void put_pair(const DevParamSet& P, const PairTab& Q, double r, double rinv, double ex,
+                                         int R, FxEnt* tab, double* scal) {
+    double fc, fcd, gs;
+    pair_setup_x(P, Q, r, ex, R, fx_kd(R), fc, fcd, gs, [&](int n, const Fx& t, const Fx& d) { tab[n] = fx_quad(t, d); });
+    const int flags = (r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0);
+    reinterpret_cast<double2*>(scal)[0] = make_double2(fc, fc * gs * rinv);
+    reinterpret_cast<double2*>(scal)[1] = make_double2(fcd * rinv, (double)flags);
+}
+
+// Bound by the FP64 pipe (geometry, square root, exponential and the three
+// cutoffs' sines; the polynomial sums are fixed-point).
+__global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owner, int rs3, int rs4) {
+    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
+    EAcc acc, acc1;   // 2-body, 1-body (an atom and an entry of the same number are mostly of different systems)
+    const long long ntot = n2 > B.n_atoms_total ? n2 : B.n_atoms_total;
+    // one contiguous range of entries per block, as k_force2
+    const long long per = ((ntot + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
+    const long long e_end = min(ntot, per * (blockIdx.x + 1));
+    for (long long e = per * blockIdx.x + threadIdx.x; e < e_end; e += blockDim.x) {
+        if (e < B.n_atoms_total) {   // compute_1B (chimesFF.cpp:1636-1641)
+            const int s = B.atom_sys[e];
+            acc1.add(B, s, B.psets[B.sys[s].pset].eoff[B.atom_type[e]]);
+        }
+        if (e >= n2) continue;
+        const int a = l2_owner[e];
+        const int s = B.atom_sys[a];
+        const SysDesc& d = B.sys[s];
+        const DevParamSet& P = B.psets[d.pset];
+        const int gj = B.l2_ghost[e];
+        int pt = P.pair_map[B.atom_type[a] * P.ntypes + B.atom_type[B.ghost_parent[gj]]];
+        if (!ck_bound(B, pt >= 0 && pt < P.npairs)) pt = 0;
+        const PairRec& pr = P.pairs[pt];
+        double dr[3], r;
+        pair_geom(B, d.h, B.atom_self[a], gj, dr, r);
+        const double rinv = r > 0.0 ? 1.0 / r : 1e20;
+        const double ex = exp(-r * pr.inv_lam);
+        double E = 0.0, fs = 0.0;
+        if (r < pr.rout) {
+            if (pr.fx_amp != 0.0) pair_2b_x(P, pr, r, rinv, ex, B.flags, E, fs);
+            else pair_2b<double>(P, pr, r, B.flags, E, fs);
+            acc.add(B, s, E);
+        }
+        reinterpret_cast<double2*>(B.pe + 4 * e)[0] = make_double2(dr[0], dr[1]);
+        reinterpret_cast<double2*>(B.pe + 4 * e)[1] = make_double2(dr[2], fs);
+        // (a pair jk of some cluster can lie at the cutoff itself, to rounding, in this list)
+        const double dist = B.l2_dist[e] - 1e-6;
+        if (rs3 > 0 && d.has3 && dist < d.c3)
+            put_pair(P, P.pt3[pt], r, rinv, ex, P.R3, reinterpret_cast<FxEnt*>(B.pct3) + e * rs3, B.pcd3 + 4 * e);
+        if (rs4 > 0 && d.has4 && dist < d.c4)
+            put_pair(P, P.pt4[pt], r, rinv, ex, P.R4, reinterpret_cast<FxEnt*>(B.pct4) + e * rs4, B.pcd4 + 4 * e);
+    }
+    acc.flush_warp(B);
+    acc1.flush_warp(B);
+}
+
+// Forces and virial of every list entry from its summed force scalar: eight
+// lanes per atom, its entries in turn; the atom's own force is summed over the
+// lanes, the neighbours' go out as atomics.
+__global__ void __launch_bounds__(256) k_pair_forces(BatchView B) {
+    const int gl = threadIdx.x & 7;
+    const long long ngrp = (long long)gridDim.x * (blockDim.x / 8);
+    const long long per = (B.n_atoms_total + ngrp - 1) / ngrp;
+    const long long a0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 8 * per;
+    EVAcc acc;
+    for (long long k = 0; k < per; k++) {   // (all lanes of a warp make every round)
+        const long long a = a0 + k;
+        const bool have = a < B.n_atoms_total;
+        const long long b0 = have ? min(B.l2_off[a], B.n2_cap) : 0, b1 = have ? min(B.l2_off[a + 1], B.n2_cap) : 0;
+        double f[3] = {0.0, 0.0, 0.0};
+        if (have) {
+            const int s = B.atom_sys[a];
+            if (s != acc.s) { acc.flush(B); acc.s = s; }
+        }
+        for (long long e = b0 + gl; e < b1; e += 8) {
+            const double2 p = reinterpret_cast<const double2*>(B.pe + 4 * e)[0];
+            const double2 q = reinterpret_cast<const double2*>(B.pe + 4 * e)[1];
+            const double fs = q.y;
+            if (fs == 0.0) continue;
+            const double d[3] = {p.x, p.y, q.x}, g[3] = {fs * p.x, fs * p.y, fs * q.x};
+            for (int c = 0; c < 3; c++) f[c] += g[c];
+            add_force(B, B.l2_ghost[e], -g[0], -g[1], -g[2]);
+            acc.v[1] -= g[0] * d[0];
+            acc.v[2] -= g[0] * d[1];
+            acc.v[3] -= g[0] * d[2];
+            acc.v[4] -= g[1] * d[1];
+            acc.v[5] -= g[1] * d[2];
+            acc.v[6] -= g[2] * d[2];
+        }
+        for (int off = 4; off; off >>= 1)
+            for (int c = 0; c < 3; c++) f[c] += __shfl_xor_sync(kFull, f[c], off);
+        if (have && gl == 0) add_force(B, B.atom_self[a], f[0], f[1], f[2]);
+    }
+    acc.flush_warp(B);
+}
+
+// ---------------------------------------------------------------------------
+// Set-up and finish of a tile
+// ---------------------------------------------------------------------------
+// Shared memory of a block (all of it dynamic: allow_max_smem's limit leaves
+// no room for static arrays): the claimed tile, then interleaved
+// [entry][cluster]
+//   ENT:  double miss[NM * 4]         fc, fc gs / r, fc'/r, flags of pairs that no list holds
+//   else: double geo[NP * 4], fc[NP], fcd[NP], gs[NP]
+//   long long part[NW][NP + 1]        the warps' S and G
+//   FxEnt  tab[NT * rs]               T and dT limbs (3-body ENT: pairs ik, jk; else all pairs)
+template <int NB, int NW, bool ENT>
+struct FxSmem {
+    static constexpr int NP = Topo<NB>::NP;
+    static constexpr int KC = NB - 1;                       // pairs of the first atom
+    static constexpr int P0 = NB == 3 && ENT ? 1 : 0;       // first pair with a table here
+    static constexpr int ND = ENT ? (NP - KC) * 4 : NP * 7;
+    long long* tile;
+    double* d;
+    long long* part;
+    FxEnt* tab;
+    unsigned char* rest;
+    __device__ FxSmem(unsigned char* smem, int rs) {
+        tile = reinterpret_cast<long long*>(smem);
+        d = reinterpret_cast<double*>(smem + 16);
+        part = reinterpret_cast<long long*>(d + ND * kFxTile);
+        tab = reinterpret_cast<FxEnt*>(part + NW * (NP + 1) * kFxTile);
+        rest = reinterpret_cast<unsigned char*>(tab + (NP - P0) * rs * kFxTile);
+    }
+    __device__ FxEnt* table(int p, int rs) const { return tab + (p - P0) * rs * kFxTile; }
+    static size_t bytes(int rs) {
+        return 16 + sizeof(double) * (size_t)(ND + NW * (NP + 1)) * kFxTile +
+               sizeof(FxEnt) * (size_t)(NP - P0) * rs * kFxTile;
+    }
+};
+
+// ENT, cold path: a pair that its list does not hold (within rounding of the
+// search radius): its tables and scalars from the atoms themselves.
+template <int NB>
+__device__ __noinline__ void missing_pair(const BatchView& B, const DevParamSet& P, const TupleRec& R, int p,
+                                          const int* id, FxEnt* tab, double* scal) {
+    const int s = B.atom_sys[B.ghost_parent[id[0]]];
+    double dr[3], r, fc, fcd, gs;
+    pair_geom(B, B.sys[s].h, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], dr, r);
+    const int Rp = NB == 3 ? P.R3 : P.R4;
+    const PairTab Q = tuple_pair_x(R, p);
+    pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
+                 [&](int n, const Fx& t, const Fx& d) { tab[n * kFxTile] = fx_quad(t, d); });
+    scal[0] = fc;
+    scal[kFxTile] = fc * gs / r;
+    scal[2 * kFxTile] = fcd / r;
+    scal[3 * kFxTile] = (double)((r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0));
+}
+__device__ __noinline__ void missing_force(const BatchView& B, int ga, int gb, int s, double fs) {
+    double dr[3], r, vir[6] = {0, 0, 0, 0, 0, 0};
+    pair_geom(B, B.sys[s].h, ga, gb, dr, r);
+    add_force(B, ga, fs * dr[0], fs * dr[1], fs * dr[2]);
+    add_force(B, gb, -fs * dr[0], -fs * dr[1], -fs * dr[2]);
+    virial_add(vir, fs, dr);
+    for (int k = 0; k < 6; k++) atomicAdd(&B.ev[8 * s + 1 + k], vir[k]);
+}
+
+// Tables of this lane's cluster c into shared memory, spread over the warps.
+// ENT: gathered from the list entries ent[] (lanes without a cluster take entry
+// 0; which clusters are evaluated is known at the finish).  Else computed;
+// returns whether the cluster is evaluated (compute_3B/4B's early-outs).
+template <int NB, int NW, bool ENT>
 __device__ __forceinline__ bool fx_setup(const BatchView& B, const int* clusters, int c, const DevParamSet& P,
-                                         const TupleRec& R, int rs, const FxSmem<NB, NW>& m, int* id, int& s) {
-    constexpr int NP = Topo<NB>::NP, KC = NB - 1;
+                                         const TupleRec& R, int rs, const FxSmem<NB, NW, ENT>& m, int* ent) {
+    using M = FxSmem<NB, NW, ENT>;
+    constexpr int NP = M::NP, KC = M::KC;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const bool use_pc = NB == 3 ? B.use_pc3 : B.use_pc4;
-    const int* ce = NB == 3 ? B.c3e : B.c4e;
-    const double* pcd = NB == 3 ? B.pcd3 : B.pcd4;
-    const FxPair* pct = reinterpret_cast<const FxPair*>(NB == 3 ? B.pct3 : B.pct4);
     const int Rp = NB == 3 ? P.R3 : P.R4;
     bool active = c >= 0;
-    s = 0;
-    if (active) {
-        for (int k = 0; k < NB; k++) id[k] = clusters[(long long)NB * c + k];
-        s = B.atom_sys[B.ghost_parent[id[0]]];
-        const double* h = B.sys[s].h;
-        for (int sl = w; sl < NP; sl += NW) {
-            // with the cache the evaluated pairs come first, spread over the warps
-            const int p = use_pc ? (sl < NP - KC ? KC + sl : sl - (NP - KC)) : sl;
-            double dr[3], r;
-            if (use_pc && p < KC) {
-                const double* g = pcd + 8 * (long long)ce[(long long)KC * c + p];
-                dr[0] = g[0]; dr[1] = g[1]; dr[2] = g[2]; r = g[3];
-            } else {
+    if constexpr (ENT) {
+        const int* ce = NB == 3 ? B.c3e : B.c4e;
+        const FxEnt* pct = reinterpret_cast<const FxEnt*>(NB == 3 ? B.pct3 : B.pct4);
+#pragma unroll
+        for (int p = 0; p < NP; p++) ent[p] = active ? ce[(long long)NP * c + p] : 0;
+        for (int k = w; k < (NP - M::P0) * Rp; k += NW) {
+            const int p = M::P0 + k / Rp, n = k % Rp;
+            int e = ent[0];
+#pragma unroll
+            for (int q = 1; q < NP; q++) e = p == q ? ent[q] : e;
+            if (e >= 0) m.table(p, rs)[n * kFxTile + lane] = pct[(long long)e * rs + n];
+        }
+#pragma unroll
+        for (int p = KC; p < NP; p++)
+            if (ent[p] < 0 && w == 0) {
+                int id[NB];
+                for (int k = 0; k < NB; k++) id[k] = clusters[(long long)NB * c + k];
+                missing_pair<NB>(B, P, R, p, id, m.table(p, rs) + lane, m.d + (p - KC) * 4 * kFxTile + lane);
+            }
+        __syncthreads();
+    } else {
+        double* geo = m.d;
+        if (active) {
+            int id[NB];
+            for (int k = 0; k < NB; k++) id[k] = clusters[(long long)NB * c + k];
+            const double* h = B.sys[B.atom_sys[B.ghost_parent[id[0]]]].h;
+            for (int p = w; p < NP; p += NW) {
+                double dr[3], r;
                 pair_geom(B, h, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], dr, r);
+                for (int k = 0; k < 3; k++) geo[(4 * p + k) * kFxTile + lane] = dr[k];
+                geo[(4 * p + 3) * kFxTile + lane] = r;
             }
-            m.geo[(4 * p + 0) * kFxTile + lane] = dr[0];
-            m.geo[(4 * p + 1) * kFxTile + lane] = dr[1];
-            m.geo[(4 * p + 2) * kFxTile + lane] = dr[2];
-            m.geo[(4 * p + 3) * kFxTile + lane] = r;
         }
+        __syncthreads();
+        if (active)
+            for (int p = 0; p < NP; p++)
+                if (geo[(4 * p + 3) * kFxTile + lane] >= R.rout[p]) active = false;
+        if (active)
+            for (int p = w; p < NP; p += NW) {
+                FxEnt* tab = m.table(p, rs) + lane;
+                const double r = geo[(4 * p + 3) * kFxTile + lane];
+                const PairTab Q = tuple_pair_x(R, p);
+                if (r < Q.rin) atomicAdd(&B.flags[4], 1);
+                double fc, fcd, gs;
+                pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
+                             [&](int n, const Fx& t, const Fx& d) { tab[n * kFxTile] = fx_quad(t, d); });
+                geo[(4 * NP + p) * kFxTile + lane] = fc;
+                geo[(5 * NP + p) * kFxTile + lane] = fcd;
+                geo[(6 * NP + p) * kFxTile + lane] = gs;
+            }
+        __syncthreads();
     }
-    __syncthreads();
-    if (active)
-        for (int p = 0; p < NP; p++)
-            if (m.geo[(4 * p + 3) * kFxTile + lane] >= R.rout[p]) active = false;
-    if (active)
-        for (int sl = w; sl < NP; sl += NW) {
-            const int p = use_pc ? (sl < NP - KC ? KC + sl : sl - (NP - KC)) : sl;
-            FxPair* T = m.T + p * rs * kFxTile + lane;
-            FxPair* D = m.D + p * rs * kFxTile + lane;
-            double fc, fcd, gs;
-            if (use_pc && p < KC) {
-                const long long ent = ce[(long long)KC * c + p];
-                const double* g = pcd + 8 * ent;
-                const FxPair* tab = pct + ent * 2 * rs;
-                for (int n = 0; n < Rp; n++) {
-                    T[n * kFxTile] = tab[n];
-                    D[n * kFxTile] = tab[rs + n];
-                }
-                fc = g[4];
-                fcd = g[5];
-                gs = g[7];
-                if (g[6] != 0.0) atomicAdd(&B.flags[4], 1);
-            } else {
-                pair_setup_x(P, tuple_pair_x(R, p), m.geo[(4 * p + 3) * kFxTile + lane], T, D, kFxTile, Rp, fx_kd(Rp),
-                             fc, fcd, gs, B.flags);
-            }
-            m.fc[p * kFxTile + lane] = fc;
-            m.fcd[p * kFxTile + lane] = fcd;
-            m.gs[p * kFxTile + lane] = gs;
-        }
-    __syncthreads();
     return active;
 }
 
-// The warps' parts of S and the G's, added and turned into forces by warp 0.
-template <int NB, int NW>
-__device__ __forceinline__ void fx_finish(const BatchView& B, const FxSmem<NB, NW>& m, const TupleRec& R, bool active,
-                                          const int* id, int s, EVAcc& acc) {
+// The warps' parts of S and the G's, added and turned into force scalars (ENT,
+// added to the pairs' entries) or forces by warp 0.
+//   f_p = (prod_{q != p} fc_q / r_p) (fc_p G_p + fc'_p S), E = prod fc S
+template <int NB, int NW, bool ENT, typename Acc>
+__device__ __forceinline__ void fx_finish(const BatchView& B, const int* clusters, int c,
+                                          const FxSmem<NB, NW, ENT>& m, const TupleRec& R, bool active,
+                                          const int* ent, const long long* own, Acc& acc) {
     constexpr int NP = Topo<NB>::NP;
-    const int lane = threadIdx.x & 31;
-    if (NW > 1) __syncthreads();
-    if (threadIdx.x < 32 && active) {
-        double S = 0.0, dr[NP][4], fc[NP], fcd[NP], G[NP];
-        for (int w = 0; w < NW; w++) S += m.part[w * (NP + 1) * kFxTile + lane];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (NW > 1) {
+        for (int k = 0; k <= NP; k++) m.part[(w * (NP + 1) + k) * kFxTile + lane] = own[k];
+        __syncthreads();
+        if (w > 0) return;
+    }
+    double S, G[NP];
+    for (int k = 0; k <= NP; k++) {
+        long long v = own[k];
+        for (int u = 1; u < NW; u++) v += m.part[(u * (NP + 1) + k) * kFxTile + lane];
+        (k == 0 ? S : G[k - 1]) = (double)v;
+    }
+    const double unit = R.fx_amp * kFxUnit;
+    int s = 0;
+    if (active) s = B.atom_sys[B.ghost_parent[clusters[(long long)NB * c]]];
+    if constexpr (ENT) {
+        constexpr int KC = NB - 1;
+        const double* pcd = NB == 3 ? B.pcd3 : B.pcd4;
+        double fc[NP], ga[NP], ca[NP];
+        int flags = 0, oor = 0;
+#pragma unroll
         for (int p = 0; p < NP; p++) {
-            double g = 0.0;
-            for (int w = 0; w < NW; w++) g += m.part[(w * (NP + 1) + 1 + p) * kFxTile + lane];
-            G[p] = g * m.gs[p * kFxTile + lane] * R.fx_amp;
-            for (int k = 0; k < 4; k++) dr[p][k] = m.geo[(4 * p + k) * kFxTile + lane];
-            fc[p] = m.fc[p * kFxTile + lane];
-            fcd[p] = m.fcd[p * kFxTile + lane];
+            double fl;
+            if (p >= KC && ent[p] < 0) {
+                const double* q = m.d + (p - KC) * 4 * kFxTile + lane;
+                fc[p] = q[0]; ga[p] = q[kFxTile]; ca[p] = q[2 * kFxTile]; fl = q[3 * kFxTile];
+            } else {
+                const double2* q = reinterpret_cast<const double2*>(pcd + 4 * (long long)ent[p]);
+                const double2 x = q[0], y = q[1];
+                fc[p] = x.x; ga[p] = x.y; ca[p] = y.x; fl = y.y;
+            }
+            const int f = (int)fl;
+            flags |= f;
+            oor += f & kPairOor ? 1 : 0;
         }
-        cluster_epilogue<NB>(B, id, s, dr, fc, fcd, S * R.fx_amp, G, acc);
+        active = active && !(flags & kPairFar);   // compute_3B/4B's early-outs
+        double E = 0.0;
+        if (active) {
+            if (oor) atomicAdd(&B.flags[4], oor);
+            double rest[NP];   // unit times the other pairs' cutoffs
+            if constexpr (NB == 3) {
+                const double u0 = unit * fc[0];
+                rest[0] = unit * fc[1] * fc[2];
+                rest[1] = u0 * fc[2];
+                rest[2] = u0 * fc[1];
+            } else {
+                double suf = 1.0, pre = unit;
+#pragma unroll
+                for (int p = NP - 1; p > 0; p--) { rest[p] = suf; suf *= fc[p]; }
+                rest[0] = suf * unit;
+#pragma unroll
+                for (int p = 1; p < NP; p++) { pre *= fc[p - 1]; rest[p] *= pre; }
+            }
+            E = rest[NP - 1] * fc[NP - 1] * S;
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                const double fs = rest[p] * (ga[p] * G[p] + ca[p] * S);
+                if (p >= KC && ent[p] < 0) {
+                    const int* id = clusters + (long long)NB * c;
+                    missing_force(B, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], s, fs);
+                } else {
+                    atomicAdd(&B.pe[4 * (long long)ent[p] + 3], fs);
+                }
+            }
+        }
+        acc.add_warp(B, s, E, active);
+    } else if (active) {
+        const double* geo = m.d;
+        double dr[NP][4], fc[NP], fcd[NP];
+        int id[NB];
+        for (int k = 0; k < NB; k++) id[k] = clusters[(long long)NB * c + k];
+        for (int p = 0; p < NP; p++) {
+            for (int k = 0; k < 4; k++) dr[p][k] = geo[(4 * p + k) * kFxTile + lane];
+            fc[p] = geo[(4 * NP + p) * kFxTile + lane];
+            fcd[p] = geo[(5 * NP + p) * kFxTile + lane];
+            G[p] *= unit * geo[(6 * NP + p) * kFxTile + lane];
+        }
+        cluster_epilogue<NB>(B, id, s, dr, fc, fcd, S * unit, G, acc);
     }
 }
 
@@ -200,29 +418,40 @@ __device__ __forceinline__ long long fx_claim(unsigned long long* head, long lon
     return t;
 }
 
+template <bool ENT>
+struct AccOf {
+    using type = EVAcc;
+};
+template <>
+struct AccOf<true> {
+    using type = EAcc;
+};
+
+// ---------------------------------------------------------------------------
 // 3-body.  X = T_ij and the row sums z stay in registers (RX powers, unrolled;
-// a column's mask says which of them it has), Y_J is formed per column, and
-// the column sums w_J are folded over q_jk within a run of q_ik.
-template <int RX, int NW>
+// a column's mask says which pairs of them it has), Y_J is formed per column,
+// and the column sums w_J are folded over q_jk within a run of q_ik.
+// ---------------------------------------------------------------------------
+template <int RX, int NW, bool ENT>
 __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clusters, const int* perm,
                                                      const long long* perm_n, long long perm_cap, int rs) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const FxSmem<3, NW> m(smem, rs);
+    const FxSmem<3, NW, ENT> m(smem, rs);
     FxEnt* strm = reinterpret_cast<FxEnt*>(m.rest);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long ntiles = min(*perm_n, perm_cap) / kFxTile;
     int loaded = -1;
     const DevParamSet* loaded_set = nullptr;
-    EVAcc acc;
+    typename AccOf<ENT>::type acc;
     for (;;) {
         const long long tile = fx_claim(&B.queue[0], m.tile);
         if (tile >= ntiles) break;
         const long long base = tile * kFxTile;
         const int c0 = perm[base];
         if (c0 < 0) continue;   // uniform: a tile never starts in a bucket's padding
-        int id[3], s, u;
+        int id0[3], s0, u, ent[3];
         const DevParamSet* P;
-        const TupleRec* R = cluster_tuple<3>(B, clusters, c0, id, s, P, u);
+        const TupleRec* R = cluster_tuple<3>(B, clusters, c0, id0, s0, P, u);
         int len = R->fx_split[8];
         if (!ck_bound(B, R->fx_off >= 0 && R->fx_off + (long long)len <= P->n_fx3)) len = 0;
         if (R->fx_off != loaded || P != loaded_set) {
@@ -230,36 +459,37 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
             loaded = R->fx_off;
             loaded_set = P;
         }
-        const bool active = fx_setup<3, NW>(B, clusters, perm[base + lane], *P, *R, rs, m, id, s);
+        const int c = perm[base + lane];
+        const bool active = fx_setup<3, NW, ENT>(B, clusters, c, *P, *R, rs, m, ent);
         const int Rp = P->R3;
-        const FxPair *T0 = m.T + lane, *T1 = T0 + rs * kFxTile, *T2 = T1 + rs * kFxTile;
-        const FxPair *D0 = m.D + lane, *D1 = D0 + rs * kFxTile, *D2 = D1 + rs * kFxTile;
+        const FxEnt* t0 = ENT ? reinterpret_cast<const FxEnt*>(B.pct3) + (long long)ent[0] * rs : m.table(0, rs) + lane;
+        constexpr int st0 = ENT ? 1 : kFxTile;
+        const FxEnt *t1 = m.table(1, rs) + lane, *t2 = m.table(2, rs) + lane;
         Fx X[RX];
         FxAcc z[RX];
 #pragma unroll
-        for (int q = 0; q < RX; q++) X[q] = q < Rp ? fx_load(T0[q * kFxTile]) : Fx{0, 0};
+        for (int q = 0; q < RX; q++) X[q] = q < Rp ? quad_t(t0 + q * st0) : Fx{0, 0};
         FxAcc g1, g2, ca, cb;
-        Fx tb{0, 0}, db{0, 0};
+        FxEnt tb{0, 0, 0, 0};
         int qb = -1;
         int o = len ? R->fx_split[8 * w / NW] : 0;
         const int o1 = len ? R->fx_split[8 * (w + 1) / NW] : 0;
         FxEnt hd = strm[o];   // (the buffer has room for a header past the stream)
         while (o < o1) {
-            const int b = hd.x, c = hd.y, mask = hd.z;
+            const int b = hd.x, mask = hd.z;
+            const FxEnt tc = t2[hd.y * kFxTile];
             const FxEnt* q4 = strm + o + 1;
             o += 1 + __popc(mask);
             hd = strm[o];
             if (b != qb) {   // uniform: a new run of q_ik
-                g1.mac(db, ca.value<0>());
-                g2.mac(tb, cb.value<0>());
+                g1.mac(Fx{tb.z, tb.w}, ca.value<0>());
+                g2.mac(Fx{tb.x, tb.y}, cb.value<0>());
                 ca = FxAcc();
                 cb = FxAcc();
-                tb = fx_load(T1[b * kFxTile]);
-                db = fx_load(D1[b * kFxTile]);
+                tb = t1[b * kFxTile];
                 qb = b;
             }
-            const Fx tc = fx_load(T2[c * kFxTile]), dc = fx_load(D2[c * kFxTile]);
-            const Fx Y = fx_mul(tb, tc);
+            const Fx Y = fx_mul(Fx{tb.x, tb.y}, Fx{tc.x, tc.y});
             FxAcc wj;
 #pragma unroll
             for (int g = 0; g < RX / 2; g++)
@@ -271,55 +501,56 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
                     z[2 * g + 1].mac(Fx{a.z, a.w}, Y);
                 }
             const Fx wv = wj.value<kFxDown>();
-            ca.mac(tc, wv);
-            cb.mac(dc, wv);
+            ca.mac(Fx{tc.x, tc.y}, wv);
+            cb.mac(Fx{tc.z, tc.w}, wv);
         }
-        g1.mac(db, ca.value<0>());
-        g2.mac(tb, cb.value<0>());
+        g1.mac(Fx{tb.z, tb.w}, ca.value<0>());
+        g2.mac(Fx{tb.x, tb.y}, cb.value<0>());
         FxAcc S, g0;
 #pragma unroll
         for (int q = 0; q < RX; q++)
             if (q < Rp) {
+                const FxEnt t = t0[q * st0];
                 const Fx zv = z[q].template value<kFxDown>();
-                S.mac(X[q], zv);
-                g0.mac(fx_load(D0[q * kFxTile]), zv);
+                S.mac(Fx{t.x, t.y}, zv);
+                g0.mac(Fx{t.z, t.w}, zv);
             }
-        double* part = m.part + w * 4 * kFxTile + lane;
-        part[0 * kFxTile] = S.real(kFxUnit);
-        part[1 * kFxTile] = g0.real(kFxUnit);
-        part[2 * kFxTile] = g1.real(kFxUnit);
-        part[3 * kFxTile] = g2.real(kFxUnit);
-        fx_finish<3, NW>(B, m, *R, active, id, s, acc);
+        const long long own[4] = {S.sum(), g0.sum(), g1.sum(), g2.sum()};
+        fx_finish<3, NW, ENT>(B, clusters, c, m, *R, active, ent, own, acc);
     }
     if (w == 0) acc.flush_warp(B);
 }
 
-// One side of the 4-body contraction: the entries [o, o1) of its stream, V the
-// other side's products, t / d the side's three pair tables.  The record sums
-// are folded over the last pair's power, then the middle one's, then the
-// first one's, as their records are sorted: out[0] = sum_I X_I z_I, out[1..3]
-// = the three pairs' gradients.
-__device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, int o1, const FxPair* V, const FxPair* t,
-                                        const FxPair* d, int rs, double* out) {
-    const FxPair *t1 = t + rs * kFxTile, *t2 = t1 + rs * kFxTile, *d1 = d + rs * kFxTile, *d2 = d1 + rs * kFxTile;
+// ---------------------------------------------------------------------------
+// 4-body
+// ---------------------------------------------------------------------------
+// One side: the records [o, o1) of its stream, V the other side's products, t
+// the side's three pair tables.  The record sums are folded over the last
+// pair's power, then the middle one's, then the first one's, as their records
+// are sorted: out[0] = sum_I X_I z_I, out[1..3] = the three pairs' gradients.
+__device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, int o1, const FxPair* V, const FxEnt* t,
+                                        int rs, long long* out) {
+    const FxEnt *t1 = t + rs * kFxTile, *t2 = t1 + rs * kFxTile;
     FxAcc S, g0, g1, g2, ra, rb, rP, rQ, rR;
     int q0 = -1, q1 = -1;
     auto fold1 = [&]() {
         if (q1 < 0) return;
-        const Fx a = ra.value<0>(), b = rb.value<0>(), tv = fx_load(t1[q1 * kFxTile]);
-        rP.mac(tv, a);
-        rQ.mac(fx_load(d1[q1 * kFxTile]), a);
-        rR.mac(tv, b);
+        const Fx a = ra.value<0>(), b = rb.value<0>();
+        const FxEnt v = t1[q1 * kFxTile];
+        rP.mac(Fx{v.x, v.y}, a);
+        rQ.mac(Fx{v.z, v.w}, a);
+        rR.mac(Fx{v.x, v.y}, b);
         ra = FxAcc();
         rb = FxAcc();
     };
     auto fold0 = [&]() {
         if (q0 < 0) return;
-        const Fx p = rP.value<0>(), tv = fx_load(t[q0 * kFxTile]);
-        S.mac(tv, p);
-        g0.mac(fx_load(d[q0 * kFxTile]), p);
-        g1.mac(tv, rQ.value<0>());
-        g2.mac(tv, rR.value<0>());
+        const Fx p = rP.value<0>();
+        const FxEnt v = t[q0 * kFxTile];
+        S.mac(Fx{v.x, v.y}, p);
+        g0.mac(Fx{v.z, v.w}, p);
+        g1.mac(Fx{v.x, v.y}, rQ.value<0>());
+        g2.mac(Fx{v.x, v.y}, rR.value<0>());
         rP = FxAcc();
         rQ = FxAcc();
         rR = FxAcc();
@@ -342,73 +573,73 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
             q1 = r1;
         }
         const Fx zv = z.value<kFxDown>();
-        ra.mac(fx_load(t2[r2 * kFxTile]), zv);
-        rb.mac(fx_load(d2[r2 * kFxTile]), zv);
+        const FxEnt v = t2[r2 * kFxTile];
+        ra.mac(Fx{v.x, v.y}, zv);
+        rb.mac(Fx{v.z, v.w}, zv);
     }
     fold1();
     fold0();
-    out[0] = S.real(kFxUnit);
-    out[1] = g0.real(kFxUnit);
-    out[2] = g1.real(kFxUnit);
-    out[3] = g2.real(kFxUnit);
+    out[0] = S.sum();
+    out[1] = g0.sum();
+    out[2] = g1.sum();
+    out[3] = g2.sum();
 }
 
-// 4-body.  With one warp it takes the rows, then the columns; with more, half
-// of the warps take the rows and half the columns.
-template <int NW>
+// With one warp it takes the rows, then the columns; with more, half of the
+// warps take the rows and half the columns.
+template <int NW, bool ENT>
 __global__ void __launch_bounds__(32 * NW) k_forcex4(BatchView B, const int* clusters, const int* perm,
                                                      const long long* perm_n, long long perm_cap, int rs) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const FxSmem<4, NW> m(smem, rs);
-    FxPair* X = m.rest;
+    const FxSmem<4, NW, ENT> m(smem, rs);
+    FxPair* X = reinterpret_cast<FxPair*>(m.rest);
     FxPair* Y = X + rs * rs * rs * kFxTile;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long ntiles = min(*perm_n, perm_cap) / kFxTile;
-    EVAcc acc;
+    typename AccOf<ENT>::type acc;
     for (;;) {
         const long long tile = fx_claim(&B.queue[1], m.tile);
         if (tile >= ntiles) break;
         const long long base = tile * kFxTile;
         const int c0 = perm[base];
         if (c0 < 0) continue;   // uniform
-        int id[4], s, u;
+        int id0[4], s0, u, ent6[6];
         const DevParamSet* P;
-        const TupleRec* R = cluster_tuple<4>(B, clusters, c0, id, s, P, u);
-        const bool active = fx_setup<4, NW>(B, clusters, perm[base + lane], *P, *R, rs, m, id, s);
+        const TupleRec* R = cluster_tuple<4>(B, clusters, c0, id0, s0, P, u);
+        const int c = perm[base + lane];
+        const bool active = fx_setup<4, NW, ENT>(B, clusters, c, *P, *R, rs, m, ent6);
         const int Rp = P->R4;
-        const FxPair *T = m.T + lane, *D = m.D + lane;
+        const FxEnt* T = m.tab + lane;
         // the products X_I, Y_J: the first two pairs' product per (q0, q1), spread over the warps
         for (int k = w; k < 2 * Rp * Rp; k += NW) {
             const int side = k >= Rp * Rp ? 1 : 0, q01 = k - side * Rp * Rp;
-            const FxPair* t = T + 3 * side * rs * kFxTile;
-            const Fx v = fx_mul(fx_load(t[(q01 / Rp) * kFxTile]), fx_load(t[(rs + q01 % Rp) * kFxTile]));
+            const FxEnt* t = T + 3 * side * rs * kFxTile;
+            const Fx v = fx_mul(quad_t(t + (q01 / Rp) * kFxTile), quad_t(t + (rs + q01 % Rp) * kFxTile));
             FxPair* dst = (side ? Y : X) + q01 * Rp * kFxTile + lane;
-            for (int q = 0; q < Rp; q++) dst[q * kFxTile] = fx_store(fx_mul(v, fx_load(t[(2 * rs + q) * kFxTile])));
+            for (int q = 0; q < Rp; q++) dst[q * kFxTile] = fx_store(fx_mul(v, quad_t(t + (2 * rs + q) * kFxTile)));
         }
         __syncthreads();
         const bool ok = ck_bound(B, R->fx_off >= 0 && R->fx_off + (long long)R->fx_split[8] <= P->n_fx4);
         const FxEnt* ent = P->fx4 + R->fx_off;
-        double* part = m.part + w * 7 * kFxTile + lane;
+        long long own[7] = {0, 0, 0, 0, 0, 0, 0};
         if (NW == 1) {
-            double a[4], b[4];
-            fx_side(ent, ok ? R->fx_split[0] : 0, ok ? R->fx_split[4] : 0, Y + lane, T, D, rs, a);
-            fx_side(ent, ok ? R->fx_split[4] : 0, ok ? R->fx_split[8] : 0, X + lane, T + 3 * rs * kFxTile,
-                    D + 3 * rs * kFxTile, rs, b);
-            for (int k = 0; k < 4; k++) part[k * kFxTile] = a[k];
-            for (int k = 1; k < 4; k++) part[(3 + k) * kFxTile] = b[k];
+            long long b[4];
+            fx_side(ent, ok ? R->fx_split[0] : 0, ok ? R->fx_split[4] : 0, Y + lane, T, rs, own);
+            fx_side(ent, ok ? R->fx_split[4] : 0, ok ? R->fx_split[8] : 0, X + lane, T + 3 * rs * kFxTile, rs, b);
+            for (int k = 1; k < 4; k++) own[3 + k] = b[k];
         } else {
             constexpr int H = NW > 1 ? NW / 2 : 1;   // warps per side
             const int side = w / H, k0 = 4 * side + 4 * (w % H) / H, k1 = 4 * side + 4 * (w % H + 1) / H;
-            double a[4];
+            long long a[4];
             fx_side(ent, ok ? R->fx_split[k0] : 0, ok ? R->fx_split[k1] : 0, (side ? X : Y) + lane,
-                    T + 3 * side * rs * kFxTile, D + 3 * side * rs * kFxTile, rs, a);
-            part[0] = side ? 0.0 : a[0];
+                    T + 3 * side * rs * kFxTile, rs, a);
+            own[0] = side ? 0 : a[0];
             for (int k = 1; k < 4; k++) {
-                part[k * kFxTile] = side ? 0.0 : a[k];
-                part[(3 + k) * kFxTile] = side ? a[k] : 0.0;
+                own[k] = side ? 0 : a[k];
+                own[3 + k] = side ? a[k] : 0;
             }
         }
-        fx_finish<4, NW>(B, m, *R, active, id, s, acc);
+        fx_finish<4, NW, ENT>(B, clusters, c, m, *R, active, ent6, own, acc);
     }
     if (w == 0) acc.flush_warp(B);
 }
@@ -421,61 +652,79 @@ unsigned fx_grid(const void* kern, int threads, size_t smem, long long tiles) {
     return (unsigned)(want < tiles ? want : tiles);
 }
 
-template <int RX, int NW>
+template <int RX, int NW, bool ENT>
 void launch_x3(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     const int rs = L.rf3;
-    const size_t smem = FxSmem<3, NW>::bytes(rs) + sizeof(FxEnt) * (size_t)(L.xs3 + 1);
-    auto kern = k_forcex3<RX, NW>;
+    const size_t smem = FxSmem<3, NW, ENT>::bytes(rs) + sizeof(FxEnt) * (size_t)(L.xs3 + 1);
+    auto kern = k_forcex3<RX, NW, ENT>;
     const unsigned grid = fx_grid((const void*)kern, 32 * NW, smem, (B.perm3_cap + kFxTile - 1) / kFxTile);
     count_launch(), kern<<<grid, 32 * NW, smem, st>>>(B, B.c3, B.perm3, B.bk_start + B.nbk3, B.perm3_cap, rs);
 }
 
-template <int NW>
+template <int NW, bool ENT>
 void launch_x3_nw(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    if (L.rf3 <= 4) launch_x3<4, NW>(B, L, st);
-    else if (L.rf3 <= 8) launch_x3<8, NW>(B, L, st);
-    else if (L.rf3 <= 10) launch_x3<10, NW>(B, L, st);
-    else launch_x3<12, NW>(B, L, st);
+    if (L.rf3 <= 4) launch_x3<4, NW, ENT>(B, L, st);
+    else if (L.rf3 <= 8) launch_x3<8, NW, ENT>(B, L, st);
+    else if (L.rf3 <= 10) launch_x3<10, NW, ENT>(B, L, st);
+    else launch_x3<12, NW, ENT>(B, L, st);
 }
 
-template <int NW>
+template <int NW, bool ENT>
 void launch_x4_nw(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     const int rs = L.rf4;
-    const size_t smem = FxSmem<4, NW>::bytes(rs) + sizeof(FxPair) * (size_t)2 * rs * rs * rs * kFxTile;
-    auto kern = k_forcex4<NW>;
+    const size_t smem = FxSmem<4, NW, ENT>::bytes(rs) + sizeof(FxPair) * (size_t)2 * rs * rs * rs * kFxTile;
+    auto kern = k_forcex4<NW, ENT>;
     const unsigned grid = fx_grid((const void*)kern, 32 * NW, smem, (B.perm4_cap + kFxTile - 1) / kFxTile);
     count_launch(), kern<<<grid, 32 * NW, smem, st>>>(B, B.c4, B.perm4, B.bk_start + B.nbk3 + 1 + B.nbk4,
                                                        B.perm4_cap, rs);
 }
 
+template <bool ENT>
+void launch_x3_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
+    switch (L.ftpc3) {
+        case 1: launch_x3_nw<1, ENT>(B, L, st); break;
+        case 2: launch_x3_nw<2, ENT>(B, L, st); break;
+        case 4: launch_x3_nw<4, ENT>(B, L, st); break;
+        default: launch_x3_nw<8, ENT>(B, L, st); break;
+    }
+}
+
+template <bool ENT>
+void launch_x4_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
+    switch (L.ftpc4) {
+        case 1: launch_x4_nw<1, ENT>(B, L, st); break;
+        case 2: launch_x4_nw<2, ENT>(B, L, st); break;
+        case 4: launch_x4_nw<4, ENT>(B, L, st); break;
+        default: launch_x4_nw<8, ENT>(B, L, st); break;
+    }
+}
+
 }  // namespace
 
-void launch_pair_tables_x(const BatchView& B, const int* l2_owner, int nbody, const ForceLaunch& L, cudaStream_t st) {
-    if (!(nbody == 3 ? B.use_pc3 : B.use_pc4) || B.n2_cap <= 0) return;
-    const long long want = (long long)sm_count() * 8, need = (B.n2_cap + 255) / 256;
+void launch_pairs_x(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st) {
+    const long long ntot = B.n2_cap > B.n_atoms_total ? B.n2_cap : B.n_atoms_total;
+    if (ntot <= 0) return;
+    const long long want = (long long)sm_count() * 12, need = (ntot + 127) / 128;
     const unsigned grid = (unsigned)(want < need ? want : need);
-    if (nbody == 3) count_launch(), k_pair_tables_x<3><<<grid, 256, 0, st>>>(B, l2_owner, L.rf3);
-    else count_launch(), k_pair_tables_x<4><<<grid, 256, 0, st>>>(B, l2_owner, L.rf4);
+    count_launch(), k_pairs_x<<<grid, 128, 0, st>>>(B, l2_owner, B.nbk3 > 0 ? L.rf3 : 0, B.nbk4 > 0 ? L.rf4 : 0);
+}
+
+void launch_pair_forces(const BatchView& B, cudaStream_t st) {
+    if (B.n_atoms_total <= 0) return;
+    const long long want = (long long)sm_count() * 6, need = (B.n_atoms_total + 31) / 32;
+    count_launch(), k_pair_forces<<<(unsigned)(want < need ? want : need), 256, 0, st>>>(B);
 }
 
 void launch_force3x(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     if (B.perm3_cap <= 0 || B.nbk3 <= 0 || L.rf3 <= 0) return;
-    switch (L.ftpc3) {
-        case 1: launch_x3_nw<1>(B, L, st); break;
-        case 2: launch_x3_nw<2>(B, L, st); break;
-        case 4: launch_x3_nw<4>(B, L, st); break;
-        default: launch_x3_nw<8>(B, L, st); break;
-    }
+    if (B.all_pairs) launch_x3_ent<true>(B, L, st);
+    else launch_x3_ent<false>(B, L, st);
 }
 
 void launch_force4x(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     if (B.perm4_cap <= 0 || B.nbk4 <= 0 || L.rf4 <= 0) return;
-    switch (L.ftpc4) {
-        case 1: launch_x4_nw<1>(B, L, st); break;
-        case 2: launch_x4_nw<2>(B, L, st); break;
-        case 4: launch_x4_nw<4>(B, L, st); break;
-        default: launch_x4_nw<8>(B, L, st); break;
-    }
+    if (B.all_pairs) launch_x4_ent<true>(B, L, st);
+    else launch_x4_ent<false>(B, L, st);
 }
 
 }  // namespace ck

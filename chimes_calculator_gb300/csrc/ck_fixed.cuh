@@ -52,15 +52,14 @@ struct FxAcc {
     template <int DOWN>
     __device__ __forceinline__ Fx value() const {
         if constexpr (DOWN == 0) {
-            return fx_split(hi + ((mid + (1LL << (kFxLimb - 1))) >> kFxLimb));
+            return fx_split(sum());
         } else {
             return fx_split((hi + (mid >> kFxLimb) + (1LL << (DOWN - 1))) >> DOWN);
         }
     }
-    // the sum in units of full scale, for a sum at 2^scale
-    __device__ __forceinline__ double real(double unit) const {
-        return ((double)hi + (double)mid * (1.0 / (double)(1LL << kFxLimb))) * unit;
-    }
+    // the sum as an integer at its scale, and times `unit`
+    __device__ __forceinline__ long long sum() const { return hi + ((mid + (1LL << (kFxLimb - 1))) >> kFxLimb); }
+    __device__ __forceinline__ double real(double unit) const { return (double)sum() * unit; }
 };
 constexpr int kFxDown = kFxCoef - kFxSum;   // record sums: 2^61 -> 2^59
 constexpr double kFxUnit = 1.0 / (double)(1LL << kFxSum);
@@ -72,69 +71,114 @@ __device__ __forceinline__ long long fx_2x(long long x, long long t) {
     return (hi << 3) | (long long)(lo >> 61);
 }
 
-// Chebyshev tables and cutoff of one pair (set_cheby_polys, chimesFF.h:542-628,
-// set_polys_out_of_range, chimesFF.cpp:1572-1613, get_fcut, chimesFF.h:347-386):
-// T[n] and n U_{n-1}(x) 2^-kd, n < nT, at T[n * stride], D[n * stride]; fc and
-// fc'; gs with dT_n/dr = gs D[n].  Below the inner cutoff the extrapolated
-// T_n + k dT_n can exceed one: both tables are scaled down by 2^s and fc, fc'
-// carry the 2^s (every term of S and of the G's has one factor of each pair).
-__device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab& Q, double r, FxPair* T, FxPair* D,
-                                             int stride, int nT, int kd, double& fc, double& fcd, double& gs,
-                                             int* flags) {
-    const double rin = Q.rin;
-    const bool oor = r < rin;
-    const double rr = oor ? rin : r;
-    const double e = exp(-rr * Q.inv_lam);
-    const double xd = (e - Q.xavg) * Q.inv_xdiff;
-    const double g = -e * Q.inv_lam * Q.inv_xdiff;
-    const double finv = Q.fc_inv;
-    if (!P.tersoff) {
-        const double f0 = 1.0 - r * finv;
-        fc = f0 * f0 * f0;
-        fcd = f0 * f0 * (-3.0 * finv);
-    } else {
-        const double th = Q.fc_th;
-        if (r < th) { fc = 1.0; fcd = 0.0; }
-        else if (r > Q.rout) { fc = 0.0; fcd = 0.0; }
-        else {
-            const double f0 = (r - th) * finv * kPi + kPi / 2.0;
-            double sn, cs;
-            sincos(f0, &sn, &cs);
-            fc = 0.5 + 0.5 * sn;
-            fcd = 0.5 * cs * (kPi * finv);
-        }
-    }
-    gs = g * (double)(1 << kd);
-    double k = 0.0, damp = 1.0;
-    int s = 0;
-    if (oor) {
-        if (flags) atomicAdd(&flags[4], 1);
-        damp = exp((r - rin) / P.inner_smooth);
-        k = P.inner_smooth * (damp - 1.0) * g;
-        double bound = 1.0 + fabs(k) * (double)(1 << kd);
-        while (bound > 1.0 && s < 40) { bound *= 0.5; s++; }
-        const double up = (double)(1LL << s);
-        fc *= up;
-        fcd *= up;
-    }
+// The Chebyshev recursions at x (in [-1, 1]): f(n, T_n, n U_{n-1} 2^-kd), n =
+// 0..nT-1, both at 2^56 (T is kept at 2^60 and U, below 64, at 2^57 on the way).
+template <typename F>
+__device__ __forceinline__ void fx_chebyshev(double xd, int nT, int kd, F&& f) {
     const long long x = __double2ll_rn(xd * (double)(1LL << 62));
-    // T at 2^60 and U at 2^58 along their recursions: tn, tp = T_n, T_{n+1}; um, un = U_{n-1}, U_n
-    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 58;
+    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 57;   // T_n, T_{n+1}, U_{n-1}, U_n
     for (int n = 0; n < nT; n++) {
-        long long t = (tn + 8) >> 4;
-        long long d = __mul64hi(um, (long long)n << (62 - kd));
-        if (oor) {
-            const double dn = 1.0 / (double)(1LL << s);
-            t = __double2ll_rn(((double)t + k * (double)(1 << kd) * (double)d) * dn);
-            d = __double2ll_rn((double)d * damp * dn);
-        }
-        T[n * stride] = fx_store(fx_split(t));
-        D[n * stride] = fx_store(fx_split(d));
+        f(n, (tn + 8) >> 4, __mul64hi(um, (long long)n << (63 - kd)));
         const long long t2 = fx_2x(x, tp) - tn, u2 = fx_2x(x, un) - um;
         tn = tp;
         tp = t2;
         um = un;
         un = u2;
+    }
+}
+
+// get_fcut (chimesFF.h:347-386) with the precomputed threshold and reciprocal
+__device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double rout, double th, double finv,
+                                       double& fc, double& fcd) {
+    if (!P.tersoff) {
+        const double f0 = 1.0 - r * finv;
+        fc = f0 * f0 * f0;
+        fcd = f0 * f0 * (-3.0 * finv);
+    } else if (r < th) {
+        fc = 1.0;
+        fcd = 0.0;
+    } else if (r > rout) {
+        fc = 0.0;
+        fcd = 0.0;
+    } else {
+        const double f0 = (r - th) * finv * kPi + kPi / 2.0;
+        double sn, cs;
+        sincos(f0, &sn, &cs);
+        fc = 0.5 + 0.5 * sn;
+        fcd = 0.5 * cs * (kPi * finv);
+    }
+}
+
+// Chebyshev tables and cutoff of one pair (set_cheby_polys, chimesFF.h:542-628,
+// set_polys_out_of_range, chimesFF.cpp:1572-1613): put(n, T_n, D_n) for n <
+// nT with D_n = n U_{n-1}(x) 2^-kd; fc and fc'; gs with dT_n/dr = gs D_n.
+// ex = exp(-r / lambda).  Below the inner cutoff the extrapolated T_n + k dT_n
+// can exceed one: both tables are scaled down by 2^s and fc, fc' carry the
+// 2^s (every term of S and of the G's has one factor of each pair).
+template <typename F>
+__device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab& Q, double r, double ex, int nT,
+                                             int kd, double& fc, double& fcd, double& gs, F&& put) {
+    const bool oor = r < Q.rin;
+    if (oor) ex = exp(-Q.rin * Q.inv_lam);
+    const double xd = (ex - Q.xavg) * Q.inv_xdiff;
+    const double g = -ex * Q.inv_lam * Q.inv_xdiff;
+    fcut_x(P, r, Q.rout, Q.fc_th, Q.fc_inv, fc, fcd);
+    gs = g * (double)(1 << kd);
+    if (!oor) {
+        fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
+        return;
+    }
+    const double damp = exp((r - Q.rin) / P.inner_smooth);
+    const double k = P.inner_smooth * (damp - 1.0) * gs;
+    int s = 0;
+    for (double bound = 1.0 + fabs(k); bound > 1.0 && s < 40; s++) bound *= 0.5;
+    const double up = (double)(1LL << s), down = 1.0 / up;
+    fc *= up;
+    fcd *= up;
+    fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) {
+        put(n, fx_split(__double2ll_rn(((double)t + k * (double)d) * down)),
+            fx_split(__double2ll_rn((double)d * damp * down)));
+    });
+}
+
+// compute_2B (chimesFF.cpp:1644-1775) of one pair below its outer cutoff, as
+// pair_2b: energy and force scalar over r, the Chebyshev sum in fixed point.
+// ex = exp(-r / lambda), rinv = 1 / r.
+__device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& pr, double r, double rinv, double ex,
+                                          int* flags, double& E, double& fs) {
+    const bool oor = r < pr.rin;
+    if (oor) ex = exp(-pr.rin * pr.inv_lam);
+    const double xd = (ex - pr.xavg) * pr.inv_xdiff;
+    const int kd = fx_kd(P.o2 + 1);
+    const double gs = -ex * pr.inv_lam * pr.inv_xdiff * (double)(1 << kd);
+    const FxPair* a = P.fx2 + pr.coef_off;
+    FxAcc s, g;
+    fx_chebyshev(xd, P.o2 + 1, kd, [&](int n, long long t, long long d) {
+        const Fx c = fx_load(a[n]);
+        s.mac(c, fx_split(t));
+        g.mac(c, fx_split(d));
+    });
+    const double unit = pr.fx_amp * (1.0 / (double)(1LL << kFxCoef));
+    double S = s.real(unit), G = g.real(unit) * gs;
+    if (oor) {
+        atomicAdd(&flags[4], 1);
+        const double damp = exp((r - pr.rin) / P.inner_smooth);
+        S += P.inner_smooth * (damp - 1.0) * G;
+        G *= damp;
+    }
+    double fc, fcd;
+    fcut_x(P, r, pr.rout, pr.fc_th, pr.fc_inv, fc, fcd);
+    E = fc * S;
+    fs = (fc * G + fcd * S) * rinv;
+    // get_penalty (chimesFF.h:388-419)
+    if (r - P.pen_dist < pr.rin) {
+        const double rp = pr.rin + P.pen_dist - r;
+        atomicMax(&flags[2], r < pr.rin ? 2 : 1);
+        if (rp > 0.0) {
+            atomicAdd(&flags[3], 1);
+            E += rp * rp * rp * P.pen_scale;
+            fs += (-3.0 * rp * rp * P.pen_scale) / r;
+        }
     }
 }
 

@@ -73,7 +73,11 @@ void launch_pair_tables(const BatchView& B, const int* l2_owner, int nbody, cons
 void launch_force3f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 // The FP64 form of the factored contraction, in 64-bit fixed point (ck_fixed.cu).
-void launch_pair_tables_x(const BatchView& B, const int* l2_owner, int nbody, const ForceLaunch& L, cudaStream_t st);
+// Pair-entry form (B.all_pairs): launch_pairs_x does the 1-body and 2-body terms
+// and the pairs' tables before the contractions, launch_pair_forces the forces
+// and virial of every pair after them.
+void launch_pairs_x(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st);
+void launch_pair_forces(const BatchView& B, cudaStream_t st);
 void launch_force3x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 // Tensor-core 3-body contraction (ck_tensor.cu): mixed form, R3 powers per

@@ -156,6 +156,7 @@ __global__ void k_atoms(BatchView B) {
         }
         B.ghost_parent[q] = (int)r;
         B.ghost_id[q] = rl;
+        if (B.ghost_sh) B.ghost_sh[q] = kShiftBias;
         B.atom_self[r] = (int)q;
         B.atom_sys[r] = s;
         B.atom_type[r] = B.in_type[d.in_off + a];
@@ -243,6 +244,7 @@ __global__ void k_ghosts(BatchView B) {
         B.ghost_xf[3 * q + c] = (float)xn[c];
     }
     B.ghost_parent[q] = (int)r;
+    if (B.ghost_sh) B.ghost_sh[q] = pack_shift(i0, i1, i2);
     B.ghost_id[q] = image_index(i0, i1, i2, d.n_layers, d.side) * d.n_atoms + rl;
 }
 
@@ -480,6 +482,7 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, const long long* b
                 B.l2_ghost[pos] = ajj;
                 B.l2_dist[pos] = dd;
                 l2_owner[pos] = (int)r;
+                if (B.l2_key) B.l2_key[pos] = (long long)par << 32 | B.ghost_sh[ajj];
                 // x, y, z: FP32 displacement for the enumeration's prefilter;
                 // w: the neighbour's parent atom (int bits; saves the
                 // enumeration a dependent load per candidate) with the exact
@@ -684,6 +687,58 @@ __global__ void k_enum(BatchView B, const int* l2_owner) {
     }
 }
 
+// List entry of the pair (j, k) of two images in one atom's list: the entry of
+// j's parent whose neighbour is k's parent at the shift of k relative to j
+// (key_j, key_k: the images' l2_key).  The list of the parent holds every pair
+// below the search radius whose parents are in this order, so only a pair
+// within rounding of the radius itself can be missing: -1.
+__device__ __forceinline__ int find_entry(const BatchView& B, long long key_j, long long key_k) {
+    const long long want = (key_k & ~0xffffffffLL) | (unsigned)((int)key_k - (int)key_j + kShiftBias);
+    const int pj = (int)(key_j >> 32);
+    const long long b1 = min(B.l2_off[pj + 1], B.n2_cap);
+    for (long long e = min(B.l2_off[pj], B.n2_cap); e < b1; e += 4) {
+        long long q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) q[u] = e + u < b1 ? B.l2_key[e + u] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (q[u] == want) return (int)e + u;
+    }
+    return -1;
+}
+
+// The list entries of a triplet's / quadruplet's pairs (entries a, b[, c] of
+// the first atom): those of the first atom alone, or all of them (all_pairs).
+__device__ __forceinline__ void put_c3e(const BatchView& B, long long q, long long a, long long b) {
+    if (!B.c3e) return;
+    if (!B.all_pairs) {
+        B.c3e[2 * q] = (int)a;
+        B.c3e[2 * q + 1] = (int)b;
+        return;
+    }
+    int* o = B.c3e + 3 * q;
+    o[0] = (int)a;
+    o[1] = (int)b;
+    o[2] = find_entry(B, B.l2_key[a], B.l2_key[b]);
+}
+__device__ __forceinline__ void put_c4e(const BatchView& B, long long q, long long a, long long b, long long c) {
+    if (!B.c4e) return;
+    if (!B.all_pairs) {
+        B.c4e[3 * q] = (int)a;
+        B.c4e[3 * q + 1] = (int)b;
+        B.c4e[3 * q + 2] = (int)c;
+        return;
+    }
+    const long long ka = B.l2_key[a], kb = B.l2_key[b], kc = B.l2_key[c];
+    int* o = B.c4e + 6 * q;
+    o[0] = (int)a;
+    o[1] = (int)b;
+    o[2] = (int)c;
+    o[3] = find_entry(B, ka, kb);
+    o[4] = find_entry(B, ka, kc);
+    o[5] = find_entry(B, kb, kc);
+}
+
 // Per-entry warp form of the same enumeration.  When the 4-body outer cutoff
 // does not exceed the 3-body one (or a system lacks one of the two), the
 // valid_3mer / valid_4mer flags are restored before every k (the reference's
@@ -732,7 +787,7 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
                 if (q < B.n3_cap) {
                     int* out = B.c3 + 3 * q;
                     out[0] = gi; out[1] = jj; out[2] = kk;
-                    if (B.c3e) { B.c3e[2 * q] = (int)e; B.c3e[2 * q + 1] = (int)k; }
+                    put_c3e(B, q, e, k);
                 }
             }
             n3 += __popc(m3);
@@ -774,11 +829,7 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
                         if (q < B.n4_cap) {
                             int* out = B.c4 + 4 * q;
                             out[0] = gi; out[1] = jj; out[2] = ks; out[3] = ll;
-                            if (B.c4e) {
-                                B.c4e[3 * q] = (int)e;
-                                B.c4e[3 * q + 1] = (int)(kb + src);
-                                B.c4e[3 * q + 2] = (int)l;
-                            }
+                            put_c4e(B, q, e, kb + src, l);
                         }
                     }
                     n4 += __popc(ml);
@@ -990,7 +1041,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
             if (q < B.n3_cap) {
                 int* out = B.c3 + 3 * q;
                 out[0] = gi; out[1] = sg[a]; out[2] = sg[bk];
-                if (B.c3e) { B.c3e[2 * q] = (int)(b0 + a); B.c3e[2 * q + 1] = (int)(b0 + bk); }
+                put_c3e(B, q, b0 + a, b0 + bk);
             }
         }
         for (int t = 32 * w + lane; t < t4; t += 32 * G) {
@@ -1019,11 +1070,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
             if (q < B.n4_cap) {
                 int* out = B.c4 + 4 * q;
                 out[0] = gi; out[1] = sg[a]; out[2] = sg[bk]; out[3] = sg[lk];
-                if (B.c4e) {
-                    B.c4e[3 * q] = (int)(b0 + a);
-                    B.c4e[3 * q + 1] = (int)(b0 + bk);
-                    B.c4e[3 * q + 2] = (int)(b0 + lk);
-                }
+                put_c4e(B, q, b0 + a, b0 + bk, b0 + lk);
             }
         }
     }

@@ -962,6 +962,7 @@ ParamImage pack_params(const HostParams& P) {
     std::vector<double> c2d;
     std::vector<float> c2f;
     std::vector<int> p2;
+    std::vector<FxPair> fx2;
     for (int p = 0; p < P.npairs; p++) {
         pr[p].rin = P.rin[p]; pr[p].rout = P.rout[p]; pr[p].lam = P.lam[p];
         morse_consts(P.rin[p], P.rout[p], P.lam[p], pr[p].xavg, pr[p].xdiff);
@@ -987,7 +988,20 @@ ParamImage pack_params(const HostParams& P) {
             c2d.push_back(dense[n]);
             c2f.push_back((float)dense[n]);
         }
+        std::vector<FxCoef> q;
+        bool finite = true;
+        for (int n = 0; n <= P.o2; n++) {
+            q.push_back(FxCoef{n, 0, 0, 0, dense[n]});
+            finite = finite && std::isfinite(dense[n]);
+        }
+        pr[p].fx_amp = finite ? fx_amplitude(q) : 0.0;   // 0: summed in FP64
+        for (int n = 0; n <= P.o2; n++) {
+            FxPair v{0, 0};
+            if (finite) fx_limbs(dense[n], pr[p].fx_amp, v.x, v.y);
+            fx2.push_back(v);
+        }
     }
+    H.fx2 = as_off<const FxPair>(B.add(fx2.data(), fx2.size()));
     H.pairs = as_off<const PairRec>(B.add(pr.data(), pr.size()));
     H.c2d = as_off<const double>(B.add(c2d.data(), c2d.size()));
     H.c2f = as_off<const float>(B.add(c2f.data(), c2f.size()));
