@@ -316,9 +316,11 @@ int ck_tuple_factored(void* h, int slot, int nbody, int* nrow, int* ncol, int* R
 
 int ck_get_tuning(void* h, int* out) {
     if (int st = check_handle(h)) return st;
-    const ck::ForceLaunch& L = static_cast<Instance*>(h)->eng.tuning;
-    const int v[11] = {L.tpc3,  L.tpc4,  L.blocks_per_sm, L.fact3, L.fact4, L.ftpc3,
-                       L.ftpc4, L.fbps3, L.fbps4,         L.noy3,  L.tc3 | (L.tc4 << 1)};
+    const ck::Engine& e = static_cast<Instance*>(h)->eng;
+    const ck::ForceLaunch& L = e.tuning;
+    const bool fx = e.precision == ck::kFP64;
+    const int v[11] = {L.tpc3,  L.tpc4,  L.blocks_per_sm, L.fact3, L.fact4, fx ? L.xw3 : L.ftpc3,
+                       fx ? L.xw4 : L.ftpc4, L.fbps3, L.fbps4,         L.noy3,  L.tc3 | (L.tc4 << 1)};
     for (int k = 0; k < 11; k++) out[k] = v[k];
     return ck::kOk;
 }
@@ -349,6 +351,8 @@ int ck_set_tuning(void* h, int tpc3, int tpc4, int blocks_per_sm) {
     // factored kernels: 1, 2 or 4 lanes per cluster, one-warp blocks
     e.tuning.ftpc3 = tpc3 < 4 ? tpc3 : 4;
     e.tuning.ftpc4 = tpc4 < 4 ? tpc4 : 4;
+    e.tuning.xw3 = tpc3 < 8 ? tpc3 : 8;
+    e.tuning.xw4 = tpc4 < 8 ? tpc4 : 8;
     e.tuning.fbps3 = e.tuning.fbps4 = 4 * blocks_per_sm;
     return ck::kOk;
 }

@@ -116,13 +116,14 @@ constexpr int kFactMaxDim = 128;   // largest R^K and R^(P-K) kept in shared mem
 // sum |a| <= 0.9 fx_amp and max |a| <= 0.24 fx_amp, and kept at 2^kFxCoef as two
 // limbs {h, l}, a = h 2^kFxLimb + l.
 //   3-body: per column J = (q_ik, q_jk) with coefficients, in ascending order, a
-//   header {q_ik, q_jk, mask of its groups, 0}, then per group g of its mask the
-//   coefficients of q_ij = 2g and 2g + 1 {h, l, h, l} (zero where absent);
-//   fx_split[k], k = 0..8: eight parts of about equal work.
-//   4-body: per row I with coefficients a header {entries / 4, I's powers, 0,
-//   0}, then its entries {h, l, J, 0}, padded with zeros to a multiple of four;
+//   header {q_ik, q_jk, mask of its groups, 0}, then for g = 0..(R + 1) / 2 - 1
+//   the coefficients of q_ij = 2g and 2g + 1 {h, l, h, l} (zero where absent, the
+//   mask bit of an all-zero group clear); fx_split[k], k = 0..8: eight parts.
+//   4-body: per row I with coefficients its entries {h, l, J, -1}, padded with
+//   zeros to a multiple of four, the last with I's powers in place of the -1;
 //   then the columns likewise (rows and columns exchanged); fx_split[0..4] /
-//   [4..8]: four parts of the rows / columns.
+//   [4..8]: four parts of the rows / columns.  Four spare entries end the
+//   array.
 // Splits are offsets from fx_off, at record boundaries.
 struct __attribute__((aligned(8))) FxPair {
     int x, y;
@@ -242,7 +243,7 @@ struct DevParamSet {
     // table lengths, for the index checks of the checked build (CK_BOUNDS):
     // 3-/4-body coefficients, factored entries, tensor-core image floats
     long long n_c3, n_c4, n_fe3, n_fe4, n_tc3, n_tc4;
-    // fixed-point streams (FP64 form); fx3_max = longest 3-body stream
+    // fixed-point streams (FP64 form); fx3_max = most columns of a 3-body stream
     const FxPair* fx2; const FxEnt* fx3; const FxEnt* fx4;
     long long n_fx3, n_fx4;
     int fx3_max, fx_pad;

@@ -579,7 +579,7 @@ Status Engine::launch(std::string& err) {
     std::vector<long long> key = {(long long)V_.n_sys, V_.n_in_total, V_.n_atoms_total, V_.n_ghost_total,
                                   V_.n_bins_total, n2_cap_, n3_cap_, n4_cap_, precision, tuning.tpc3, tuning.tpc4,
                                   tuning.stride3, tuning.stride4, tuning.blocks_per_sm, profile ? 1 : 0,
-                                  tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4,
+                                  tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4, tuning.xw3, tuning.xw4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
                                   tuning.tc3, tuning.tc4, V_.all_pairs};
     for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
@@ -707,8 +707,9 @@ Status Engine::autotune(int* chosen, std::string& err) {
     const std::string key = tune_key();
     auto report = [&]() {
         if (chosen) {
-            chosen[0] = tuning.fact3 ? tuning.ftpc3 : tuning.tpc3;
-            chosen[1] = tuning.fact4 ? tuning.ftpc4 : tuning.tpc4;
+            const bool fx = precision == kFP64;
+            chosen[0] = tuning.fact3 ? (fx ? tuning.xw3 : tuning.ftpc3) : tuning.tpc3;
+            chosen[1] = tuning.fact4 ? (fx ? tuning.xw4 : tuning.ftpc4) : tuning.tpc4;
             chosen[2] = tuning.blocks_per_sm;
         }
     };
@@ -719,6 +720,8 @@ Status Engine::autotune(int* chosen, std::string& err) {
             tuning.blocks_per_sm = kv.second.blocks_per_sm;
             tuning.ftpc3 = kv.second.ftpc3;
             tuning.ftpc4 = kv.second.ftpc4;
+            tuning.xw3 = kv.second.xw3;
+            tuning.xw4 = kv.second.xw4;
             tuning.fbps3 = kv.second.fbps3;
             tuning.fbps4 = kv.second.fbps4;
             tuning.want_fact3 = kv.second.want_fact3;
@@ -791,20 +794,20 @@ Status Engine::autotune(int* chosen, std::string& err) {
     auto apply = [&](int nb, const Cand& c) {
         if (nb == 3) {
             tuning.fact3 = c.fact;
-            (c.fact ? tuning.ftpc3 : tuning.tpc3) = c.tpc;
+            (c.fact ? (mixed ? tuning.ftpc3 : tuning.xw3) : tuning.tpc3) = c.tpc;
             tuning.noy3 = c.noy;
             tuning.tc3 = c.tc;
             if (c.fbps > 0) tuning.fbps3 = c.fbps;
         } else {
             tuning.fact4 = c.fact;
-            (c.fact ? tuning.ftpc4 : tuning.tpc4) = c.tpc;
+            (c.fact ? (mixed ? tuning.ftpc4 : tuning.xw4) : tuning.tpc4) = c.tpc;
             tuning.tc4 = c.tc;
             if (c.fbps > 0) tuning.fbps4 = c.fbps;
         }
     };
     double best3 = 1e300, best4 = 1e300;
-    Cand b3 = {tuning.fact3, tuning.fact3 ? tuning.ftpc3 : tuning.tpc3, tuning.noy3, tuning.fbps3, tuning.tc3};
-    Cand b4 = {tuning.fact4, tuning.fact4 ? tuning.ftpc4 : tuning.tpc4, 0, tuning.fbps4, tuning.tc4};
+    Cand b3 = {tuning.fact3, tuning.fact3 ? (mixed ? tuning.ftpc3 : tuning.xw3) : tuning.tpc3, tuning.noy3, tuning.fbps3, tuning.tc3};
+    Cand b4 = {tuning.fact4, tuning.fact4 ? (mixed ? tuning.ftpc4 : tuning.xw4) : tuning.tpc4, 0, tuning.fbps4, tuning.tc4};
     const size_t nc = std::max(c3.size(), c4.size());
     for (size_t i = 0; i < nc && st == kOk; i++) {
         const bool need3 = do3 && i < c3.size(), need4 = do4 && i < c4.size();

@@ -28,6 +28,13 @@
 // turns each entry's scalar into forces and virial, once per entry and not once
 // per cluster.  Otherwise (caller's neighbour lists, per-tuple cutoffs) a
 // cluster's pairs are set up and its forces scattered in the cluster kernel.
+//
+// Measured (GB300, 384 configurations of 8-512 atoms, 12/10/4, 1.81 M triplets
+// and 358 k quadruplets): 3-body 1.48 ms and 4-body 0.86 ms, against 5.91 and
+// 3.12 ms for the FP64 factored kernels that this form replaced and 3.27 and
+// 1.63 ms with the pairs set up per cluster.  Bound by the integer
+// multiply-adds (about half of the pipe's rate) and the latency that 16 warps
+// per SM leave exposed.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -269,13 +276,22 @@ __device__ __forceinline__ bool fx_setup(const BatchView& B, const int* clusters
         const FxEnt* pct = reinterpret_cast<const FxEnt*>(NB == 3 ? B.pct3 : B.pct4);
 #pragma unroll
         for (int p = 0; p < NP; p++) ent[p] = active ? ce[(long long)NP * c + p] : 0;
-        for (int k = w; k < (NP - M::P0) * Rp; k += NW) {
-            const int p = M::P0 + k / Rp, n = k % Rp;
-            int e = ent[0];
+        // a warp takes every NW-th power of each pair, four loads in flight
 #pragma unroll
-            for (int q = 1; q < NP; q++) e = p == q ? ent[q] : e;
-            if (e >= 0) m.table(p, rs)[n * kFxTile + lane] = pct[(long long)e * rs + n];
+        for (int p = M::P0; p < NP; p++) {
+            const FxEnt* src = pct + (long long)(ent[p] < 0 ? 0 : ent[p]) * rs;
+            FxEnt* dst = m.table(p, rs) + lane;
+            for (int n0 = w; n0 < Rp; n0 += 4 * NW) {
+                FxEnt t[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (n0 + k * NW < Rp) t[k] = src[n0 + k * NW];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (n0 + k * NW < Rp) dst[(n0 + k * NW) * kFxTile] = t[k];
+            }
         }
+        if (KC < NP) __syncthreads();   // (a missing pair's tables replace what was copied for it)
 #pragma unroll
         for (int p = KC; p < NP; p++)
             if (ent[p] < 0 && w == 0) {
@@ -429,11 +445,14 @@ struct AccOf<true> {
 
 // ---------------------------------------------------------------------------
 // 3-body.  X = T_ij and the row sums z stay in registers (RX powers, unrolled;
-// a column's mask says which pairs of them it has), Y_J is formed per column,
+// a column's mask says which groups of two it has), Y_J is formed per column,
 // and the column sums w_J are folded over q_jk within a run of q_ik.
 // ---------------------------------------------------------------------------
+// 16 warps per SM (128 registers): 384 configurations 1.70 -> 1.61 ms for the
+// stage; all groups' loads ahead of the masked sums and not inside them, and
+// plain masks against unmasked sums over zeros, measured the same.
 template <int RX, int NW, bool ENT>
-__global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clusters, const int* perm,
+__global__ void __launch_bounds__(32 * NW, RX <= 10 ? 16 / NW : 1) k_forcex3(BatchView B, const int* clusters, const int* perm,
                                                      const long long* perm_n, long long perm_cap, int rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     const FxSmem<3, NW, ENT> m(smem, rs);
@@ -452,10 +471,15 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
         int id0[3], s0, u, ent[3];
         const DevParamSet* P;
         const TupleRec* R = cluster_tuple<3>(B, clusters, c0, id0, s0, P, u);
-        int len = R->fx_split[8];
-        if (!ck_bound(B, R->fx_off >= 0 && R->fx_off + (long long)len <= P->n_fx3)) len = 0;
+        constexpr int CL = 1 + RX / 2;   // a column here: header, then every group
+        const int cl = 1 + (P->R3 + 1) / 2;   // and as stored
+        int ncol = R->fx_split[8] / cl;
+        if (!ck_bound(B, R->fx_off >= 0 && R->fx_off + (long long)R->fx_split[8] <= P->n_fx3)) ncol = 0;
         if (R->fx_off != loaded || P != loaded_set) {
-            for (int q = threadIdx.x; q < len; q += 32 * NW) strm[q] = P->fx3[R->fx_off + q];
+            for (int q = threadIdx.x; q < ncol * CL; q += 32 * NW) {
+                const int col = q / CL, k = q % CL;
+                strm[q] = k < cl ? P->fx3[R->fx_off + col * cl + k] : FxEnt{0, 0, 0, 0};
+            }
             loaded = R->fx_off;
             loaded_set = P;
         }
@@ -466,52 +490,50 @@ __global__ void __launch_bounds__(32 * NW) k_forcex3(BatchView B, const int* clu
         constexpr int st0 = ENT ? 1 : kFxTile;
         const FxEnt *t1 = m.table(1, rs) + lane, *t2 = m.table(2, rs) + lane;
         Fx X[RX];
-        FxAcc z[RX];
+        FxRec z[RX];
 #pragma unroll
         for (int q = 0; q < RX; q++) X[q] = q < Rp ? quad_t(t0 + q * st0) : Fx{0, 0};
         FxAcc g1, g2, ca, cb;
         FxEnt tb{0, 0, 0, 0};
         int qb = -1;
-        int o = len ? R->fx_split[8 * w / NW] : 0;
-        const int o1 = len ? R->fx_split[8 * (w + 1) / NW] : 0;
-        FxEnt hd = strm[o];   // (the buffer has room for a header past the stream)
-        while (o < o1) {
-            const int b = hd.x, mask = hd.z;
+        int o = ncol ? R->fx_split[8 * w / NW] / cl * CL : 0;
+        const int o1 = ncol ? R->fx_split[8 * (w + 1) / NW] / cl * CL : 0;
+        for (; o < o1; o += 1 + RX / 2) {
+            const FxEnt hd = strm[o];
+            FxEnt a[RX / 2];
+#pragma unroll
+            for (int g = 0; g < RX / 2; g++) a[g] = strm[o + 1 + g];
             const FxEnt tc = t2[hd.y * kFxTile];
-            const FxEnt* q4 = strm + o + 1;
-            o += 1 + __popc(mask);
-            hd = strm[o];
-            if (b != qb) {   // uniform: a new run of q_ik
-                g1.mac(Fx{tb.z, tb.w}, ca.value<0>());
-                g2.mac(Fx{tb.x, tb.y}, cb.value<0>());
+            if (hd.x != qb) {   // uniform: a new run of q_ik
+                g1.mac(Fx{tb.z, tb.w}, ca.value());
+                g2.mac(Fx{tb.x, tb.y}, cb.value());
                 ca = FxAcc();
                 cb = FxAcc();
-                tb = t1[b * kFxTile];
-                qb = b;
+                tb = t1[hd.x * kFxTile];
+                qb = hd.x;
             }
             const Fx Y = fx_mul(Fx{tb.x, tb.y}, Fx{tc.x, tc.y});
-            FxAcc wj;
+            FxRec wj;
 #pragma unroll
             for (int g = 0; g < RX / 2; g++)
-                if (mask & (1 << g)) {   // uniform
-                    const FxEnt a = *q4++;
-                    wj.mac(Fx{a.x, a.y}, X[2 * g]);
-                    wj.mac(Fx{a.z, a.w}, X[2 * g + 1]);
-                    z[2 * g].mac(Fx{a.x, a.y}, Y);
-                    z[2 * g + 1].mac(Fx{a.z, a.w}, Y);
+                if (hd.z & (1 << g)) {   // uniform
+                    wj.mac(Fx{a[g].x, a[g].y}, X[2 * g]);
+                    wj.mac(Fx{a[g].z, a[g].w}, X[2 * g + 1]);
+                    z[2 * g].mac(Fx{a[g].x, a[g].y}, Y);
+                    z[2 * g + 1].mac(Fx{a[g].z, a[g].w}, Y);
                 }
-            const Fx wv = wj.value<kFxDown>();
+            const Fx wv = wj.value();
             ca.mac(Fx{tc.x, tc.y}, wv);
             cb.mac(Fx{tc.z, tc.w}, wv);
         }
-        g1.mac(Fx{tb.z, tb.w}, ca.value<0>());
-        g2.mac(Fx{tb.x, tb.y}, cb.value<0>());
+        g1.mac(Fx{tb.z, tb.w}, ca.value());
+        g2.mac(Fx{tb.x, tb.y}, cb.value());
         FxAcc S, g0;
 #pragma unroll
         for (int q = 0; q < RX; q++)
             if (q < Rp) {
                 const FxEnt t = t0[q * st0];
-                const Fx zv = z[q].template value<kFxDown>();
+                const Fx zv = z[q].value();
                 S.mac(Fx{t.x, t.y}, zv);
                 g0.mac(Fx{t.z, t.w}, zv);
             }
@@ -535,7 +557,7 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
     int q0 = -1, q1 = -1;
     auto fold1 = [&]() {
         if (q1 < 0) return;
-        const Fx a = ra.value<0>(), b = rb.value<0>();
+        const Fx a = ra.value(), b = rb.value();
         const FxEnt v = t1[q1 * kFxTile];
         rP.mac(Fx{v.x, v.y}, a);
         rQ.mac(Fx{v.z, v.w}, a);
@@ -545,37 +567,45 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
     };
     auto fold0 = [&]() {
         if (q0 < 0) return;
-        const Fx p = rP.value<0>();
+        const Fx p = rP.value();
         const FxEnt v = t[q0 * kFxTile];
         S.mac(Fx{v.x, v.y}, p);
         g0.mac(Fx{v.z, v.w}, p);
-        g1.mac(Fx{v.x, v.y}, rQ.value<0>());
-        g2.mac(Fx{v.x, v.y}, rR.value<0>());
+        g1.mac(Fx{v.x, v.y}, rQ.value());
+        g2.mac(Fx{v.x, v.y}, rR.value());
         rP = FxAcc();
         rQ = FxAcc();
         rR = FxAcc();
     };
+    FxRec z;
+    FxEnt q[4], n[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) q[k] = ent[o + k];   // (a side without entries reads its neighbour's: in bounds)
     while (o < o1) {
-        const FxEnt hd = ent[o++];
-        FxAcc z;
-        for (const int end = o + 4 * hd.x; o < end; o += 4) {
-            FxEnt q[4];
+        o += 4;
+        if (o < o1) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) q[k] = ent[o + k];
+            for (int k = 0; k < 4; k++) n[k] = ent[o + k];   // the next four in flight
+        }
 #pragma unroll
-            for (int k = 0; k < 4; k++) z.mac(Fx{q[k].x, q[k].y}, fx_load(V[q[k].z * kFxTile]));
+        for (int k = 0; k < 4; k++) z.mac(Fx{q[k].x, q[k].y}, fx_load(V[q[k].z * kFxTile]));
+        const int pows = q[3].w;
+        if (pows >= 0) {   // uniform: the record's end
+            const int r0 = pows & 31, r1 = (pows >> kPowBits) & 31, r2 = (pows >> (2 * kPowBits)) & 31;
+            if (r0 != q0 || r1 != q1) {
+                fold1();
+                if (r0 != q0) fold0();
+                q0 = r0;
+                q1 = r1;
+            }
+            const Fx zv = z.value();
+            const FxEnt v = t2[r2 * kFxTile];
+            ra.mac(Fx{v.x, v.y}, zv);
+            rb.mac(Fx{v.z, v.w}, zv);
+            z = FxRec();
         }
-        const int r0 = hd.y & 31, r1 = (hd.y >> kPowBits) & 31, r2 = (hd.y >> (2 * kPowBits)) & 31;
-        if (r0 != q0 || r1 != q1) {   // uniform
-            fold1();
-            if (r0 != q0) fold0();
-            q0 = r0;
-            q1 = r1;
-        }
-        const Fx zv = z.value<kFxDown>();
-        const FxEnt v = t2[r2 * kFxTile];
-        ra.mac(Fx{v.x, v.y}, zv);
-        rb.mac(Fx{v.z, v.w}, zv);
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = n[k];
     }
     fold1();
     fold0();
@@ -655,7 +685,7 @@ unsigned fx_grid(const void* kern, int threads, size_t smem, long long tiles) {
 template <int RX, int NW, bool ENT>
 void launch_x3(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
     const int rs = L.rf3;
-    const size_t smem = FxSmem<3, NW, ENT>::bytes(rs) + sizeof(FxEnt) * (size_t)(L.xs3 + 1);
+    const size_t smem = FxSmem<3, NW, ENT>::bytes(rs) + sizeof(FxEnt) * (size_t)L.xs3 * (1 + RX / 2);
     auto kern = k_forcex3<RX, NW, ENT>;
     const unsigned grid = fx_grid((const void*)kern, 32 * NW, smem, (B.perm3_cap + kFxTile - 1) / kFxTile);
     count_launch(), kern<<<grid, 32 * NW, smem, st>>>(B, B.c3, B.perm3, B.bk_start + B.nbk3, B.perm3_cap, rs);
@@ -681,7 +711,7 @@ void launch_x4_nw(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
 
 template <bool ENT>
 void launch_x3_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    switch (L.ftpc3) {
+    switch (L.xw3) {
         case 1: launch_x3_nw<1, ENT>(B, L, st); break;
         case 2: launch_x3_nw<2, ENT>(B, L, st); break;
         case 4: launch_x3_nw<4, ENT>(B, L, st); break;
@@ -691,7 +721,7 @@ void launch_x3_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
 
 template <bool ENT>
 void launch_x4_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    switch (L.ftpc4) {
+    switch (L.xw4) {
         case 1: launch_x4_nw<1, ENT>(B, L, st); break;
         case 2: launch_x4_nw<2, ENT>(B, L, st); break;
         case 4: launch_x4_nw<4, ENT>(B, L, st); break;

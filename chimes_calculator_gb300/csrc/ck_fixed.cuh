@@ -12,7 +12,7 @@
 //
 //   Fx    value h 2^28 + l, |l| <= 2^27: T, dT, X and Y at 2^56, record sums
 //         at 2^59, coefficients at 2^61
-//   FxAcc sum of products: hi += a.h b.h, mid += a.h b.l + a.l b.h (the
+//   FxRec, FxAcc sums of products: hi += a.h b.h, mid += a.h b.l + a.l b.h (the
 //         low x low product, below 2^-62 of full scale, is dropped)
 #pragma once
 #include <cuda_runtime.h>
@@ -34,34 +34,59 @@ __device__ __forceinline__ Fx fx_split(long long v) {
 __device__ __forceinline__ Fx fx_load(const FxPair& q) { return Fx{q.x, q.y}; }
 __device__ __forceinline__ FxPair fx_store(const Fx& v) { return FxPair{v.h, v.l}; }
 
-// product of two values, at the sum of their scales less 2^56
-__device__ __forceinline__ Fx fx_mul(const Fx& a, const Fx& b) {
-    long long m = (long long)a.h * b.l + (1LL << (kFxLimb - 1));
-    m += (long long)a.l * b.h;
-    return fx_split((long long)a.h * b.h + (m >> kFxLimb));
+// v + 2^(kFxLimb - 1) -> the limbs of v (the rounding constant is added by the
+// caller where an accumulator starts, so that it costs nothing)
+__device__ __forceinline__ Fx fx_limbs(long long v) {
+    return Fx{(int)(v >> kFxLimb), (int)((unsigned)v & ((1u << kFxLimb) - 1u)) - (1 << (kFxLimb - 1))};
 }
 
+// acc += a b: one IMAD.WIDE (written out: the compiler otherwise splits some
+// of these products from their sums, which took a third more instructions)
+__device__ __forceinline__ void imad(long long& acc, int a, int b) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
+}
+
+// product of two values, at the sum of their scales less 2^56
+__device__ __forceinline__ Fx fx_mul(const Fx& a, const Fx& b) {
+    // (rounding of the shift, and fx_limbs' constant above it)
+    long long m = (1LL << (kFxLimb - 1)) + (1LL << (2 * kFxLimb - 1));
+    imad(m, a.h, b.l);
+    imad(m, a.l, b.h);
+    m >>= kFxLimb;
+    imad(m, a.h, b.h);
+    return fx_limbs(m);
+}
+
+// A record sum, kept at 2^kFxCoef with the constants of `value` already in it.
+struct FxRec {
+    long long hi = 1LL << (kFxCoef - kFxSum + kFxLimb - 1), mid = 0;
+    __device__ __forceinline__ void mac(const Fx& a, const Fx& b) {
+        imad(hi, a.h, b.h);
+        imad(mid, a.h, b.l);
+        imad(mid, a.l, b.h);
+    }
+    // the sum as a value at 2^kFxSum
+    __device__ __forceinline__ Fx value() const {
+        constexpr int D = kFxCoef - kFxSum;
+        const long long v = hi + (mid >> kFxLimb);
+        return Fx{(int)(v >> (kFxLimb + D)),
+                  (int)(((unsigned)v & ((1u << (kFxLimb + D)) - 1u)) >> D) - (1 << (kFxLimb - 1))};
+    }
+};
+
+// A sum of products with record sums or of tables, at the scale of its terms.
 struct FxAcc {
     long long hi = 0, mid = 0;
     __device__ __forceinline__ void mac(const Fx& a, const Fx& b) {
-        hi += (long long)a.h * b.h;
-        mid += (long long)a.h * b.l;
-        mid += (long long)a.l * b.h;
+        imad(hi, a.h, b.h);
+        imad(mid, a.h, b.l);
+        imad(mid, a.l, b.h);
     }
-    // the sum as a value, down = bits dropped from its scale
-    template <int DOWN>
-    __device__ __forceinline__ Fx value() const {
-        if constexpr (DOWN == 0) {
-            return fx_split(sum());
-        } else {
-            return fx_split((hi + (mid >> kFxLimb) + (1LL << (DOWN - 1))) >> DOWN);
-        }
-    }
-    // the sum as an integer at its scale, and times `unit`
+    // the sum as an integer at its scale, as a value, and times `unit`
     __device__ __forceinline__ long long sum() const { return hi + ((mid + (1LL << (kFxLimb - 1))) >> kFxLimb); }
+    __device__ __forceinline__ Fx value() const { return fx_limbs(sum() + (1LL << (kFxLimb - 1))); }
     __device__ __forceinline__ double real(double unit) const { return (double)sum() * unit; }
 };
-constexpr int kFxDown = kFxCoef - kFxSum;   // record sums: 2^61 -> 2^59
 constexpr double kFxUnit = 1.0 / (double)(1LL << kFxSum);
 
 // 2 x t for x at 2^62 and t at 2^k: at 2^k

@@ -45,10 +45,12 @@ struct ForceLaunch {
     int fact3 = 0, fact4 = 0;
     int want_fact3 = 1, want_fact4 = 1;   // preference (autotuner); fact = want && tables present
     int rf3 = 0, rf4 = 0;  // powers per pair (max over the batch's sets)
-    int xs3 = 0;           // longest 3-body fixed-point stream over the batch's sets (FP64 form)
-    // mixed form: threads per cluster, 1, 2 or 4; FP64 form (ck_fixed.cu):
-    // warps per 32 clusters, 1, 2, 4 or 8
+    int xs3 = 0;           // most columns of a 3-body fixed-point stream over the batch's sets (FP64 form)
+    // mixed form: threads per cluster, 1, 2 or 4
     int ftpc3 = 1, ftpc4 = 4;
+    // FP64 form (ck_fixed.cu): warps per 32 clusters, 1, 2, 4 or 8 (defaults: the
+    // fastest of 1024 atoms and of 384 configurations alike)
+    int xw3 = 2, xw4 = 4;
     int fbps3 = 8, fbps4 = 8;      // mixed form: resident one-warp blocks per SM (capped by occupancy)
     int noy3 = 0;                  // mixed form: 3-body without the Y table (products per entry)
     // tensor-core 3-body contraction (mixed form only; ck_tensor.cu): tc3 = in

@@ -863,18 +863,18 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& 
         const size_t at = out.size();
         const int col = c[k].col;
         out.push_back(FxEnt{col / Rp, col % Rp, 0, 0});
+        out.resize(at + 1 + (Rp + 1) / 2);
         while (k < c.size() && c[k].col == col) {
             const int grp = c[k].row / 2;
             double a[2] = {0.0, 0.0};
             for (; k < c.size() && c[k].col == col && c[k].row / 2 == grp; k++) a[c[k].row % 2] += c[k].a;
-            FxEnt q;
+            FxEnt& q = out[at + 1 + grp];
             fx_limbs(a[0], R.fx_amp, q.x, q.y);
             fx_limbs(a[1], R.fx_amp, q.z, q.w);
-            out.push_back(q);
             out[at].z |= 1 << grp;
         }
         ends.push_back((int)out.size() - R.fx_off);
-        weight.push_back(2.0 + (double)(out.size() - at - 1));
+        weight.push_back(1.0);
     }
     R.fx_split[0] = 0;
     fx_parts(ends, weight, 8, R.fx_split);
@@ -897,17 +897,16 @@ void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
         split[0] = (int)out.size() - R.fx_off;
         for (size_t k = 0; k < c.size();) {
             const size_t at = out.size();
-            const int row = c[k].row;
-            out.push_back(FxEnt{0, c[k].rowp, 0, 0});
+            const int row = c[k].row, pows = c[k].rowp;
             for (; k < c.size() && c[k].row == row; k++) {
-                FxEnt q{0, 0, c[k].col, 0};
+                FxEnt q{0, 0, c[k].col, -1};
                 fx_limbs(c[k].a, R.fx_amp, q.x, q.y);
                 out.push_back(q);
             }
-            while ((out.size() - at - 1) % 4) out.push_back(FxEnt{0, 0, 0, 0});
-            out[at].x = (int)(out.size() - at - 1) / 4;
+            while ((out.size() - at) % 4) out.push_back(FxEnt{0, 0, 0, -1});
+            out.back().w = pows;
             ends.push_back((int)out.size() - R.fx_off);
-            weight.push_back(4.0 + (double)(out.size() - at - 1));
+            weight.push_back(4.0 + (double)(out.size() - at));
         }
         fx_parts(ends, weight, 4, split);
     }
@@ -1153,7 +1152,7 @@ ParamImage pack_params(const HostParams& P) {
                 for (int c = 0; c < R.ncoef; c++) q[c] = FxCoef{rowi[c], coli[c], rowp[c], colp[c], Bd.coef[ti][c]};
                 if (nb == 3) {
                     fx3_stream(std::move(q), R_pow, R, fx3);
-                    fx3_max = std::max(fx3_max, R.fx_split[8]);
+                    fx3_max = std::max(fx3_max, R.fx_split[8] / (1 + (R_pow + 1) / 2));
                 } else {
                     fx4_stream(std::move(q), R, fx4);
                 }
@@ -1208,6 +1207,7 @@ ParamImage pack_params(const HostParams& P) {
             H.fx3_max = fx3_max;
         }
         if (nb == 4 && !fx4.empty()) {
+            fx4.resize(fx4.size() + 4);
             H.fx4 = as_off<const FxEnt>(B.add(fx4.data(), fx4.size()));
             H.n_fx4 = (long long)fx4.size();
         }

@@ -185,7 +185,7 @@ public:
             std::lock_guard<std::mutex> ge(*engine_mu_[w]);
             ForceLaunch& d = engines_[w]->tuning;
             d.tpc3 = t.tpc3, d.tpc4 = t.tpc4, d.blocks_per_sm = t.blocks_per_sm;
-            d.ftpc3 = t.ftpc3, d.ftpc4 = t.ftpc4, d.fbps3 = t.fbps3, d.fbps4 = t.fbps4;
+            d.ftpc3 = t.ftpc3, d.ftpc4 = t.ftpc4, d.xw3 = t.xw3, d.xw4 = t.xw4, d.fbps3 = t.fbps3, d.fbps4 = t.fbps4;
             d.want_fact3 = t.want_fact3, d.want_fact4 = t.want_fact4, d.noy3 = t.noy3;
             d.want_tc3 = t.want_tc3;
             d.want_tc4 = t.want_tc4;

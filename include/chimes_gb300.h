@@ -62,8 +62,9 @@ int ck_tuple_table(void *h, int slot, int nbody, int *valid, int *ncoef, double 
  * and *R, the powers per pair (0 when the set has no factored tables). */
 int ck_tuple_factored(void *h, int slot, int nbody, int *nrow, int *ncol, int *R);
 /* out[11] = tpc3, tpc4, blocks_per_sm (per-coefficient kernels), factored 3B and
- * 4B in use for the staged batch (0/1), their threads per cluster and one-warp
- * blocks per SM (ftpc3, ftpc4, fbps3, fbps4), whether the factored 3-body
+ * 4B in use for the staged batch (0/1), their threads per cluster (FP64: warps
+ * per 32 clusters) and one-warp blocks per SM (ftpc3, ftpc4, fbps3, fbps4; the
+ * last two in the mixed form only), whether the factored 3-body
  * kernel forms its column products per coefficient instead of keeping a table
  * of them (noy3), and which contractions run on the tensor cores (mixed
  * form): bit 0 the 3-body one, bit 1 the 4-body one */
@@ -77,7 +78,8 @@ int ck_set_precision(void *h, int precision);
 /* threads per 3-body and 4-body cluster (1,2,4,8,16,32) and resident 4-warp
  * blocks per SM of the per-coefficient kernels; the factored kernels take
  * min(tpc, 4) threads per cluster and 4 * blocks_per_sm one-warp blocks
- * (capped by their shared-memory occupancy). */
+ * (capped by their shared-memory occupancy) in the mixed form, and min(tpc, 8)
+ * warps per 32 clusters in FP64. */
 int ck_set_tuning(void *h, int tpc3, int tpc4, int blocks_per_sm);
 /* 3-/4-body contraction kernels: 1 (default) = factored (coefficients grouped
  * by row and column products, two multiply-adds per coefficient) wherever every
