@@ -36,6 +36,7 @@ namespace ck {
 constexpr int kMaxOrder = 31;      // powers are packed 5 bits per pair
 constexpr int kMaxTypes = 8;       // nt^4 4-body tuple records
 constexpr int kPowBits = 5;
+constexpr int kBkSmem = 1024;      // cluster buckets counted in shared memory (more: in global memory)
 
 enum Status : int {
     kOk = 0,
@@ -223,6 +224,9 @@ struct DevParamSet {
     const double* c2d; const float* c2f; const int* p2;
     const TupleRec* t3;        // [nt^3] (null when o3 == 0)
     const double* c3d; const float* c3f; const uint32_t* p3;
+    // bucket key of each tuple within the set (its index, or -1 without
+    // coefficients or factored tables)
+    const int* key3; const int* key4;
     const TupleRec* t4;        // [nt^4] (null when o4 == 0)
     const double* c4d; const float* c4f; const uint32_t* p4;
     // factored lists (FactRow); R3/R4 = powers per pair, 0 when the tables are
@@ -265,7 +269,7 @@ struct SysDesc {
     double h[9], hi[9];        // cell of the (replicated) system and inverse: r = h * s
     double hn[9], hni[9];      // reoriented cell used for the neighbour lists
     double h0[9], h0i[9];      // unreplicated cell (replication step)
-    double search;             // max(rc2, rc3, rc4)
+    double search, inv_search; // max(rc2, rc3, rc4) and its reciprocal
     double c3, c4;             // max 3B / 4B outer cutoffs (0 when the order is 0)
     int n_in;                  // caller atoms
     int n_rep;                 // n_replicates
@@ -279,12 +283,13 @@ struct SysDesc {
     double ulo[3], uhi[3];     // kept fractional range per axis of the reoriented cell
     double eps;                // margin of the FP32 distance prefilter (Angstrom)
     float c3lo, c3hi, c4lo, c4hi;   // c3 -/+ eps and c4 -/+ eps as FP32, rounded outward
-    float far2, near2;         // (search +/- eps)^2 as FP32: the pair lists' squared-distance prefilter
+    float far2;                // (search + eps)^2 as FP32: the pair lists' squared-distance prefilter
     float c3lo2, c3hi2, c4lo2, c4hi2;   // the same thresholds squared, rounded outward (-1: none below)
     // device-completed
     double minpos[3];
     int nb[3];
     int err;
+    int done;                  // atoms whose bounding box has been taken in
 };
 
 // Flat views of a batch workspace (all device pointers).
@@ -306,28 +311,34 @@ struct BatchView {
     int* ghost_parent;             // [q] atom index (global)
     int* ghost_sh;                 // [q] image shift, packed (pack_shift), or null
     double* ghost_fs;              // [q][3] fractional coords, input cell
-    double* ghost_xn;              // [q][3] Cartesian coords, reoriented cell
     double* ghost_fn;              // [q][3] fractional coords, reoriented cell
-    float* ghost_xf;               // [q][3] ghost_xn rounded to FP32 (distance prefilter)
+    float* ghost_xf;               // [q][3] Cartesian coords, reoriented cell, rounded to FP32 (distance prefilter)
     // bins (per system, offset bin_off)
     unsigned long long* minmax;    // [n_sys][6] order-preserving keys
     int* ghost_bin;                // [g] local bin id
     int* bin_count;                // [n_bins_total]
-    long long* bin_start;          // [n_bins_total+1] positions in bin_items (global exclusive scan)
+    long long* bin_start;          // [n_bins_total] position of each bin's members in bin_items
     int* bin_fill;
     int* bin_items;                // [g] global ghost ids sorted by (bin, id)
     float* bin_xp;                 // [g][4] ghost_xf and ghost_parent (int bits) of bin_items, same order; or null
     // 2B lists
+    // (an atom's entries are contiguous; the atoms come in the order in which
+    // their blocks reserved room)
     int* l2_count;                 // [n_atoms_total]
-    long long* l2_off;             // [n_atoms_total+1]
+    long long* l2_off;             // [n_atoms_total]
     int* l2_ghost;                 // [n2] ghost slot of the neighbour
     double* l2_dist;               // [n2] distance in the reoriented frame
     float* l2_vec;                 // [n2][4] displacement from the list's atom (FP32), for the prefilter
     long long* l2_key;             // [n2] neighbour's parent atom << 32 | its packed image shift, or null
     long long n2_cap;
     // 3B/4B enumeration
+    // (an atom's clusters are contiguous, at a_off[2 r], a_off[2 r + 1]; the
+    // sequential enumeration scans per-entry counts instead, which also serve
+    // as scratch for atoms with long lists)
     int* e_cnt3; int* e_cnt4;      // [n2]
     long long* e_off3; long long* e_off4;   // [n2+1]
+    long long* a_off;              // [n_atoms_total][2]
+    int* a_cnt;                    // [n_atoms_total][2]
     int* c3;                       // [n3][3] ghost slots (i, j, k)
     int* c4;                       // [n4][4]
     long long n3_cap, n4_cap;
@@ -366,20 +377,34 @@ struct BatchView {
                                    //     3 penalty count, 4 below-rin count, 5 table look-ups,
                                    //     6 inputs (no-alloc entry), 7 bounded wait expired
     unsigned long long* queue;     // [2] work-queue heads of the 3-body and 4-body force kernels
+    long long* totals;             // [4] list entries, triplets, quadruplets, binned ghosts
+    const long long* n3_ptr;       // the triplet and quadruplet counts (in totals or at the end of a scan)
+    const long long* n4_ptr;
     // cluster buckets by (parameter set, ordered type tuple), for the factored
     // contraction: bucket key = pset.bk{3,4} + tuple index; each bucket padded
     // to a multiple of 32 slots with -1, so a warp's clusters share one tuple
     // (3-body: of bk_pad3 slots, 128 for the tensor-core form's 128-cluster tiles)
     int nbk3, nbk4;
     int bk_pad3;
-    int* bk_key3;                  // [n3_cap] / [n4_cap] or null: each cluster's bucket key,
-    int* bk_key4;                  //   written by the count pass and read by the scatter pass
+    int* bk_key3;                  // [n3_cap], [n4_cap]: each cluster's bucket key, written by the
+    int* bk_key4;                  //   enumeration (keyed = 1) or by the count pass
+    int keyed;
     int* bk_count;                 // [nbk3 + nbk4]
     int* bk_fill;                  // [nbk3 + nbk4]
     long long* bk_start;           // [nbk3 + 1] then [nbk4 + 1]; last = slots in use
     int* perm3; int* perm4;        // [perm*_cap] cluster index or -1
     long long perm3_cap, perm4_cap;
 };
+
+#if defined(__CUDACC__)
+// The entries [b0, b1) of an atom, as far as the lists hold them.
+__device__ __forceinline__ void list_range(const BatchView& B, long long r, long long& b0, long long& b1) {
+    const long long o = B.l2_off[r];
+    b0 = min(o, B.n2_cap);
+    b1 = min(o + B.l2_count[r], B.n2_cap);
+}
+__device__ __forceinline__ long long list_total(const BatchView& B) { return min(B.totals[0], B.n2_cap); }
+#endif
 
 // A caller's full neighbour list with ghost atoms (LAMMPS layout), for the
 // pair-style path (ck_neigh.cu): local atoms ilist[inum], entries of atom

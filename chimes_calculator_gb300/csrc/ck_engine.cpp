@@ -78,7 +78,7 @@ Status Engine::init_device(std::string& err) {
     CK_TRY(h_flags_.reserve(8));
     CK_TRY(h_counts_.reserve(4));
     CK_TRY(d_flags_.reserve(8));
-    CK_TRY(d_queue_.reserve(2));
+    CK_TRY(d_queue_.reserve(6));
     ready_ = true;
     return kOk;
 }
@@ -123,6 +123,7 @@ int Engine::load_params(const std::string& path, std::string& err) {
     rel(h.pt3); rel(h.pt4);
     rel(h.tc3);
     rel(h.tc4);
+    rel(h.key3); rel(h.key4);
     rel(h.fx2); rel(h.fx3); rel(h.fx4);
     rel(h.t2rec); rel(h.tab2r); rel(h.tab2c);
     rel(h.t3rec); rel(h.tab3r); rel(h.tab3v);
@@ -291,16 +292,17 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     CK_TRY(d_ghost_parent_.reserve(ghost_off));
     CK_TRY(d_ghost_bin_.reserve(ghost_off));
     CK_TRY(d_ghost_fs_.reserve(3 * ghost_off));
-    CK_TRY(d_ghost_xn_.reserve(3 * ghost_off));
     CK_TRY(d_ghost_fn_.reserve(3 * ghost_off));
     CK_TRY(d_bin_items_.reserve(ghost_off));
     CK_TRY(d_bin_xp_.reserve(4 * ghost_off));
     CK_TRY(d_minmax_.reserve(6 * S));
     CK_TRY(d_bin_count_.reserve(bin_off));
     CK_TRY(d_bin_fill_.reserve(bin_off));
-    CK_TRY(d_bin_start_.reserve(bin_off + 1));
+    CK_TRY(d_bin_start_.reserve(bin_off));
     CK_TRY(d_l2_count_.reserve(atom_off));
-    CK_TRY(d_l2_off_.reserve(atom_off + 1));
+    CK_TRY(d_l2_off_.reserve(atom_off));
+    CK_TRY(d_a_off_.reserve(2 * atom_off));
+    CK_TRY(d_a_cnt_.reserve(2 * atom_off));
     CK_TRY(d_force_.reserve(3 * in_off));
     CK_TRY(d_ev_.reserve(8 * S));
     CK_TRY(h_in_pos_.reserve(3 * in_off));
@@ -324,6 +326,7 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
 
 Status Engine::ensure_lists(std::string& err) {
     CK_TRY(d_l2_ghost_.reserve(n2_cap_));
+    CK_TRY(d_pe_.reserve(4 * n2_cap_));
     CK_TRY(d_l2_owner_.reserve(n2_cap_));
     CK_TRY(d_l2_dist_.reserve(n2_cap_));
     CK_TRY(d_l2_vec_.reserve(4 * n2_cap_));
@@ -338,13 +341,14 @@ Status Engine::ensure_lists(std::string& err) {
     const long long p4cap = nbk4_ > 0 ? n4_cap_ + 32LL * nbk4_ : 0;
     CK_TRY(d_perm3_.reserve(std::max(1LL, p3cap)));
     CK_TRY(d_perm4_.reserve(std::max(1LL, p4cap)));
+    CK_TRY(d_bk_key3_.reserve(std::max(1LL, nbk3_ > 0 ? n3_cap_ : 0)));
+    CK_TRY(d_bk_key4_.reserve(std::max(1LL, nbk4_ > 0 ? n4_cap_ : 0)));
     CK_TRY(d_bk_count_.reserve(nbk3_ + nbk4_ + 1));
     CK_TRY(d_bk_fill_.reserve(nbk3_ + nbk4_ + 1));
     CK_TRY(d_bk_start_.reserve(nbk3_ + nbk4_ + 2));
     if (avail_ent_) {
         CK_TRY(d_ghost_sh_.reserve(V_.n_ghost_total));
         CK_TRY(d_l2_key_.reserve(n2_cap_));
-        CK_TRY(d_pe_.reserve(4 * n2_cap_));
         if (tuning.rf3 > 0) {
             CK_TRY(d_c3e_.reserve(3 * n3_cap_));
             CK_TRY(d_pcd3_.reserve(4 * n2_cap_));
@@ -366,8 +370,7 @@ Status Engine::ensure_lists(std::string& err) {
         CK_TRY(d_pcd4_.reserve(8 * n2_cap_));
         CK_TRY(d_pct4_.reserve((long long)sizeof(double) * 2 * tuning.rf4 * n2_cap_));
     }
-    long long scan_n = std::max(std::max(V_.n_bins_total, V_.n_atoms_total), n2_cap_);
-    CK_TRY(d_scan_tmp_.reserve(scan_tmp_bytes(scan_n)));
+    if (enum_serial_) CK_TRY(d_scan_tmp_.reserve(scan_tmp_bytes(n2_cap_)));
     BatchView& B = V_;
     B.sys = d_sys_.p;
     B.psets = dsets_.p;
@@ -378,7 +381,7 @@ Status Engine::ensure_lists(std::string& err) {
     B.ghost_id = d_ghost_id_.p;
     B.ghost_xf = d_ghost_xf_.p;
     B.ghost_parent = d_ghost_parent_.p;
-    B.ghost_fs = d_ghost_fs_.p; B.ghost_xn = d_ghost_xn_.p; B.ghost_fn = d_ghost_fn_.p;
+    B.ghost_fs = d_ghost_fs_.p; B.ghost_fn = d_ghost_fn_.p;
     B.minmax = d_minmax_.p;
     B.ghost_bin = d_ghost_bin_.p;
     B.bin_count = d_bin_count_.p; B.bin_start = d_bin_start_.p; B.bin_fill = d_bin_fill_.p;
@@ -388,10 +391,14 @@ Status Engine::ensure_lists(std::string& err) {
     B.l2_vec = d_l2_vec_.p;
     B.n2_cap = n2_cap_;
     B.e_cnt3 = d_e_cnt3_.p; B.e_cnt4 = d_e_cnt4_.p; B.e_off3 = d_e_off3_.p; B.e_off4 = d_e_off4_.p;
+    B.a_off = d_a_off_.p; B.a_cnt = d_a_cnt_.p;
     B.c3 = d_c3_.p; B.c4 = d_c4_.p;
     B.n3_cap = n3_cap_; B.n4_cap = n4_cap_;
     B.force = d_force_.p; B.ev = d_ev_.p; B.flags = d_flags_.p; B.queue = d_queue_.p;
     B.enum_serial = enum_serial_ ? 1 : 0;
+    B.totals = reinterpret_cast<long long*>(d_queue_.p + 2);
+    B.n3_ptr = enum_serial_ ? B.e_off3 + B.n2_cap : B.totals + 1;
+    B.n4_ptr = enum_serial_ ? B.e_off4 + B.n2_cap : B.totals + 2;
     B.c3e = avail_pc3_ || (avail_ent_ && tuning.rf3 > 0) ? d_c3e_.p : nullptr;
     B.c4e = avail_pc4_ || (avail_ent_ && tuning.rf4 > 0) ? d_c4e_.p : nullptr;
     B.all_pairs = avail_ent_ ? 1 : 0;
@@ -403,6 +410,7 @@ Status Engine::ensure_lists(std::string& err) {
     B.use_pc3 = B.use_pc4 = 0;   // set per launch from the contraction form
     B.nbk3 = nbk3_; B.nbk4 = nbk4_;
     B.bk_count = d_bk_count_.p; B.bk_fill = d_bk_fill_.p; B.bk_start = d_bk_start_.p;
+    B.bk_key3 = d_bk_key3_.p; B.bk_key4 = d_bk_key4_.p;
     B.perm3 = d_perm3_.p; B.perm4 = d_perm4_.p;
     B.perm3_cap = p3cap; B.perm4_cap = p4cap;
     return kOk;
@@ -439,6 +447,8 @@ Status Engine::enqueue(std::string& err) {
     B.use_pc3 = avail_pc3_ && tuning.fact3 && (tuning.tc3 || pc_small_) ? 1 : 0;
     B.bk_pad3 = tuning.tc3 ? 128 : 32;
     B.use_pc4 = avail_pc4_ && tuning.fact4 && !tuning.tc4 ? 1 : 0;
+    // the enumeration writes and counts the bucket keys when a contraction reads them
+    B.keyed = !B.enum_serial && ((tuning.stride3 > 0 && tuning.fact3) || (tuning.stride4 > 0 && tuning.fact4)) ? 1 : 0;
     cudaStream_t st = stream_;
     const long long k0 = launch_counter();
     if (profile) {
@@ -447,29 +457,18 @@ Status Engine::enqueue(std::string& err) {
         CK_TRY(record_stage_event(ev_[0], st));
     }
     NvtxRange lists_range("chimes: list build");
-    CK_TRY(cudaMemsetAsync(B.bin_count, 0, sizeof(int) * B.n_bins_total, st));
-    CK_TRY(cudaMemsetAsync(B.bin_fill, 0, sizeof(int) * B.n_bins_total, st));
     launch_reset(B, st);
     launch_atoms(B, st);
     launch_ghosts(B, st);
-    launch_bin_setup(B, st);
-    launch_bin_count(B, st);
-    exclusive_scan(B.bin_count, B.bin_start, B.n_bins_total, d_scan_tmp_.p, st);
+    launch_bin_alloc(B, st);
     launch_bin_scatter(B, st);
     launch_bin_sort(B, st);
-    launch_l2(B, d_l2_owner_.p, false, st);
-    exclusive_scan(B.l2_count, B.l2_off, B.n_atoms_total, d_scan_tmp_.p, st);
-    launch_l2(B, d_l2_owner_.p, true, st);
+    launch_l2(B, d_l2_owner_.p, st);
     ForceLaunch L = tuning;
     L.precision = precision;
     // pair-entry form: every body order present runs in fixed point (an order
     // that the tuning gave to the per-coefficient kernel scatters its own forces)
     const bool ent = avail_ent_ && precision == kFP64 && ((L.stride3 > 0 && L.fact3) || (L.stride4 > 0 && L.fact4));
-    auto pairs12 = [&](cudaStream_t q) {
-        NvtxRange r("chimes: 1B+2B");
-        if (ent) launch_pairs_x(B, d_l2_owner_.p, L, q);
-        else launch_force2(B, d_l2_owner_.p, L, q);
-    };
     // Concurrent form: the second stream takes 1B+2B (it needs only the pair
     // lists) while the first enumerates the clusters, then the 4-body branch
     // while the first runs the 3-body one; both join before the copies out.
@@ -478,33 +477,23 @@ Status Engine::enqueue(std::string& err) {
     if (conc) {
         CK_TRY(cudaEventRecord(fork_, st));
         CK_TRY(cudaStreamWaitEvent(stream2_, fork_, 0));
-        pairs12(stream2_);
+        NvtxRange r("chimes: 1B+2B");
+        launch_pairs(B, d_l2_owner_.p, L, stream2_);
         CK_TRY(cudaEventRecord(pairs_, stream2_));
+        if (!ent) launch_pair_forces(B, stream2_);
     }
-    launch_enum(B, d_l2_owner_.p, false, st);
-    exclusive_scan2(B.e_cnt3, B.e_off3, B.e_cnt4, B.e_off4, B.n2_cap, d_scan_tmp_.p, st);
-    launch_enum(B, d_l2_owner_.p, true, st);
-    launch_check(B, st);
+    launch_enum(B, d_l2_owner_.p, d_scan_tmp_.p, st);
+    launch_bucket(B, L.stride3 > 0 && L.fact3, L.stride4 > 0 && L.fact4, st);
     lists_range.end();
     if (profile) CK_TRY(record_stage_event(ev_[1], st));
-    if ((L.stride3 > 0 && L.fact3) || (L.stride4 > 0 && L.fact4)) {
-        CK_TRY(cudaMemsetAsync(B.bk_count, 0, sizeof(int) * (B.nbk3 + B.nbk4), st));
-        CK_TRY(cudaMemsetAsync(B.bk_fill, 0, sizeof(int) * (B.nbk3 + B.nbk4), st));
-    }
     auto body3 = [&](cudaStream_t q) {
         if (L.stride3 <= 0) return;
         NvtxRange r("chimes: 3B");
         if (L.fact3 && L.tc3) {
-            launch_pair_tables(B, d_l2_owner_.p, 3, L, q);
-            launch_bucket(B, 3, q);
             launch_force3tc(B, L, q);
         } else if (L.fact3 && L.precision == kFP64) {
-            launch_bucket(B, 3, q);
-            if (ent && conc) (void)cudaStreamWaitEvent(q, pairs_, 0);
             launch_force3x(B, L, q);
         } else if (L.fact3) {
-            launch_pair_tables(B, d_l2_owner_.p, 3, L, q);
-            launch_bucket(B, 3, q);
             launch_force3f(B, L, q);
         } else {
             launch_force3(B, L, q);
@@ -514,14 +503,10 @@ Status Engine::enqueue(std::string& err) {
         if (L.stride4 <= 0) return;
         NvtxRange r("chimes: 4B");
         if (L.fact4 && L.tc4) {
-            launch_bucket(B, 4, q);
             launch_force4tc(B, L, q);
         } else if (L.fact4 && L.precision == kFP64) {
-            launch_bucket(B, 4, q);
             launch_force4x(B, L, q);
         } else if (L.fact4) {
-            launch_pair_tables(B, d_l2_owner_.p, 4, L, q);
-            launch_bucket(B, 4, q);
             launch_force4f(B, L, q);
         } else {
             launch_force4(B, L, q);
@@ -534,11 +519,16 @@ Status Engine::enqueue(std::string& err) {
         CK_TRY(cudaStreamWaitEvent(stream2_, fork2_, 0));
         body4(stream2_);
         CK_TRY(cudaEventRecord(join_, stream2_));
+        CK_TRY(cudaStreamWaitEvent(st, pairs_, 0));   // the pairs' tables
         body3(st);
         CK_TRY(cudaStreamWaitEvent(st, join_, 0));
         if (ent) launch_pair_forces(B, st);
     } else {
-        pairs12(st);
+        {
+            NvtxRange r("chimes: 1B+2B");
+            launch_pairs(B, d_l2_owner_.p, L, st);
+            if (!ent) launch_pair_forces(B, st);
+        }
         if (profile) CK_TRY(record_stage_event(ev_[2], st));
         body3(st);
         if (profile) CK_TRY(record_stage_event(ev_[3], st));
@@ -551,9 +541,11 @@ Status Engine::enqueue(std::string& err) {
     CK_TRY(cudaMemcpyAsync(h_force_.p, B.force, sizeof(double) * 3 * B.n_in_total, cudaMemcpyDeviceToHost, st));
     CK_TRY(cudaMemcpyAsync(h_ev_.p, B.ev, sizeof(double) * 8 * B.n_sys, cudaMemcpyDeviceToHost, st));
     CK_TRY(cudaMemcpyAsync(h_flags_.p, B.flags, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_counts_.p + 0, B.l2_off + B.n_atoms_total, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_counts_.p + 1, B.e_off3 + B.n2_cap, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_counts_.p + 2, B.e_off4 + B.n2_cap, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    CK_TRY(cudaMemcpyAsync(h_counts_.p, B.totals, sizeof(long long) * 3, cudaMemcpyDeviceToHost, st));
+    if (B.enum_serial) {
+        CK_TRY(cudaMemcpyAsync(h_counts_.p + 1, B.n3_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
+        CK_TRY(cudaMemcpyAsync(h_counts_.p + 2, B.n4_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    }
     CK_TRY(cudaGetLastError());
     return kOk;
 }
@@ -581,7 +573,7 @@ Status Engine::launch(std::string& err) {
                                   tuning.stride3, tuning.stride4, tuning.blocks_per_sm, profile ? 1 : 0,
                                   tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4, tuning.xw3, tuning.xw4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
-                                  tuning.tc3, tuning.tc4, V_.all_pairs};
+                                  tuning.tc3, tuning.tc4, V_.all_pairs, V_.enum_serial};
     for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
                           (const void*)V_.bin_items, (const void*)V_.l2_ghost, (const void*)V_.c3,
                           (const void*)V_.c4, (const void*)V_.force, (const void*)d_scan_tmp_.p,
@@ -589,7 +581,7 @@ Status Engine::launch(std::string& err) {
                           (const void*)V_.e_off3, (const void*)V_.psets, (const void*)V_.perm3,
                           (const void*)V_.perm4, (const void*)V_.bk_count, (const void*)V_.bk_fill,
                           (const void*)V_.bk_start, (const void*)V_.c3e, (const void*)V_.c4e,
-                          (const void*)V_.pe, (const void*)V_.l2_key, (const void*)V_.ghost_sh,
+                          (const void*)V_.pe, (const void*)V_.a_off, (const void*)V_.l2_off, (const void*)V_.l2_key, (const void*)V_.ghost_sh,
                           (const void*)V_.pcd3, (const void*)V_.pcd4, (const void*)V_.pct3, (const void*)V_.pct4})
         key.push_back((long long)(uintptr_t)p);
     if (key != graph_key_) {
@@ -629,7 +621,7 @@ Status Engine::collect(double* force_out, std::vector<SystemResult>& res, std::s
         err = "bin grid larger than its reserved capacity";
         return kErrGeometry;
     }
-    if ((f[0] & (2 | 4 | 8)) || c[0] > n2_cap_ || c[1] > n3_cap_ || c[2] > n4_cap_) {
+    if (c[0] > n2_cap_ || c[1] > n3_cap_ || c[2] > n4_cap_) {
         if (c[0] > n2_cap_) n2_cap_ = c[0] + c[0] / 8 + 1024;
         else {
             if (c[1] > n3_cap_) n3_cap_ = c[1] + c[1] / 8 + 1024;
@@ -949,16 +941,45 @@ Status Engine::export_lists(std::vector<int>& l2, std::vector<int>& l3, std::vec
     std::vector<int> gid(V_.n_ghost_total);
     if (V_.n_ghost_total)
         CK_TRY(cudaMemcpy(gid.data(), V_.ghost_id, sizeof(int) * V_.n_ghost_total, cudaMemcpyDeviceToHost));
-    l2.resize(2 * n2);
-    for (long long e = 0; e < n2; e++) {
-        const SysDesc& d = hsys_[asys[own[e]]];
-        l2[2 * e] = (int)(own[e] - d.atom_off);
-        l2[2 * e + 1] = gid[g2[e]];
+    // the reference's order: atom by atom (each atom's entries and clusters are
+    // contiguous and in order, wherever its block found room)
+    const long long na = V_.n_atoms_total;
+    std::vector<int> cnt(na), ccnt(2 * na);
+    std::vector<long long> off(na), coff(2 * na), e3, e4;
+    if (na) {
+        CK_TRY(cudaMemcpy(cnt.data(), V_.l2_count, sizeof(int) * na, cudaMemcpyDeviceToHost));
+        CK_TRY(cudaMemcpy(off.data(), V_.l2_off, sizeof(long long) * na, cudaMemcpyDeviceToHost));
     }
-    l3.resize(3 * n3);
-    for (long long q = 0; q < 3 * n3; q++) l3[q] = gid[g3[q]];
-    l4.resize(4 * n4);
-    for (long long q = 0; q < 4 * n4; q++) l4[q] = gid[g4[q]];
+    if (V_.enum_serial) {
+        e3.resize(n2 + 1);
+        e4.resize(n2 + 1);
+        CK_TRY(cudaMemcpy(e3.data(), V_.e_off3, sizeof(long long) * (n2 + 1), cudaMemcpyDeviceToHost));
+        CK_TRY(cudaMemcpy(e4.data(), V_.e_off4, sizeof(long long) * (n2 + 1), cudaMemcpyDeviceToHost));
+        for (long long r = 0; r < na; r++) {
+            coff[2 * r] = e3[off[r]];
+            coff[2 * r + 1] = e4[off[r]];
+            ccnt[2 * r] = (int)(e3[off[r] + cnt[r]] - e3[off[r]]);
+            ccnt[2 * r + 1] = (int)(e4[off[r] + cnt[r]] - e4[off[r]]);
+        }
+    } else if (na) {
+        CK_TRY(cudaMemcpy(coff.data(), V_.a_off, sizeof(long long) * 2 * na, cudaMemcpyDeviceToHost));
+        CK_TRY(cudaMemcpy(ccnt.data(), V_.a_cnt, sizeof(int) * 2 * na, cudaMemcpyDeviceToHost));
+    }
+    l2.clear();
+    l3.clear();
+    l4.clear();
+    l2.reserve(2 * n2);
+    l3.reserve(3 * n3);
+    l4.reserve(4 * n4);
+    for (long long r = 0; r < na; r++) {
+        for (long long e = off[r]; e < off[r] + cnt[r]; e++) {
+            l2.push_back((int)(own[e] - hsys_[asys[own[e]]].atom_off));
+            l2.push_back(gid[g2[e]]);
+        }
+        for (long long q = 3 * coff[2 * r]; q < 3 * (coff[2 * r] + ccnt[2 * r]); q++) l3.push_back(gid[g3[q]]);
+        for (long long q = 4 * coff[2 * r + 1]; q < 4 * (coff[2 * r + 1] + ccnt[2 * r + 1]); q++)
+            l4.push_back(gid[g4[q]]);
+    }
     return kOk;
 }
 

@@ -179,7 +179,7 @@ private:
     DevBuf<int> d_atom_self_, d_ghost_id_;
     DevBuf<float> d_ghost_xf_, d_l2_vec_, d_bin_xp_;
     DevBuf<int> d_ghost_parent_, d_ghost_bin_;
-    DevBuf<double> d_ghost_fs_, d_ghost_xn_, d_ghost_fn_;
+    DevBuf<double> d_ghost_fs_, d_ghost_fn_;
     DevBuf<unsigned long long> d_minmax_;
     DevBuf<int> d_bin_count_, d_bin_fill_, d_bin_items_;
     DevBuf<long long> d_bin_start_;
@@ -200,7 +200,8 @@ private:
     DevBuf<int> d_c3e_, d_c4e_;
     DevBuf<double> d_pcd3_, d_pcd4_, d_pe_;
     DevBuf<int> d_ghost_sh_;
-    DevBuf<long long> d_l2_key_;
+    DevBuf<long long> d_l2_key_, d_a_off_;
+    DevBuf<int> d_a_cnt_, d_bk_key3_, d_bk_key4_;
     DevBuf<unsigned char> d_pct3_, d_pct4_;
     DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_;
     DevBuf<long long> d_bk_start_;

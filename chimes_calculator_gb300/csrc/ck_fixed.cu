@@ -51,10 +51,6 @@ namespace {
 
 constexpr int kFxTile = 32;   // clusters per block
 
-__device__ __forceinline__ PairTab tuple_pair_x(const TupleRec& R, int p) {
-    return PairTab{R.rin[p], R.rout[p], R.xavg[p], R.xdiff[p], R.inv_lam[p], R.inv_xdiff[p], R.fc_th[p], R.fc_inv[p]};
-}
-
 __device__ __forceinline__ FxEnt fx_quad(const Fx& t, const Fx& d) { return FxEnt{t.h, t.l, d.h, d.l}; }
 __device__ __forceinline__ Fx quad_t(const FxEnt* q) { return fx_load(*reinterpret_cast<const FxPair*>(q)); }
 
@@ -72,18 +68,19 @@ struct EAcc {
         v += e;
     }
     // warp-collective, one interaction per valid lane: lane 0 takes the warp's
-    // sum when the lanes hold one system (see EVAcc::add_warp)
+    // sum per system (see EVAcc::add_warp)
     __device__ void add_warp(const BatchView& B, int sys, double e, bool valid) {
-        const unsigned have = __ballot_sync(kFull, valid);
-        if (!have) return;
-        const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
-        if (__all_sync(kFull, !valid || sys == s0)) {
-            double x = valid ? e : 0.0;
+        unsigned have = __ballot_sync(kFull, valid);
+        for (int round = 0; have && round < 4; round++) {
+            const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
+            const bool mine = valid && sys == s0;
+            have &= ~__ballot_sync(kFull, mine);
+            double x = mine ? e : 0.0;
             for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
             if ((threadIdx.x & 31) == 0) add(B, s0, x);
-        } else if (valid) {
-            add(B, sys, e);
+            if (mine) valid = false;
         }
+        if (valid) add(B, sys, e);
     }
     // end of kernel: one atomic per warp when the warp holds one system
     __device__ void flush_warp(const BatchView& B) {
@@ -112,13 +109,29 @@ __device__ __forceinline__ void put_pair(const DevParamSet& P, const PairTab& Q,
     reinterpret_cast<double2*>(scal)[1] = make_double2(fcd * rinv, (double)flags);
 }
 
-// Bound by the FP64 pipe (geometry, square root, exponential and the three
-// cutoffs' sines; the polynomial sums are fixed-point).
+// The mixed form's pair-table cache: the values the cluster kernel would compute
+// for a pair ij, ik or il, once per entry.
+__device__ __forceinline__ void put_pair_f(const DevParamSet& P, const PairTab& Q, const double* dr, double r, double ex,
+                                           int R, int rs, float* tab, double* g) {
+    float fc, fcd;
+    pair_setup<float>(P, Q, r, ex, tab, tab + rs, 1, R, fc, fcd, nullptr);
+    g[0] = dr[0]; g[1] = dr[1]; g[2] = dr[2]; g[3] = r;
+    g[4] = double(fc); g[5] = double(fcd); g[6] = r < Q.rin ? 1.0 : 0.0; g[7] = 0.0;
+}
+
+// Bound by the FP64 pipe (geometry, square root, exponential and the cutoffs'
+// sines; the polynomial sums are fixed-point).  Measured: 5.23 M entries mixed
+// 1.32 ms and 0.41 ms for their forces, against 1.84 ms for the 2-body kernel
+// and 0.59 ms for a separate pass over the tables.  rs3, rs4: stride of the tables of
+// a body order, 0 for none.  (Entries one by one: with an atom's entries spread
+// over eight lanes instead, 384 configurations took 941 us and not 456, the
+// lanes' rounds being one long dependent chain each.)
+template <bool MIXED>
 __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owner, int rs3, int rs4) {
-    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
+    const long long n2 = list_total(B);
     EAcc acc, acc1;   // 2-body, 1-body (an atom and an entry of the same number are mostly of different systems)
     const long long ntot = n2 > B.n_atoms_total ? n2 : B.n_atoms_total;
-    // one contiguous range of entries per block, as k_force2
+    // one contiguous range of entries per block, so that the energy changes system seldom
     const long long per = ((ntot + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
     const long long e_end = min(ntot, per * (blockIdx.x + 1));
     for (long long e = per * blockIdx.x + threadIdx.x; e < e_end; e += blockDim.x) {
@@ -147,12 +160,16 @@ __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owne
         }
         reinterpret_cast<double2*>(B.pe + 4 * e)[0] = make_double2(dr[0], dr[1]);
         reinterpret_cast<double2*>(B.pe + 4 * e)[1] = make_double2(dr[2], fs);
-        // (a pair jk of some cluster can lie at the cutoff itself, to rounding, in this list)
-        const double dist = B.l2_dist[e] - 1e-6;
-        if (rs3 > 0 && d.has3 && dist < d.c3)
-            put_pair(P, P.pt3[pt], r, rinv, ex, P.R3, reinterpret_cast<FxEnt*>(B.pct3) + e * rs3, B.pcd3 + 4 * e);
-        if (rs4 > 0 && d.has4 && dist < d.c4)
-            put_pair(P, P.pt4[pt], r, rinv, ex, P.R4, reinterpret_cast<FxEnt*>(B.pct4) + e * rs4, B.pcd4 + 4 * e);
+        // (FP64: a pair jk of some cluster can lie at the cutoff itself, to rounding, in this list)
+        const double dist = MIXED ? B.l2_dist[e] : B.l2_dist[e] - 1e-6;
+        if (rs3 > 0 && d.has3 && dist < d.c3) {
+            if (MIXED) put_pair_f(P, P.pt3[pt], dr, r, ex, P.R3, rs3, reinterpret_cast<float*>(B.pct3) + e * 2 * rs3, B.pcd3 + 8 * e);
+            else put_pair(P, P.pt3[pt], r, rinv, ex, P.R3, reinterpret_cast<FxEnt*>(B.pct3) + e * rs3, B.pcd3 + 4 * e);
+        }
+        if (rs4 > 0 && d.has4 && dist < d.c4) {
+            if (MIXED) put_pair_f(P, P.pt4[pt], dr, r, ex, P.R4, rs4, reinterpret_cast<float*>(B.pct4) + e * 2 * rs4, B.pcd4 + 8 * e);
+            else put_pair(P, P.pt4[pt], r, rinv, ex, P.R4, reinterpret_cast<FxEnt*>(B.pct4) + e * rs4, B.pcd4 + 4 * e);
+        }
     }
     acc.flush_warp(B);
     acc1.flush_warp(B);
@@ -170,7 +187,8 @@ __global__ void __launch_bounds__(256) k_pair_forces(BatchView B) {
     for (long long k = 0; k < per; k++) {   // (all lanes of a warp make every round)
         const long long a = a0 + k;
         const bool have = a < B.n_atoms_total;
-        const long long b0 = have ? min(B.l2_off[a], B.n2_cap) : 0, b1 = have ? min(B.l2_off[a + 1], B.n2_cap) : 0;
+        long long b0 = 0, b1 = 0;
+        if (have) list_range(B, a, b0, b1);
         double f[3] = {0.0, 0.0, 0.0};
         if (have) {
             const int s = B.atom_sys[a];
@@ -242,7 +260,7 @@ __device__ __noinline__ void missing_pair(const BatchView& B, const DevParamSet&
     double dr[3], r, fc, fcd, gs;
     pair_geom(B, B.sys[s].h, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], dr, r);
     const int Rp = NB == 3 ? P.R3 : P.R4;
-    const PairTab Q = tuple_pair_x(R, p);
+    const PairTab Q = tuple_pair(R, p);
     pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
                  [&](int n, const Fx& t, const Fx& d) { tab[n * kFxTile] = fx_quad(t, d); });
     scal[0] = fc;
@@ -321,7 +339,7 @@ __device__ __forceinline__ bool fx_setup(const BatchView& B, const int* clusters
             for (int p = w; p < NP; p += NW) {
                 FxEnt* tab = m.table(p, rs) + lane;
                 const double r = geo[(4 * p + 3) * kFxTile + lane];
-                const PairTab Q = tuple_pair_x(R, p);
+                const PairTab Q = tuple_pair(R, p);
                 if (r < Q.rin) atomicAdd(&B.flags[4], 1);
                 double fc, fcd, gs;
                 pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
@@ -731,12 +749,18 @@ void launch_x4_ent(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
 
 }  // namespace
 
-void launch_pairs_x(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st) {
+void launch_pairs(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st) {
     const long long ntot = B.n2_cap > B.n_atoms_total ? B.n2_cap : B.n_atoms_total;
     if (ntot <= 0) return;
     const long long want = (long long)sm_count() * 12, need = (ntot + 127) / 128;
     const unsigned grid = (unsigned)(want < need ? want : need);
-    count_launch(), k_pairs_x<<<grid, 128, 0, st>>>(B, l2_owner, B.nbk3 > 0 ? L.rf3 : 0, B.nbk4 > 0 ? L.rf4 : 0);
+    if (L.precision == kMixed) {
+        count_launch(), k_pairs_x<true><<<grid, 128, 0, st>>>(B, l2_owner, B.use_pc3 ? L.rf3 : 0, B.use_pc4 ? L.rf4 : 0);
+    } else {
+        const bool ent = B.all_pairs;
+        count_launch(), k_pairs_x<false><<<grid, 128, 0, st>>>(B, l2_owner, ent && B.nbk3 > 0 ? L.rf3 : 0,
+                                                             ent && B.nbk4 > 0 ? L.rf4 : 0);
+    }
 }
 
 void launch_pair_forces(const BatchView& B, cudaStream_t st) {

@@ -45,7 +45,7 @@ namespace {
 // ---------------------------------------------------------------------------
 template <typename CT>
 __global__ void __launch_bounds__(256) k_force2(BatchView B, const int* l2_owner) {
-    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
+    const long long n2 = list_total(B);
     EVAcc acc;
     const long long ntot = n2 > B.n_atoms_total ? n2 : B.n_atoms_total;
     // each block takes one contiguous range of entries (threads striding by
@@ -396,13 +396,13 @@ void launch_force2(const BatchView& B, const int* l2_owner, const ForceLaunch& L
 }
 
 void launch_force3(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    const long long* np = B.e_off3 + B.n2_cap;
+    const long long* np = B.n3_ptr;
     if (L.precision == kMixed) launch_n<3, float>(B, B.c3, np, B.n3_cap, L.tpc3, L.stride3, L, st);
     else launch_n<3, double>(B, B.c3, np, B.n3_cap, L.tpc3, L.stride3, L, st);
 }
 
 void launch_force4(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {
-    const long long* np = B.e_off4 + B.n2_cap;
+    const long long* np = B.n4_ptr;
     if (L.precision == kMixed) launch_n<4, float>(B, B.c4, np, B.n4_cap, L.tpc4, L.stride4, L, st);
     else launch_n<4, double>(B, B.c4, np, B.n4_cap, L.tpc4, L.stride4, L, st);
 }

@@ -96,15 +96,24 @@ __device__ __forceinline__ void tally_atoms(const BatchView& B, const int* ghost
     }
 }
 
-// Per-lane energy/virial accumulator for one system at a time.
+// Energy/virial accumulator for one system at a time: per lane (add), and per
+// warp (add_warp), where lane 4 k holds value k of the warp's sum.
 struct EVAcc {
     int s = -1;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    int ws = -1;      // the warp sum's system (uniform)
+    double wv = 0.0;
     __device__ void flush(const BatchView& B) {
         if (s >= 0)
             for (int k = 0; k < 7; k++) atomicAdd(&B.ev[8 * s + k], v[k]);
         s = -1;
         for (int k = 0; k < 7; k++) v[k] = 0;
+    }
+    __device__ void flush_sum(const BatchView& B) {
+        const int lane = threadIdx.x & 31;
+        if (ws >= 0 && (lane & 3) == 0 && lane < 28) atomicAdd(&B.ev[8 * ws + (lane >> 2)], wv);
+        ws = -1;
+        wv = 0.0;
     }
     __device__ void add(const BatchView& B, int sys, double e, const double* vir) {
         if (sys != s) { flush(B); s = sys; }
@@ -112,50 +121,98 @@ struct EVAcc {
         for (int k = 0; k < 6; k++) v[1 + k] += vir[k];
     }
     // Warp-collective (all 32 lanes call it): one interaction's energy and
-    // virial per lane (valid lanes), summed over the warp first when every
-    // valid lane's interaction belongs to one system, so that one lane's
-    // accumulator takes the sum (atomics only when that lane changes system);
-    // otherwise each valid lane adds its own.  Keeps batches of many systems
-    // from turning every interaction into seven atomics on a few addresses.
+    // virial per lane (valid lanes), summed over the warp per system -- the
+    // lanes of a warp mostly hold one, or few.  The seven sums are folded
+    // together (a lane keeps half of its values and hands over the rest at each
+    // step: 9 additions, where seven butterflies take 35; GB300 issues an FP64
+    // addition per 16 cycles and SM), so each costs 10 FP64 instructions.
     __device__ void add_warp(const BatchView& B, int sys, double e, const double* vir, bool valid) {
         const int lane = threadIdx.x & 31;
-        const unsigned have = __ballot_sync(kFull, valid);
-        if (!have) return;
-        const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
-        if (__all_sync(kFull, !valid || sys == s0)) {
-            double x[7];
-            x[0] = valid ? e : 0.0;
-            for (int k = 0; k < 6; k++) x[1 + k] = valid ? vir[k] : 0.0;
-            for (int k = 0; k < 7; k++)
-                for (int off = 16; off; off >>= 1) x[k] += __shfl_xor_sync(kFull, x[k], off);
-            if (lane == 0) add(B, s0, x[0], x + 1);
-        } else if (valid) {
-            add(B, sys, e, vir);
+        unsigned have = __ballot_sync(kFull, valid);
+        for (int round = 0; have && round < 4; round++) {
+            const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
+            const bool mine = valid && sys == s0;
+            have &= ~__ballot_sync(kFull, mine);
+            double x[8];
+            x[0] = mine ? e : 0.0;
+#pragma unroll
+            for (int k = 0; k < 6; k++) x[1 + k] = mine ? vir[k] : 0.0;
+            x[7] = 0.0;
+#pragma unroll
+            for (int n = 4, off = 16; n >= 1; n >>= 1, off >>= 1) {
+                const bool up = lane & off;
+#pragma unroll
+                for (int k = 0; k < n; k++) {
+                    const double give = up ? x[k] : x[k + n], keep = up ? x[k + n] : x[k];
+                    x[k] = keep + __shfl_xor_sync(kFull, give, off);
+                }
+            }
+            x[0] += __shfl_xor_sync(kFull, x[0], 2);
+            x[0] += __shfl_xor_sync(kFull, x[0], 1);
+            if (s0 != ws) {
+                flush_sum(B);
+                ws = s0;
+            }
+            wv += x[0];
+            if (mine) valid = false;
         }
+        if (valid) add(B, sys, e, vir);   // a warp of many systems
     }
-    // end of kernel: one set of atomics per warp when the warp holds one system
+    // end of kernel: the sums, one set of atomics per warp when its lanes hold one system
     __device__ void flush_warp(const BatchView& B) {
+        flush_sum(B);
         const int lane = threadIdx.x & 31;
-        int key = s;
-        int s0 = -1;
-        for (int l = 0; l < 32; l++) {
-            int t = __shfl_sync(kFull, key, l);
-            if (t >= 0) { s0 = t; break; }
-        }
-        const bool uniform = __all_sync(kFull, s < 0 || s == s0);
-        if (uniform) {
+        const unsigned have = __ballot_sync(kFull, s >= 0);
+        if (!have) return;
+        const int s0 = __shfl_sync(kFull, s, __ffs(have) - 1);
+        if (__all_sync(kFull, s < 0 || s == s0)) {
             for (int k = 0; k < 7; k++) {
                 double x = v[k];
                 for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
                 v[k] = x;
             }
-            if (lane == 0 && s0 >= 0)
+            if (lane == 0)
                 for (int k = 0; k < 7; k++) atomicAdd(&B.ev[8 * s0 + k], v[k]);
         } else {
             flush(B);
         }
     }
 };
+
+// Chebyshev tables and cutoff of pair p of a tuple (set_cheby_polys,
+// chimesFF.h:542-628; get_fcut, chimesFF.h:347-386) with the tuple's
+// precomputed reciprocals in place of the divisions; ex = exp(-r / lambda).
+__device__ __forceinline__ PairTab tuple_pair(const TupleRec& R, int p) {
+    return PairTab{R.rin[p], R.rout[p], R.xavg[p], R.xdiff[p], R.inv_lam[p], R.inv_xdiff[p], R.fc_th[p], R.fc_inv[p]};
+}
+
+template <typename CT>
+__device__ __forceinline__ void pair_setup(const DevParamSet& P, const PairTab& Q, double r, double ex, CT* T, CT* D,
+                                           int stride, int nT, CT& fc, CT& fcd, int* flags) {
+    const double rin = Q.rin;
+    const bool oor = r < rin;
+    const double e = oor ? exp(-rin * Q.inv_lam) : ex;
+    const double xd = (e - Q.xavg) * Q.inv_xdiff;
+    const double dxdr = -e * Q.inv_lam * Q.inv_xdiff;
+    cheby_fill_strided<CT>(T, D, stride, nT, xd, dxdr, oor, r, rin, P.inner_smooth, flags);
+    const double finv = Q.fc_inv;
+    if (!P.tersoff) {
+        const CT f0 = CT(1.0) - CT(r) * CT(finv);
+        fc = f0 * f0 * f0;
+        fcd = f0 * f0 * (CT(-3.0) * CT(finv));
+    } else {
+        const double th = Q.fc_th;
+        if (r < th) { fc = CT(1); fcd = CT(0); }
+        else if (r > Q.rout) { fc = CT(0); fcd = CT(0); }
+        else {
+            const CT f0 = CT(r - th) * CT(finv) * CT(kPi) + CT(kPi / 2.0);
+            CT sn, cs;
+            csincos<CT>(f0, &sn, &cs);
+            fc = CT(0.5) + CT(0.5) * sn;
+            fcd = CT(0.5) * cs * (CT(kPi) * CT(finv));
+        }
+    }
+}
 
 __device__ __forceinline__ void virial_add(double* vir, double f, const double* d) {
     vir[0] -= f * d[0] * d[0];

@@ -164,6 +164,7 @@ Status system_geometry(const double* ca, const double* cb, const double* cc, int
     d.search = c2;
     if (c3 > d.search) d.search = c3;
     if (c4 > d.search) d.search = c4;
+    d.inv_search = 1.0 / d.search;
     d.c3 = has3 ? c3 : 0.0;
     d.c4 = has4 ? c4 : 0.0;
     d.n_in = n_in;
@@ -248,7 +249,6 @@ Status system_geometry(const double* ca, const double* cb, const double* cc, int
     d.c4lo2 = sq_down(d.c4lo);
     d.c4hi2 = sq_up(d.c4hi);
     d.far2 = (float)((d.search + d.eps) * (d.search + d.eps));
-    d.near2 = d.search > d.eps ? (float)((d.search - d.eps) * (d.search - d.eps)) : 0.0f;
     return kOk;
 }
 

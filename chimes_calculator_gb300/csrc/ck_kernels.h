@@ -9,16 +9,14 @@ namespace ck {
 // ---- cluster-list build (ck_lists.cu) -------------------------------------
 void launch_atoms(const BatchView& B, cudaStream_t st);
 void launch_ghosts(const BatchView& B, cudaStream_t st);
-void launch_bin_setup(const BatchView& B, cudaStream_t st);
-void launch_bin_count(const BatchView& B, cudaStream_t st);
+void launch_bin_alloc(const BatchView& B, cudaStream_t st);
 void launch_bin_scatter(const BatchView& B, cudaStream_t st);
 void launch_bin_sort(const BatchView& B, cudaStream_t st);
-void launch_l2(const BatchView& B, int* l2_owner, bool fill, cudaStream_t st);
-// Runs over the list capacity B.n2_cap; the live count is read on the device.
-void launch_enum(const BatchView& B, const int* l2_owner, bool fill, cudaStream_t st);
-// Sets capacity flags when a live count exceeds its buffer.
-void launch_check(const BatchView& B, cudaStream_t st);
-// Clears bounding boxes, accumulators and flags.
+void launch_l2(const BatchView& B, int* l2_owner, cudaStream_t st);
+// Sequential enumeration (B.enum_serial): runs over the list capacity B.n2_cap,
+// with two scans in scan_tmp; the live count is read on the device.
+void launch_enum(const BatchView& B, const int* l2_owner, void* scan_tmp, cudaStream_t st);
+// Clears bounding boxes, accumulators, counters, bins, buckets and flags.
 void launch_reset(const BatchView& B, cudaStream_t st);
 
 // Exclusive scan of n ints into n+1 int64 (out[n] = total).  `tmp` must hold
@@ -60,25 +58,24 @@ struct ForceLaunch {
     int tc4 = 0, want_tc4 = 0;
 };
 
-// Cluster counts are read on the device (l2_off[n_atoms], e_off3/4[n2_cap]) and
+// Cluster counts are read on the device (totals, n3_ptr, n4_ptr) and
 // clamped to the capacities, so launches need no host round trip.
 void launch_force2(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st);
 void launch_force3(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 
-// Factored contraction of the mixed form (ck_factored.cu): bucket the clusters of one body
-// order by (parameter set, type tuple), then contract.  Both read their
+// Factored contraction of the mixed form (ck_factored.cu): bucket the clusters of one or both
+// body orders by (parameter set, type tuple), then contract.  Both read their
 // counts on the device.
-void launch_bucket(const BatchView& B, int nbody, cudaStream_t st);
-// Pair-table cache of body order nbody (when B.use_pc3 / use_pc4): one pass over the list entries.
-void launch_pair_tables(const BatchView& B, const int* l2_owner, int nbody, const ForceLaunch& L, cudaStream_t st);
+void launch_bucket(const BatchView& B, bool three, bool four, cudaStream_t st);
 void launch_force3f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4f(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 // The FP64 form of the factored contraction, in 64-bit fixed point (ck_fixed.cu).
-// Pair-entry form (B.all_pairs): launch_pairs_x does the 1-body and 2-body terms
-// and the pairs' tables before the contractions, launch_pair_forces the forces
-// and virial of every pair after them.
-void launch_pairs_x(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st);
+// Once per list entry, both forms: launch_pairs does the 1-body and 2-body terms
+// and the pairs' tables (FP64 pair-entry form, mixed pair-table cache),
+// launch_pair_forces the forces and virial of every entry's force scalar (in the
+// pair-entry form after the contractions, which add theirs to it).
+void launch_pairs(const BatchView& B, const int* l2_owner, const ForceLaunch& L, cudaStream_t st);
 void launch_pair_forces(const BatchView& B, cudaStream_t st);
 void launch_force3x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);
 void launch_force4x(const BatchView& B, const ForceLaunch& L, cudaStream_t st);

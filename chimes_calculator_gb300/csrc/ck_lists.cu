@@ -24,6 +24,7 @@
 //    distance that is stored, is evaluated exactly in FP64.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 
@@ -112,6 +113,23 @@ __device__ __forceinline__ void shift_box(const SysDesc& d, const double* fn, Sh
     }
 }
 
+// bin grid of a system from its bounding box (build_neigh_lists :622-642)
+__device__ __forceinline__ void bin_setup(const BatchView& B, int s, SysDesc& d) {
+    long long total = 1;
+    for (int c = 0; c < 3; c++) {
+        const double mn = okey_inv(__ldcg(&B.minmax[6 * s + c])), mx = okey_inv(__ldcg(&B.minmax[6 * s + 3 + c]));
+        d.minpos[c] = mn;
+        int nb = (int)ceil(__ddiv_rn(sub(mx, mn), d.search));
+        if (nb < 1) nb = 1;
+        d.nb[c] = nb;
+        total *= nb;
+    }
+    if (total > d.bin_cap) {
+        d.err = kErrCapacity;
+        atomicOr(&B.flags[0], 1);
+    }
+}
+
 // --- 1. atoms: replicate (small=true), wrap, reorient, bounding box --------
 // simulation_system::init (:196-322) and reorient (:352-405).  The bounding box
 // of all ghost images (build_neigh_lists :590-610) comes from each atom, its
@@ -150,7 +168,6 @@ __global__ void k_atoms(BatchView B) {
         const long long q = d.ghost_off + (long long)rl * d.gstride + (j0 < d.gstride ? j0 : 0);
         for (int c = 0; c < 3; c++) {
             B.ghost_fs[3 * q + c] = fa[c];
-            B.ghost_xn[3 * q + c] = xn[c];
             B.ghost_fn[3 * q + c] = fn[c];
             B.ghost_xf[3 * q + c] = (float)xn[c];
         }
@@ -184,6 +201,7 @@ __global__ void k_atoms(BatchView B) {
         kmin[c] = valid ? okey(lo[c]) : ~0ull;
         kmax[c] = valid ? okey(hi[c]) : 0ull;
     }
+    int mine = valid ? 1 : 0;   // atoms this lane reports
     if (uniform) {
         for (int off = 16; off; off >>= 1)
             for (int c = 0; c < 3; c++) {
@@ -192,23 +210,37 @@ __global__ void k_atoms(BatchView B) {
                 kmin[c] = a < kmin[c] ? a : kmin[c];
                 kmax[c] = b > kmax[c] ? b : kmax[c];
             }
-        if (lane == 0)
-            for (int c = 0; c < 3; c++) {
-                atomicMin(&B.minmax[6 * s0 + c], kmin[c]);
-                atomicMax(&B.minmax[6 * s0 + 3 + c], kmax[c]);
-            }
-    } else if (valid) {
-        for (int c = 0; c < 3; c++) {
-            atomicMin(&B.minmax[6 * s + c], kmin[c]);
-            atomicMax(&B.minmax[6 * s + 3 + c], kmax[c]);
-        }
+        mine = __popc(__ballot_sync(kFull, valid));
+        if (lane != 0) mine = 0;
+        s = s0;
     }
+    if (mine == 0) return;
+    for (int c = 0; c < 3; c++) {
+        atomicMin(&B.minmax[6 * s + c], kmin[c]);
+        atomicMax(&B.minmax[6 * s + 3 + c], kmax[c]);
+    }
+    // the lane that completes its system sets the system's bin grid
+    __threadfence();
+    SysDesc& d = B.sys[s];
+    if (atomicAdd(&d.done, mine) + mine != d.n_atoms) return;
+    __threadfence();
+    bin_setup(B, s, d);
 }
 
 // --- 2. kept ghost images, one thread per slot -----------------------------
 // build_layered_system (:546-585) for both the input-cell system (fractional
 // coordinates for the force evaluation) and the reoriented system (Cartesian
 // and fractional coordinates for the lists).
+// floor((x - min) / search) as the reference computes it, with the correctly
+// rounded FP64 quotient: the FP32 quotient decides unless it lies within its
+// error (several times the rounding of the coordinates) of an integer.
+__device__ __forceinline__ int bin_axis(double x, double mn, double search, float inv) {
+    const float xf = (float)x, mf = (float)mn;
+    const float q = (xf - mf) * inv, f = floorf(q);
+    const float m = 1e-6f + 1e-6f * (fabsf(xf) + fabsf(mf)) * inv;
+    if (q - f > m && q - f < 1.0f - m) return (int)f;
+    return (int)floor(__ddiv_rn(sub(x, mn), search));
+}
 __global__ void k_ghosts(BatchView B) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= B.n_ghost_total) return;
@@ -218,78 +250,84 @@ __global__ void k_ghosts(BatchView B) {
     const int rl = (int)(ql / d.gstride), j = (int)(ql % d.gstride);
     const long long r = d.atom_off + rl;
     const long long qs = B.atom_self[r];
-    if (q == qs) return;   // the atom itself, written by k_atoms
-    const double fa[3] = {B.ghost_fs[3 * qs], B.ghost_fs[3 * qs + 1], B.ghost_fs[3 * qs + 2]};
     const double fn[3] = {B.ghost_fn[3 * qs], B.ghost_fn[3 * qs + 1], B.ghost_fn[3 * qs + 2]};
-    ShiftBox sb;
-    shift_box(d, fn, sb);
-    if (j >= sb.count) {
-        B.ghost_id[q] = -1;
-        return;
+    double t[3], xn[3];
+    if (q == qs) {   // the atom itself: the rest was written by k_atoms, from the wrapped coordinates
+        const double fa[3] = {B.ghost_fs[3 * qs], B.ghost_fs[3 * qs + 1], B.ghost_fs[3 * qs + 2]};
+        mv(d.hn, fa[0], fa[1], fa[2], xn);
+    } else {
+        ShiftBox sb;
+        shift_box(d, fn, sb);
+        if (j >= sb.count) {
+            B.ghost_id[q] = -1;
+            B.ghost_bin[q] = -1;
+            return;
+        }
+        const int i0 = sb.lo[0] + j / (sb.cnt[1] * sb.cnt[2]);
+        const int i1 = sb.lo[1] + (j / sb.cnt[2]) % sb.cnt[1];
+        const int i2 = sb.lo[2] + j % sb.cnt[2];
+        // input cell: only the forces' distances use these, so the image's
+        // fractional coordinates are the shifted ones themselves (the reference
+        // takes them through Cartesian ones and back, which rounds them)
+        B.ghost_fs[3 * q] = add(B.ghost_fs[3 * qs], (double)i0);
+        B.ghost_fs[3 * q + 1] = add(B.ghost_fs[3 * qs + 1], (double)i1);
+        B.ghost_fs[3 * q + 2] = add(B.ghost_fs[3 * qs + 2], (double)i2);
+        // reoriented cell: these decide list membership
+        double o[3];
+        t[0] = add(fn[0], (double)i0); t[1] = add(fn[1], (double)i1); t[2] = add(fn[2], (double)i2);
+        mv(d.hn, t[0], t[1], t[2], xn);
+        mv(d.hni, xn[0], xn[1], xn[2], o);
+        for (int c = 0; c < 3; c++) {
+            B.ghost_fn[3 * q + c] = o[c];
+            B.ghost_xf[3 * q + c] = (float)xn[c];
+        }
+        B.ghost_parent[q] = (int)r;
+        if (B.ghost_sh) B.ghost_sh[q] = pack_shift(i0, i1, i2);
+        B.ghost_id[q] = image_index(i0, i1, i2, d.n_layers, d.side) * d.n_atoms + rl;
     }
-    const int i0 = sb.lo[0] + j / (sb.cnt[1] * sb.cnt[2]);
-    const int i1 = sb.lo[1] + (j / sb.cnt[2]) % sb.cnt[1];
-    const int i2 = sb.lo[2] + j % sb.cnt[2];
-    double t[3], p[3], o[3], xn[3];
-    t[0] = add(fa[0], (double)i0); t[1] = add(fa[1], (double)i1); t[2] = add(fa[2], (double)i2);
-    mv(d.h, t[0], t[1], t[2], p);
-    mv(d.hi, p[0], p[1], p[2], o);
-    B.ghost_fs[3 * q] = o[0]; B.ghost_fs[3 * q + 1] = o[1]; B.ghost_fs[3 * q + 2] = o[2];
-    t[0] = add(fn[0], (double)i0); t[1] = add(fn[1], (double)i1); t[2] = add(fn[2], (double)i2);
-    mv(d.hn, t[0], t[1], t[2], xn);
-    mv(d.hni, xn[0], xn[1], xn[2], o);
-    for (int c = 0; c < 3; c++) {
-        B.ghost_xn[3 * q + c] = xn[c];
-        B.ghost_fn[3 * q + c] = o[c];
-        B.ghost_xf[3 * q + c] = (float)xn[c];
+    // bin population (:644-678)
+    int ib = -1;
+    if (!d.err) {
+        const float inv = (float)d.inv_search;
+        const int bx = bin_axis(xn[0], d.minpos[0], d.search, inv);
+        const int by = bin_axis(xn[1], d.minpos[1], d.search, inv);
+        const int bz = bin_axis(xn[2], d.minpos[2], d.search, inv);
+        const long long total = (long long)d.nb[0] * d.nb[1] * d.nb[2];
+        const long long b = bx + (long long)by * d.nb[0] + (long long)bz * d.nb[0] * d.nb[1];
+        if (bx < 0 || by < 0 || bz < 0) atomicExch(&B.flags[1], 1);
+        else if (b >= total) atomicExch(&B.flags[1], 2);
+        else ib = (int)b;
     }
-    B.ghost_parent[q] = (int)r;
-    if (B.ghost_sh) B.ghost_sh[q] = pack_shift(i0, i1, i2);
-    B.ghost_id[q] = image_index(i0, i1, i2, d.n_layers, d.side) * d.n_atoms + rl;
+    B.ghost_bin[q] = ib;
+    if (ib >= 0) atomicAdd(&B.bin_count[d.bin_off + ib], 1);
 }
 
-// --- 3. bin grid per system (build_neigh_lists :622-642) -------------------
-__global__ void k_bin_setup(BatchView B) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B.n_sys) return;
-    SysDesc& d = B.sys[s];
-    long long total = 1;
-    for (int c = 0; c < 3; c++) {
-        const double mn = okey_inv(B.minmax[6 * s + c]), mx = okey_inv(B.minmax[6 * s + 3 + c]);
-        d.minpos[c] = mn;
-        int nb = (int)ceil(__ddiv_rn(sub(mx, mn), d.search));
-        if (nb < 1) nb = 1;
-        d.nb[c] = nb;
-        total *= nb;
+// Room for every bin's members in bin_items: which bin comes first does not
+// matter, so a block scans its bins and reserves their sum.
+__global__ void __launch_bounds__(1024) k_bin_alloc(BatchView B) {
+    __shared__ int wsum[32];
+    __shared__ long long base;
+    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int v = b < B.n_bins_total ? B.bin_count[b] : 0;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
     }
-    if (total > d.bin_cap) {
-        d.err = kErrCapacity;
-        atomicOr(&B.flags[0], 1);
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        int t = wsum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, t, o);
+            if (lane >= o) t += y;
+        }
+        wsum[lane] = t;
+        if (lane == 31) base = t > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[3], (unsigned long long)t) : 0;
     }
-}
-
-__device__ __forceinline__ void bin_of(const SysDesc& d, const double* x, int& bx, int& by, int& bz) {
-    bx = (int)floor(__ddiv_rn(sub(x[0], d.minpos[0]), d.search));
-    by = (int)floor(__ddiv_rn(sub(x[1], d.minpos[1]), d.search));
-    bz = (int)floor(__ddiv_rn(sub(x[2], d.minpos[2]), d.search));
-}
-
-// --- 4. bin population (:644-678) -------------------------------------------
-__global__ void k_bin_count(BatchView B) {
-    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= B.n_ghost_total) return;
-    if (B.ghost_id[q] < 0) { B.ghost_bin[q] = -1; return; }
-    const int s = find_sys_ghost(B.sys, B.n_sys, q);
-    const SysDesc& d = B.sys[s];
-    if (d.err) { B.ghost_bin[q] = -1; return; }
-    int bx, by, bz;
-    bin_of(d, &B.ghost_xn[3 * q], bx, by, bz);
-    const long long total = (long long)d.nb[0] * d.nb[1] * d.nb[2];
-    if (bx < 0 || by < 0 || bz < 0) { atomicExch(&B.flags[1], 1); B.ghost_bin[q] = -1; return; }
-    const long long ib = bx + (long long)by * d.nb[0] + (long long)bz * d.nb[0] * d.nb[1];
-    if (ib >= total) { atomicExch(&B.flags[1], 2); B.ghost_bin[q] = -1; return; }
-    B.ghost_bin[q] = (int)ib;
-    atomicAdd(&B.bin_count[d.bin_off + ib], 1);
+    __syncthreads();
+    if (b < B.n_bins_total) B.bin_start[b] = base + x - v + (w ? wsum[w - 1] : 0);
 }
 
 __global__ void k_bin_scatter(BatchView B, const long long* bin_start) {
@@ -400,159 +438,201 @@ __global__ void __launch_bounds__(256) k_bin_rank(BatchView B, const long long* 
 // decides most candidates; the exact FP64 distance (which the list keeps) is
 // taken only for the candidates that survive it, queued in candidate order in
 // shared memory and evaluated 32 at a time, so the FP64 pipe (1/64 of the
-// FP32 rate) runs full warps instead of one or two live lanes per chunk.  The
-// count pass counts the candidates the FP32 test places inside the cutoff by
-// more than the margin without an FP64 distance.
+// FP32 rate) runs full warps instead of one or two live lanes per chunk.
+// One pass: a warp keeps its members in shared memory (up to kL2Hold; an atom
+// with more walks its candidates again), the block reserves room for its
+// warps' members with one atomic, and the members are written there.  (A
+// counting pass, a scan over the atoms and a filling pass took 402 + 863 us and
+// 10 us of scans on 2000 configurations of 8-512 atoms; this takes 906 us.)
 constexpr int kL2Block = 256;
+constexpr int kL2Hold = 96;
 // bits of l2_vec.w above the parent atom index (atom indices are below 2^30)
 constexpr unsigned kL2Parent = 0x3FFFFFFFu, kL2In3 = 1u << 30, kL2In4 = 1u << 31;
-template <bool FILL>
-__global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, const long long* bin_start, int* l2_owner) {
-    __shared__ int queue[kL2Block / 32][64];
-    __shared__ int qpar[kL2Block / 32][64];
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+struct L2Hold {
+    double dist[kL2Hold];
+    float x[3][kL2Hold];
+    int ghost[kL2Hold];
+    unsigned w[kL2Hold];
+};
+// An entry: x, y, z the FP32 displacement for the enumeration's prefilter; w the
+// neighbour's parent atom (int bits; saves the enumeration a dependent load per
+// candidate) with the exact tests dist < c3 and dist < c4 in bits 30 and 31, so
+// the enumeration compares no FP64 distances.
+__device__ __forceinline__ void put_l2(const BatchView& B, int* l2_owner, long long pos, int r, int ghost, double dist,
+                                       float x, float y, float z, unsigned w) {
+    if (pos >= B.n2_cap) return;
+    B.l2_ghost[pos] = ghost;
+    B.l2_dist[pos] = dist;
+    l2_owner[pos] = r;
+    if (B.l2_key) B.l2_key[pos] = (long long)(w & kL2Parent) << 32 | B.ghost_sh[ghost];
+    reinterpret_cast<float4*>(B.l2_vec)[pos] = make_float4(x, y, z, __uint_as_float(w));
+}
+
+__global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
+    constexpr int NWARP = kL2Block / 32;
+    __shared__ int queue[NWARP][64];
+    __shared__ int qpar[NWARP][64];
+    __shared__ L2Hold hold[NWARP];
+    __shared__ int s_cnt[NWARP];
+    __shared__ long long s_base;
+    const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    if (warp >= B.n_atoms_total) return;
-    const long long r = warp;
-    const int s = B.atom_sys[r];
+    const bool have = r < B.n_atoms_total;
+    const int s = have ? B.atom_sys[r] : 0;
     const SysDesc& d = B.sys[s];
-    if (d.err) { if (!FILL && lane == 0) B.l2_count[r] = 0; return; }
-    const long long gi = B.atom_self[r];
-    const double fi[3] = {B.ghost_fn[3 * gi], B.ghost_fn[3 * gi + 1], B.ghost_fn[3 * gi + 2]};
-    const float xi[3] = {B.ghost_xf[3 * gi], B.ghost_xf[3 * gi + 1], B.ghost_xf[3 * gi + 2]};
-    double hn[9];
-    for (int c = 0; c < 9; c++) hn[c] = d.hn[c];
-    const double sd = d.search;
-    const float far2 = d.far2, near2 = d.near2;
-    // the atom's bin, as k_bin_count placed it (bin_of of the same coordinates;
-    // recomputing it would cost three FP64 divisions per atom)
-    const int ib0 = B.ghost_bin[gi];
-    int bx = -1, by = -1, bz = -1;
-    if (ib0 >= 0) {
-        bx = ib0 % d.nb[0];
-        by = (ib0 / d.nb[0]) % d.nb[1];
-        bz = ib0 / (d.nb[0] * d.nb[1]);
-    }
-    if (bx < 1 || by < 1 || bz < 1) {
-        if (lane == 0) { atomicExch(&B.flags[1], 3); if (!FILL) B.l2_count[r] = 0; }
-        return;
-    }
-    const long long total = (long long)d.nb[0] * d.nb[1] * d.nb[2];
-    long long base = FILL ? B.l2_off[r] : 0;
+    const long long gi = have ? B.atom_self[r] : 0;
     int count = 0;
-    long long bst = 0;
-    int nbin = 0;
-    if (lane < 27) {
-        const int i = bx - 1 + lane / 9, j = by - 1 + (lane / 3) % 3, k = bz - 1 + lane % 3;
-        const long long ib = i + (long long)j * d.nb[0] + (long long)k * d.nb[0] * d.nb[1];
-        if (ib >= total) {
-            atomicExch(&B.flags[1], 4);
-        } else {
-            const long long b = d.bin_off + ib;
-            bst = bin_start[b];
-            nbin = B.bin_count[b];
+    long long base = -1;   // where entries go: < 0 into shared memory
+    L2Hold& H = hold[wib];
+    auto walk = [&]() {
+        const double fi[3] = {B.ghost_fn[3 * gi], B.ghost_fn[3 * gi + 1], B.ghost_fn[3 * gi + 2]};
+        const float xi[3] = {B.ghost_xf[3 * gi], B.ghost_xf[3 * gi + 1], B.ghost_xf[3 * gi + 2]};
+        double hn[9];
+        for (int c = 0; c < 9; c++) hn[c] = d.hn[c];
+        const double sd = d.search;
+        const float far2 = d.far2;
+        count = 0;
+        // the atom's bin, as k_ghosts placed it
+        const int ib0 = B.ghost_bin[gi];
+        int bx = -1, by = -1, bz = -1;
+        if (ib0 >= 0) {
+            bx = ib0 % d.nb[0];
+            by = (ib0 / d.nb[0]) % d.nb[1];
+            bz = ib0 / (d.nb[0] * d.nb[1]);
         }
-    }
-    int incl = nbin;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-    }
-    const int excl = incl - nbin;
-    const int ncand = __shfl_sync(kFull, incl, 31);
-    int* q = queue[wib];
-    int* qp = qpar[wib];
-    int qn = 0;   // queued candidates (warp-uniform)
-    // exact distances of the first n queued candidates; members counted / written in order
-    auto drain = [&](int n) {
-        bool pred = false;
-        int ajj = -1, par = -1;
-        double dd = 0.0, rv[3] = {0, 0, 0};
-        if (lane < n) {
-            ajj = q[lane];
-            par = qp[lane];
-            dd = dist_frac(hn, fi, &B.ghost_fn[3 * (long long)ajj], rv);
-            pred = dd < sd;
+        if (bx < 1 || by < 1 || bz < 1) {
+            if (lane == 0) atomicExch(&B.flags[1], 3);
+            return;
         }
-        const unsigned bal = __ballot_sync(kFull, pred);
-        if (FILL && pred) {
-            const long long pos = base + count + __popc(bal & lt);
-            if (pos < B.n2_cap) {
-                B.l2_ghost[pos] = ajj;
-                B.l2_dist[pos] = dd;
-                l2_owner[pos] = (int)r;
-                if (B.l2_key) B.l2_key[pos] = (long long)par << 32 | B.ghost_sh[ajj];
-                // x, y, z: FP32 displacement for the enumeration's prefilter;
-                // w: the neighbour's parent atom (int bits; saves the
-                // enumeration a dependent load per candidate) with the exact
-                // tests dd < c3 and dd < c4 in bits 30 and 31, so the
-                // enumeration compares no FP64 distances
-                const unsigned w = (unsigned)par | (dd < d.c3 ? kL2In3 : 0u) | (dd < d.c4 ? kL2In4 : 0u);
-                float4 v = make_float4((float)rv[0], (float)rv[1], (float)rv[2], __uint_as_float(w));
-                reinterpret_cast<float4*>(B.l2_vec)[pos] = v;
-            }
-        }
-        count += __popc(bal);
-        // move the rest of the queue to its front
-        __syncwarp();
-        const int rest = qn - n;
-        int mv = -1, mp = -1;
-        if (lane < rest) { mv = q[n + lane]; mp = qp[n + lane]; }
-        __syncwarp();
-        if (lane < rest) { q[lane] = mv; qp[lane] = mp; }
-        __syncwarp();
-        qn = rest;
-    };
-    for (int t0 = 0; t0 < ncand; t0 += 32) {
-        const int t = t0 + lane;
-        // bin of candidate t: the last bin whose first candidate is <= t
-        int lo = 0;
-        for (int step = 16; step >= 1; step >>= 1) {
-            const int cand = lo + step;
-            const int ex = __shfl_sync(kFull, excl, cand & 31);
-            if (cand < 27 && ex <= t) lo = cand;
-        }
-        const long long st = __shfl_sync(kFull, bst, lo);
-        const int first = __shfl_sync(kFull, excl, lo);
-        bool exact = false, sure = false;
-        int ajj = -1, par = -1;
-        if (t < ncand) {
-            const long long it = st + (t - first);
-            ajj = B.bin_items[it];
-            float xj[3];
-            if (B.bin_xp) {   // the candidate's coordinates and parent stored in bin order
-                const float4 p = reinterpret_cast<const float4*>(B.bin_xp)[it];
-                xj[0] = p.x; xj[1] = p.y; xj[2] = p.z;
-                par = __float_as_int(p.w);
+        const long long total = (long long)d.nb[0] * d.nb[1] * d.nb[2];
+        long long bst = 0;
+        int nbin = 0;
+        if (lane < 27) {
+            const int i = bx - 1 + lane / 9, j = by - 1 + (lane / 3) % 3, k = bz - 1 + lane % 3;
+            const long long ib = i + (long long)j * d.nb[0] + (long long)k * d.nb[0] * d.nb[1];
+            if (ib >= total) {
+                atomicExch(&B.flags[1], 4);
             } else {
-                par = B.ghost_parent[ajj];
-                xj[0] = B.ghost_xf[3 * (long long)ajj];
-                xj[1] = B.ghost_xf[3 * (long long)ajj + 1];
-                xj[2] = B.ghost_xf[3 * (long long)ajj + 2];
+                const long long b = d.bin_off + ib;
+                bst = B.bin_start[b];
+                nbin = B.bin_count[b];
             }
-            if (ajj != gi && r <= par) {
-                const float ex = xj[0] - xi[0], ey = xj[1] - xi[1], ez = xj[2] - xi[2];
-                const float e2 = ex * ex + ey * ey + ez * ez;
-                if (e2 < far2) {   // else certainly >= sd
-                    if (!FILL && e2 < near2) sure = true;   // certainly < sd
-                    else exact = true;
+        }
+        int incl = nbin;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int excl = incl - nbin;
+        const int ncand = __shfl_sync(kFull, incl, 31);
+        int* q = queue[wib];
+        int* qp = qpar[wib];
+        int qn = 0;   // queued candidates (warp-uniform)
+        // exact distances of the first n queued candidates; members kept in order
+        auto drain = [&](int n) {
+            bool pred = false;
+            int ajj = -1, par = -1;
+            double dd = 0.0, rv[3] = {0, 0, 0};
+            if (lane < n) {
+                ajj = q[lane];
+                par = qp[lane];
+                dd = dist_frac(hn, fi, &B.ghost_fn[3 * (long long)ajj], rv);
+                pred = dd < sd;
+            }
+            const unsigned bal = __ballot_sync(kFull, pred);
+            if (pred) {
+                const int k = count + __popc(bal & lt);
+                const unsigned w = (unsigned)par | (dd < d.c3 ? kL2In3 : 0u) | (dd < d.c4 ? kL2In4 : 0u);
+                if (base >= 0) {
+                    put_l2(B, l2_owner, base + k, (int)r, ajj, dd, (float)rv[0], (float)rv[1], (float)rv[2], w);
+                } else if (k < kL2Hold) {
+                    H.dist[k] = dd;
+                    H.x[0][k] = (float)rv[0];
+                    H.x[1][k] = (float)rv[1];
+                    H.x[2][k] = (float)rv[2];
+                    H.ghost[k] = ajj;
+                    H.w[k] = w;
                 }
             }
+            count += __popc(bal);
+            // move the rest of the queue to its front
+            __syncwarp();
+            const int rest = qn - n;
+            int mv = -1, mp = -1;
+            if (lane < rest) { mv = q[n + lane]; mp = qp[n + lane]; }
+            __syncwarp();
+            if (lane < rest) { q[lane] = mv; qp[lane] = mp; }
+            __syncwarp();
+            qn = rest;
+        };
+        for (int t0 = 0; t0 < ncand; t0 += 32) {
+            const int t = t0 + lane;
+            // bin of candidate t: the last bin whose first candidate is <= t
+            int lo = 0;
+            for (int step = 16; step >= 1; step >>= 1) {
+                const int cand = lo + step;
+                const int ex = __shfl_sync(kFull, excl, cand & 31);
+                if (cand < 27 && ex <= t) lo = cand;
+            }
+            const long long st = __shfl_sync(kFull, bst, lo);
+            const int first = __shfl_sync(kFull, excl, lo);
+            bool near = false;
+            int ajj = -1, par = -1;
+            if (t < ncand) {
+                const long long it = st + (t - first);
+                ajj = B.bin_items[it];
+                float xj[3];
+                if (B.bin_xp) {   // the candidate's coordinates and parent stored in bin order
+                    const float4 p = reinterpret_cast<const float4*>(B.bin_xp)[it];
+                    xj[0] = p.x; xj[1] = p.y; xj[2] = p.z;
+                    par = __float_as_int(p.w);
+                } else {
+                    par = B.ghost_parent[ajj];
+                    xj[0] = B.ghost_xf[3 * (long long)ajj];
+                    xj[1] = B.ghost_xf[3 * (long long)ajj + 1];
+                    xj[2] = B.ghost_xf[3 * (long long)ajj + 2];
+                }
+                if (ajj != gi && r <= par) {
+                    const float ex = xj[0] - xi[0], ey = xj[1] - xi[1], ez = xj[2] - xi[2];
+                    near = ex * ex + ey * ey + ez * ez < far2;   // else certainly >= sd
+                }
+            }
+            const unsigned m = __ballot_sync(kFull, near);
+            if (near) {
+                const int pos = qn + __popc(m & lt);
+                q[pos] = ajj;
+                qp[pos] = par;
+            }
+            qn += __popc(m);
+            __syncwarp();
+            if (qn >= 32) drain(32);
         }
-        if (!FILL) count += __popc(__ballot_sync(kFull, sure));
-        const unsigned m = __ballot_sync(kFull, exact);
-        if (exact) {
-            const int pos = qn + __popc(m & lt);
-            q[pos] = ajj;
-            qp[pos] = par;
-        }
-        qn += __popc(m);
-        __syncwarp();
-        if (qn >= 32) drain(32);
+        if (qn > 0) drain(qn);
+    };
+    if (have && !d.err) walk();
+    if (lane == 0) s_cnt[wib] = count;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int k = 0; k < NWARP; k++) sum += s_cnt[k];
+        s_base = sum > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[0], (unsigned long long)sum) : 0;
     }
-    if (qn > 0) drain(qn);
-    if (!FILL && lane == 0) B.l2_count[r] = count;
+    __syncthreads();
+    if (!have) return;
+    long long at = s_base;
+    for (int k = 0; k < wib; k++) at += s_cnt[k];
+    if (lane == 0) {
+        B.l2_off[r] = at;
+        B.l2_count[r] = count;
+    }
+    if (count > kL2Hold) {
+        base = at;
+        walk();
+        return;
+    }
+    for (int k = lane; k < count; k += 32)
+        put_l2(B, l2_owner, at + k, (int)r, H.ghost[k], H.dist[k], H.x[0][k], H.x[1][k], H.x[2][k], H.w[k]);
 }
 
 // Exact test "distance >= c" for a ghost pair of one atom's list, deciding
@@ -606,7 +686,8 @@ __device__ void enum_entry(const BatchView& B, const int* l2_owner, long long e)
         double hn[9];
         for (int c = 0; c < 9; c++) hn[c] = d.hn[c];
         const int gi = B.atom_self[r];
-        const long long b0 = min(B.l2_off[r], B.n2_cap), b1 = min(B.l2_off[r + 1], B.n2_cap);
+        long long b0, b1;
+        list_range(B, r, b0, b1);
         const float4* vec = reinterpret_cast<const float4*>(B.l2_vec);
         const int jj = B.l2_ghost[e];
         const double dij = B.l2_dist[e];
@@ -676,7 +757,7 @@ __device__ void enum_entry(const BatchView& B, const int* l2_owner, long long e)
 
 template <bool FILL>
 __global__ void k_enum(BatchView B, const int* l2_owner) {
-    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
+    const long long n2 = list_total(B);
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < B.n2_cap;
          e += (long long)gridDim.x * blockDim.x) {
         if (e >= n2) {
@@ -694,9 +775,9 @@ __global__ void k_enum(BatchView B, const int* l2_owner) {
 // within rounding of the radius itself can be missing: -1.
 __device__ __forceinline__ int find_entry(const BatchView& B, long long key_j, long long key_k) {
     const long long want = (key_k & ~0xffffffffLL) | (unsigned)((int)key_k - (int)key_j + kShiftBias);
-    const int pj = (int)(key_j >> 32);
-    const long long b1 = min(B.l2_off[pj + 1], B.n2_cap);
-    for (long long e = min(B.l2_off[pj], B.n2_cap); e < b1; e += 4) {
+    long long b0, b1;
+    list_range(B, key_j >> 32, b0, b1);
+    for (long long e = b0; e < b1; e += 4) {
         long long q[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) q[u] = e + u < b1 ? B.l2_key[e + u] : -1;
@@ -748,7 +829,8 @@ __device__ __forceinline__ void put_c4e(const BatchView& B, long long q, long lo
 // 4-body terms and rc4 > rc3 keep the sequential carry-over (k_enum).  Used
 // by k_enuma for atoms whose list is longer than its bit matrices hold.
 template <bool FILL>
-__device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDesc& d, int lane, unsigned lt) {
+__device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDesc& d, int lane, unsigned lt,
+                            long long at3 = 0, long long at4 = 0) {
     const float4* vec = reinterpret_cast<const float4*>(B.l2_vec);
     const double c3 = d.c3, c4 = d.c4;
     const float4 vj = vec[e];
@@ -756,12 +838,13 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
     const bool want3 = d.has3 && (wj & kL2In3), want4 = d.has4 && (wj & kL2In4);
     long long n3 = 0, n4 = 0;
     long long o3 = 0, o4 = 0;
-    if (FILL) { o3 = B.e_off3[e]; o4 = B.e_off4[e]; }
+    if (FILL) { o3 = at3 + B.e_off3[e]; o4 = at4 + B.e_off4[e]; }
     if (want3 || want4) {
         const double* hn = d.hn;   // read in place: the exact distances are rare
         const float c3lo = d.c3lo, c3hi = d.c3hi, c4lo = d.c4lo, c4hi = d.c4hi;
         const int gi = B.atom_self[r];
-        const long long b0 = min(B.l2_off[r], B.n2_cap), b1 = min(B.l2_off[r + 1], B.n2_cap);
+        long long b0, b1;
+        list_range(B, r, b0, b1);
         const int jj = B.l2_ghost[e];
         const double* fj = &B.ghost_fn[3 * (long long)jj];
         const int pj = (int)(wj & kL2Parent);
@@ -850,13 +933,14 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
 // The warps test every ordered pair of entries once -- the FP32 distance with
 // the same thresholds and, inside the margin, the same exact FP64 distance as
 // the per-entry form -- and keep the rows T[j], Q[j] as bit masks in shared
-// memory.  The count pass then takes n3(j) = popc T[j] and n4(j) = sum over
-// k in Q[j] of popc(Q[j] & Q[k]); the fill pass emits the clusters from the
-// masks in the same order (k ascending, then l ascending), each entry at the
-// offset of the atom's first entry plus the counts of the entries before it
-// (which the masks give).  The per-entry form walks k and, for every 4-body
-// k, all l again, once per pass; here both passes cost one test per ordered
-// pair.  G = 1 for batches with many atoms; small ones spread an atom over
+// memory.  The masks give the counts, n3(j) = popc T[j] and n4(j) = sum over k in
+// Q[j] of popc(Q[j] & Q[k]), room for the atom's clusters is reserved with one
+// atomic per body order, and the clusters are emitted from the masks in the
+// same order (k ascending, then l ascending), each entry's after the counts of
+// the entries before it.  One pass over the atoms: two passes with a scan over
+// the entries between them tested every pair twice (2000 configurations: 625 +
+// 860 us and about 180 us of scans; this takes 875 us, and 930 with the bucket
+// keys).  G = 1 for batches with many atoms; small ones spread an atom over
 // up to a whole block so that the launch still fills the GPU.
 constexpr int kEnumRows = 96;
 constexpr int kEnumWords = kEnumRows / 32;   // odd: column reads of the masks hit distinct banks
@@ -894,51 +978,121 @@ __device__ __forceinline__ void mask_counts(const unsigned* rt, const unsigned* 
     }
 }
 
-template <bool FILL, int G>
+// Bucket key of a cluster from its atoms' types, counted in the block's
+// histogram (kBkSmem buckets) or, with more buckets, in B.bk_count.  Called by
+// whole warps; on: the lane has a cluster.
+__device__ __forceinline__ void count_key(const BatchView& B, int* hist, int at, int key) {
+    const unsigned peers = __match_any_sync(kFull, key);
+    if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) {
+        if (hist) atomicAdd(&hist[at + key], __popc(peers));
+        else atomicAdd(&B.bk_count[at + key], __popc(peers));
+    }
+}
+
+template <int G>
 __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
     constexpr int NG = kEnumWarps / G;   // atoms a block works on at a time
     __shared__ float4 s_v[NG][kEnumRows];
     __shared__ int s_g[NG][kEnumRows];
     __shared__ unsigned s_t[NG][kEnumRows * kEnumWords];
     __shared__ unsigned s_q[NG][kEnumRows * kEnumWords];
-    __shared__ int s_o[FILL ? NG : 1][FILL ? 2 * kEnumRows + 2 : 1];   // per-entry offsets, then the totals
+    __shared__ int s_o[NG][2 * kEnumRows + 2];   // per-entry offsets, then the totals
+    __shared__ long long s_at[NG][2];            // where the atom's clusters go
+    __shared__ unsigned char s_ty[NG][kEnumRows];   // the entries' types
+    extern __shared__ int s_hist[];              // bucket counts of this block (when B.keyed and few buckets)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int grp = wib / G, w = wib % G;
-    const unsigned lt = (1u << lane) - 1u;
-    const long long n2 = min(B.l2_off[B.n_atoms_total], B.n2_cap);
-    if (!FILL) {
-        for (long long e = n2 + (long long)blockIdx.x * blockDim.x + threadIdx.x; e < B.n2_cap;
-             e += (long long)gridDim.x * blockDim.x) {
-            B.e_cnt3[e] = 0;
-            B.e_cnt4[e] = 0;
-        }
+    const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
+    int* hist = nbk > 0 && nbk <= kBkSmem ? s_hist : nullptr;
+    if (hist) {
+        for (int k = threadIdx.x; k < nbk; k += blockDim.x) hist[k] = 0;
+        __syncthreads();
     }
+    const unsigned lt = (1u << lane) - 1u;
     const float4* vec = reinterpret_cast<const float4*>(B.l2_vec);
     float4* sv = s_v[grp];
     int* sg = s_g[grp];
     unsigned* rt = s_t[grp];
     unsigned* rq = s_q[grp];
+    int* so = s_o[grp];
+    // room for an atom's t3 triplets and t4 quadruplets (one lane of the group)
+    auto reserve = [&](long long r, long long t3, long long t4) {
+        const long long a3 = t3 > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[1], (unsigned long long)t3) : 0;
+        const long long a4 = t4 > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[2], (unsigned long long)t4) : 0;
+        B.a_off[2 * r] = s_at[grp][0] = a3;
+        B.a_off[2 * r + 1] = s_at[grp][1] = a4;
+        B.a_cnt[2 * r] = (int)t3;
+        B.a_cnt[2 * r + 1] = (int)t4;
+    };
     const long long ngroups = (long long)gridDim.x * NG;
     for (long long r = (long long)blockIdx.x * NG + grp; r < B.n_atoms_total; r += ngroups) {
-        const long long b0 = min(B.l2_off[r], B.n2_cap), b1 = min(B.l2_off[r + 1], B.n2_cap);
+        long long b0, b1;
+        list_range(B, r, b0, b1);
         const int L = (int)(b1 - b0);
-        if (L <= 0) continue;
         const SysDesc& d = B.sys[B.atom_sys[r]];
-        if (!d.has3 && !d.has4) {
-            if (!FILL)
-                for (int a = 32 * w + lane; a < L; a += 32 * G) { B.e_cnt3[b0 + a] = 0; B.e_cnt4[b0 + a] = 0; }
+        if (L <= 0 || (!d.has3 && !d.has4)) {
+            if (w == 0 && lane == 0) {
+                B.a_off[2 * r] = B.a_off[2 * r + 1] = 0;
+                B.a_cnt[2 * r] = B.a_cnt[2 * r + 1] = 0;
+            }
             continue;
         }
+        group_sync<G>(grp);   // the previous atom's masks and offsets are no longer read
         if (L > kEnumRows) {
-            for (long long e = b0 + w; e < b1; e += G) enumw_entry<FILL>(B, e, (int)r, d, lane, lt);
+            // counts per entry, their offsets, then the clusters
+            for (long long e = b0 + w; e < b1; e += G) enumw_entry<false>(B, e, (int)r, d, lane, lt);
+            __threadfence_block();
+            group_sync<G>(grp);
+            if (w == 0) {
+                long long c3 = 0, c4 = 0;
+                for (long long e0 = b0; e0 < b1; e0 += 32) {
+                    const long long e = e0 + lane;
+                    const int n3 = e < b1 ? B.e_cnt3[e] : 0, n4 = e < b1 ? B.e_cnt4[e] : 0;
+                    int i3 = n3, i4 = n4;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y3 = __shfl_up_sync(kFull, i3, o), y4 = __shfl_up_sync(kFull, i4, o);
+                        if (lane >= o) { i3 += y3; i4 += y4; }
+                    }
+                    if (e < b1) { B.e_off3[e] = c3 + i3 - n3; B.e_off4[e] = c4 + i4 - n4; }
+                    c3 += __shfl_sync(kFull, i3, 31);
+                    c4 += __shfl_sync(kFull, i4, 31);
+                }
+                if (lane == 0) reserve(r, c3, c4);
+            }
+            __threadfence_block();
+            group_sync<G>(grp);
+            for (long long e = b0 + w; e < b1; e += G)
+                enumw_entry<true>(B, e, (int)r, d, lane, lt, s_at[grp][0], s_at[grp][1]);
+            if (nbk > 0) {
+                // their keys, from the clusters as written
+                __threadfence_block();
+                group_sync<G>(grp);
+                const DevParamSet& P = B.psets[d.pset];
+                auto type = [&](int g) { return B.atom_type[B.ghost_parent[g]]; };
+                for (int nb = 3; nb <= 4; nb++) {
+                    const long long at = s_at[grp][nb - 3], n = B.a_cnt[2 * r + nb - 3], cap = nb == 3 ? B.n3_cap : B.n4_cap;
+                    const int* cl = nb == 3 ? B.c3 : B.c4;
+                    for (long long t0 = 32 * w; t0 < n; t0 += 32 * G) {
+                        const long long q = at + t0 + lane;
+                        int key = -1;
+                        if (t0 + lane < n && q < cap) {
+                            int u = 0;
+                            for (int k = 0; k < nb; k++) u = u * P.ntypes + type(cl[nb * q + k]);
+                            key = (nb == 3 ? P.key3 : P.key4)[u];
+                            if (key >= 0) key += nb == 3 ? P.bk3 : P.bk4;
+                            (nb == 3 ? B.bk_key3 : B.bk_key4)[q] = key;
+                        }
+                        count_key(B, hist, nb == 3 ? 0 : B.nbk3, key);
+                    }
+                }
+            }
             continue;
         }
-        long long o3 = 0, o4 = 0;
-        if (FILL) { o3 = B.e_off3[b0]; o4 = B.e_off4[b0]; }
-        group_sync<G>(grp);   // the previous atom's masks are no longer read
         for (int a = 32 * w + lane; a < L; a += 32 * G) {
-            sv[a] = vec[b0 + a];
+            const float4 v = vec[b0 + a];
+            sv[a] = v;
             sg[a] = B.l2_ghost[b0 + a];
+            s_ty[grp][a] = (unsigned char)B.atom_type[__float_as_uint(v.w) & kL2Parent];
         }
         group_sync<G>(grp);
         const int nw = (L + 31) >> 5;
@@ -986,18 +1140,8 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
             }
         }
         group_sync<G>(grp);
-        if (!FILL) {
-            for (int a = 32 * w + lane; a < L; a += 32 * G) {
-                int n3, n4;
-                mask_counts(rt, rq, a, nw, n3, n4);
-                B.e_cnt3[b0 + a] = n3;
-                B.e_cnt4[b0 + a] = n4;
-            }
-            continue;
-        }
         // offsets of the entries within the atom (triplets, quadruplets) and
-        // the atom's totals
-        int* so = s_o[FILL ? grp : 0];
+        // room for the atom's totals
         if (w == 0) {
             int c3 = 0, c4 = 0;
             for (int a0 = 0; a0 < L; a0 += 32) {
@@ -1013,7 +1157,11 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
                 c3 += __shfl_sync(kFull, i3, 31);
                 c4 += __shfl_sync(kFull, i4, 31);
             }
-            if (lane == 0) { so[2 * L] = c3; so[2 * L + 1] = c4; }
+            if (lane == 0) {
+                so[2 * L] = c3;
+                so[2 * L + 1] = c4;
+                reserve(r, c3, c4);
+            }
         }
         group_sync<G>(grp);
         // the atom's clusters in the reference's order, one per lane: the t-th
@@ -1021,85 +1169,124 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
         // entry's (t - offset)-th set bit of T; the t-th quadruplet likewise,
         // walking the entry's k in Q and the set bits of Q[j] & Q[k]
         const int gi = B.atom_self[r];
-        const long long base3 = B.e_off3[b0], base4 = B.e_off4[b0];
+        const long long base3 = s_at[grp][0], base4 = s_at[grp][1];
         const int t3 = so[2 * L], t4 = so[2 * L + 1];
-        for (int t = 32 * w + lane; t < t3; t += 32 * G) {
-            int lo = 0, hi = L - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (so[2 * mid] <= t) lo = mid; else hi = mid - 1;
-            }
-            const int a = lo;
-            int rk = t - so[2 * a], bk = 0;
-            for (int c = 0; c < nw; c++) {
-                const unsigned m = rt[a * kEnumWords + c];
-                const int pc = __popc(m);
-                if (rk < pc) { bk = 32 * c + select_bit(m, rk); break; }
-                rk -= pc;
-            }
-            const long long q = base3 + t;
-            if (q < B.n3_cap) {
-                int* out = B.c3 + 3 * q;
-                out[0] = gi; out[1] = sg[a]; out[2] = sg[bk];
-                put_c3e(B, q, b0 + a, b0 + bk);
-            }
-        }
-        for (int t = 32 * w + lane; t < t4; t += 32 * G) {
-            int lo = 0, hi = L - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (so[2 * mid + 1] <= t) lo = mid; else hi = mid - 1;
-            }
-            const int a = lo;
-            int rk = t - so[2 * a + 1], bk = 0, lk = 0;
-            bool found = false;
-            for (int c = 0; c < nw && !found; c++) {
-                unsigned mb = rq[a * kEnumWords + c];
-                while (mb && !found) {
-                    const int bb = 32 * c + __ffs(mb) - 1;
-                    mb &= mb - 1;
-                    for (int c2 = 0; c2 < nw; c2++) {
-                        const unsigned x = rq[a * kEnumWords + c2] & rq[bb * kEnumWords + c2];
-                        const int pc = __popc(x);
-                        if (rk < pc) { bk = bb; lk = 32 * c2 + select_bit(x, rk); found = true; break; }
-                        rk -= pc;
+        const DevParamSet& P = B.psets[d.pset];
+        const int nt = P.ntypes, ti = B.atom_type[r];
+        for (int t0 = 32 * w; t0 < t3; t0 += 32 * G) {
+            const int t = t0 + lane;
+            int key = -1;
+            if (t < t3) {
+                int lo = 0, hi = L - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (so[2 * mid] <= t) lo = mid; else hi = mid - 1;
+                }
+                const int a = lo;
+                int rk = t - so[2 * a], bk = 0;
+                for (int c = 0; c < nw; c++) {
+                    const unsigned m = rt[a * kEnumWords + c];
+                    const int pc = __popc(m);
+                    if (rk < pc) { bk = 32 * c + select_bit(m, rk); break; }
+                    rk -= pc;
+                }
+                const long long q = base3 + t;
+                if (q < B.n3_cap) {
+                    int* out = B.c3 + 3 * q;
+                    out[0] = gi; out[1] = sg[a]; out[2] = sg[bk];
+                    put_c3e(B, q, b0 + a, b0 + bk);
+                    if (nbk > 0) {
+                        key = P.key3[(ti * nt + s_ty[grp][a]) * nt + s_ty[grp][bk]];
+                        if (key >= 0) key += P.bk3;
+                        B.bk_key3[q] = key;
                     }
                 }
             }
-            const long long q = base4 + t;
-            if (q < B.n4_cap) {
-                int* out = B.c4 + 4 * q;
-                out[0] = gi; out[1] = sg[a]; out[2] = sg[bk]; out[3] = sg[lk];
-                put_c4e(B, q, b0 + a, b0 + bk, b0 + lk);
-            }
+            if (nbk > 0) count_key(B, hist, 0, key);
         }
+        for (int t0 = 32 * w; t0 < t4; t0 += 32 * G) {
+            const int t = t0 + lane;
+            int key = -1;
+            if (t < t4) {
+                int lo = 0, hi = L - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (so[2 * mid + 1] <= t) lo = mid; else hi = mid - 1;
+                }
+                const int a = lo;
+                int rk = t - so[2 * a + 1], bk = 0, lk = 0;
+                bool found = false;
+                for (int c = 0; c < nw && !found; c++) {
+                    unsigned mb = rq[a * kEnumWords + c];
+                    while (mb && !found) {
+                        const int bb = 32 * c + __ffs(mb) - 1;
+                        mb &= mb - 1;
+                        for (int c2 = 0; c2 < nw; c2++) {
+                            const unsigned x = rq[a * kEnumWords + c2] & rq[bb * kEnumWords + c2];
+                            const int pc = __popc(x);
+                            if (rk < pc) { bk = bb; lk = 32 * c2 + select_bit(x, rk); found = true; break; }
+                            rk -= pc;
+                        }
+                    }
+                }
+                const long long q = base4 + t;
+                if (q < B.n4_cap) {
+                    int* out = B.c4 + 4 * q;
+                    out[0] = gi; out[1] = sg[a]; out[2] = sg[bk]; out[3] = sg[lk];
+                    put_c4e(B, q, b0 + a, b0 + bk, b0 + lk);
+                    if (nbk > 0) {
+                        key = P.key4[((ti * nt + s_ty[grp][a]) * nt + s_ty[grp][bk]) * nt + s_ty[grp][lk]];
+                        if (key >= 0) key += P.bk4;
+                        B.bk_key4[q] = key;
+                    }
+                }
+            }
+            if (nbk > 0) count_key(B, hist, B.nbk3, key);
+        }
+    }
+    if (hist) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < nbk; k += blockDim.x)
+            if (hist[k]) atomicAdd(&B.bk_count[k], hist[k]);
     }
 }
 
-template <bool FILL, int G>
+template <int G>
 void launch_enuma(const BatchView& B, cudaStream_t st) {
     constexpr int NG = kEnumWarps / G;
     const long long want = (long long)sm_count() * 4;   // 4 blocks of 8 warps per SM
     const long long need = (B.n_atoms_total + NG - 1) / NG;
     const unsigned grid = (unsigned)(want < need ? want : need);
-    count_launch(), k_enuma<FILL, G><<<grid, 32 * kEnumWarps, 0, st>>>(B);
+    const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
+    const size_t smem = nbk <= kBkSmem ? sizeof(int) * (size_t)nbk : 0;
+    count_launch(), k_enuma<G><<<grid, 32 * kEnumWarps, smem, st>>>(B);
 }
 
-// --- capacity checks and accumulator reset ---------------------------------
-__global__ void k_check(BatchView B) {
-    if (B.l2_off[B.n_atoms_total] > B.n2_cap) atomicOr(&B.flags[0], 2);
-    if (B.e_off3[B.n2_cap] > B.n3_cap) atomicOr(&B.flags[0], 4);
-    if (B.e_off4[B.n2_cap] > B.n4_cap) atomicOr(&B.flags[0], 8);
-}
-
+// --- reset of accumulators, counters and bins -------------------------------
 __global__ void k_reset(BatchView B) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 6LL * B.n_sys) B.minmax[i] = (i % 6) < 3 ? ~0ull : 0ull;
-    if (i < 8LL * B.n_sys) B.ev[i] = 0.0;
-    if (i < 3 * B.n_in_total) B.force[i] = 0.0;
-    if (i < 8) B.flags[i] = 0;
-    if (i < 2) B.queue[i] = 0ull;
-    if (i < B.n_sys) B.sys[i].err = 0;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = t; i < B.n_bins_total; i += stride) {
+        B.bin_count[i] = 0;
+        B.bin_fill[i] = 0;
+    }
+    for (long long i = t; i < 3 * B.n_in_total; i += stride) B.force[i] = 0.0;
+    for (long long i = t; i < 8LL * B.n_sys; i += stride) {
+        B.ev[i] = 0.0;
+        if (i < 6LL * B.n_sys) B.minmax[i] = (i % 6) < 3 ? ~0ull : 0ull;
+        if (i < B.n_sys) {
+            B.sys[i].err = 0;
+            B.sys[i].done = 0;
+        }
+    }
+    if (B.bk_count)
+        for (long long i = t; i < B.nbk3 + B.nbk4; i += stride) {
+            B.bk_count[i] = 0;
+            B.bk_fill[i] = 0;
+        }
+    if (t < 8) B.flags[t] = 0;
+    if (t < 2) B.queue[t] = 0ull;
+    if (t < 4 && B.totals) B.totals[t] = 0;
 }
 
 // --- exclusive scan (three phases, recursive on block sums) -----------------
@@ -1273,11 +1460,8 @@ void launch_atoms(const BatchView& B, cudaStream_t st) {
 void launch_ghosts(const BatchView& B, cudaStream_t st) {
     if (B.n_ghost_total) count_launch(), k_ghosts<<<grid_for(B.n_ghost_total, 64), 64, 0, st>>>(B);
 }
-void launch_bin_setup(const BatchView& B, cudaStream_t st) {
-    count_launch(), k_bin_setup<<<grid_for(B.n_sys, 128), 128, 0, st>>>(B);
-}
-void launch_bin_count(const BatchView& B, cudaStream_t st) {
-    if (B.n_ghost_total) count_launch(), k_bin_count<<<grid_for(B.n_ghost_total, 256), 256, 0, st>>>(B);
+void launch_bin_alloc(const BatchView& B, cudaStream_t st) {
+    if (B.n_bins_total) count_launch(), k_bin_alloc<<<grid_for(B.n_bins_total, 1024), 1024, 0, st>>>(B);
 }
 void launch_bin_scatter(const BatchView& B, cudaStream_t st) {
     if (B.n_ghost_total) count_launch(), k_bin_scatter<<<grid_for(B.n_ghost_total, 256), 256, 0, st>>>(B, B.bin_start);
@@ -1291,20 +1475,19 @@ void launch_bin_sort(const BatchView& B, cudaStream_t st) {
     const long long warps = (B.n_bins_total + per - 1) / per;
     count_launch(), k_bin_rank<<<grid_for(warps * 32, 256), 256, 0, st>>>(B, B.bin_start, per);
 }
-void launch_l2(const BatchView& B, int* l2_owner, bool fill, cudaStream_t st) {
-    if (!B.n_atoms_total) return;
-    const unsigned grid = grid_for(B.n_atoms_total * 32, kL2Block);
-    if (fill) count_launch(), k_l2<true><<<grid, kL2Block, 0, st>>>(B, B.bin_start, l2_owner);
-    else count_launch(), k_l2<false><<<grid, kL2Block, 0, st>>>(B, B.bin_start, l2_owner);
+void launch_l2(const BatchView& B, int* l2_owner, cudaStream_t st) {
+    if (B.n_atoms_total)
+        count_launch(), k_l2<<<grid_for(B.n_atoms_total * 32, kL2Block), kL2Block, 0, st>>>(B, l2_owner);
 }
-void launch_enum(const BatchView& B, const int* l2_owner, bool fill, cudaStream_t st) {
+void launch_enum(const BatchView& B, const int* l2_owner, void* scan_tmp, cudaStream_t st) {
     if (!B.n2_cap) return;
     if (B.enum_serial) {
         long long want = (long long)sm_count() * 16;
         long long need = (B.n2_cap + 127) / 128;
         const unsigned grid = (unsigned)(want < need ? want : need);
-        if (fill) count_launch(), k_enum<true><<<grid, 128, 0, st>>>(B, l2_owner);
-        else count_launch(), k_enum<false><<<grid, 128, 0, st>>>(B, l2_owner);
+        count_launch(), k_enum<false><<<grid, 128, 0, st>>>(B, l2_owner);
+        exclusive_scan2(B.e_cnt3, B.e_off3, B.e_cnt4, B.e_off4, B.n2_cap, scan_tmp, st);
+        count_launch(), k_enum<true><<<grid, 128, 0, st>>>(B, l2_owner);
         return;
     }
     // warps per atom: the fewest that still give about two warps per
@@ -1313,18 +1496,16 @@ void launch_enum(const BatchView& B, const int* l2_owner, bool fill, cudaStream_
     const long long n = B.n_atoms_total;
     const int G = n >= target ? 1 : 2 * n >= target ? 2 : 4 * n >= target ? 4 : 8;
     switch (G) {
-    case 1: fill ? launch_enuma<true, 1>(B, st) : launch_enuma<false, 1>(B, st); break;
-    case 2: fill ? launch_enuma<true, 2>(B, st) : launch_enuma<false, 2>(B, st); break;
-    case 4: fill ? launch_enuma<true, 4>(B, st) : launch_enuma<false, 4>(B, st); break;
-    default: fill ? launch_enuma<true, 8>(B, st) : launch_enuma<false, 8>(B, st); break;
+    case 1: launch_enuma<1>(B, st); break;
+    case 2: launch_enuma<2>(B, st); break;
+    case 4: launch_enuma<4>(B, st); break;
+    default: launch_enuma<8>(B, st); break;
     }
 }
-void launch_check(const BatchView& B, cudaStream_t st) { count_launch(), k_check<<<1, 1, 0, st>>>(B); }
 void launch_reset(const BatchView& B, cudaStream_t st) {
-    long long n = 8LL * B.n_sys;
-    if (3 * B.n_in_total > n) n = 3 * B.n_in_total;
-    if (n < 8) n = 8;
-    count_launch(), k_reset<<<grid_for(n, 256), 256, 0, st>>>(B);
+    long long n = std::max(std::max(8LL * B.n_sys, 3 * B.n_in_total), std::max(B.n_bins_total, 8LL));
+    n = std::min((n + 255) / 256, 16LL * sm_count());
+    count_launch(), k_reset<<<(unsigned)n, 256, 0, st>>>(B);
 }
 
 }  // namespace ck

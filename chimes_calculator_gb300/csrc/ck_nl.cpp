@@ -147,6 +147,7 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
     B.e_cnt3 = d_e_cnt3_.p; B.e_cnt4 = d_e_cnt4_.p; B.e_off3 = d_e_off3_.p; B.e_off4 = d_e_off4_.p;
     B.force = d_force_.p; B.ev = d_ev_.p; B.flags = d_flags_.p; B.queue = d_queue_.p;
     B.enum_serial = 0;
+    B.n3_ptr = B.e_off3 + nent; B.n4_ptr = B.e_off4 + nent;
     NeighView& N = N_;
     N.inum = inum;
     N.nent = nent;
@@ -245,12 +246,7 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
     // a tabulated 3-body term is looked up per listed triplet (no buckets)
     const bool tab3 = P.tab3 && L.stride3 > 0;
     const bool bk3 = L.stride3 > 0 && L.fact3 && n3_ > 0 && !tab3;
-    if (bk3 || (L.stride4 > 0 && L.fact4 && n4_ > 0)) {
-        NL_TRY(cudaMemsetAsync(B.bk_count, 0, sizeof(int) * (nbk3 + nbk4), s));
-        NL_TRY(cudaMemsetAsync(B.bk_fill, 0, sizeof(int) * (nbk3 + nbk4), s));
-        if (bk3) launch_bucket(B, 3, s);
-        if (L.stride4 > 0 && L.fact4 && n4_ > 0) launch_bucket(B, 4, s);
-    }
+    launch_bucket(B, bk3, L.stride4 > 0 && L.fact4 && n4_ > 0, s);
     launch_nl_pairs(B, N, L.precision, s);
     if (L.stride3 > 0 && n3_ > 0) {
         if (tab3) {

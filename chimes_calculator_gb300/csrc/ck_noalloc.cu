@@ -50,7 +50,7 @@ constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // byte layout of the scratch array
 struct Layout {
     size_t sys, minmax, ev, flags, queue, in_pos, in_type, atom_sys, atom_type, atom_orig, atom_self;
-    size_t ghost_id, ghost_parent, ghost_bin, ghost_fs, ghost_xn, ghost_fn, ghost_xf, bin_items;
+    size_t ghost_id, ghost_parent, ghost_bin, ghost_fs, ghost_fn, ghost_xf, bin_items;
     size_t bin_count, bin_fill, bin_start, l2_count, l2_off;
     size_t l2_ghost, l2_owner, l2_dist, l2_vec, e_cnt3, e_cnt4, e_off3, e_off4, c3, c4, force, scan, total;
 };
@@ -65,7 +65,7 @@ constexpr Layout make_layout() {
     L.minmax = take(6 * sizeof(unsigned long long));
     L.ev = take(8 * sizeof(double));
     L.flags = take(8 * sizeof(int));
-    L.queue = take(2 * sizeof(unsigned long long));
+    L.queue = take(6 * sizeof(unsigned long long));   // queue heads, then the list totals
     L.in_pos = take(3 * kNaAtoms * sizeof(double));
     L.in_type = take(kNaAtoms * sizeof(int));
     L.atom_sys = take(kNaAtoms * sizeof(int));
@@ -76,15 +76,14 @@ constexpr Layout make_layout() {
     L.ghost_parent = take(kNaGhosts * sizeof(int));
     L.ghost_bin = take(kNaGhosts * sizeof(int));
     L.ghost_fs = take(3 * kNaGhosts * sizeof(double));
-    L.ghost_xn = take(3 * kNaGhosts * sizeof(double));
     L.ghost_fn = take(3 * kNaGhosts * sizeof(double));
     L.ghost_xf = take(3 * kNaGhosts * sizeof(float));
     L.bin_items = take(kNaGhosts * sizeof(int));
     L.bin_count = take(kNaBins * sizeof(int));
     L.bin_fill = take(kNaBins * sizeof(int));
-    L.bin_start = take((kNaBins + 1) * sizeof(long long));
+    L.bin_start = take(kNaBins * sizeof(long long));
     L.l2_count = take(kNaAtoms * sizeof(int));
-    L.l2_off = take((kNaAtoms + 1) * sizeof(long long));
+    L.l2_off = take(kNaAtoms * sizeof(long long));
     L.l2_ghost = take(kNaPairs * sizeof(int));
     L.l2_owner = take(kNaPairs * sizeof(int));
     L.l2_dist = take(kNaPairs * sizeof(double));
@@ -173,7 +172,7 @@ __global__ void k_noalloc_finish(const double* ev, const double* force, int n, d
 Status calculate_noalloc(Engine& eng, int slot, int natom, const double* d_pos, const int* d_types,
                          const double* cell, bool small, double* d_energy, double* d_force, double* d_stress,
                          cudaStream_t st, std::string& err) {
-    if (scan_tmp_bytes(kNaGhosts) > kScanBytes) {   // the largest scan is no longer than kNaGhosts
+    if (scan_tmp_bytes(kNaPairs) > kScanBytes) {
         err = "ck_calculate_noalloc: scan workspace too small";
         return kErrState;
     }
@@ -240,7 +239,6 @@ Status calculate_noalloc(Engine& eng, int slot, int natom, const double* d_pos, 
     B.ghost_xf = reinterpret_cast<float*>(base + kLayout.ghost_xf);
     B.ghost_parent = reinterpret_cast<int*>(base + kLayout.ghost_parent);
     B.ghost_fs = reinterpret_cast<double*>(base + kLayout.ghost_fs);
-    B.ghost_xn = reinterpret_cast<double*>(base + kLayout.ghost_xn);
     B.ghost_fn = reinterpret_cast<double*>(base + kLayout.ghost_fn);
     B.minmax = reinterpret_cast<unsigned long long*>(base + kLayout.minmax);
     B.ghost_bin = reinterpret_cast<int*>(base + kLayout.ghost_bin);
@@ -266,6 +264,9 @@ Status calculate_noalloc(Engine& eng, int slot, int natom, const double* d_pos, 
     B.ev = reinterpret_cast<double*>(base + kLayout.ev);
     B.flags = reinterpret_cast<int*>(base + kLayout.flags);
     B.queue = reinterpret_cast<unsigned long long*>(base + kLayout.queue);
+    B.totals = reinterpret_cast<long long*>(B.queue + 2);
+    B.n3_ptr = B.e_off3 + B.n2_cap;
+    B.n4_ptr = B.e_off4 + B.n2_cap;
     int* l2_owner = reinterpret_cast<int*>(base + kLayout.l2_owner);
     void* scan = base + kLayout.scan;
 
@@ -283,27 +284,17 @@ Status calculate_noalloc(Engine& eng, int slot, int natom, const double* d_pos, 
     NA_TRY(cudaMemcpyAsync((void*)B.in_pos, d_pos, sizeof(double) * 3 * natom, cudaMemcpyDeviceToDevice, st));
     NA_TRY(cudaMemcpyAsync((void*)B.in_type, d_types, sizeof(int) * natom, cudaMemcpyDeviceToDevice, st));
     // what must start at zero (the array keeps the previous call's contents)
-    NA_TRY(cudaMemsetAsync(B.bin_count, 0, sizeof(int) * B.n_bins_total, st));
-    NA_TRY(cudaMemsetAsync(B.bin_fill, 0, sizeof(int) * B.n_bins_total, st));
-    launch_reset(B, st);   // bounding box, energy/virial, forces, flags, system error word
+    launch_reset(B, st);   // bounding box, bins, totals, energy/virial, forces, flags, system words
     count_launch(), k_noalloc_check_inputs<<<(natom + 255) / 256, 256, 0, st>>>(
         reinterpret_cast<double*>(base + kLayout.in_pos), reinterpret_cast<int*>(base + kLayout.in_type), natom,
         P.ntypes, B.flags);
     launch_atoms(B, st);
     launch_ghosts(B, st);
-    launch_bin_setup(B, st);
-    launch_bin_count(B, st);
-    exclusive_scan(B.bin_count, B.bin_start, B.n_bins_total, scan, st);
+    launch_bin_alloc(B, st);
     launch_bin_scatter(B, st);
     launch_bin_sort(B, st);
-    launch_l2(B, l2_owner, false, st);
-    exclusive_scan(B.l2_count, B.l2_off, B.n_atoms_total, scan, st);
-    launch_l2(B, l2_owner, true, st);
-    launch_enum(B, l2_owner, false, st);
-    exclusive_scan(B.e_cnt3, B.e_off3, B.n2_cap, scan, st);
-    exclusive_scan(B.e_cnt4, B.e_off4, B.n2_cap, scan, st);
-    launch_enum(B, l2_owner, true, st);
-    launch_check(B, st);
+    launch_l2(B, l2_owner, st);
+    launch_enum(B, l2_owner, scan, st);
     ForceLaunch L = eng.tuning;
     L.precision = eng.precision;
     L.stride3 = P.o3 > 0 ? P.o3 + 1 : 0;
@@ -318,9 +309,9 @@ Status calculate_noalloc(Engine& eng, int slot, int natom, const double* d_pos, 
     int flags[8];
     long long counts[3];
     NA_TRY(cudaMemcpyAsync(flags, B.flags, sizeof(flags), cudaMemcpyDeviceToHost, st));
-    NA_TRY(cudaMemcpyAsync(&counts[0], B.l2_off + B.n_atoms_total, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    NA_TRY(cudaMemcpyAsync(&counts[1], B.e_off3 + B.n2_cap, sizeof(long long), cudaMemcpyDeviceToHost, st));
-    NA_TRY(cudaMemcpyAsync(&counts[2], B.e_off4 + B.n2_cap, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    NA_TRY(cudaMemcpyAsync(&counts[0], B.totals, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    NA_TRY(cudaMemcpyAsync(&counts[1], B.n3_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
+    NA_TRY(cudaMemcpyAsync(&counts[2], B.n4_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
     NA_TRY(cudaStreamSynchronize(st));
 #undef NA_TRY
     eng.last.n2 = counts[0];

@@ -1190,6 +1190,9 @@ ParamImage pack_params(const HostParams& P) {
             ffo = B.add(fef.data(), fef.size());
         }
         const int Rf = (fact && !fed.empty()) ? R_pow : 0;
+        std::vector<int> keys(ntup);
+        for (int u = 0; u < ntup; u++) keys[u] = tr[u].valid && Rf > 0 ? u : -1;
+        (nb == 3 ? H.key3 : H.key4) = as_off<const int>(B.add(keys.data(), keys.size()));
         if (nb == 3 && tc && Rf > 0 && !tcimg.empty()) {
             H.tc3_k = tc3_kpad(R_pow);
             H.tc3_n = tc3_npad(R_pow);

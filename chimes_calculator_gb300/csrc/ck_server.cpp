@@ -308,8 +308,8 @@ private:
         // pair lists ~70 B per pair plus the factored kernels' per-entry table cache
         // (~350 B per pair in FP64 for the 3- and 4-body orders), cluster lists
         // with their entry indices
-        return (double)d.n_atoms * d.gstride * 110.0 + (double)d.bin_cap * 20.0 + n2 * 420.0 + n3 * 28.0 +
-               n4 * 44.0 + d.n_atoms * 120.0;
+        return (double)d.n_atoms * d.gstride * 110.0 + (double)d.bin_cap * 20.0 + n2 * 420.0 + n3 * 32.0 +
+               n4 * 48.0 + d.n_atoms * 120.0;
     }
 
     void worker(int w) {
