@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
                 } else {
                     CT fc, fcd;
                     const double r = geo[(4 * p + 3) * G + grp];
-                    pair_setup<CT>(*P, tuple_pair(*R, p), r, exp(-r * R->inv_lam[p]), Tt + p * rs * G + grp,
+                    pair_setup<CT>(*P, tuple_pair(*R, p), r, exp_neg(r * R->inv_lam[p]), Tt + p * rs * G + grp,
                                    Dt + p * rs * G + grp, G, Rp, fc, fcd, B.flags);
                     fcs[p * G + grp] = double(fc);
                     fcds[p * G + grp] = double(fcd);

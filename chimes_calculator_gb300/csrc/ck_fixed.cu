@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owne
         double dr[3], r;
         pair_geom(B, d.h, B.atom_self[a], gj, dr, r);
         const double rinv = r > 0.0 ? 1.0 / r : 1e20;
-        const double ex = exp(-r * pr.inv_lam);
+        const double ex = exp_neg(r * pr.inv_lam);
         double E = 0.0, fs = 0.0;
         if (r < pr.rout) {
             if (pr.fx_amp != 0.0) pair_2b_x(P, pr, r, rinv, ex, B.flags, E, fs);
@@ -261,7 +261,7 @@ __device__ __noinline__ void missing_pair(const BatchView& B, const DevParamSet&
     pair_geom(B, B.sys[s].h, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], dr, r);
     const int Rp = NB == 3 ? P.R3 : P.R4;
     const PairTab Q = tuple_pair(R, p);
-    pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
+    pair_setup_x(P, Q, r, exp_neg(r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
                  [&](int n, const Fx& t, const Fx& d) { tab[n * kFxTile] = fx_quad(t, d); });
     scal[0] = fc;
     scal[kFxTile] = fc * gs / r;
@@ -342,7 +342,7 @@ __device__ __forceinline__ bool fx_setup(const BatchView& B, const int* clusters
                 const PairTab Q = tuple_pair(R, p);
                 if (r < Q.rin) atomicAdd(&B.flags[4], 1);
                 double fc, fcd, gs;
-                pair_setup_x(P, Q, r, exp(-r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
+                pair_setup_x(P, Q, r, exp_neg(r * Q.inv_lam), Rp, fx_kd(Rp), fc, fcd, gs,
                              [&](int n, const Fx& t, const Fx& d) { tab[n * kFxTile] = fx_quad(t, d); });
                 geo[(4 * NP + p) * kFxTile + lane] = fc;
                 geo[(5 * NP + p) * kFxTile + lane] = fcd;

@@ -126,11 +126,11 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
         fc = 0.0;
         fcd = 0.0;
     } else {
-        const double f0 = (r - th) * finv * kPi + kPi / 2.0;
-        double sn, cs;
-        sincos(f0, &sn, &cs);
-        fc = 0.5 + 0.5 * sn;
-        fcd = 0.5 * cs * (kPi * finv);
+        // f0 = (r - th) finv kPi + kPi / 2 = pi + psi, with kPi - pi = 2.07e-13
+        long long sn, cs;
+        sincos_fx(((r - th) * finv - 0.5) * kPi + 2.0682310711021444e-13, sn, cs);
+        fc = (double)((1LL << 61) - sn) * 0x1p-62;
+        fcd = (double)cs * (-0x1p-62 * kPi * finv);
     }
 }
 
@@ -144,7 +144,7 @@ template <typename F>
 __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab& Q, double r, double ex, int nT,
                                              int kd, double& fc, double& fcd, double& gs, F&& put) {
     const bool oor = r < Q.rin;
-    if (oor) ex = exp(-Q.rin * Q.inv_lam);
+    if (oor) ex = exp_neg(Q.rin * Q.inv_lam);
     const double xd = (ex - Q.xavg) * Q.inv_xdiff;
     const double g = -ex * Q.inv_lam * Q.inv_xdiff;
     fcut_x(P, r, Q.rout, Q.fc_th, Q.fc_inv, fc, fcd);
@@ -172,7 +172,7 @@ __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab
 __device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& pr, double r, double rinv, double ex,
                                           int* flags, double& E, double& fs) {
     const bool oor = r < pr.rin;
-    if (oor) ex = exp(-pr.rin * pr.inv_lam);
+    if (oor) ex = exp_neg(pr.rin * pr.inv_lam);
     const double xd = (ex - pr.xavg) * pr.inv_xdiff;
     const int kd = fx_kd(P.o2 + 1);
     const double gs = -ex * pr.inv_lam * pr.inv_xdiff * (double)(1 << kd);

@@ -191,7 +191,7 @@ __device__ __forceinline__ void pair_setup(const DevParamSet& P, const PairTab& 
                                            int stride, int nT, CT& fc, CT& fcd, int* flags) {
     const double rin = Q.rin;
     const bool oor = r < rin;
-    const double e = oor ? exp(-rin * Q.inv_lam) : ex;
+    const double e = oor ? exp_neg(rin * Q.inv_lam) : ex;
     const double xd = (e - Q.xavg) * Q.inv_xdiff;
     const double dxdr = -e * Q.inv_lam * Q.inv_xdiff;
     cheby_fill_strided<CT>(T, D, stride, nT, xd, dxdr, oor, r, rin, P.inner_smooth, flags);

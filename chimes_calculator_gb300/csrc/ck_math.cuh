@@ -13,6 +13,57 @@ namespace {
 
 constexpr double kPi = 3.14159265359;   // the reference's `pi` macro (chimesFF.h:22)
 
+// exp(-y) and the sine and cosine of the cutoffs in 64-bit integer arithmetic.
+// GB300 issues an FP64 warp instruction per 16 cycles and SM: exp took 304 SM
+// cycles a warp and sincos 455 (measured), a 64 x 64 bit product's high half
+// about 2.  Taylor series after an exact reduction; every product is truncated
+// at 2^-62 or below.
+//
+// exp(-y): y log2(e) = k + j / 4 + f with f < 1/4, exp(-y) = 2^-k 2^(-j/4)
+// exp(-f ln 2), twelve terms (z^13 / 13! < 2^-65 for z < 0.1733).  The result is
+// within 2^-56 of exp(-y) relatively for y < 64, before its rounding to a double.
+__device__ __forceinline__ double exp_neg(double y) {
+    if (!(y >= 0.0 && y < 64.0)) return exp(-y);
+    const unsigned long long v = (unsigned long long)__double2ll_rn(y * 144115188075855872.0);   // 2^57
+    const unsigned long long t = __umul64hi(v, 0xb8aa3b295c17f0bcull);                           // y log2(e) at 2^56
+    const int k = (int)(t >> 56), j = (int)(t >> 54) & 3;
+    const unsigned long long z = __umul64hi((t & ((1ull << 54) - 1)) << 8, 0xb17217f7d1cf79acull);   // f ln 2 at 2^64
+    constexpr unsigned long long c[12] = {0x8000000000000000ull, 0x8000000000000000ull, 0x4000000000000000ull,
+                                          0x1555555555555555ull, 0x0555555555555555ull, 0x0111111111111111ull,
+                                          0x002d82d82d82d82eull, 0x0006806806806807ull, 0x0000d00d00d00d01ull,
+                                          0x0000171de3a556c7ull, 0x0000024fc9f6ef14ull, 0x00000035cc8acfebull};   // 2^63 / n!
+    unsigned long long p = 0x47bb63bfeull;
+#pragma unroll
+    for (int n = 11; n >= 0; n--) p = c[n] - __umul64hi(z, p);
+    const unsigned long long q0 = j & 1 ? 0x6ba27e656b4eb57aull : 0x8000000000000000ull;   // 2^63 2^(-j/4)
+    const unsigned long long q1 = j & 1 ? 0x4c1bf828c6dc54b8ull : 0x5a827999fcef3242ull;
+    const unsigned long long m = __umul64hi(p, j & 2 ? q1 : q0);                            // at 2^62
+    return __ull2double_rn(m) * __longlong_as_double((long long)(1023 - 62 - k) << 52);
+}
+
+// sin and cos of psi, |psi| < 2, at 2^61 (both within 2^-59): series of the half
+// angle to x^19 and x^18 (remainders below 2^-63), then the double angle.
+__device__ __forceinline__ void sincos_fx(double psi, long long& sn, long long& cs) {
+    const unsigned long long x = (unsigned long long)__double2ll_rn(fabs(psi) * 4611686018427387904.0) << 1;   // |psi| / 2 at 2^64
+    const unsigned long long w = __umul64hi(x, x);
+    constexpr unsigned long long s[9] = {0x8000000000000000ull, 0x1555555555555555ull, 0x0111111111111111ull,
+                                         0x0006806806806807ull, 0x0000171de3a556c7ull, 0x00000035cc8acfebull,
+                                         0x000000005849184full, 0x00000000006b9fd0ull, 0x000000000000654bull};   // 2^63 / (2n + 1)!
+    constexpr unsigned long long c[9] = {0x8000000000000000ull, 0x4000000000000000ull, 0x0555555555555555ull,
+                                         0x002d82d82d82d82eull, 0x0000d00d00d00d01ull, 0x0000024fc9f6ef14ull,
+                                         0x000000047bb63bfeull, 0x00000000064e5d2aull, 0x000000000006b9fdull};   // 2^63 / (2n)!
+    unsigned long long p = 0x4cull, q = 0x5a1ull;
+#pragma unroll
+    for (int n = 8; n >= 0; n--) {
+        p = s[n] - __umul64hi(w, p);
+        q = c[n] - __umul64hi(w, q);
+    }
+    const unsigned long long h = __umul64hi(x, p);        // sin(|psi| / 2) at 2^63
+    const long long sv = (long long)__umul64hi(h, q);     // sin cos at 2^62: sin(psi) at 2^61
+    sn = psi < 0.0 ? -sv : sv;
+    cs = (1LL << 61) - (long long)__umul64hi(h, h);
+}
+
 template <typename CT> __device__ __forceinline__ void csincos(CT x, CT* s, CT* c);
 template <> __device__ __forceinline__ void csincos<double>(double x, double* s, double* c) { sincos(x, s, c); }
 template <> __device__ __forceinline__ void csincos<float>(float x, float* s, float* c) { sincosf(x, s, c); }

@@ -20,6 +20,7 @@
 #include <cstdint>
 
 #include "ck_common.h"
+#include "ck_fixed.cuh"
 #include "ck_force_common.cuh"
 #include "ck_kernels.h"
 #include "ck_math.cuh"
@@ -118,6 +119,8 @@ __global__ void __launch_bounds__(256) k_nl_pairs(BatchView B, NeighView N) {
                 atomicMax(&B.flags[2], dist < pr.rin ? 2 : 1);
                 if (pr.rin + P.pen_dist - dist > 0.0) atomicAdd(&B.flags[3], 1);
             }
+        } else if (pr.fx_amp != 0.0) {
+            pair_2b_x(P, pr, dist, dist > 0.0 ? 1.0 / dist : 1e20, exp_neg(dist * pr.inv_lam), B.flags, E, fs);
         } else {
             pair_2b<CT>(P, pr, dist, B.flags, E, fs);
         }

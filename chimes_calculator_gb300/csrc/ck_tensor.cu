@@ -105,7 +105,7 @@ __device__ __forceinline__ void pair_regs(const DevParamSet& P, const TupleRec& 
     const double rin = Q.rin[p];
     const bool oor = r < rin;
     const double rr = oor ? rin : r;
-    const double e = exp(-rr * Q.inv_lam[p]);
+    const double e = exp_neg(rr * Q.inv_lam[p]);
     const double xd = (e - Q.xavg[p]) * Q.inv_xdiff[p];
     const double dxdr = -e * Q.inv_lam[p] * Q.inv_xdiff[p];
     const float x = float(xd), tx = 2.0f * x, g = float(dxdr);
