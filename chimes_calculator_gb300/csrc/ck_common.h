@@ -36,6 +36,8 @@ namespace ck {
 constexpr int kMaxOrder = 31;      // powers are packed 5 bits per pair
 constexpr int kMaxTypes = 8;       // nt^4 4-body tuple records
 constexpr int kPowBits = 5;
+// bits of l2_vec.w above the parent atom index (atom indices are below 2^30)
+constexpr unsigned kL2Parent = 0x3FFFFFFFu, kL2In3 = 1u << 30, kL2In4 = 1u << 31;
 constexpr int kBkSmem = 1024;      // cluster buckets counted in shared memory (more: in global memory)
 
 enum Status : int {
@@ -283,7 +285,7 @@ struct SysDesc {
     double ulo[3], uhi[3];     // kept fractional range per axis of the reoriented cell
     double eps;                // margin of the FP32 distance prefilter (Angstrom)
     float c3lo, c3hi, c4lo, c4hi;   // c3 -/+ eps and c4 -/+ eps as FP32, rounded outward
-    float far2;                // (search + eps)^2 as FP32: the pair lists' squared-distance prefilter
+    float far2, near2;         // (search +/- eps)^2 as FP32: the pair lists' squared-distance prefilter
     float c3lo2, c3hi2, c4lo2, c4hi2;   // the same thresholds squared, rounded outward (-1: none below)
     // device-completed
     double minpos[3];
@@ -327,9 +329,11 @@ struct BatchView {
     int* l2_count;                 // [n_atoms_total]
     long long* l2_off;             // [n_atoms_total]
     int* l2_ghost;                 // [n2] ghost slot of the neighbour
-    double* l2_dist;               // [n2] distance in the reoriented frame
+    double* l2_dist;               // [n2] distance in the reoriented frame (sequential enumeration only)
     float* l2_vec;                 // [n2][4] displacement from the list's atom (FP32), for the prefilter
     long long* l2_key;             // [n2] neighbour's parent atom << 32 | its packed image shift, or null
+    int* l2_hash;                  // [l2_slots] entry index or -1, by atom and key, or null (see put_hash)
+    long long l2_slots;
     long long n2_cap;
     // 3B/4B enumeration
     // (an atom's clusters are contiguous, at a_off[2 r], a_off[2 r + 1]; the

@@ -349,6 +349,9 @@ Status Engine::ensure_lists(std::string& err) {
     if (avail_ent_) {
         CK_TRY(d_ghost_sh_.reserve(V_.n_ghost_total));
         CK_TRY(d_l2_key_.reserve(n2_cap_));
+        l2_slots_ = 1024;   // a power of two, twice the list's capacity or more
+        while (l2_slots_ < 2 * n2_cap_) l2_slots_ *= 2;
+        CK_TRY(d_l2_hash_.reserve(l2_slots_));
         if (tuning.rf3 > 0) {
             CK_TRY(d_c3e_.reserve(3 * n3_cap_));
             CK_TRY(d_pcd3_.reserve(4 * n2_cap_));
@@ -404,6 +407,8 @@ Status Engine::ensure_lists(std::string& err) {
     B.all_pairs = avail_ent_ ? 1 : 0;
     B.ghost_sh = avail_ent_ ? d_ghost_sh_.p : nullptr;
     B.l2_key = avail_ent_ ? d_l2_key_.p : nullptr;
+    B.l2_hash = avail_ent_ ? d_l2_hash_.p : nullptr;
+    B.l2_slots = l2_slots_;
     B.pe = d_pe_.p;
     B.pcd3 = d_pcd3_.p; B.pcd4 = d_pcd4_.p;
     B.pct3 = d_pct3_.p; B.pct4 = d_pct4_.p;
@@ -581,7 +586,7 @@ Status Engine::launch(std::string& err) {
                           (const void*)V_.e_off3, (const void*)V_.psets, (const void*)V_.perm3,
                           (const void*)V_.perm4, (const void*)V_.bk_count, (const void*)V_.bk_fill,
                           (const void*)V_.bk_start, (const void*)V_.c3e, (const void*)V_.c4e,
-                          (const void*)V_.pe, (const void*)V_.a_off, (const void*)V_.l2_off, (const void*)V_.l2_key, (const void*)V_.ghost_sh,
+                          (const void*)V_.pe, (const void*)V_.a_off, (const void*)V_.l2_off, (const void*)V_.l2_key, (const void*)V_.l2_hash, (const void*)V_.ghost_sh,
                           (const void*)V_.pcd3, (const void*)V_.pcd4, (const void*)V_.pct3, (const void*)V_.pct4})
         key.push_back((long long)(uintptr_t)p);
     if (key != graph_key_) {

@@ -170,6 +170,7 @@ private:
     std::vector<double> vols_;
     BatchView V_{};
     long long n2_cap_ = 0, n3_cap_ = 0, n4_cap_ = 0;
+    long long l2_slots_ = 0;
     bool staged_ = false;
 
     DevBuf<SysDesc> d_sys_;
@@ -201,7 +202,7 @@ private:
     DevBuf<double> d_pcd3_, d_pcd4_, d_pe_;
     DevBuf<int> d_ghost_sh_;
     DevBuf<long long> d_l2_key_, d_a_off_;
-    DevBuf<int> d_a_cnt_, d_bk_key3_, d_bk_key4_;
+    DevBuf<int> d_a_cnt_, d_bk_key3_, d_bk_key4_, d_l2_hash_;
     DevBuf<unsigned char> d_pct3_, d_pct4_;
     DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_;
     DevBuf<long long> d_bk_start_;

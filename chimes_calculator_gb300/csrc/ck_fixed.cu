@@ -161,12 +161,12 @@ __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owne
         reinterpret_cast<double2*>(B.pe + 4 * e)[0] = make_double2(dr[0], dr[1]);
         reinterpret_cast<double2*>(B.pe + 4 * e)[1] = make_double2(dr[2], fs);
         // (FP64: a pair jk of some cluster can lie at the cutoff itself, to rounding, in this list)
-        const double dist = MIXED ? B.l2_dist[e] : B.l2_dist[e] - 1e-6;
-        if (rs3 > 0 && d.has3 && dist < d.c3) {
+        const unsigned w = MIXED ? reinterpret_cast<const unsigned*>(B.l2_vec)[4 * e + 3] : 0u;
+        if (rs3 > 0 && d.has3 && (MIXED ? (w & kL2In3) != 0 : r < d.c3 + 1e-6)) {
             if (MIXED) put_pair_f(P, P.pt3[pt], dr, r, ex, P.R3, rs3, reinterpret_cast<float*>(B.pct3) + e * 2 * rs3, B.pcd3 + 8 * e);
             else put_pair(P, P.pt3[pt], r, rinv, ex, P.R3, reinterpret_cast<FxEnt*>(B.pct3) + e * rs3, B.pcd3 + 4 * e);
         }
-        if (rs4 > 0 && d.has4 && dist < d.c4) {
+        if (rs4 > 0 && d.has4 && (MIXED ? (w & kL2In4) != 0 : r < d.c4 + 1e-6)) {
             if (MIXED) put_pair_f(P, P.pt4[pt], dr, r, ex, P.R4, rs4, reinterpret_cast<float*>(B.pct4) + e * 2 * rs4, B.pcd4 + 8 * e);
             else put_pair(P, P.pt4[pt], r, rinv, ex, P.R4, reinterpret_cast<FxEnt*>(B.pct4) + e * rs4, B.pcd4 + 4 * e);
         }

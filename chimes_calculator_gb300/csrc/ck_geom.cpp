@@ -249,6 +249,7 @@ Status system_geometry(const double* ca, const double* cb, const double* cc, int
     d.c4lo2 = sq_down(d.c4lo);
     d.c4hi2 = sq_up(d.c4hi);
     d.far2 = (float)((d.search + d.eps) * (d.search + d.eps));
+    d.near2 = d.search > d.eps ? (float)((d.search - d.eps) * (d.search - d.eps)) : 0.0f;
     return kOk;
 }
 

@@ -434,44 +434,60 @@ __global__ void __launch_bounds__(256) k_bin_rank(BatchView B, const long long* 
 // Lane b < 27 owns neighbour bin b in the reference's loop order (x bins
 // outermost, z innermost); the candidates of all 27 bins are numbered bin by
 // bin and the warp walks them 32 at a time, so the emitted order is the
-// reference's and short bins leave no lanes idle.  The FP32 displacement
-// decides most candidates; the exact FP64 distance (which the list keeps) is
-// taken only for the candidates that survive it, queued in candidate order in
-// shared memory and evaluated 32 at a time, so the FP64 pipe (1/64 of the
-// FP32 rate) runs full warps instead of one or two live lanes per chunk.
+// reference's and short bins leave no lanes idle.  The FP32 distance decides
+// membership and the 3-/4-body range bits of nearly every candidate; the exact
+// FP64 distance is taken only within the margin of one of the cutoffs (FP64
+// distances of all members bound this kernel before: its pipe at 62%).
 // One pass: a warp keeps its members in shared memory (up to kL2Hold; an atom
 // with more walks its candidates again), the block reserves room for its
-// warps' members with one atomic, and the members are written there.  (A
-// counting pass, a scan over the atoms and a filling pass took 402 + 863 us and
-// 10 us of scans on 2000 configurations of 8-512 atoms; this takes 906 us.)
+// warps' members with one atomic, and the members are written there.
+// Measured, 2000 configurations of 8-512 atoms: 402 + 863 us for a counting and
+// a filling pass, and 10 us of scans between; 906 in one pass; 465 us without
+// the members' FP64 distances.
 constexpr int kL2Block = 256;
 constexpr int kL2Hold = 96;
-// bits of l2_vec.w above the parent atom index (atom indices are below 2^30)
-constexpr unsigned kL2Parent = 0x3FFFFFFFu, kL2In3 = 1u << 30, kL2In4 = 1u << 31;
 struct L2Hold {
-    double dist[kL2Hold];
     float x[3][kL2Hold];
     int ghost[kL2Hold];
     unsigned w[kL2Hold];
 };
+// Open-addressing table of the list entries within the 3- or 4-body range, by
+// atom and neighbour key; a slot holds an entry's index (B.l2_slots a power of two,
+// at least twice those entries).  (Scanning the atom's list instead, by a lane or
+// by a warp, made the enumeration of 384 configurations 440-510 us; with the
+// table it takes 258, and the insertions 16 us of the list kernel.)
+__device__ __forceinline__ unsigned entry_hash(const BatchView& B, int r, long long key) {
+    unsigned long long x = (unsigned long long)key * 0x9e3779b97f4a7c15ull + (unsigned)r * 0xc2b2ae3d27d4eb4full;
+    x ^= x >> 29;
+    x *= 0xbf58476d1ce4e5b9ull;
+    return (unsigned)(x >> 32) & (unsigned)(B.l2_slots - 1);
+}
+__device__ __forceinline__ void put_hash(const BatchView& B, int r, long long key, long long e) {
+    unsigned h = entry_hash(B, r, key);
+    // (never full: bounded all the same)
+    for (long long n = 0; n < B.l2_slots; n++, h = (h + 1) & (unsigned)(B.l2_slots - 1))
+        if (atomicCAS(&B.l2_hash[h], -1, (int)e) == -1) return;
+}
+
 // An entry: x, y, z the FP32 displacement for the enumeration's prefilter; w the
 // neighbour's parent atom (int bits; saves the enumeration a dependent load per
 // candidate) with the exact tests dist < c3 and dist < c4 in bits 30 and 31, so
 // the enumeration compares no FP64 distances.
-__device__ __forceinline__ void put_l2(const BatchView& B, int* l2_owner, long long pos, int r, int ghost, double dist,
-                                       float x, float y, float z, unsigned w) {
+__device__ __forceinline__ void put_l2(const BatchView& B, int* l2_owner, long long pos, int r, int ghost, float x,
+                                       float y, float z, unsigned w) {
     if (pos >= B.n2_cap) return;
     B.l2_ghost[pos] = ghost;
-    B.l2_dist[pos] = dist;
     l2_owner[pos] = r;
-    if (B.l2_key) B.l2_key[pos] = (long long)(w & kL2Parent) << 32 | B.ghost_sh[ghost];
+    if (B.l2_key) {
+        const long long key = (long long)(w & kL2Parent) << 32 | B.ghost_sh[ghost];
+        B.l2_key[pos] = key;
+        if (w & (kL2In3 | kL2In4)) put_hash(B, r, key, pos);
+    }
     reinterpret_cast<float4*>(B.l2_vec)[pos] = make_float4(x, y, z, __uint_as_float(w));
 }
 
 __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
     constexpr int NWARP = kL2Block / 32;
-    __shared__ int queue[NWARP][64];
-    __shared__ int qpar[NWARP][64];
     __shared__ L2Hold hold[NWARP];
     __shared__ int s_cnt[NWARP];
     __shared__ long long s_base;
@@ -486,12 +502,11 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
     long long base = -1;   // where entries go: < 0 into shared memory
     L2Hold& H = hold[wib];
     auto walk = [&]() {
-        const double fi[3] = {B.ghost_fn[3 * gi], B.ghost_fn[3 * gi + 1], B.ghost_fn[3 * gi + 2]};
         const float xi[3] = {B.ghost_xf[3 * gi], B.ghost_xf[3 * gi + 1], B.ghost_xf[3 * gi + 2]};
-        double hn[9];
-        for (int c = 0; c < 9; c++) hn[c] = d.hn[c];
-        const double sd = d.search;
-        const float far2 = d.far2;
+        const double sd = d.search, c3 = d.c3, c4 = d.c4;
+        const float far2 = d.far2, near2 = B.enum_serial ? -1.0f : d.near2;   // (the sequential form reads l2_dist)
+        const float c3lo2 = d.c3lo2, c3hi2 = d.c3hi2, c4lo2 = d.c4lo2, c4hi2 = d.c4hi2;
+        const bool has3 = d.has3, has4 = d.has4;
         count = 0;
         // the atom's bin, as k_ghosts placed it
         const int ib0 = B.ghost_bin[gi];
@@ -526,46 +541,6 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
         }
         const int excl = incl - nbin;
         const int ncand = __shfl_sync(kFull, incl, 31);
-        int* q = queue[wib];
-        int* qp = qpar[wib];
-        int qn = 0;   // queued candidates (warp-uniform)
-        // exact distances of the first n queued candidates; members kept in order
-        auto drain = [&](int n) {
-            bool pred = false;
-            int ajj = -1, par = -1;
-            double dd = 0.0, rv[3] = {0, 0, 0};
-            if (lane < n) {
-                ajj = q[lane];
-                par = qp[lane];
-                dd = dist_frac(hn, fi, &B.ghost_fn[3 * (long long)ajj], rv);
-                pred = dd < sd;
-            }
-            const unsigned bal = __ballot_sync(kFull, pred);
-            if (pred) {
-                const int k = count + __popc(bal & lt);
-                const unsigned w = (unsigned)par | (dd < d.c3 ? kL2In3 : 0u) | (dd < d.c4 ? kL2In4 : 0u);
-                if (base >= 0) {
-                    put_l2(B, l2_owner, base + k, (int)r, ajj, dd, (float)rv[0], (float)rv[1], (float)rv[2], w);
-                } else if (k < kL2Hold) {
-                    H.dist[k] = dd;
-                    H.x[0][k] = (float)rv[0];
-                    H.x[1][k] = (float)rv[1];
-                    H.x[2][k] = (float)rv[2];
-                    H.ghost[k] = ajj;
-                    H.w[k] = w;
-                }
-            }
-            count += __popc(bal);
-            // move the rest of the queue to its front
-            __syncwarp();
-            const int rest = qn - n;
-            int mv = -1, mp = -1;
-            if (lane < rest) { mv = q[n + lane]; mp = qp[n + lane]; }
-            __syncwarp();
-            if (lane < rest) { q[lane] = mv; qp[lane] = mp; }
-            __syncwarp();
-            qn = rest;
-        };
         for (int t0 = 0; t0 < ncand; t0 += 32) {
             const int t = t0 + lane;
             // bin of candidate t: the last bin whose first candidate is <= t
@@ -577,8 +552,11 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
             }
             const long long st = __shfl_sync(kFull, bst, lo);
             const int first = __shfl_sync(kFull, excl, lo);
-            bool near = false;
+            bool in = false;
             int ajj = -1, par = -1;
+            float ex = 0.f, ey = 0.f, ez = 0.f;
+            unsigned w = 0;
+            double dd = 0.0;
             if (t < ncand) {
                 const long long it = st + (t - first);
                 ajj = B.bin_items[it];
@@ -593,22 +571,36 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
                     xj[1] = B.ghost_xf[3 * (long long)ajj + 1];
                     xj[2] = B.ghost_xf[3 * (long long)ajj + 2];
                 }
-                if (ajj != gi && r <= par) {
-                    const float ex = xj[0] - xi[0], ey = xj[1] - xi[1], ez = xj[2] - xi[2];
-                    near = ex * ex + ey * ey + ez * ez < far2;   // else certainly >= sd
+                ex = xj[0] - xi[0]; ey = xj[1] - xi[1]; ez = xj[2] - xi[2];
+                const float e2 = ex * ex + ey * ey + ez * ez;
+                in = ajj != gi && r <= par && e2 < far2;   // else certainly >= sd
+                if (in) {
+                    bool in3 = has3 && e2 < c3lo2, in4 = has4 && e2 < c4lo2;
+                    if (!(e2 < near2) || (has3 && !in3 && !(e2 >= c3hi2)) || (has4 && !in4 && !(e2 >= c4hi2))) {
+                        dd = dist_frac(d.hn, &B.ghost_fn[3 * gi], &B.ghost_fn[3 * (long long)ajj]);
+                        in = dd < sd;
+                        in3 = dd < c3;   // (c3, c4 are 0 for an absent order)
+                        in4 = dd < c4;
+                    }
+                    w = (unsigned)par | (in3 ? kL2In3 : 0u) | (in4 ? kL2In4 : 0u);
                 }
             }
-            const unsigned m = __ballot_sync(kFull, near);
-            if (near) {
-                const int pos = qn + __popc(m & lt);
-                q[pos] = ajj;
-                qp[pos] = par;
+            const unsigned m = __ballot_sync(kFull, in);
+            if (in) {
+                const int k = count + __popc(m & lt);
+                if (base >= 0) {
+                    put_l2(B, l2_owner, base + k, (int)r, ajj, ex, ey, ez, w);
+                    if (B.enum_serial && base + k < B.n2_cap) B.l2_dist[base + k] = dd;
+                } else if (k < kL2Hold) {
+                    H.x[0][k] = ex;
+                    H.x[1][k] = ey;
+                    H.x[2][k] = ez;
+                    H.ghost[k] = ajj;
+                    H.w[k] = w;
+                }
             }
-            qn += __popc(m);
-            __syncwarp();
-            if (qn >= 32) drain(32);
+            count += __popc(m);
         }
-        if (qn > 0) drain(qn);
     };
     if (have && !d.err) walk();
     if (lane == 0) s_cnt[wib] = count;
@@ -626,13 +618,14 @@ __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
         B.l2_off[r] = at;
         B.l2_count[r] = count;
     }
-    if (count > kL2Hold) {
+    if (count > kL2Hold || B.enum_serial) {
         base = at;
         walk();
         return;
     }
+    __syncwarp();
     for (int k = lane; k < count; k += 32)
-        put_l2(B, l2_owner, at + k, (int)r, H.ghost[k], H.dist[k], H.x[0][k], H.x[1][k], H.x[2][k], H.w[k]);
+        put_l2(B, l2_owner, at + k, (int)r, H.ghost[k], H.x[0][k], H.x[1][k], H.x[2][k], H.w[k]);
 }
 
 // Exact test "distance >= c" for a ghost pair of one atom's list, deciding
@@ -770,54 +763,52 @@ __global__ void k_enum(BatchView B, const int* l2_owner) {
 
 // List entry of the pair (j, k) of two images in one atom's list: the entry of
 // j's parent whose neighbour is k's parent at the shift of k relative to j
-// (key_j, key_k: the images' l2_key).  The list of the parent holds every pair
-// below the search radius whose parents are in this order, so only a pair
-// within rounding of the radius itself can be missing: -1.
-__device__ __forceinline__ int find_entry(const BatchView& B, long long key_j, long long key_k) {
-    const long long want = (key_k & ~0xffffffffLL) | (unsigned)((int)key_k - (int)key_j + kShiftBias);
-    long long b0, b1;
-    list_range(B, key_j >> 32, b0, b1);
-    for (long long e = b0; e < b1; e += 4) {
-        long long q[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) q[u] = e + u < b1 ? B.l2_key[e + u] : -1;
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (q[u] == want) return (int)e + u;
+// (w_j, w_k: their l2_vec.w; sh: packed shifts).  The list of the parent holds
+// every pair below the search radius whose parents are in this order, so only a
+// pair within rounding of a cutoff can be missing: -1.
+__device__ __forceinline__ int find_entry(const BatchView& B, const int* l2_owner, unsigned w_j, int sh_j, unsigned w_k,
+                                          int sh_k) {
+    const int pj = (int)(w_j & kL2Parent);
+    const long long want = (long long)(w_k & kL2Parent) << 32 | (unsigned)(sh_k - sh_j + kShiftBias);
+    unsigned h = entry_hash(B, pj, want);
+    for (long long n = 0; n < B.l2_slots; n++, h = (h + 1) & (unsigned)(B.l2_slots - 1)) {
+        const int e = B.l2_hash[h];
+        if (e < 0) return -1;
+        if (B.l2_key[e] == want && l2_owner[e] == pj) return e;
     }
     return -1;
 }
 
-// The list entries of a triplet's / quadruplet's pairs (entries a, b[, c] of
-// the first atom): those of the first atom alone, or all of them (all_pairs).
-__device__ __forceinline__ void put_c3e(const BatchView& B, long long q, long long a, long long b) {
-    if (!B.c3e) return;
-    if (!B.all_pairs) {
-        B.c3e[2 * q] = (int)a;
-        B.c3e[2 * q + 1] = (int)b;
-        return;
-    }
-    int* o = B.c3e + 3 * q;
-    o[0] = (int)a;
-    o[1] = (int)b;
-    o[2] = find_entry(B, B.l2_key[a], B.l2_key[b]);
+// The list entries of a cluster's pairs (entries e[0..n) of the first atom):
+// those of the first atom alone, or all of them (all_pairs).
+template <int N>
+__device__ __forceinline__ void put_entries(const BatchView& B, const int* l2_owner, long long q, const int* e,
+                                            const unsigned* w, const int* sh) {
+    int* out = N == 2 ? B.c3e : B.c4e;
+    if (!out) return;
+    constexpr int ALL = N * (N + 1) / 2;
+    out += (B.all_pairs ? ALL : N) * q;
+#pragma unroll
+    for (int k = 0; k < N; k++) out[k] = e[k];
+    if (!B.all_pairs) return;
+    int n = N;
+#pragma unroll
+    for (int a = 0; a < N; a++)
+#pragma unroll
+        for (int b = a + 1; b < N; b++) out[n++] = find_entry(B, l2_owner, w[a], sh[a], w[b], sh[b]);
 }
-__device__ __forceinline__ void put_c4e(const BatchView& B, long long q, long long a, long long b, long long c) {
-    if (!B.c4e) return;
-    if (!B.all_pairs) {
-        B.c4e[3 * q] = (int)a;
-        B.c4e[3 * q + 1] = (int)b;
-        B.c4e[3 * q + 2] = (int)c;
-        return;
+__device__ __forceinline__ void put_entries_of(const BatchView& B, const int* l2_owner, long long q, int n, long long a,
+                                               long long b, long long c) {
+    const long long at[3] = {a, b, c};
+    int e[3], sh[3] = {0, 0, 0};
+    unsigned w[3];
+    for (int k = 0; k < n; k++) {
+        e[k] = (int)at[k];
+        w[k] = reinterpret_cast<const unsigned*>(B.l2_vec)[4 * at[k] + 3];
+        if (B.all_pairs) sh[k] = (int)B.l2_key[at[k]];
     }
-    const long long ka = B.l2_key[a], kb = B.l2_key[b], kc = B.l2_key[c];
-    int* o = B.c4e + 6 * q;
-    o[0] = (int)a;
-    o[1] = (int)b;
-    o[2] = (int)c;
-    o[3] = find_entry(B, ka, kb);
-    o[4] = find_entry(B, ka, kc);
-    o[5] = find_entry(B, kb, kc);
+    if (n == 2) put_entries<2>(B, l2_owner, q, e, w, sh);
+    else put_entries<3>(B, l2_owner, q, e, w, sh);
 }
 
 // Per-entry warp form of the same enumeration.  When the 4-body outer cutoff
@@ -829,7 +820,7 @@ __device__ __forceinline__ void put_c4e(const BatchView& B, long long q, long lo
 // 4-body terms and rc4 > rc3 keep the sequential carry-over (k_enum).  Used
 // by k_enuma for atoms whose list is longer than its bit matrices hold.
 template <bool FILL>
-__device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDesc& d, int lane, unsigned lt,
+__device__ void enumw_entry(const BatchView& B, const int* l2_owner, long long e, int r, const SysDesc& d, int lane, unsigned lt,
                             long long at3 = 0, long long at4 = 0) {
     const float4* vec = reinterpret_cast<const float4*>(B.l2_vec);
     const double c3 = d.c3, c4 = d.c4;
@@ -870,7 +861,7 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
                 if (q < B.n3_cap) {
                     int* out = B.c3 + 3 * q;
                     out[0] = gi; out[1] = jj; out[2] = kk;
-                    put_c3e(B, q, e, k);
+                    put_entries_of(B, l2_owner, q, 2, e, k, 0);
                 }
             }
             n3 += __popc(m3);
@@ -912,7 +903,7 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
                         if (q < B.n4_cap) {
                             int* out = B.c4 + 4 * q;
                             out[0] = gi; out[1] = jj; out[2] = ks; out[3] = ll;
-                            put_c4e(B, q, e, kb + src, l);
+                            put_entries_of(B, l2_owner, q, 3, e, kb + src, l);
                         }
                     }
                     n4 += __popc(ml);
@@ -924,7 +915,8 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
 }
 
 // Bit-matrix form (G warps per atom i, atoms with at most kEnumRows list
-// entries).  With the reset semantics above, membership depends only on pair
+// entries within the 3- or 4-body range; the others of the list start and join
+// no cluster).  With the reset semantics above, membership depends only on pair
 // tests among the entries of i's list:
 //   T[j][k] = want3(j) && in3(k) && j != k && parent(j) <= parent(k) && |r_jk| < rc3
 //   Q[j][k] = want4(j) && in4(k) && j != k && parent(j) <= parent(k) && |r_jk| < rc4
@@ -939,8 +931,9 @@ __device__ void enumw_entry(const BatchView& B, long long e, int r, const SysDes
 // same order (k ascending, then l ascending), each entry's after the counts of
 // the entries before it.  One pass over the atoms: two passes with a scan over
 // the entries between them tested every pair twice (2000 configurations: 625 +
-// 860 us and about 180 us of scans; this takes 875 us, and 930 with the bucket
-// keys).  G = 1 for batches with many atoms; small ones spread an atom over
+// 860 us and about 180 us of scans; 875 us in one pass, 930 with the bucket
+// keys, 633 since each atom's list is compacted to its entries in range).
+// G = 1 for batches with many atoms; small ones spread an atom over
 // up to a whole block so that the launch still fills the GPU.
 constexpr int kEnumRows = 96;
 constexpr int kEnumWords = kEnumRows / 32;   // odd: column reads of the masks hit distinct banks
@@ -990,7 +983,7 @@ __device__ __forceinline__ void count_key(const BatchView& B, int* hist, int at,
 }
 
 template <int G>
-__global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
+__global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B, const int* l2_owner) {
     constexpr int NG = kEnumWarps / G;   // atoms a block works on at a time
     __shared__ float4 s_v[NG][kEnumRows];
     __shared__ int s_g[NG][kEnumRows];
@@ -999,6 +992,8 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
     __shared__ int s_o[NG][2 * kEnumRows + 2];   // per-entry offsets, then the totals
     __shared__ long long s_at[NG][2];            // where the atom's clusters go
     __shared__ unsigned char s_ty[NG][kEnumRows];   // the entries' types
+    __shared__ unsigned short s_e[NG][kEnumRows];   // their numbers in the atom's list
+    __shared__ int s_sh[NG][kEnumRows];             // their image shifts
     extern __shared__ int s_hist[];              // bucket counts of this block (when B.keyed and few buckets)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int grp = wib / G, w = wib % G;
@@ -1015,6 +1010,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
     unsigned* rt = s_t[grp];
     unsigned* rq = s_q[grp];
     int* so = s_o[grp];
+    unsigned short* se = s_e[grp];
     // room for an atom's t3 triplets and t4 quadruplets (one lane of the group)
     auto reserve = [&](long long r, long long t3, long long t4) {
         const long long a3 = t3 > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[1], (unsigned long long)t3) : 0;
@@ -1028,19 +1024,38 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
     for (long long r = (long long)blockIdx.x * NG + grp; r < B.n_atoms_total; r += ngroups) {
         long long b0, b1;
         list_range(B, r, b0, b1);
-        const int L = (int)(b1 - b0);
         const SysDesc& d = B.sys[B.atom_sys[r]];
-        if (L <= 0 || (!d.has3 && !d.has4)) {
+        // the entries within the 3- or 4-body range, in order (about half of the list)
+        int L = 0;
+        if (d.has3 || d.has4) {
+            group_sync<G>(grp);   // the previous atom's masks and offsets are no longer read
+            for (long long e0 = b0; e0 < b1; e0 += 32) {   // (every warp of the group counts; the first one keeps)
+                const long long e = e0 + lane;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (e < b1) v = vec[e];
+                const bool in = e < b1 && (__float_as_uint(v.w) & (kL2In3 | kL2In4));
+                const unsigned m = __ballot_sync(kFull, in);
+                const int k = L + __popc(m & lt);
+                if (in && w == 0 && k < kEnumRows) {
+                    sv[k] = v;
+                    se[k] = (int)(e - b0);
+                    sg[k] = B.l2_ghost[e];
+                    s_ty[grp][k] = (unsigned char)B.atom_type[__float_as_uint(v.w) & kL2Parent];
+                    if (B.all_pairs) s_sh[grp][k] = (int)B.l2_key[e];
+                }
+                L += __popc(m);
+            }
+        }
+        if (L <= 0) {
             if (w == 0 && lane == 0) {
                 B.a_off[2 * r] = B.a_off[2 * r + 1] = 0;
                 B.a_cnt[2 * r] = B.a_cnt[2 * r + 1] = 0;
             }
             continue;
         }
-        group_sync<G>(grp);   // the previous atom's masks and offsets are no longer read
         if (L > kEnumRows) {
             // counts per entry, their offsets, then the clusters
-            for (long long e = b0 + w; e < b1; e += G) enumw_entry<false>(B, e, (int)r, d, lane, lt);
+            for (long long e = b0 + w; e < b1; e += G) enumw_entry<false>(B, l2_owner, e, (int)r, d, lane, lt);
             __threadfence_block();
             group_sync<G>(grp);
             if (w == 0) {
@@ -1062,7 +1077,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
             __threadfence_block();
             group_sync<G>(grp);
             for (long long e = b0 + w; e < b1; e += G)
-                enumw_entry<true>(B, e, (int)r, d, lane, lt, s_at[grp][0], s_at[grp][1]);
+                enumw_entry<true>(B, l2_owner, e, (int)r, d, lane, lt, s_at[grp][0], s_at[grp][1]);
             if (nbk > 0) {
                 // their keys, from the clusters as written
                 __threadfence_block();
@@ -1087,12 +1102,6 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
                 }
             }
             continue;
-        }
-        for (int a = 32 * w + lane; a < L; a += 32 * G) {
-            const float4 v = vec[b0 + a];
-            sv[a] = v;
-            sg[a] = B.l2_ghost[b0 + a];
-            s_ty[grp][a] = (unsigned char)B.atom_type[__float_as_uint(v.w) & kL2Parent];
         }
         group_sync<G>(grp);
         const int nw = (L + 31) >> 5;
@@ -1194,7 +1203,12 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
                 if (q < B.n3_cap) {
                     int* out = B.c3 + 3 * q;
                     out[0] = gi; out[1] = sg[a]; out[2] = sg[bk];
-                    put_c3e(B, q, b0 + a, b0 + bk);
+                    if (B.c3e) {
+                        const int e[2] = {(int)b0 + se[a], (int)b0 + se[bk]};
+                        const unsigned wv[2] = {__float_as_uint(sv[a].w), __float_as_uint(sv[bk].w)};
+                        const int sh[2] = {s_sh[grp][a], s_sh[grp][bk]};
+                        put_entries<2>(B, l2_owner, q, e, wv, sh);
+                    }
                     if (nbk > 0) {
                         key = P.key3[(ti * nt + s_ty[grp][a]) * nt + s_ty[grp][bk]];
                         if (key >= 0) key += P.bk3;
@@ -1233,7 +1247,13 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
                 if (q < B.n4_cap) {
                     int* out = B.c4 + 4 * q;
                     out[0] = gi; out[1] = sg[a]; out[2] = sg[bk]; out[3] = sg[lk];
-                    put_c4e(B, q, b0 + a, b0 + bk, b0 + lk);
+                    if (B.c4e) {
+                        const int e[3] = {(int)b0 + se[a], (int)b0 + se[bk], (int)b0 + se[lk]};
+                        const unsigned wv[3] = {__float_as_uint(sv[a].w), __float_as_uint(sv[bk].w),
+                                                __float_as_uint(sv[lk].w)};
+                        const int sh[3] = {s_sh[grp][a], s_sh[grp][bk], s_sh[grp][lk]};
+                        put_entries<3>(B, l2_owner, q, e, wv, sh);
+                    }
                     if (nbk > 0) {
                         key = P.key4[((ti * nt + s_ty[grp][a]) * nt + s_ty[grp][bk]) * nt + s_ty[grp][lk]];
                         if (key >= 0) key += P.bk4;
@@ -1252,14 +1272,14 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B) {
 }
 
 template <int G>
-void launch_enuma(const BatchView& B, cudaStream_t st) {
+void launch_enuma(const BatchView& B, const int* l2_owner, cudaStream_t st) {
     constexpr int NG = kEnumWarps / G;
     const long long want = (long long)sm_count() * 4;   // 4 blocks of 8 warps per SM
     const long long need = (B.n_atoms_total + NG - 1) / NG;
     const unsigned grid = (unsigned)(want < need ? want : need);
     const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
     const size_t smem = nbk <= kBkSmem ? sizeof(int) * (size_t)nbk : 0;
-    count_launch(), k_enuma<G><<<grid, 32 * kEnumWarps, smem, st>>>(B);
+    count_launch(), k_enuma<G><<<grid, 32 * kEnumWarps, smem, st>>>(B, l2_owner);
 }
 
 // --- reset of accumulators, counters and bins -------------------------------
@@ -1284,6 +1304,8 @@ __global__ void k_reset(BatchView B) {
             B.bk_count[i] = 0;
             B.bk_fill[i] = 0;
         }
+    if (B.l2_hash)
+        for (long long i = t; i < B.l2_slots / 4; i += stride) reinterpret_cast<int4*>(B.l2_hash)[i] = make_int4(-1, -1, -1, -1);
     if (t < 8) B.flags[t] = 0;
     if (t < 2) B.queue[t] = 0ull;
     if (t < 4 && B.totals) B.totals[t] = 0;
@@ -1496,14 +1518,15 @@ void launch_enum(const BatchView& B, const int* l2_owner, void* scan_tmp, cudaSt
     const long long n = B.n_atoms_total;
     const int G = n >= target ? 1 : 2 * n >= target ? 2 : 4 * n >= target ? 4 : 8;
     switch (G) {
-    case 1: launch_enuma<1>(B, st); break;
-    case 2: launch_enuma<2>(B, st); break;
-    case 4: launch_enuma<4>(B, st); break;
-    default: launch_enuma<8>(B, st); break;
+    case 1: launch_enuma<1>(B, l2_owner, st); break;
+    case 2: launch_enuma<2>(B, l2_owner, st); break;
+    case 4: launch_enuma<4>(B, l2_owner, st); break;
+    default: launch_enuma<8>(B, l2_owner, st); break;
     }
 }
 void launch_reset(const BatchView& B, cudaStream_t st) {
     long long n = std::max(std::max(8LL * B.n_sys, 3 * B.n_in_total), std::max(B.n_bins_total, 8LL));
+    if (B.l2_hash) n = std::max(n, B.l2_slots / 4);
     n = std::min((n + 255) / 256, 16LL * sm_count());
     count_launch(), k_reset<<<(unsigned)n, 256, 0, st>>>(B);
 }
