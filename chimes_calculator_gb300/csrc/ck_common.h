@@ -175,6 +175,17 @@ struct PairTab {
     double rin, rout, xavg, xdiff, inv_lam, inv_xdiff, fc_th, fc_inv;
 };
 
+// Mixed pair-table cache: one list entry's pair at a body order's cutoffs.
+struct PairCache {
+    double d[3], r;
+    float df[3];      // d in FP32
+    float rinv;       // 1 / r
+    float fc, fcd;
+    int flags;        // kPairOor, kPairFar
+    float pad;
+};
+static_assert(sizeof(PairCache) == 64, "eight doubles a list entry");
+
 // One factored-list entry: coefficient and the other side's record, in one
 // 16-byte (FP64) or 8-byte (FP32) load.  idx = linear index (bits 0-15) |
 // the other side's powers packed kPowBits per pair (bits 16-30) | bit 31 set on

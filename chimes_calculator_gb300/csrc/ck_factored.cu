@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
         constexpr int KC = NB - 1;
         const bool use_pc = NB == 3 ? B.use_pc3 : B.use_pc4;
         const int* ce = NB == 3 ? B.c3e : B.c4e;
-        const double* pcd = NB == 3 ? B.pcd3 : B.pcd4;
+        const PairCache* pcd = reinterpret_cast<const PairCache*>(NB == 3 ? B.pcd3 : B.pcd4);
         const CT* pct = reinterpret_cast<const CT*>(NB == 3 ? B.pct3 : B.pct4);
         if (active) {
             for (int k = 0; k < NB; k++) id[k] = clusters[(long long)NB * c + k];
@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
                 const int p = use_pc ? (sl < NP - KC ? KC + sl : sl - (NP - KC)) : sl;
                 double dr[3], r;
                 if (use_pc && p < KC) {
-                    const double* g = pcd + 8 * (long long)ce[(long long)KC * c + p];
-                    dr[0] = g[0]; dr[1] = g[1]; dr[2] = g[2]; r = g[3];
+                    const PairCache& g = pcd[ce[(long long)KC * c + p]];
+                    dr[0] = g.d[0]; dr[1] = g.d[1]; dr[2] = g.d[2]; r = g.r;
                 } else {
                     pair_geom(B, h, id[Topo<NB>::a(p)], id[Topo<NB>::b(p)], dr, r);
                 }
@@ -389,15 +389,15 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
                 const int p = use_pc ? (sl < NP - KC ? KC + sl : sl - (NP - KC)) : sl;
                 if (use_pc && p < KC) {
                     const long long ent = ce[(long long)KC * c + p];
-                    const double* g = pcd + 8 * ent;
+                    const PairCache& g = pcd[ent];
                     const CT* tab = pct + ent * 2 * rs;
                     for (int n = 0; n < Rp; n++) {
                         Tt[(p * rs + n) * G + grp] = tab[n];
                         Dt[(p * rs + n) * G + grp] = tab[rs + n];
                     }
-                    fcs[p * G + grp] = g[4];
-                    fcds[p * G + grp] = g[5];
-                    if (g[6] != 0.0) atomicAdd(&B.flags[4], 1);
+                    fcs[p * G + grp] = double(g.fc);
+                    fcds[p * G + grp] = double(g.fcd);
+                    if (g.flags & kPairOor) atomicAdd(&B.flags[4], 1);
                 } else {
                     CT fc, fcd;
                     const double r = geo[(4 * p + 3) * G + grp];
@@ -642,7 +642,9 @@ __global__ void __launch_bounds__(32) k_forcef(BatchView B, const int* clusters,
                 Gf[p] = float(Gp[p]);
             }
             double e_c, vir_c[6];
-            cluster_epilogue_f32<NB>(B, id, drf, rinv, fcf, fcdf, float(S), Gf, e_c, vir_c);
+            int at[NB];
+            for (int k = 0; k < NB; k++) at[k] = B.atom_orig[B.ghost_parent[id[k]]];
+            cluster_epilogue_f32<NB>(B, at, drf, rinv, fcf, fcdf, float(S), Gf, e_c, vir_c);
             acc.add(B, s, e_c, vir_c);
         }
         __syncwarp();

@@ -115,14 +115,20 @@ __device__ __forceinline__ void put_pair_f(const DevParamSet& P, const PairTab& 
                                            int R, int rs, float* tab, double* g) {
     float fc, fcd;
     pair_setup<float>(P, Q, r, ex, tab, tab + rs, 1, R, fc, fcd, nullptr);
-    g[0] = dr[0]; g[1] = dr[1]; g[2] = dr[2]; g[3] = r;
-    g[4] = double(fc); g[5] = double(fcd); g[6] = r < Q.rin ? 1.0 : 0.0; g[7] = 0.0;
+    for (int n = R; n < rs; n++) tab[n] = tab[rs + n] = 0.0f;
+    PairCache& c = *reinterpret_cast<PairCache*>(g);
+    c.d[0] = dr[0]; c.d[1] = dr[1]; c.d[2] = dr[2]; c.r = r;
+    const float rf = float(r);
+    c.df[0] = float(dr[0]); c.df[1] = float(dr[1]); c.df[2] = float(dr[2]); c.rinv = 1.0f / rf;
+    c.fc = fc; c.fcd = fcd;
+    c.flags = (r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0);
+    c.pad = 0.0f;
 }
 
 // Bound by the FP64 pipe (geometry, square root, exponential and the cutoffs'
 // sines; the polynomial sums are fixed-point).  Measured: 5.23 M entries mixed
-// 1.32 ms and 0.41 ms for their forces, against 1.84 ms for the 2-body kernel
-// and 0.59 ms for a separate pass over the tables.  rs3, rs4: stride of the tables of
+// 1.37 ms with the tables of both body orders and 0.40 ms for their forces, against
+// 1.84 ms for a 2-body kernel and 0.59 ms for a pass over the 3-body tables alone.  rs3, rs4: stride of the tables of
 // a body order, 0 for none.  (Entries one by one: with an atom's entries spread
 // over eight lanes instead, 384 configurations took 941 us and not 456, the
 // lanes' rounds being one long dependent chain each.)

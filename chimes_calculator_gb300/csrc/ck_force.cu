@@ -248,7 +248,9 @@ __global__ void __launch_bounds__(128) k_forcen(BatchView B, const int* clusters
                     Gf[p] = float(Gp[p]);
                 }
                 double e_c, vir_c[6];
-                cluster_epilogue_f32<NB>(B, id, drf, rinv, fcf, fcdf, float(S), Gf, e_c, vir_c);
+                int at[NB];
+                for (int k = 0; k < NB; k++) at[k] = B.atom_orig[B.ghost_parent[id[k]]];
+                cluster_epilogue_f32<NB>(B, at, drf, rinv, fcf, fcdf, float(S), Gf, e_c, vir_c);
                 acc.add(B, s, e_c, vir_c);
             }
         } else if (nc > 0 && gl == 0) {

@@ -67,22 +67,26 @@ __device__ __forceinline__ const TupleRec* cluster_tuple(const BatchView& B, con
     return (NB == 3 ? P->t3 : P->t4) + u;
 }
 
-__device__ __forceinline__ void add_force(const BatchView& B, int ghost, double fx, double fy, double fz) {
-    const int o = B.atom_orig[B.ghost_parent[ghost]];
+// (o: one of the caller's atoms)
+__device__ __forceinline__ void add_force_atom(const BatchView& B, int o, double fx, double fy, double fz) {
     if (!ck_bound(B, o >= 0 && o < B.n_in_total)) return;
     atomicAdd(&B.force[3 * (long long)o + 0], fx);
     atomicAdd(&B.force[3 * (long long)o + 1], fy);
     atomicAdd(&B.force[3 * (long long)o + 2], fz);
 }
+__device__ __forceinline__ void add_force(const BatchView& B, int ghost, double fx, double fy, double fz) {
+    add_force_atom(B, B.atom_orig[B.ghost_parent[ghost]], fx, fy, fz);
+}
 
 // Per-atom energy and virial of one n-atom interaction, shared equally by its
 // atoms (Pair::ev_tally_mb, etc/lmp/etc/pair.cpp); vir in the order
 // xx xy xz yy yz zz, stored as xx yy zz xy xz yz.  Only when requested.
-__device__ __forceinline__ void tally_atoms(const BatchView& B, const int* ghosts, int n, double e, const double* vir) {
+// (at: the caller's atoms)
+__device__ __forceinline__ void tally_at(const BatchView& B, const int* at, int n, double e, const double* vir) {
     if (!B.eatom && !B.vatom) return;
     const double w = 1.0 / n;
     for (int k = 0; k < n; k++) {
-        const long long o = B.atom_orig[B.ghost_parent[ghosts[k]]];
+        const long long o = at[k];
         if (B.eatom) atomicAdd(&B.eatom[o], e * w);
         if (B.vatom) {
             double* v = &B.vatom[6 * o];
@@ -96,40 +100,71 @@ __device__ __forceinline__ void tally_atoms(const BatchView& B, const int* ghost
     }
 }
 
-// Energy/virial accumulator for one system at a time: per lane (add), and per
-// warp (add_warp), where lane 4 k holds value k of the warp's sum.
+// The same for ghosts or atoms of the list.
+__device__ __forceinline__ void tally_atoms(const BatchView& B, const int* ghosts, int n, double e, const double* vir) {
+    if (!B.eatom && !B.vatom) return;
+    int at[4];
+    for (int k = 0; k < n; k++) at[k] = B.atom_orig[B.ghost_parent[ghosts[k]]];
+    tally_at(B, at, n, e, vir);
+}
+
+// Energy/virial accumulator for one system at a time, per lane.
 struct EVAcc {
     int s = -1;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
-    int ws = -1;      // the warp sum's system (uniform)
-    double wv = 0.0;
     __device__ void flush(const BatchView& B) {
         if (s >= 0)
             for (int k = 0; k < 7; k++) atomicAdd(&B.ev[8 * s + k], v[k]);
         s = -1;
         for (int k = 0; k < 7; k++) v[k] = 0;
     }
-    __device__ void flush_sum(const BatchView& B) {
-        const int lane = threadIdx.x & 31;
-        if (ws >= 0 && (lane & 3) == 0 && lane < 28) atomicAdd(&B.ev[8 * ws + (lane >> 2)], wv);
-        ws = -1;
-        wv = 0.0;
-    }
     __device__ void add(const BatchView& B, int sys, double e, const double* vir) {
         if (sys != s) { flush(B); s = sys; }
         v[0] += e;
         for (int k = 0; k < 6; k++) v[1 + k] += vir[k];
     }
-    // Warp-collective (all 32 lanes call it): one interaction's energy and
-    // virial per lane (valid lanes), summed over the warp per system -- the
-    // lanes of a warp mostly hold one, or few.  The seven sums are folded
-    // together (a lane keeps half of its values and hands over the rest at each
-    // step: 9 additions, where seven butterflies take 35; GB300 issues an FP64
-    // addition per 16 cycles and SM), so each costs 10 FP64 instructions.
-    __device__ void add_warp(const BatchView& B, int sys, double e, const double* vir, bool valid) {
+    // end of kernel: one set of atomics per warp when its lanes hold one system
+    __device__ void flush_warp(const BatchView& B) {
+        const int lane = threadIdx.x & 31;
+        const unsigned have = __ballot_sync(kFull, s >= 0);
+        if (!have) return;
+        const int s0 = __shfl_sync(kFull, s, __ffs(have) - 1);
+        if (__all_sync(kFull, s < 0 || s == s0)) {
+            for (int k = 0; k < 7; k++) {
+                double x = v[k];
+                for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
+                v[k] = x;
+            }
+            if (lane == 0)
+                for (int k = 0; k < 7; k++) atomicAdd(&B.ev[8 * s0 + k], v[k]);
+        } else {
+            flush(B);
+        }
+    }
+};
+
+// The same per warp (all 32 lanes call it): lane 4 k holds value k of the sum of
+// one system at a time.
+struct EVWarp {
+    int ws = -1;      // the sum's system (uniform)
+    double wv = 0.0;
+    __device__ void flush(const BatchView& B) {
+        const int lane = threadIdx.x & 31;
+        if (ws >= 0 && (lane & 3) == 0 && lane < 28) atomicAdd(&B.ev[8 * ws + (lane >> 2)], wv);
+        ws = -1;
+        wv = 0.0;
+    }
+    // One interaction's energy and virial per lane (valid lanes), summed over
+    // the warp per system -- the lanes of a warp mostly hold one, or few; more than
+    // kRounds add theirs one by one.  The seven sums are folded together (a
+    // lane keeps half of its values and hands over the rest at each step: 9
+    // additions, where seven butterflies take 35; GB300 issues an FP64 addition
+    // per 16 cycles and SM), so each costs 10 FP64 instructions.
+    static constexpr int kRounds = 6;
+    __device__ void add(const BatchView& B, int sys, double e, const double* vir, bool valid) {
         const int lane = threadIdx.x & 31;
         unsigned have = __ballot_sync(kFull, valid);
-        for (int round = 0; have && round < 4; round++) {
+        for (int round = 0; have && round < kRounds; round++) {
             const int s0 = __shfl_sync(kFull, sys, __ffs(have) - 1);
             const bool mine = valid && sys == s0;
             have &= ~__ballot_sync(kFull, mine);
@@ -150,31 +185,15 @@ struct EVAcc {
             x[0] += __shfl_xor_sync(kFull, x[0], 2);
             x[0] += __shfl_xor_sync(kFull, x[0], 1);
             if (s0 != ws) {
-                flush_sum(B);
+                flush(B);
                 ws = s0;
             }
             wv += x[0];
             if (mine) valid = false;
         }
-        if (valid) add(B, sys, e, vir);   // a warp of many systems
-    }
-    // end of kernel: the sums, one set of atomics per warp when its lanes hold one system
-    __device__ void flush_warp(const BatchView& B) {
-        flush_sum(B);
-        const int lane = threadIdx.x & 31;
-        const unsigned have = __ballot_sync(kFull, s >= 0);
-        if (!have) return;
-        const int s0 = __shfl_sync(kFull, s, __ffs(have) - 1);
-        if (__all_sync(kFull, s < 0 || s == s0)) {
-            for (int k = 0; k < 7; k++) {
-                double x = v[k];
-                for (int off = 16; off; off >>= 1) x += __shfl_xor_sync(kFull, x, off);
-                v[k] = x;
-            }
-            if (lane == 0)
-                for (int k = 0; k < 7; k++) atomicAdd(&B.ev[8 * s0 + k], v[k]);
-        } else {
-            flush(B);
+        if (valid) {
+            atomicAdd(&B.ev[8 * sys], e);
+            for (int k = 0; k < 6; k++) atomicAdd(&B.ev[8 * sys + 1 + k], vir[k]);
         }
     }
 };
@@ -315,9 +334,11 @@ __device__ __forceinline__ void cluster_epilogue(const BatchView& B, const int* 
         }
         virial_add(vir, fsp, dr[p]);
     }
-    for (int k = 0; k < NB; k++) add_force(B, id[k], f[k][0], f[k][1], f[k][2]);
+    int at[NB];
+    for (int k = 0; k < NB; k++) at[k] = B.atom_orig[B.ghost_parent[id[k]]];
+    for (int k = 0; k < NB; k++) add_force_atom(B, at[k], f[k][0], f[k][1], f[k][2]);
     acc.add(B, sys, pre[NP] * S, vir);
-    tally_atoms(B, id, NB, pre[NP] * S, vir);
+    tally_at(B, at, NB, pre[NP] * S, vir);
 }
 
 // The same for the mixed form, in FP32: the cluster's force scalars, forces
@@ -327,9 +348,9 @@ __device__ __forceinline__ void cluster_epilogue(const BatchView& B, const int* 
 // per-atom forces (FP64 atomics) and the system's energy and virial (FP64)
 // are accumulated in FP64.  dr: the pairs' vectors, rinv: 1 / distance.
 // The cluster's energy and virial are returned for the caller's (warp-wide)
-// accumulation.
+// accumulation.  at: the cluster's atoms among the caller's.
 template <int NB>
-__device__ __forceinline__ void cluster_epilogue_f32(const BatchView& B, const int* id, const float (*dr)[3],
+__device__ __forceinline__ void cluster_epilogue_f32(const BatchView& B, const int* at, const float (*dr)[3],
                                                      const float* rinv, const float* fc, const float* fcd, float S,
                                                      const float* G, double& e_out, double* vir_out) {
     constexpr int NP = Topo<NB>::NP;
@@ -361,10 +382,10 @@ __device__ __forceinline__ void cluster_epilogue_f32(const BatchView& B, const i
         v[5] -= fsp * dr[p][2] * dr[p][2];
     }
 #pragma unroll
-    for (int k = 0; k < NB; k++) add_force(B, id[k], double(f[k][0]), double(f[k][1]), double(f[k][2]));
-    for (int k = 0; k < 6; k++) vir_out[k] = double(v[k]);
-    e_out = double(pre[NP] * S);
-    tally_atoms(B, id, NB, e_out, vir_out);
+    for (int k = 0; k < NB; k++) add_force_atom(B, at[k], widen(f[k][0]), widen(f[k][1]), widen(f[k][2]));
+    for (int k = 0; k < 6; k++) vir_out[k] = widen(v[k]);
+    e_out = widen(pre[NP] * S);
+    tally_at(B, at, NB, e_out, vir_out);
 }
 
 }  // namespace

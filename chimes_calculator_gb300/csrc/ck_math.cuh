@@ -13,6 +13,15 @@ namespace {
 
 constexpr double kPi = 3.14159265359;   // the reference's `pi` macro (chimesFF.h:22)
 
+// double(x) without the FP64 pipe, which takes 16 cycles per SM for a warp's
+// conversion: the exponent rebased and the significand shifted (zero, subnormal and
+// non-finite values convert).
+__device__ __forceinline__ double widen(float x) {
+    const unsigned b = __float_as_uint(x);
+    if (((b >> 23) & 0xffu) - 1u >= 254u) return b << 1 ? double(x) : __hiloint2double((int)b, 0);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
 // exp(-y) and the sine and cosine of the cutoffs in 64-bit integer arithmetic.
 // GB300 issues an FP64 warp instruction per 16 cycles and SM: exp took 304 SM
 // cycles a warp and sincos 455 (measured), a 64 x 64 bit product's high half
