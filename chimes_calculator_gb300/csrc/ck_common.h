@@ -90,6 +90,7 @@ struct TupleRec {
     // fixed-point form (FP64; see FxStream): the tuple's stream in fx3 / fx4,
     // its parts' boundaries and the power of two its coefficients are scaled by
     int fx_off, fx_split[9];
+    int fx_zbits;      // bits that a group's sum stays below the whole tuple's (see ck_direct.cu)
     double fx_amp;
     double rin[6], rout[6], lam[6], xavg[6], xdiff[6];
     // reciprocals for the factored kernels: 1/lam, 1/xdiff, and the cutoff's
@@ -122,9 +123,9 @@ constexpr int kFactMaxDim = 128;   // largest R^K and R^(P-K) kept in shared mem
 //   header {q_ik, q_jk, mask of its groups, 0}, then for g = 0..(R + 1) / 2 - 1
 //   the coefficients of q_ij = 2g and 2g + 1 {h, l, h, l} (zero where absent, the
 //   mask bit of an all-zero group clear); fx_split[k], k = 0..8: eight parts.
-//   4-body: per row I with coefficients its entries {h, l, J, -1}, padded with
-//   zeros to a multiple of four, the last with I's powers in place of the -1;
-//   then the columns likewise (rows and columns exchanged); fx_split[0..4] /
+//   4-body: per row I with coefficients its entries {h, l, J, I's powers}, padded
+//   with zeros to a multiple of four, kFxMore set in the powers of all but the
+//   last; then the columns likewise (rows and columns exchanged); fx_split[0..4] /
 //   [4..8]: four parts of the rows / columns.  Four spare entries end the
 //   array.
 // Splits are offsets from fx_off, at record boundaries.
@@ -135,6 +136,7 @@ struct __attribute__((aligned(16))) FxEnt {
     int x, y, z, w;
 };
 constexpr int kPairFar = 1, kPairOor = 2;   // pair-entry flags: at or beyond the outer cutoff, below the inner one
+constexpr int kFxMore = (int)0x80000000u;
 constexpr int kFxLimb = 28;
 constexpr int kFxCoef = 61;
 constexpr int kFxSum = 59;

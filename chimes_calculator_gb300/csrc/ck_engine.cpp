@@ -915,8 +915,10 @@ Status Engine::compute_clusters(int slot, int nbody, int n, const double* dx, co
     CK_TRY(cudaMemcpyAsync(ddx, dx, sizeof(double) * n * np, cudaMemcpyHostToDevice, stream_));
     CK_TRY(cudaMemcpyAsync(ddr, dr, sizeof(double) * n * np * 3, cudaMemcpyHostToDevice, stream_));
     CK_TRY(cudaMemcpyAsync(dtyp, typ, sizeof(int) * n * nbody, cudaMemcpyHostToDevice, stream_));
+    const DevParamSet& V = sets_[slot].view;
+    const int fx_powers = nbody == 3 && V.fx3 ? V.R3 : nbody == 4 && V.fx4 ? V.R4 : 0;
     launch_direct(dsets_.p + slot, nbody, nbody == 2 ? P.o2 : nbody == 3 ? P.o3 : P.o4, n, ddx, ddr, dtyp, dforce,
-                  dstress, denergy, dfscal, dstatus, stream_, tab);
+                  dstress, denergy, dfscal, dstatus, stream_, tab, fx_powers);
     CK_TRY(cudaGetLastError());
     CK_TRY(cudaMemcpyAsync(force, dforce, sizeof(double) * n * 3 * nbody, cudaMemcpyDeviceToHost, stream_));
     CK_TRY(cudaMemcpyAsync(stress, dstress, sizeof(double) * n * 6, cudaMemcpyDeviceToHost, stream_));

@@ -134,6 +134,27 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
     }
 }
 
+// T_n and D_n of a pair from its x and dx/dr 2^kd (see pair_setup_x).
+template <typename F>
+__device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, double rin, double xd, double gs, int nT,
+                                              int kd, double& fc, double& fcd, F&& put) {
+    if (!(r < rin)) {
+        fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
+        return;
+    }
+    const double damp = exp((r - rin) / P.inner_smooth);
+    const double k = P.inner_smooth * (damp - 1.0) * gs;
+    int s = 0;
+    for (double bound = 1.0 + fabs(k); bound > 1.0 && s < 40; s++) bound *= 0.5;
+    const double up = (double)(1LL << s), down = 1.0 / up;
+    fc *= up;
+    fcd *= up;
+    fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) {
+        put(n, fx_split(__double2ll_rn(((double)t + k * (double)d) * down)),
+            fx_split(__double2ll_rn((double)d * damp * down)));
+    });
+}
+
 // Chebyshev tables and cutoff of one pair (set_cheby_polys, chimesFF.h:542-628,
 // set_polys_out_of_range, chimesFF.cpp:1572-1613): put(n, T_n, D_n) for n <
 // nT with D_n = n U_{n-1}(x) 2^-kd; fc and fc'; gs with dT_n/dr = gs D_n.
@@ -149,21 +170,7 @@ __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab
     const double g = -ex * Q.inv_lam * Q.inv_xdiff;
     fcut_x(P, r, Q.rout, Q.fc_th, Q.fc_inv, fc, fcd);
     gs = g * (double)(1 << kd);
-    if (!oor) {
-        fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
-        return;
-    }
-    const double damp = exp((r - Q.rin) / P.inner_smooth);
-    const double k = P.inner_smooth * (damp - 1.0) * gs;
-    int s = 0;
-    for (double bound = 1.0 + fabs(k); bound > 1.0 && s < 40; s++) bound *= 0.5;
-    const double up = (double)(1LL << s), down = 1.0 / up;
-    fc *= up;
-    fcd *= up;
-    fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) {
-        put(n, fx_split(__double2ll_rn(((double)t + k * (double)d) * down)),
-            fx_split(__double2ll_rn((double)d * damp * down)));
-    });
+    pair_tables_x(P, r, Q.rin, xd, gs, nT, kd, fc, fcd, put);
 }
 
 // compute_2B (chimesFF.cpp:1644-1775) of one pair below its outer cutoff, as

@@ -106,10 +106,11 @@ void launch_nl_fp(const BatchView& B, const NeighView& N, int nbody, long long n
                   const long long* off, double* d, int* t, cudaStream_t st);
 
 // Per-cluster evaluation (caller-owned cluster loop), FP64; order = the body
-// order's polynomial order of the set (sizes the 3-/4-body kernels' tables).
+// order's polynomial order of the set (sizes the 3-/4-body kernels' tables);
+// fx_powers = its powers per pair where it has fixed-point streams, else 0.
 void launch_direct(const DevParamSet* P, int nbody, int order, int n, const double* dx, const double* dr,
                    const int* typ, double* force, double* stress, double* energy, double* fscal, int* status,
-                   cudaStream_t st, bool tab = false);
+                   cudaStream_t st, bool tab, int fx_powers);
 
 int sm_count();
 

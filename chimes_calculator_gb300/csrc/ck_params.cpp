@@ -840,6 +840,13 @@ double fx_amplitude(const std::vector<FxCoef>& c) {
     std::frexp(need, &e);   // need <= 2^e
     return std::ldexp(1.0, e);
 }
+
+// Whole bits between a tuple's amplitude and its largest group sum.
+int fx_zbits(double amp, double group) {
+    int e = 0;
+    while (e < 10 && group * std::ldexp(2.0, e) <= 0.9 * amp) e++;
+    return e;
+}
 // splits of [0, total) into n parts at the record ends `ends` (ascending, the last = total), by weight
 void fx_parts(const std::vector<int>& ends, const std::vector<double>& weight, int n, int* split) {
     double all = 0.0, w = 0.0;
@@ -857,6 +864,7 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& 
     std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
         return x.col != y.col ? x.col < y.col : x.row < y.row;
     });
+    double top = 0.0;
     std::vector<int> ends;
     std::vector<double> weight;
     for (size_t k = 0; k < c.size();) {
@@ -864,6 +872,7 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& 
         const int col = c[k].col;
         out.push_back(FxEnt{col / Rp, col % Rp, 0, 0});
         out.resize(at + 1 + (Rp + 1) / 2);
+        double sum = 0.0;
         while (k < c.size() && c[k].col == col) {
             const int grp = c[k].row / 2;
             double a[2] = {0.0, 0.0};
@@ -872,16 +881,20 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& 
             fx_limbs(a[0], R.fx_amp, q.x, q.y);
             fx_limbs(a[1], R.fx_amp, q.z, q.w);
             out[at].z |= 1 << grp;
+            sum += std::fabs(a[0]) + std::fabs(a[1]);
         }
+        top = std::max(top, sum);
         ends.push_back((int)out.size() - R.fx_off);
         weight.push_back(1.0);
     }
     R.fx_split[0] = 0;
     fx_parts(ends, weight, 8, R.fx_split);
+    R.fx_zbits = fx_zbits(R.fx_amp, top);
 }
 void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
     R.fx_amp = fx_amplitude(c);
     R.fx_off = (int)out.size();
+    double top = 0.0;
     for (int side = 0; side < 2; side++) {
         if (side == 1)
             for (FxCoef& q : c) {
@@ -898,18 +911,22 @@ void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
         for (size_t k = 0; k < c.size();) {
             const size_t at = out.size();
             const int row = c[k].row, pows = c[k].rowp;
+            double sum = 0.0;
             for (; k < c.size() && c[k].row == row; k++) {
-                FxEnt q{0, 0, c[k].col, -1};
+                if ((out.size() - at) % 4 == 0) sum = 0.0;
+                top = std::max(top, sum += std::fabs(c[k].a));
+                FxEnt q{0, 0, c[k].col, pows | kFxMore};
                 fx_limbs(c[k].a, R.fx_amp, q.x, q.y);
                 out.push_back(q);
             }
-            while ((out.size() - at) % 4) out.push_back(FxEnt{0, 0, 0, -1});
+            while ((out.size() - at) % 4) out.push_back(FxEnt{0, 0, 0, pows | kFxMore});
             out.back().w = pows;
             ends.push_back((int)out.size() - R.fx_off);
             weight.push_back(4.0 + (double)(out.size() - at));
         }
         fx_parts(ends, weight, 4, split);
     }
+    R.fx_zbits = fx_zbits(R.fx_amp, top);
 }
 
 // set_cheby_polys' Morse-map constants (chimesFF.h:553-559)
