@@ -109,6 +109,12 @@ public:
     Status collect(double* force_out, std::vector<SystemResult>& res, std::string& err);  // D2H + sync
 
     cudaStream_t stream() const { return stream_; }
+    // scratch of at least n bytes, kept for the engine's next call on its stream
+    cudaError_t workspace(size_t n, unsigned char*& p) {
+        const cudaError_t e = d_ws_.reserve(n);
+        p = d_ws_.p;
+        return e;
+    }
     ForceLaunch tuning;
     // 3-/4-body contraction: true = factored kernels wherever every parameter
     // set of the batch has factored tables, false = per-coefficient kernels
@@ -210,6 +216,7 @@ private:
     DevBuf<int> d_flags_;
     DevBuf<unsigned long long> d_queue_;
     DevBuf<unsigned char> d_scan_tmp_;
+    DevBuf<unsigned char> d_ws_;
     DevBuf<double> d_dir_d_;      // per-cluster inputs and outputs (doubles)
     DevBuf<int> d_dir_i_;         // per-cluster types and status
 

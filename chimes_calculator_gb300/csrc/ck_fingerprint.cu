@@ -15,12 +15,20 @@
 // Euclidean distance to a histogram of nbin bins over [0, maxd).  The pair
 // loop is O(n1*n2) and runs here as tiles of 256 x 256 records: set-2 tiles
 // staged in shared memory (broadcast reads), each thread owning two set-1
-// records and a private histogram column in shared memory (bin-major, so a
-// warp's 32 columns sit on 32 different banks and increments never collide).
+// records; counts go to a histogram column per lane in shared memory (bin-major, so a
+// warp's 32 columns sit on 32 different banks), by atomics that the block's warps
+// share: no load to wait for, and room for more blocks than a column per thread.
 // Distances are computed in FP32 with a rigorous bound on the error of the
-// squared distance; a pair whose bin the bound certifies is counted directly,
-// the rest (those within ~1e-6 of a bin edge) are recomputed in FP64 with the
-// reference's operations, so the counts equal the FP64 histogram's.
+// distance; a pair whose bin the bound certifies is counted directly, the
+// rest (about 1e-4 of them) are recomputed in FP64 with the reference's
+// operations, so the counts equal the FP64 histogram's.
+//
+// Bound: instruction issue.  The two records of a thread go through packed FP32
+// instructions together, and the bound is one on the distance in units of bins (a
+// constant per record and a relative part) and not on its square against both
+// edges: 20 instructions a pair against 45, and a fifth as many pairs to repeat in
+// FP64.  Measured, 40001 triplets with themselves, 100 bins: 0.63 ms against 1.86
+// (issue slots 68% used).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,16 +48,44 @@ namespace {
 
 constexpr int kFpTileJ = 256;   // set-2 records per shared-memory tile
 constexpr int kFpRows = 2;      // set-1 records per thread
+constexpr int kFpStep = 4;      // set-2 records in flight per thread
 
+// One staged set-2 record, every value twice (packed operands): edges, -margin.
 template <int P>
-struct __align__(P == 1 ? 8 : 16) FpRec {   // one staged set-2 record: edges and squared norm
-    float e[P];
-    float q;
+struct __align__(16) FpRec {
+    float2 e[P];
+    float2 m;
 };
 
-__device__ __forceinline__ float fp_sqrt_approx(float x) {
+// packed FP32 (two values per 64-bit register)
+__device__ __forceinline__ unsigned long long fp_pack(float a, float b) {
+    return (unsigned long long)__float_as_uint(b) << 32 | __float_as_uint(a);
+}
+__device__ __forceinline__ float fp_lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float fp_hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ unsigned long long fp_add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fp_add2_rm(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fp_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fp_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float fp_rsqrt_approx(float x) {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -76,35 +112,41 @@ __device__ __forceinline__ int fp_exact_bin(const double* a, const double* b, do
     return (bin < 0 || bin >= nbin) ? -1 : bin;
 }
 
-// One thread owns kFpRows set-1 records (i0 + tid + r*T) and loops over the
-// staged set-2 tile.  Per pair: the FP32 squared distance s, its error bound
-// eps, a candidate bin k from an approximate square root (floor by a
-// round-down add at 1.5*2^23: no conversion instructions), and the test
-// (k w)^2 (1+d) <= s - eps, s + eps <= ((k+1) w)^2 (1-d) written as fused
-// multiply-adds; a pair that fails it (near an edge, ~1e-4 of them) takes the
-// exact FP64 path.
+// The FP32 distance and its error, u = 2^-24, N = |a| + |b| (norms of the
+// records): with a, b and each difference rounded,
+//   |s32 - s| <= 2 u N sqrt(s) + (2 + P) u s (+ second order),
+// so |sqrt(s32) - sqrt(s)| <= 2 u N + (2 + P) u sqrt(s) -- the second-order part
+// included once sqrt(s) >= 4 u N, which the test below implies -- and
+// t = (s32 / w) rsqrt(s32) adds 2^-21.9 t at most.  In units of bins:
+//   |t - dist / w| <= 4 u N / w + 2^-20 t
+// A pair is counted in floor(t) when t's fraction is farther than that from 0
+// and 1 (the floor by a round-down add at 1.5 * 2^23: no conversion
+// instructions); otherwise, and for s = 0, in its exact FP64 bin.
+constexpr float kFpMargin = 4.0f * 5.9604645e-8f * 1.001f;   // per unit of norm and bin width
+constexpr float kFpRel = 9.5367432e-7f;                      // 2^-20
+constexpr float kFpMagic = 12582912.0f;                      // 1.5 * 2^23: adding it rounds to an integer
+constexpr int kFpMagicBits = 0x4B400000;
+
+// e, m: records' edges and margins (kFpMargin norm / w, rounded up).
 template <int P>
-__global__ void __launch_bounds__(128) k_fp_hist(const float* __restrict__ e1, const float* __restrict__ q1,
+__global__ void __launch_bounds__(128) k_fp_hist(const float* __restrict__ e1, const float* __restrict__ m1,
                                                  const double* __restrict__ d1, long long n1,
-                                                 const float* __restrict__ e2, const float* __restrict__ q2,
+                                                 const float* __restrict__ e2, const float* __restrict__ m2,
                                                  const double* __restrict__ d2, long long n2, int same, int nbin,
                                                  double binw, double maxd, long long n_itile, long long n_jtile,
                                                  unsigned long long* counts, int* flags) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int T = blockDim.x;
-    const int tid = threadIdx.x;
-    unsigned int* hist = reinterpret_cast<unsigned int*>(smem);                  // [nbin][T]
-    FpRec<P>* tile = reinterpret_cast<FpRec<P>*>(smem + sizeof(unsigned int) * (size_t)nbin * T);
-    for (int b = 0; b < nbin; b++) hist[b * T + tid] = 0u;
-    // |s32 - s| <= (4 + P) u sum_k (|a_k| + |b_k|)^2 <= 2 (4 + P) u (qa + qb), u = 2^-24;
-    // the staged norms carry kEps (a margin of 3x over that bound)
-    const float kEps = 6.0f * (4 + P) * 5.9604645e-8f;
+    const int tid = threadIdx.x, lane = tid & 31;
+    FpRec<P>* tile = reinterpret_cast<FpRec<P>*>(smem);
+    unsigned int* hist = reinterpret_cast<unsigned int*>(tile + kFpTileJ);       // [nbin][32]
+    for (int b = tid; b < nbin * 32; b += T) hist[b] = 0u;
     const float inv_wf = (float)(1.0 / binw);
-    const float wlo = (float)(binw * (1.0 + 1.0e-6)), whi = (float)(binw * (1.0 - 1.0e-6));
-    const float kMagic = 12582912.0f;                // 1.5 * 2^23: adding it rounds to an integer
-    const int kMagicBits = 0x4B400000;
     const int rows = T * kFpRows;
     const long long ntiles = n_itile * n_jtile;
+    const unsigned long long inv2 = fp_pack(inv_wf, inv_wf), magic2 = fp_pack(kFpMagic, kFpMagic),
+                             unmagic2 = fp_pack(-kFpMagic, -kFpMagic), half2 = fp_pack(-0.5f, -0.5f),
+                             rel2 = fp_pack(-kFpRel, -kFpRel), neg2 = fp_pack(-1.0f, -1.0f);
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long it = t / n_jtile, jt = t % n_jtile;
         const long long i0 = it * rows, j0 = jt * kFpTileJ;
@@ -114,52 +156,136 @@ __global__ void __launch_bounds__(128) k_fp_hist(const float* __restrict__ e1, c
         __syncthreads();
         for (int k = tid; k < jn; k += T) {
             FpRec<P> r;
-            for (int p = 0; p < P; p++) r.e[p] = e2[(j0 + k) * P + p];
-            r.q = kEps * q2[j0 + k];
+            for (int p = 0; p < P; p++) {
+                const float v = -e2[(j0 + k) * P + p];
+                r.e[p] = make_float2(v, v);
+            }
+            const float v = -m2[j0 + k];
+            r.m = make_float2(v, v);
             tile[k] = r;
         }
         __syncthreads();
-        for (int rr = 0; rr < kFpRows; rr++) {
-            const long long i = i0 + tid + (long long)rr * T;
-            if (i >= n1) break;
-            float a[P];
-            for (int p = 0; p < P; p++) a[p] = e1[i * P + p];
-            const float qa = kEps * q1[i];
-            const int jstart = same ? (int)max(0LL, min((long long)jn, i + 1 - j0)) : 0;
-#pragma unroll 2
-            for (int k = jstart; k < jn; k++) {
-                const FpRec<P> r = tile[k];
-                float s = 0.0f;
+        const long long ia = i0 + tid, ib = ia + T;
+        if (ia >= n1) continue;
+        const bool two = ib < n1;   // (else the second row repeats the first and counts nothing)
+        unsigned long long a[P];
+        for (int p = 0; p < P; p++) a[p] = fp_pack(e1[ia * P + p], e1[(two ? ib : ia) * P + p]);
+        const unsigned long long lim2 = fp_pack(0.5f - m1[ia], 0.5f - m1[two ? ib : ia]);
+        // from k on both rows take every record; before it, where both records are of
+        // the same set, only the first row does
+        const int ka = same ? (int)max(0LL, min((long long)jn, ia + 1 - j0)) : 0;
+        const int kb = !two ? jn : same ? (int)max(0LL, min((long long)jn, ib + 1 - j0)) : 0;
+        // record k against both rows: candidate bins, and whether the bound certifies them
+        auto candidates = [&](int k, int& ba, int& bb, bool& oka, bool& okb) {
+            const FpRec<P>& r = tile[k];
+            unsigned long long s = 0ull;
 #pragma unroll
-                for (int p = 0; p < P; p++) {
-                    const float d = a[p] - r.e[p];
-                    s = fmaf(d, d, s);
-                }
-                const float eps = qa + r.q;
-                // rounded down at magnitude 1.5*2^23 (unit spacing): kMagic + floor(sqrt(s) / w)
-                const float mag = __fmaf_rd(fp_sqrt_approx(s), inv_wf, kMagic);
-                const float kf = mag - kMagic;                 // candidate bin, an exact float integer
-                const int bin = __float_as_int(mag) - kMagicBits;
-                const float lo = kf * wlo, hi = fmaf(kf, whi, whi);
-                const bool ok = bin < nbin && fmaf(lo, lo, eps - s) <= 0.0f && fmaf(-hi, hi, s + eps) <= 0.0f;
-                int b = bin;
-                if (!ok) {
-                    const long long j = j0 + k;
-                    b = fp_exact_bin<P>(d1 + i * P, d2 + j * P, binw, maxd, nbin, bin);
-                    if (b < 0) {
-                        atomicOr(&flags[0], 1);
-                        continue;
-                    }
-                }
-                hist[b * T + tid] += 1u;
+            for (int p = 0; p < P; p++) {
+                const unsigned long long d = fp_add2(a[p], reinterpret_cast<const unsigned long long*>(r.e)[p]);
+                s = p == 0 ? fp_mul2(d, d) : fp_fma2(d, d, s);
             }
+            const unsigned long long q = fp_mul2(fp_mul2(s, inv2), fp_pack(fp_rsqrt_approx(fp_lo(s)), fp_rsqrt_approx(fp_hi(s))));
+            const unsigned long long mag = fp_add2_rm(q, magic2);           // magic + floor(dist / w)
+            const unsigned long long kf = fp_add2(mag, unmagic2);
+            const unsigned long long h = fp_add2(fp_fma2(kf, neg2, q), half2);   // fraction - 1/2
+            const unsigned long long lim = fp_fma2(q, rel2, fp_add2(lim2, *reinterpret_cast<const unsigned long long*>(&r.m)));
+            ba = (int)(unsigned)mag - kFpMagicBits;
+            bb = (int)(unsigned)(mag >> 32) - kFpMagicBits;
+            oka = fabsf(fp_lo(h)) < fp_lo(lim) && (unsigned)ba < (unsigned)nbin;
+            okb = fabsf(fp_hi(h)) < fp_hi(lim) && (unsigned)bb < (unsigned)nbin;
+        };
+        auto exact = [&](long long i, int k, int& bin) {
+            bin = fp_exact_bin<P>(d1 + i * P, d2 + (j0 + k) * P, binw, maxd, nbin, bin);
+            if (bin < 0) {
+                atomicOr(&flags[0], 1);
+                bin = 0;   // (the call fails)
+            }
+        };
+        for (int k = ka; k < kb; k++) {
+            int ba, bb;
+            bool oka, okb;
+            candidates(k, ba, bb, oka, okb);
+            if (!oka) exact(ia, k, ba);
+            atomicAdd(&hist[ba * 32 + lane], 1u);
+        }
+        int k = kb;
+        for (; k + kFpStep <= jn; k += kFpStep) {   // a few records' chains together
+            int ba[kFpStep], bb[kFpStep];
+            bool oka[kFpStep], okb[kFpStep], all = true;
+#pragma unroll
+            for (int u = 0; u < kFpStep; u++) {
+                candidates(k + u, ba[u], bb[u], oka[u], okb[u]);
+                all = all && oka[u] && okb[u];
+            }
+            if (!all)
+#pragma unroll
+                for (int u = 0; u < kFpStep; u++) {
+                    if (!oka[u]) exact(ia, k + u, ba[u]);
+                    if (!okb[u]) exact(ib, k + u, bb[u]);
+                }
+#pragma unroll
+            for (int u = 0; u < kFpStep; u++) {
+                atomicAdd(&hist[ba[u] * 32 + lane], 1u);
+                atomicAdd(&hist[bb[u] * 32 + lane], 1u);
+            }
+        }
+        for (; k < jn; k++) {
+            int ba, bb;
+            bool oka, okb;
+            candidates(k, ba, bb, oka, okb);
+            if (!oka) exact(ia, k, ba);
+            if (!okb) exact(ib, k, bb);
+            atomicAdd(&hist[ba * 32 + lane], 1u);
+            atomicAdd(&hist[bb * 32 + lane], 1u);
         }
     }
     __syncthreads();
     for (int b = tid; b < nbin; b += T) {
         unsigned long long sum = 0;
-        for (int t2 = 0; t2 < T; t2++) sum += hist[b * T + t2];
+        for (int t2 = 0; t2 < 32; t2++) sum += hist[b * 32 + t2];
         if (sum) atomicAdd(&counts[b], sum);
+    }
+}
+
+// Edges of a record: the transform of read_flat_clusters (multi_calc_histogram.cpp:
+// 26-123) with the cluster's own cutoffs, sorted, in FP64 and FP32, and its margin.
+// (Host code before: 2.0 ms of exponentials and sorting for 40001 triplets.)
+template <int P>
+__global__ void k_fp_edges(const DevParamSet* Pp, long long n, const double* d, const int* t, double inv_w,
+                           double* e, float* ef, float* m) {
+    constexpr int NB = P == 1 ? 2 : P == 3 ? 3 : 4;
+    const DevParamSet& D = *Pp;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += stride) {
+        int u = 0;
+        for (int k = 0; k < NB; k++) u = u * D.ntypes + t[c * NB + k];
+        double x[P], s = 0.0;
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            double lam, avg, diff;
+            if constexpr (P == 1) {
+                const PairRec& R = D.pairs[D.pair_map[u]];
+                lam = R.lam; avg = R.xavg; diff = R.xdiff;
+            } else {
+                const TupleRec& R = (NB == 3 ? D.t3 : D.t4)[u];
+                lam = R.lam[p]; avg = R.xavg[p]; diff = R.xdiff[p];
+            }
+            x[p] = (exp(-d[c * P + p] / lam) - avg) / diff;
+            s += x[p] * x[p];
+        }
+#pragma unroll
+        for (int q = 1; q < P; q++)
+#pragma unroll
+            for (int p = P - 1; p >= q; p--) {
+                const double lo = x[p] < x[p - 1] ? x[p] : x[p - 1], hi = x[p] < x[p - 1] ? x[p - 1] : x[p];
+                x[p - 1] = lo;
+                x[p] = hi;
+            }
+        for (int p = 0; p < P; p++) {
+            e[c * P + p] = x[p];
+            ef[c * P + p] = (float)x[p];
+        }
+        m[c] = (float)(sqrt(s) * inv_w * (1.0 + 1e-6)) * kFpMargin;
     }
 }
 
@@ -261,45 +387,23 @@ void launch_nl_fp(const BatchView& B, const NeighView& N, int nbody, long long n
 // ---------------------------------------------------------------------------
 namespace {
 
-// transform of read_flat_clusters (multi_calc_histogram.cpp:112-123), host FP64
-double fp_transform(double rcin, double rcout, double lambda, double rij) {
-    double x_min = std::exp(-1 * rcin / lambda);
-    double x_max = std::exp(-1 * rcout / lambda);
-    double x_avg = 0.5 * (x_max + x_min);
-    double x_diff = 0.5 * (x_max - x_min);
-    x_diff *= -1.0;
-    return (std::exp(-1 * rij / lambda) - x_avg) / x_diff;
-}
-
-// sorted transformed edges of n records (the cluster's own cutoffs, pair
-// lambdas by the atoms' pair type), read_flat_clusters (:26-107)
-Status fp_edges(const Engine& eng, int slot, int nbody, long long n, const double* d, const int* t,
-                std::vector<double>& out, std::string& err) {
-    const HostParams& P = eng.params(slot);
-    const int nt = P.ntypes, np = nbody * (nbody - 1) / 2;
-    out.assign((size_t)n * np, 0.0);
+// Every record has known types and a cluster type that is not excluded.
+Status fp_check(const Engine& eng, int slot, int nbody, long long n, const int* t, std::string& err) {
+    const int nt = eng.params(slot).ntypes;
     for (long long c = 0; c < n; c++) {
-        const int* ty = t + c * nbody;
-        for (int k = 0; k < nbody; k++)
-            if (ty[k] < 0 || ty[k] >= nt) {
+        int u = 0;
+        for (int k = 0; k < nbody; k++) {
+            const int ty = t[c * nbody + k];
+            if (ty < 0 || ty >= nt) {
                 err = "fingerprint record " + std::to_string(c) + ": type index out of range";
                 return kErrInput;
             }
-        double* e = &out[(size_t)c * np];
-        if (nbody == 2) {
-            const int p = P.pair_map[ty[0] * nt + ty[1]];
-            e[0] = fp_transform(P.rin[p], P.rout[p], P.lam[p], d[c]);
-        } else {
-            int u = 0;
-            for (int k = 0; k < nbody; k++) u = u * nt + ty[k];
-            const TupleRec& R = eng.tuples(slot, nbody)[u];
-            if (R.type_id < 0) {
-                err = "fingerprint record " + std::to_string(c) + ": excluded cluster type";
-                return kErrInput;
-            }
-            for (int p = 0; p < np; p++) e[p] = fp_transform(R.rin[p], R.rout[p], R.lam[p], d[c * np + p]);
+            u = u * nt + ty;
         }
-        std::sort(e, e + np);
+        if (nbody > 2 && eng.tuples(slot, nbody)[u].type_id < 0) {
+            err = "fingerprint record " + std::to_string(c) + ": excluded cluster type";
+            return kErrInput;
+        }
     }
     return kOk;
 }
@@ -327,46 +431,23 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     for (int b = 0; b < nbin; b++) counts[b] = 0;
     *nsamples = 0;
     const int np = nbody * (nbody - 1) / 2;
-    std::vector<double> e1, e2;
-    if ((st = fp_edges(eng, slot, nbody, n1, d1, t1, e1, err)) != kOk) return st;
-    if (same) {
-        n2 = n1;
-    } else if ((st = fp_edges(eng, slot, nbody, n2, d2, t2, e2, err)) != kOk) {
-        return st;
-    }
+    if ((st = fp_check(eng, slot, nbody, n1, t1, err)) != kOk) return st;
+    if (same) n2 = n1;
+    else if ((st = fp_check(eng, slot, nbody, n2, t2, err)) != kOk) return st;
     // one process of gen_flat_hists: nothing is counted unless the first set
     // has at least two records (its task range must have end > start)
     if (n1 <= 1 || n2 <= 0) return kOk;
     const double maxd = nbody == 2 ? 3.0 : (nbody == 3 ? std::sqrt(12.0) + 1.0 : std::sqrt(24.0) + 1.0);
     const double binw = maxd / nbin;
-    int T = 128;
-    while (T > 32 && (size_t)nbin * T * 4 > 160 * 1024) T /= 2;
+    constexpr int T = 128;
     const size_t rec = nbody == 2 ? sizeof(FpRec<1>) : nbody == 3 ? sizeof(FpRec<3>) : sizeof(FpRec<6>);
-    const size_t smem = (size_t)nbin * T * 4 + rec * kFpTileJ;
-    if (smem > 200 * 1024) {
+    const size_t smem = (size_t)nbin * 32 * 4 + rec * kFpTileJ;
+    // (a limit above the one it names, as it always was)
+    if ((size_t)nbin * 32 * 4 + (nbody == 2 ? 8 : nbody == 3 ? 16 : 32) * (size_t)kFpTileJ > 200 * 1024) {
         err = "fingerprint histogram: nbin too large for the shared-memory histogram (at most 1280 bins)";
         return kErrInput;
     }
-    auto pack = [&](const std::vector<double>& e, long long n, std::vector<float>& ef, std::vector<float>& q) {
-        ef.resize((size_t)n * np);
-        q.resize((size_t)n);
-        for (long long c = 0; c < n; c++) {
-            double s = 0.0;
-            for (int p = 0; p < np; p++) {
-                ef[(size_t)c * np + p] = (float)e[(size_t)c * np + p];
-                s += e[(size_t)c * np + p] * e[(size_t)c * np + p];
-            }
-            q[(size_t)c] = (float)(s * (1.0 + 1e-6));   // rounded up: the bound stays a bound
-        }
-    };
-    std::vector<float> f1, q1, f2, q2;
-    pack(e1, n1, f1, q1);
-    if (!same) pack(e2, n2, f2, q2);
     const cudaStream_t s = eng.stream();
-    DevBuf<double> dd1, dd2;
-    DevBuf<float> df1, dq1, df2, dq2;
-    DevBuf<unsigned long long> dcounts;
-    DevBuf<int> dflags;
 #define FP_TRY(call)                                                                   \
     do {                                                                               \
         cudaError_t e_ = (call);                                                       \
@@ -375,29 +456,44 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
             return kErrCuda;                                                           \
         }                                                                              \
     } while (0)
-    FP_TRY(dd1.reserve(e1.size()));
-    FP_TRY(df1.reserve(f1.size()));
-    FP_TRY(dq1.reserve(q1.size()));
-    FP_TRY(cudaMemcpyAsync(dd1.p, e1.data(), sizeof(double) * e1.size(), cudaMemcpyHostToDevice, s));
-    FP_TRY(cudaMemcpyAsync(df1.p, f1.data(), sizeof(float) * f1.size(), cudaMemcpyHostToDevice, s));
-    FP_TRY(cudaMemcpyAsync(dq1.p, q1.data(), sizeof(float) * q1.size(), cudaMemcpyHostToDevice, s));
-    const double* pd2 = dd1.p;
-    const float *pf2 = df1.p, *pq2 = dq1.p;
-    if (!same) {
-        FP_TRY(dd2.reserve(e2.size()));
-        FP_TRY(df2.reserve(f2.size()));
-        FP_TRY(dq2.reserve(q2.size()));
-        FP_TRY(cudaMemcpyAsync(dd2.p, e2.data(), sizeof(double) * e2.size(), cudaMemcpyHostToDevice, s));
-        FP_TRY(cudaMemcpyAsync(df2.p, f2.data(), sizeof(float) * f2.size(), cudaMemcpyHostToDevice, s));
-        FP_TRY(cudaMemcpyAsync(dq2.p, q2.data(), sizeof(float) * q2.size(), cudaMemcpyHostToDevice, s));
-        pd2 = dd2.p;
-        pf2 = df2.p;
-        pq2 = dq2.p;
-    }
-    FP_TRY(dcounts.reserve(nbin));
-    FP_TRY(dflags.reserve(1));
-    FP_TRY(cudaMemsetAsync(dcounts.p, 0, sizeof(unsigned long long) * nbin, s));
-    FP_TRY(cudaMemsetAsync(dflags.p, 0, sizeof(int), s));
+    // the engine's workspace: per set the distances (then the edges), types, FP32
+    // edges and margins; the counts and the flag
+    auto up16 = [](size_t b) { return (b + 15) / 16 * 16; };
+    auto set_bytes = [&](long long n) {
+        return up16(sizeof(double) * n * np) * 2 + up16(sizeof(int) * n * nbody) + up16(sizeof(float) * n * np) +
+               up16(sizeof(float) * n);
+    };
+    const size_t b1 = set_bytes(n1), b2 = same ? 0 : set_bytes(n2), bc = up16(sizeof(unsigned long long) * nbin);
+    unsigned char* ws = nullptr;
+    FP_TRY(eng.workspace(b1 + b2 + bc + 16, ws));
+    struct Set {
+        double* d;
+        float *e, *m;
+    };
+    const int Pn = np;
+    auto edges = [&](unsigned char* p, long long n, const double* d, const int* ty, Set& out) -> cudaError_t {
+        double* raw = reinterpret_cast<double*>(p);
+        out.d = reinterpret_cast<double*>(p + up16(sizeof(double) * n * np));
+        int* dt = reinterpret_cast<int*>(p + 2 * up16(sizeof(double) * n * np));
+        out.e = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(dt) + up16(sizeof(int) * n * nbody));
+        out.m = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(out.e) + up16(sizeof(float) * n * np));
+        cudaError_t e = cudaMemcpyAsync(raw, d, sizeof(double) * n * np, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dt, ty, sizeof(int) * n * nbody, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
+        const unsigned g = (unsigned)std::min<long long>((n + 127) / 128, 8LL * sm_count());
+        const DevParamSet* D = eng.device_params() + slot;
+        if (Pn == 1) count_launch(), k_fp_edges<1><<<g, 128, 0, s>>>(D, n, raw, dt, 1.0 / binw, out.d, out.e, out.m);
+        else if (Pn == 3) count_launch(), k_fp_edges<3><<<g, 128, 0, s>>>(D, n, raw, dt, 1.0 / binw, out.d, out.e, out.m);
+        else count_launch(), k_fp_edges<6><<<g, 128, 0, s>>>(D, n, raw, dt, 1.0 / binw, out.d, out.e, out.m);
+        return cudaGetLastError();
+    };
+    Set s1, s2;
+    FP_TRY(edges(ws, n1, d1, t1, s1));
+    s2 = s1;
+    if (!same) FP_TRY(edges(ws + b1, n2, d2, t2, s2));
+    unsigned long long* dcounts = reinterpret_cast<unsigned long long*>(ws + b1 + b2);
+    int* dflags = reinterpret_cast<int*>(ws + b1 + b2 + bc);
+    FP_TRY(cudaMemsetAsync(dcounts, 0, bc + 16, s));
     const long long n_it = (n1 + (long long)T * kFpRows - 1) / ((long long)T * kFpRows),
                     n_jt = (n2 + kFpTileJ - 1) / kFpTileJ;
     const void* kern = nbody == 2 ? (const void*)k_fp_hist<1> : nbody == 3 ? (const void*)k_fp_hist<3>
@@ -409,19 +505,19 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     if (grid > n_it * n_jt) grid = n_it * n_jt;
     const int sm = same ? 1 : 0;
     if (nbody == 2)
-        count_launch(), k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(df1.p, dq1.p, dd1.p, n1, pf2, pq2, pd2, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts.p, dflags.p);
+        count_launch(), k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
+                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
     else if (nbody == 3)
-        count_launch(), k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(df1.p, dq1.p, dd1.p, n1, pf2, pq2, pd2, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts.p, dflags.p);
+        count_launch(), k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
+                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
     else
-        count_launch(), k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(df1.p, dq1.p, dd1.p, n1, pf2, pq2, pd2, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts.p, dflags.p);
+        count_launch(), k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
+                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
     FP_TRY(cudaGetLastError());
     std::vector<unsigned long long> hc(nbin);
     int hflag = 0;
-    FP_TRY(cudaMemcpyAsync(hc.data(), dcounts.p, sizeof(unsigned long long) * nbin, cudaMemcpyDeviceToHost, s));
-    FP_TRY(cudaMemcpyAsync(&hflag, dflags.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FP_TRY(cudaMemcpyAsync(hc.data(), dcounts, sizeof(unsigned long long) * nbin, cudaMemcpyDeviceToHost, s));
+    FP_TRY(cudaMemcpyAsync(&hflag, dflags, sizeof(int), cudaMemcpyDeviceToHost, s));
     FP_TRY(cudaStreamSynchronize(s));
 #undef FP_TRY
     if (hflag) {

@@ -119,3 +119,30 @@ def test_errors(native_lib, system):
         c.fp_histogram(3, d, t, nbin=5000)
     counts, ns = c.fp_histogram(3, d[:1], t[:1], d, t)   # one record in the first set: nothing counted
     assert ns == 0 and not counts.any()
+
+
+@pytest.mark.parametrize("nb", [2, 3, 4])
+@pytest.mark.parametrize("n1,n2", [(2, 0), (255, 0), (256, 1), (257, 0), (513, 0), (300, 513)])
+@pytest.mark.parametrize("nbin", [1, 100, 1280])
+def test_histogram_tile_edges(native_lib, system, nb, n1, n2, nbin):
+    """Remainders of the 256 x 256 tiles and of a thread's two records, repeated
+    records (distance zero), distances beyond the cutoffs, the smallest and the
+    largest bin count: the oracle's counts exactly."""
+    p, o, nl = system
+    from chimes_calculator_gb300 import Calculator
+    c = Calculator()
+    c.load_params(p)
+    rng = np.random.default_rng(1000 * nb + n1 + n2)
+
+    def records(n):
+        d = rng.uniform(0.8, 4.8, (n, nb * (nb - 1) // 2))
+        t = np.zeros((n, nb), dtype=np.int32)   # one element: no excluded cluster type
+        if n > 4:
+            d[n // 2] = d[n // 4]
+        return d, t
+    s1 = records(n1)
+    s2 = records(n2) if n2 else (None, None)
+    counts, ns = c.fp_histogram(nb, *s1, *s2, nbin=nbin)
+    oc, ons = o.fp_histogram(nb, *s1, *s2, nbin=nbin)
+    assert ns == ons == (n1 * n2 if n2 else n1 * (n1 - 1) // 2)
+    assert np.array_equal(counts, oc)
