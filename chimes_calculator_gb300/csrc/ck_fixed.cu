@@ -104,9 +104,9 @@ __device__ __forceinline__ void put_pair(const DevParamSet& P, const PairTab& Q,
                                          int R, FxEnt* tab, double* scal) {
     double fc, fcd, gs;
     pair_setup_x(P, Q, r, ex, R, fx_kd(R), fc, fcd, gs, [&](int n, const Fx& t, const Fx& d) { tab[n] = fx_quad(t, d); });
-    const int flags = (r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0);
+    const int flags = (!less_pos(r, Q.rout) ? kPairFar : 0) | (less_pos(r, Q.rin) ? kPairOor : 0);
     reinterpret_cast<double2*>(scal)[0] = make_double2(fc, fc * gs * rinv);
-    reinterpret_cast<double2*>(scal)[1] = make_double2(fcd * rinv, (double)flags);
+    reinterpret_cast<double2*>(scal)[1] = make_double2(fcd * rinv, __hiloint2double(0, flags));
 }
 
 // The mixed form's pair-table cache: the values the cluster kernel would compute
@@ -118,16 +118,16 @@ __device__ __forceinline__ void put_pair_f(const DevParamSet& P, const PairTab& 
     for (int n = R; n < rs; n++) tab[n] = tab[rs + n] = 0.0f;
     PairCache& c = *reinterpret_cast<PairCache*>(g);
     c.d[0] = dr[0]; c.d[1] = dr[1]; c.d[2] = dr[2]; c.r = r;
-    const float rf = float(r);
-    c.df[0] = float(dr[0]); c.df[1] = float(dr[1]); c.df[2] = float(dr[2]); c.rinv = 1.0f / rf;
+    c.df[0] = narrow(dr[0]); c.df[1] = narrow(dr[1]); c.df[2] = narrow(dr[2]); c.rinv = 1.0f / narrow(r);
     c.fc = fc; c.fcd = fcd;
-    c.flags = (r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0);
+    c.flags = (!less_pos(r, Q.rout) ? kPairFar : 0) | (less_pos(r, Q.rin) ? kPairOor : 0);
     c.pad = 0.0f;
 }
 
-// Bound by the FP64 pipe (geometry, square root, exponential and the cutoffs'
-// sines; the polynomial sums are fixed-point).  Measured: 5.23 M entries mixed
-// 1.37 ms with the tables of both body orders and 0.40 ms for their forces, against
+// Bound by the FP64 pipe (68%: geometry, the maps, forces; polynomial sums,
+// exponential, sines, conversions and comparisons are integer arithmetic).  Measured:
+// 5.23 M entries mixed 1.19 ms with the tables of both body orders (1.37 with FP64
+// conversions and comparisons) and 0.40 ms for their forces, against
 // 1.84 ms for a 2-body kernel and 0.59 ms for a pass over the 3-body tables alone.  rs3, rs4: stride of the tables of
 // a body order, 0 for none.  (Entries one by one: with an atom's entries spread
 // over eight lanes instead, 384 configurations took 941 us and not 456, the
@@ -154,12 +154,11 @@ __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owne
         int pt = P.pair_map[B.atom_type[a] * P.ntypes + B.atom_type[B.ghost_parent[gj]]];
         if (!ck_bound(B, pt >= 0 && pt < P.npairs)) pt = 0;
         const PairRec& pr = P.pairs[pt];
-        double dr[3], r;
-        pair_geom(B, d.h, B.atom_self[a], gj, dr, r);
-        const double rinv = r > 0.0 ? 1.0 / r : 1e20;
+        double dr[3], r, rinv;
+        sqrt_rcp(pair_vec(B, d.h, B.atom_self[a], gj, dr), r, rinv);
         const double ex = exp_neg(r * pr.inv_lam);
         double E = 0.0, fs = 0.0;
-        if (r < pr.rout) {
+        if (less_pos(r, pr.rout)) {
             if (pr.fx_amp != 0.0) pair_2b_x(P, pr, r, rinv, ex, B.flags, E, fs);
             else pair_2b<double>(P, pr, r, B.flags, E, fs);
             acc.add(B, s, E);
@@ -168,11 +167,11 @@ __global__ void __launch_bounds__(128) k_pairs_x(BatchView B, const int* l2_owne
         reinterpret_cast<double2*>(B.pe + 4 * e)[1] = make_double2(dr[2], fs);
         // (FP64: a pair jk of some cluster can lie at the cutoff itself, to rounding, in this list)
         const unsigned w = MIXED ? reinterpret_cast<const unsigned*>(B.l2_vec)[4 * e + 3] : 0u;
-        if (rs3 > 0 && d.has3 && (MIXED ? (w & kL2In3) != 0 : r < d.c3 + 1e-6)) {
+        if (rs3 > 0 && d.has3 && (MIXED ? (w & kL2In3) != 0 : less_pos(r, d.c3 + 1e-6))) {
             if (MIXED) put_pair_f(P, P.pt3[pt], dr, r, ex, P.R3, rs3, reinterpret_cast<float*>(B.pct3) + e * 2 * rs3, B.pcd3 + 8 * e);
             else put_pair(P, P.pt3[pt], r, rinv, ex, P.R3, reinterpret_cast<FxEnt*>(B.pct3) + e * rs3, B.pcd3 + 4 * e);
         }
-        if (rs4 > 0 && d.has4 && (MIXED ? (w & kL2In4) != 0 : r < d.c4 + 1e-6)) {
+        if (rs4 > 0 && d.has4 && (MIXED ? (w & kL2In4) != 0 : less_pos(r, d.c4 + 1e-6))) {
             if (MIXED) put_pair_f(P, P.pt4[pt], dr, r, ex, P.R4, rs4, reinterpret_cast<float*>(B.pct4) + e * 2 * rs4, B.pcd4 + 8 * e);
             else put_pair(P, P.pt4[pt], r, rinv, ex, P.R4, reinterpret_cast<FxEnt*>(B.pct4) + e * rs4, B.pcd4 + 4 * e);
         }
@@ -204,7 +203,7 @@ __global__ void __launch_bounds__(256) k_pair_forces(BatchView B) {
             const double2 p = reinterpret_cast<const double2*>(B.pe + 4 * e)[0];
             const double2 q = reinterpret_cast<const double2*>(B.pe + 4 * e)[1];
             const double fs = q.y;
-            if (fs == 0.0) continue;
+            if (__double_as_longlong(fs) << 1 == 0) continue;
             const double d[3] = {p.x, p.y, q.x}, g[3] = {fs * p.x, fs * p.y, fs * q.x};
             for (int c = 0; c < 3; c++) f[c] += g[c];
             add_force(B, B.l2_ghost[e], -g[0], -g[1], -g[2]);
@@ -272,7 +271,7 @@ __device__ __noinline__ void missing_pair(const BatchView& B, const DevParamSet&
     scal[0] = fc;
     scal[kFxTile] = fc * gs / r;
     scal[2 * kFxTile] = fcd / r;
-    scal[3 * kFxTile] = (double)((r >= Q.rout ? kPairFar : 0) | (r < Q.rin ? kPairOor : 0));
+    scal[3 * kFxTile] = __hiloint2double(0, (!less_pos(r, Q.rout) ? kPairFar : 0) | (less_pos(r, Q.rin) ? kPairOor : 0));
 }
 __device__ __noinline__ void missing_force(const BatchView& B, int ga, int gb, int s, double fs) {
     double dr[3], r, vir[6] = {0, 0, 0, 0, 0, 0};
@@ -377,7 +376,7 @@ __device__ __forceinline__ void fx_finish(const BatchView& B, const int* cluster
     for (int k = 0; k <= NP; k++) {
         long long v = own[k];
         for (int u = 1; u < NW; u++) v += m.part[(u * (NP + 1) + k) * kFxTile + lane];
-        (k == 0 ? S : G[k - 1]) = (double)v;
+        (k == 0 ? S : G[k - 1]) = from_fixed(v, 0);
     }
     const double unit = R.fx_amp * kFxUnit;
     int s = 0;
@@ -398,7 +397,7 @@ __device__ __forceinline__ void fx_finish(const BatchView& B, const int* cluster
                 const double2 x = q[0], y = q[1];
                 fc[p] = x.x; ga[p] = x.y; ca[p] = y.x; fl = y.y;
             }
-            const int f = (int)fl;
+            const int f = __double2loint(fl);
             flags |= f;
             oor += f & kPairOor ? 1 : 0;
         }

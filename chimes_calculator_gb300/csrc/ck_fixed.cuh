@@ -82,10 +82,9 @@ struct FxAcc {
         imad(mid, a.h, b.l);
         imad(mid, a.l, b.h);
     }
-    // the sum as an integer at its scale, as a value, and times `unit`
+    // the sum as an integer at its scale and as a value
     __device__ __forceinline__ long long sum() const { return hi + ((mid + (1LL << (kFxLimb - 1))) >> kFxLimb); }
     __device__ __forceinline__ Fx value() const { return fx_limbs(sum() + (1LL << (kFxLimb - 1))); }
-    __device__ __forceinline__ double real(double unit) const { return (double)sum() * unit; }
 };
 constexpr double kFxUnit = 1.0 / (double)(1LL << kFxSum);
 
@@ -100,7 +99,7 @@ __device__ __forceinline__ long long fx_2x(long long x, long long t) {
 // 0..nT-1, both at 2^56 (T is kept at 2^60 and U, below 64, at 2^57 on the way).
 template <typename F>
 __device__ __forceinline__ void fx_chebyshev(double xd, int nT, int kd, F&& f) {
-    const long long x = __double2ll_rn(xd * (double)(1LL << 62));
+    const long long x = to_fixed(xd, 62);
     long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 57;   // T_n, T_{n+1}, U_{n-1}, U_n
     for (int n = 0; n < nT; n++) {
         f(n, (tn + 8) >> 4, __mul64hi(um, (long long)n << (63 - kd)));
@@ -119,18 +118,18 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
         const double f0 = 1.0 - r * finv;
         fc = f0 * f0 * f0;
         fcd = f0 * f0 * (-3.0 * finv);
-    } else if (r < th) {
+    } else if (less_pos(r, th)) {
         fc = 1.0;
         fcd = 0.0;
-    } else if (r > rout) {
+    } else if (!less_pos(r, rout) && r > rout) {
         fc = 0.0;
         fcd = 0.0;
     } else {
         // f0 = (r - th) finv kPi + kPi / 2 = pi + psi, with kPi - pi = 2.07e-13
         long long sn, cs;
         sincos_fx(((r - th) * finv - 0.5) * kPi + 2.0682310711021444e-13, sn, cs);
-        fc = (double)((1LL << 61) - sn) * 0x1p-62;
-        fcd = (double)cs * (-0x1p-62 * kPi * finv);
+        fc = from_fixed((1LL << 61) - sn, -62);
+        fcd = from_fixed(-cs, -62) * (kPi * finv);
     }
 }
 
@@ -138,7 +137,7 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
 template <typename F>
 __device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, double rin, double xd, double gs, int nT,
                                               int kd, double& fc, double& fcd, F&& put) {
-    if (!(r < rin)) {
+    if (!less_pos(r, rin)) {
         fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
         return;
     }
@@ -164,12 +163,12 @@ __device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, do
 template <typename F>
 __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab& Q, double r, double ex, int nT,
                                              int kd, double& fc, double& fcd, double& gs, F&& put) {
-    const bool oor = r < Q.rin;
+    const bool oor = less_pos(r, Q.rin);
     if (oor) ex = exp_neg(Q.rin * Q.inv_lam);
     const double xd = (ex - Q.xavg) * Q.inv_xdiff;
     const double g = -ex * Q.inv_lam * Q.inv_xdiff;
     fcut_x(P, r, Q.rout, Q.fc_th, Q.fc_inv, fc, fcd);
-    gs = g * (double)(1 << kd);
+    gs = g * __longlong_as_double((1023LL + kd) << 52);
     pair_tables_x(P, r, Q.rin, xd, gs, nT, kd, fc, fcd, put);
 }
 
@@ -178,11 +177,11 @@ __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab
 // ex = exp(-r / lambda), rinv = 1 / r.
 __device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& pr, double r, double rinv, double ex,
                                           int* flags, double& E, double& fs) {
-    const bool oor = r < pr.rin;
+    const bool oor = less_pos(r, pr.rin);
     if (oor) ex = exp_neg(pr.rin * pr.inv_lam);
     const double xd = (ex - pr.xavg) * pr.inv_xdiff;
     const int kd = fx_kd(P.o2 + 1);
-    const double gs = -ex * pr.inv_lam * pr.inv_xdiff * (double)(1 << kd);
+    const double gs = -ex * pr.inv_lam * pr.inv_xdiff * __longlong_as_double((1023LL + kd) << 52);
     const FxPair* a = P.fx2 + pr.coef_off;
     FxAcc s, g;
     fx_chebyshev(xd, P.o2 + 1, kd, [&](int n, long long t, long long d) {
@@ -190,8 +189,7 @@ __device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& p
         s.mac(c, fx_split(t));
         g.mac(c, fx_split(d));
     });
-    const double unit = pr.fx_amp * (1.0 / (double)(1LL << kFxCoef));
-    double S = s.real(unit), G = g.real(unit) * gs;
+    double S = from_fixed(s.sum(), -kFxCoef) * pr.fx_amp, G = from_fixed(g.sum(), -kFxCoef) * (pr.fx_amp * gs);
     if (oor) {
         atomicAdd(&flags[4], 1);
         const double damp = exp((r - pr.rin) / P.inner_smooth);

@@ -34,11 +34,11 @@ __device__ __forceinline__ bool ck_bound(const BatchView& B, bool ok) {
 #else
 __device__ __forceinline__ bool ck_bound(const BatchView&, bool) { return true; }
 #endif
-__device__ __forceinline__ void pair_geom(const BatchView& B, const double* h, int ga, int gb, double* dr, double& r) {
+// Vector between two images; its squared length.
+__device__ __forceinline__ double pair_vec(const BatchView& B, const double* h, int ga, int gb, double* dr) {
     if (!ck_bound(B, ga >= 0 && ga < B.n_ghost_total && gb >= 0 && gb < B.n_ghost_total)) {
         dr[0] = dr[1] = dr[2] = 0.0;
-        r = 1e300;   // beyond every cutoff: the cluster is dropped
-        return;
+        return 1e300;   // beyond every cutoff: the cluster is dropped
     }
     const double* fa = &B.ghost_fs[3 * (long long)ga];
     const double* fb = &B.ghost_fs[3 * (long long)gb];
@@ -46,7 +46,10 @@ __device__ __forceinline__ void pair_geom(const BatchView& B, const double* h, i
     dr[0] = h[0] * dx + h[1] * dy + h[2] * dz;
     dr[1] = h[3] * dx + h[4] * dy + h[5] * dz;
     dr[2] = h[6] * dx + h[7] * dy + h[8] * dz;
-    r = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
+    return dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2];
+}
+__device__ __forceinline__ void pair_geom(const BatchView& B, const double* h, int ga, int gb, double* dr, double& r) {
+    r = sqrt(pair_vec(B, h, ga, gb, dr));
 }
 
 // Ordered type tuple of cluster c: its ghost slots, system, parameter set and tuple index.
@@ -209,26 +212,26 @@ template <typename CT>
 __device__ __forceinline__ void pair_setup(const DevParamSet& P, const PairTab& Q, double r, double ex, CT* T, CT* D,
                                            int stride, int nT, CT& fc, CT& fcd, int* flags) {
     const double rin = Q.rin;
-    const bool oor = r < rin;
+    const bool oor = less_pos(r, rin);
     const double e = oor ? exp_neg(rin * Q.inv_lam) : ex;
     const double xd = (e - Q.xavg) * Q.inv_xdiff;
     const double dxdr = -e * Q.inv_lam * Q.inv_xdiff;
     cheby_fill_strided<CT>(T, D, stride, nT, xd, dxdr, oor, r, rin, P.inner_smooth, flags);
     const double finv = Q.fc_inv;
     if (!P.tersoff) {
-        const CT f0 = CT(1.0) - CT(r) * CT(finv);
+        const CT f0 = CT(1.0) - to_ct<CT>(r) * to_ct<CT>(finv);
         fc = f0 * f0 * f0;
-        fcd = f0 * f0 * (CT(-3.0) * CT(finv));
+        fcd = f0 * f0 * (CT(-3.0) * to_ct<CT>(finv));
     } else {
         const double th = Q.fc_th;
-        if (r < th) { fc = CT(1); fcd = CT(0); }
-        else if (r > Q.rout) { fc = CT(0); fcd = CT(0); }
+        if (less_pos(r, th)) { fc = CT(1); fcd = CT(0); }
+        else if (!less_pos(r, Q.rout) && r > Q.rout) { fc = CT(0); fcd = CT(0); }
         else {
-            const CT f0 = CT(r - th) * CT(finv) * CT(kPi) + CT(kPi / 2.0);
+            const CT f0 = to_ct<CT>(r - th) * to_ct<CT>(finv) * CT(kPi) + CT(kPi / 2.0);
             CT sn, cs;
             csincos<CT>(f0, &sn, &cs);
             fc = CT(0.5) + CT(0.5) * sn;
-            fcd = CT(0.5) * cs * (CT(kPi) * CT(finv));
+            fcd = CT(0.5) * cs * (CT(kPi) * to_ct<CT>(finv));
         }
     }
 }

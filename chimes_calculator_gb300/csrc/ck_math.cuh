@@ -22,6 +22,66 @@ __device__ __forceinline__ double widen(float x) {
     return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
 }
 
+// float(x), rounded to nearest even, the same way (out of the normal floats' range:
+// converted).
+__device__ __forceinline__ float narrow(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    if ((hi & 0x7fffffffu) - 0x38100000u >= 0x0fe00000u) return float(x);
+    const unsigned w = __funnelshift_l(lo, hi, 3);                    // significand's top 23 bits, exponent above
+    const unsigned up = ((lo & 0x1fffffffu) + 0x0fffffffu + (w & 1u)) >> 29;
+    return __uint_as_float((w - 0xc0000000u + up) | (hi & 0x80000000u));
+}
+template <typename CT>
+__device__ __forceinline__ CT to_ct(double x) {
+    if constexpr (sizeof(CT) == 4) return narrow(x);
+    else return x;
+}
+
+// a < b for a >= 0 (not -0) and numbers: the bits compare like integers.
+__device__ __forceinline__ bool less_pos(double a, double b) {
+    return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
+// v 2^S rounded to an integer, |v| 2^S < 2^63; and v 2^E as a double (in the
+// normal range), rounded to nearest.
+__device__ __forceinline__ long long to_fixed(double v, int S) {
+    const long long b = __double_as_longlong(v);
+    const int sh = (int)((unsigned long long)b >> 52 & 0x7ffull) - 1075 + S;
+    const unsigned long long m = ((unsigned long long)b & ((1ull << 52) - 1)) | 1ull << 52;
+    const int r = min(-sh, 63);
+    const long long u = (long long)(sh >= 0 ? m << sh : (m + (1ull << (r - 1))) >> r);
+    return b < 0 ? -u : u;
+}
+__device__ __forceinline__ double from_fixed(long long v, int E) {
+    unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
+    const int z = __clzll((long long)a);
+    a <<= z;
+    const long long q = (long long)((a >> 11) + ((a >> 10) & 1ull));   // 2^52 .. 2^53
+    const long long bits = ((long long)(1085 - z + E) << 52) + q;
+    return __longlong_as_double(v == 0 ? 0ll : bits | (v & (long long)0x8000000000000000ull));
+}
+
+// Square root and its reciprocal: one third-order Householder step for 1 / sqrt
+// from an FP32 estimate (relative error e^3 5/16 < 2^-60 for e < 2^-20), then
+// r = s y with one correction.  10 FP64 instructions, where sqrt and a division
+// took 19 (163 + 142 SM cycles a warp).
+__device__ __forceinline__ void sqrt_rcp(double s, double& r, double& y) {
+    if (!(s > 1e-30 && s < 1e30)) {
+        r = sqrt(s);
+        y = r > 0.0 ? 1.0 / r : 1e20;
+        if (s > 1e-300 && s < 1e300) {
+            const double t = s * y;
+            y = fma(0.5 * y, fma(-t, y, 1.0) - fma(s, y, -t) * y, y);
+        }
+        return;
+    }
+    const double y0 = widen(rsqrtf(narrow(s)));
+    const double e = fma(-s, y0 * y0, 1.0);   // (the square of an FP32 number is exact)
+    y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+    const double t = s * y;
+    r = fma(fma(-t, t, s), 0.5 * y, t);
+}
+
 // exp(-y) and the sine and cosine of the cutoffs in 64-bit integer arithmetic.
 // GB300 issues an FP64 warp instruction per 16 cycles and SM: exp took 304 SM
 // cycles a warp and sincos 455 (measured), a 64 x 64 bit product's high half
@@ -32,8 +92,8 @@ __device__ __forceinline__ double widen(float x) {
 // exp(-f ln 2), twelve terms (z^13 / 13! < 2^-65 for z < 0.1733).  The result is
 // within 2^-56 of exp(-y) relatively for y < 64, before its rounding to a double.
 __device__ __forceinline__ double exp_neg(double y) {
-    if (!(y >= 0.0 && y < 64.0)) return exp(-y);
-    const unsigned long long v = (unsigned long long)__double2ll_rn(y * 144115188075855872.0);   // 2^57
+    if ((unsigned long long)__double_as_longlong(y) >= 0x4050000000000000ull) return exp(-y);   // not in [0, 64)
+    const unsigned long long v = (unsigned long long)to_fixed(y, 57);
     const unsigned long long t = __umul64hi(v, 0xb8aa3b295c17f0bcull);                           // y log2(e) at 2^56
     const int k = (int)(t >> 56), j = (int)(t >> 54) & 3;
     const unsigned long long z = __umul64hi((t & ((1ull << 54) - 1)) << 8, 0xb17217f7d1cf79acull);   // f ln 2 at 2^64
@@ -47,13 +107,14 @@ __device__ __forceinline__ double exp_neg(double y) {
     const unsigned long long q0 = j & 1 ? 0x6ba27e656b4eb57aull : 0x8000000000000000ull;   // 2^63 2^(-j/4)
     const unsigned long long q1 = j & 1 ? 0x4c1bf828c6dc54b8ull : 0x5a827999fcef3242ull;
     const unsigned long long m = __umul64hi(p, j & 2 ? q1 : q0);                            // at 2^62
-    return __ull2double_rn(m) * __longlong_as_double((long long)(1023 - 62 - k) << 52);
+    const unsigned long long q = (m + 256) >> 9;                                            // 2^52 .. 2^53
+    return __longlong_as_double(((long long)(1021 - k) << 52) + (long long)q);
 }
 
 // sin and cos of psi, |psi| < 2, at 2^61 (both within 2^-59): series of the half
 // angle to x^19 and x^18 (remainders below 2^-63), then the double angle.
 __device__ __forceinline__ void sincos_fx(double psi, long long& sn, long long& cs) {
-    const unsigned long long x = (unsigned long long)__double2ll_rn(fabs(psi) * 4611686018427387904.0) << 1;   // |psi| / 2 at 2^64
+    const unsigned long long x = (unsigned long long)to_fixed(fabs(psi), 62) << 1;   // |psi| / 2 at 2^64
     const unsigned long long w = __umul64hi(x, x);
     constexpr unsigned long long s[9] = {0x8000000000000000ull, 0x1555555555555555ull, 0x0111111111111111ull,
                                          0x0006806806806807ull, 0x0000171de3a556c7ull, 0x00000035cc8acfebull,
@@ -67,10 +128,11 @@ __device__ __forceinline__ void sincos_fx(double psi, long long& sn, long long& 
         p = s[n] - __umul64hi(w, p);
         q = c[n] - __umul64hi(w, q);
     }
-    const unsigned long long h = __umul64hi(x, p);        // sin(|psi| / 2) at 2^63
-    const long long sv = (long long)__umul64hi(h, q);     // sin cos at 2^62: sin(psi) at 2^61
-    sn = psi < 0.0 ? -sv : sv;
-    cs = (1LL << 61) - (long long)__umul64hi(h, h);
+    // (+ 1: against the truncations' mean)
+    const unsigned long long h = __umul64hi(x, p) + 1;        // sin(|psi| / 2) at 2^63
+    const long long sv = (long long)__umul64hi(h, q) + 1;     // sin cos at 2^62: sin(psi) at 2^61
+    sn = __double_as_longlong(psi) < 0 ? -sv : sv;
+    cs = (1LL << 61) - 1 - (long long)__umul64hi(h, h);
 }
 
 template <typename CT> __device__ __forceinline__ void csincos(CT x, CT* s, CT* c);
@@ -156,7 +218,7 @@ __device__ __forceinline__ void cheby_table(CT* T, CT* D, double r, double rin, 
 template <typename CT>
 __device__ __forceinline__ void cheby_fill_strided(CT* T, CT* D, int stride, int nT, double xd, double dxdr, bool oor,
                                                    double r, double rin, double inner_smooth, int* flags) {
-    const CT x = CT(xd), tx = CT(2) * x, g = CT(dxdr);
+    const CT x = to_ct<CT>(xd), tx = CT(2) * x, g = to_ct<CT>(dxdr);
     CT k = CT(0), dm = CT(1);
     if (oor) {
         if (flags) atomicAdd(&flags[4], 1);

@@ -43,11 +43,11 @@
 // while the ik tables are read and the sums with W formed.
 //
 // Bound: latency of the gathers and of the chains through the MMAs, with the FP64
-// pipe (pair jk, virial sums) at 44%.  So four CTAs per SM (16 warps): one
+// pipe (pair jk, virial sums) at 39%.  So four CTAs per SM (16 warps): one
 // operand buffer and 128 TMEM columns each, 128 registers a thread, tables read
 // when they are needed rather than held.  Measured: 1.47 M triplets of 32768
-// atoms 556 -> 338 us, 9.15 M of 2000 configurations 3.30 -> 1.95 ms, against
-// two CTAs that hold both rows, both accumulators and all tables at once.
+// atoms 556 -> 338 us, 9.15 M of 2000 configurations 3.30 -> 1.95 ms (320 us and
+// 1.82 ms with conversions and comparisons off the FP64 pipe), against two CTAs that hold both rows, both accumulators and all tables at once.
 // A wait that runs out sets flags[7] and the CTA stops after freeing its TMEM.
 #include <cuda_runtime.h>
 
@@ -111,12 +111,12 @@ template <int R>
 __device__ __forceinline__ void pair_regs(const DevParamSet& P, const TupleRec& Q, int p, double r, float (&T)[R],
                                           float (&D)[R], float& fc, float& fcd, int* flags) {
     const double rin = Q.rin[p];
-    const bool oor = r < rin;
+    const bool oor = less_pos(r, rin);
     const double rr = oor ? rin : r;
     const double e = exp_neg(rr * Q.inv_lam[p]);
     const double xd = (e - Q.xavg[p]) * Q.inv_xdiff[p];
     const double dxdr = -e * Q.inv_lam[p] * Q.inv_xdiff[p];
-    const float x = float(xd), tx = 2.0f * x, g = float(dxdr);
+    const float x = narrow(xd), tx = 2.0f * x, g = narrow(dxdr);
     float k = 0.0f, dm = 1.0f;
     if (oor) {
         if (flags) atomicAdd(&flags[4], 1);
@@ -143,19 +143,19 @@ __device__ __forceinline__ void pair_regs(const DevParamSet& P, const TupleRec& 
     }
     const double finv = Q.fc_inv[p];
     if (!P.tersoff) {
-        const float f0 = 1.0f - float(r) * float(finv);
+        const float f0 = 1.0f - narrow(r) * narrow(finv);
         fc = f0 * f0 * f0;
-        fcd = f0 * f0 * (-3.0f * float(finv));
+        fcd = f0 * f0 * (-3.0f * narrow(finv));
     } else {
         const double th = Q.fc_th[p];
-        if (r < th) { fc = 1.0f; fcd = 0.0f; }
-        else if (r > Q.rout[p]) { fc = 0.0f; fcd = 0.0f; }
+        if (less_pos(r, th)) { fc = 1.0f; fcd = 0.0f; }
+        else if (!less_pos(r, Q.rout[p]) && r > Q.rout[p]) { fc = 0.0f; fcd = 0.0f; }
         else {
-            const float f0 = float(r - th) * float(finv) * float(kPi) + float(kPi / 2.0);
+            const float f0 = narrow(r - th) * narrow(finv) * float(kPi) + float(kPi / 2.0);
             float sn, cs;
             sincosf(f0, &sn, &cs);
             fc = 0.5f + 0.5f * sn;
-            fcd = 0.5f * cs * (float(kPi) * float(finv));
+            fcd = 0.5f * cs * (float(kPi) * narrow(finv));
         }
     }
 }
@@ -397,13 +397,13 @@ __global__ void __launch_bounds__(128, PC ? kTc3Ctas : 2)
                 }
                 double d[3], r;
                 pair_geom(B, B.sys[s].h, id[1], id[2], d, r);
-                active = !((fl0 | fl1) & kPairFar) && r < Rt->rout[2];   // compute_3B's early-outs
+                active = !((fl0 | fl1) & kPairFar) && less_pos(r, Rt->rout[2]);   // compute_3B's early-outs
                 if (active) {
                     const int oor = (fl0 & kPairOor ? 1 : 0) + (fl1 & kPairOor ? 1 : 0);
                     if (oor) atomicAdd(&B.flags[4], oor);
                     pair_regs<R>(*P, *Rt, 2, r, T2, D2, fcf[2], fcdf[2], B.flags);
-                    drf[2][0] = float(d[0]); drf[2][1] = float(d[1]); drf[2][2] = float(d[2]);
-                    rinv[2] = 1.0f / float(r);
+                    drf[2][0] = narrow(d[0]); drf[2][1] = narrow(d[1]); drf[2][2] = narrow(d[2]);
+                    rinv[2] = 1.0f / narrow(r);
                 }
             }
         }
@@ -475,11 +475,13 @@ __global__ void __launch_bounds__(128, PC ? kTc3Ctas : 2)
                 }
 #pragma unroll
                 for (int p = 0; p < 2; p++) {
-                    const PairCache& g = pcd[p == 0 ? e0 : e1];
-                    drf[p][0] = g.df[0]; drf[p][1] = g.df[1]; drf[p][2] = g.df[2];
-                    rinv[p] = g.rinv;
-                    fcf[p] = g.fc;
-                    fcdf[p] = g.fcd;
+                    const float4* g = reinterpret_cast<const float4*>(pcd + (p == 0 ? e0 : e1));
+                    const float4 u = g[2];   // (whole words: a gather costs L1 as much for one as for four)
+                    const float2 v = *reinterpret_cast<const float2*>(g + 3);
+                    drf[p][0] = u.x; drf[p][1] = u.y; drf[p][2] = u.z;
+                    rinv[p] = u.w;
+                    fcf[p] = v.x;
+                    fcdf[p] = v.y;
                 }
             }
         } else {
@@ -579,8 +581,8 @@ void launch_tc_r(const BatchView& B, cudaStream_t st) {
 // kl while the first MMAs run.  What
 // warp 0 reads for the forces is kept for two tiles, so that the other warps
 // go on to the next one.  Bound: latency of the chain tables - operand - MMAs -
-// TMEM at 12 warps an SM, the FP64 pipe at 29%.  Measured: 292 k quadruplets of
-// 32768 atoms 530 -> 280 us, 1.83 M of 2000 configurations 3.3 -> 1.6 ms, against two
+// TMEM at 12 warps an SM, the FP64 pipe at 23%.  Measured: 292 k quadruplets of
+// 32768 atoms 530 -> 276 us, 1.83 M of 2000 configurations 3.3 -> 1.69 ms, against two
 // CTAs of 128 threads with six pairs set up per cluster.
 constexpr int kTc4Tile = 32;              // clusters per tile
 constexpr size_t kTc4MinSmem = 184 * 1024;   // no room for another tensor-core CTA on the SM (TMEM)
@@ -715,7 +717,7 @@ __global__ void __launch_bounds__(128 * tc4_groups(PC), 1)
                 float T[R], D[R], fc = 0.0f, fcd = 0.0f;
 #pragma unroll
                 for (int q = 0; q < R; q++) T[q] = D[q] = 0.0f;
-                const bool far = !on || r >= Rt->rout[p];   // compute_4B's early-outs
+                const bool far = !on || !less_pos(r, Rt->rout[p]);   // compute_4B's early-outs
                 if (!far) pair_regs<R>(*P, *Rt, p, r, T, D, fc, fcd, nullptr);
                 const int R4 = P->R4;   // the set's own powers; entries above it multiply zero coefficients
 #pragma unroll
@@ -723,11 +725,11 @@ __global__ void __launch_bounds__(128 * tc4_groups(PC), 1)
                     sm.tab[p - P0][q][c] = q < R4 ? T[q] : 0.0f;
                     sm.tab[p - P0][R + q][c] = q < R4 ? D[q] : 0.0f;
                 }
-                ep.fl[p - P0][c] = (far ? kPairFar : 0) | (!far && r < Rt->rin[p] ? kPairOor : 0);
+                ep.fl[p - P0][c] = (far ? kPairFar : 0) | (!far && less_pos(r, Rt->rin[p]) ? kPairOor : 0);
                 ep.fc[p - P0][c] = fc;
                 ep.fcd[p - P0][c] = fcd;
-                ep.rinv[p - P0][c] = far ? 0.0f : 1.0f / float(r);
-                for (int k = 0; k < 3; k++) ep.dr[p - P0][k][c] = float(d[k]);
+                ep.rinv[p - P0][c] = far ? 0.0f : 1.0f / narrow(r);
+                for (int k = 0; k < 3; k++) ep.dr[p - P0][k][c] = narrow(d[k]);
             };
             if constexpr (PC) {
 #pragma unroll
@@ -901,12 +903,13 @@ __global__ void __launch_bounds__(128 * tc4_groups(PC), 1)
                     for (int p = 0; p < 6; p++) {
                         int fl;
                         if (p < P0) {
-                            const PairCache& g = pcd[e[p < 3 ? p : 0]];
-                            dr[p][0] = g.df[0]; dr[p][1] = g.df[1]; dr[p][2] = g.df[2];
-                            rinv[p] = g.rinv;
-                            fc[p] = g.fc;
-                            fcd[p] = g.fcd;
-                            fl = g.flags;
+                            const float4* g = reinterpret_cast<const float4*>(pcd + e[p < 3 ? p : 0]);
+                            const float4 u = g[2], v = g[3];
+                            dr[p][0] = u.x; dr[p][1] = u.y; dr[p][2] = u.z;
+                            rinv[p] = u.w;
+                            fc[p] = v.x;
+                            fcd[p] = v.y;
+                            fl = __float_as_int(v.z);
                         } else {
                             const int t = p < P0 ? 0 : p - P0;
                             dr[p][0] = ep.dr[t][0][c]; dr[p][1] = ep.dr[t][1][c]; dr[p][2] = ep.dr[t][2][c];
