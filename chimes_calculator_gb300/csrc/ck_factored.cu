@@ -29,6 +29,7 @@
 #include "ck_common.h"
 #include "ck_force_common.cuh"
 #include "ck_kernels.h"
+#include "ck_launch.cuh"
 #include "ck_math.cuh"
 
 namespace ck {
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(256) k_bucket_count(BatchView B, int first) {
 // start[nbk] and the padding slots of every bucket are set to -1.  One block
 // per body order.
 __global__ void __launch_bounds__(1024) k_bucket_scan(BatchView B, int first) {
+    chain_begin();
     const int nb = blockIdx.x == 0 ? first : 7 - first;
     const int nbk = nb == 3 ? B.nbk3 : B.nbk4;
     const int* count = B.bk_count + (nb == 3 ? 0 : B.nbk3);
@@ -299,6 +301,7 @@ __device__ void bucket_scatter(const BatchView& B, int chunk, int* s_cnt, long l
     }
 }
 __global__ void __launch_bounds__(256) k_bucket_scatter(BatchView B, int first, int chunk) {
+    chain_begin();
     __shared__ int s_cnt[kBkSmem];
     __shared__ long long s_pos[kBkSmem];
     if ((blockIdx.y == 0 ? first : 7 - first) == 3) bucket_scatter<3>(B, chunk, s_cnt, s_pos);
@@ -726,12 +729,12 @@ void launch_bucket(const BatchView& B, bool three, bool four, cudaStream_t st) {
         const dim3 grid((unsigned)std::min((long long)sm_count() * 8, (cap + 255) / 256), rows);
         count_launch(), k_bucket_count<<<grid, 256, 0, st>>>(B, first);
     }
-    count_launch(), k_bucket_scan<<<rows, 1024, 0, st>>>(B, first);
+    count_launch(), launch_chained(k_bucket_scan, rows, 1024, 0, st, B, first);
     const long long items = B.keyed ? B.n_atoms_total : (cap + 31) / 32;
     // 64 atoms a block, fewer (down to one a warp) while that leaves SMs without a block
     const int chunk = (int)std::max(8LL, std::min(64LL, items / (2 * sm_count())));
     const dim3 grid((unsigned)std::min((long long)sm_count() * 8, (items + chunk - 1) / chunk), rows);
-    count_launch(), k_bucket_scatter<<<grid, 256, 0, st>>>(B, first, chunk);
+    count_launch(), launch_chained(k_bucket_scatter, grid, 256, 0, st, B, first, chunk);
 }
 
 void launch_force3f(const BatchView& B, const ForceLaunch& L, cudaStream_t st) {

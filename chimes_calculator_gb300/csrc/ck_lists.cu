@@ -30,6 +30,7 @@
 
 #include "ck_common.h"
 #include "ck_kernels.h"
+#include "ck_launch.cuh"
 
 namespace ck {
 
@@ -135,6 +136,7 @@ __device__ __forceinline__ void bin_setup(const BatchView& B, int s, SysDesc& d)
 // of all ghost images (build_neigh_lists :590-610) comes from each atom, its
 // two corner images per axis, reduced per system.
 __global__ void k_atoms(BatchView B) {
+    chain_begin();
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = r < B.n_atoms_total;
     int s = -1;
@@ -242,6 +244,7 @@ __device__ __forceinline__ int bin_axis(double x, double mn, double search, floa
     return (int)floor(__ddiv_rn(sub(x, mn), search));
 }
 __global__ void k_ghosts(BatchView B) {
+    chain_begin();
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= B.n_ghost_total) return;
     const int s = find_sys_ghost(B.sys, B.n_sys, q);
@@ -305,6 +308,7 @@ __global__ void k_ghosts(BatchView B) {
 // Room for every bin's members in bin_items: which bin comes first does not
 // matter, so a block scans its bins and reserves their sum.
 __global__ void __launch_bounds__(1024) k_bin_alloc(BatchView B) {
+    chain_begin();
     __shared__ int wsum[32];
     __shared__ long long base;
     const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -331,6 +335,7 @@ __global__ void __launch_bounds__(1024) k_bin_alloc(BatchView B) {
 }
 
 __global__ void k_bin_scatter(BatchView B, const long long* bin_start) {
+    chain_begin();
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= B.n_ghost_total) return;
     const int ib = B.ghost_bin[q];
@@ -410,6 +415,7 @@ __device__ __forceinline__ void rank_bin(const BatchView& B, long long s0, int n
 }
 
 __global__ void __launch_bounds__(256) k_bin_rank(BatchView B, const long long* bin_start, int per) {
+    chain_begin();
     __shared__ int s_key[8][kRankSmem], s_val[8][kRankSmem];
     const long long b0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -487,6 +493,7 @@ __device__ __forceinline__ void put_l2(const BatchView& B, int* l2_owner, long l
 }
 
 __global__ void __launch_bounds__(kL2Block) k_l2(BatchView B, int* l2_owner) {
+    chain_begin();
     constexpr int NWARP = kL2Block / 32;
     __shared__ L2Hold hold[NWARP];
     __shared__ int s_cnt[NWARP];
@@ -984,6 +991,7 @@ __device__ __forceinline__ void count_key(const BatchView& B, int* hist, int at,
 
 template <int G>
 __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B, const int* l2_owner) {
+    chain_begin();
     constexpr int NG = kEnumWarps / G;   // atoms a block works on at a time
     __shared__ float4 s_v[NG][kEnumRows];
     __shared__ int s_g[NG][kEnumRows];
@@ -1279,11 +1287,12 @@ void launch_enuma(const BatchView& B, const int* l2_owner, cudaStream_t st) {
     const unsigned grid = (unsigned)(want < need ? want : need);
     const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
     const size_t smem = nbk <= kBkSmem ? sizeof(int) * (size_t)nbk : 0;
-    count_launch(), k_enuma<G><<<grid, 32 * kEnumWarps, smem, st>>>(B, l2_owner);
+    count_launch(), launch_chained(k_enuma<G>, grid, 32 * kEnumWarps, smem, st, B, l2_owner);
 }
 
 // --- reset of accumulators, counters and bins -------------------------------
 __global__ void k_reset(BatchView B) {
+    chain_begin();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = t; i < B.n_bins_total; i += stride) {
@@ -1477,16 +1486,16 @@ void exclusive_scan2(const int* in_a, long long* out_a, const int* in_b, long lo
 
 void launch_atoms(const BatchView& B, cudaStream_t st) {
     // small blocks: the per-atom cell algebra is FP64 work, spread over as many SMs as possible
-    if (B.n_atoms_total) count_launch(), k_atoms<<<grid_for(B.n_atoms_total, 32), 32, 0, st>>>(B);
+    if (B.n_atoms_total) count_launch(), launch_chained(k_atoms, grid_for(B.n_atoms_total, 32), 32, 0, st, B);
 }
 void launch_ghosts(const BatchView& B, cudaStream_t st) {
-    if (B.n_ghost_total) count_launch(), k_ghosts<<<grid_for(B.n_ghost_total, 64), 64, 0, st>>>(B);
+    if (B.n_ghost_total) count_launch(), launch_chained(k_ghosts, grid_for(B.n_ghost_total, 64), 64, 0, st, B);
 }
 void launch_bin_alloc(const BatchView& B, cudaStream_t st) {
-    if (B.n_bins_total) count_launch(), k_bin_alloc<<<grid_for(B.n_bins_total, 1024), 1024, 0, st>>>(B);
+    if (B.n_bins_total) count_launch(), launch_chained(k_bin_alloc, grid_for(B.n_bins_total, 1024), 1024, 0, st, B);
 }
 void launch_bin_scatter(const BatchView& B, cudaStream_t st) {
-    if (B.n_ghost_total) count_launch(), k_bin_scatter<<<grid_for(B.n_ghost_total, 256), 256, 0, st>>>(B, B.bin_start);
+    if (B.n_ghost_total) count_launch(), launch_chained(k_bin_scatter, grid_for(B.n_ghost_total, 256), 256, 0, st, B, B.bin_start);
 }
 void launch_bin_sort(const BatchView& B, cudaStream_t st) {
     if (!B.n_bins_total) return;
@@ -1495,11 +1504,11 @@ void launch_bin_sort(const BatchView& B, cudaStream_t st) {
     // batch reserves many times the bins its ghost clouds occupy)
     const int per = B.n_bins_total > 64LL * 32 * sm_count() ? 32 : 1;
     const long long warps = (B.n_bins_total + per - 1) / per;
-    count_launch(), k_bin_rank<<<grid_for(warps * 32, 256), 256, 0, st>>>(B, B.bin_start, per);
+    count_launch(), launch_chained(k_bin_rank, grid_for(warps * 32, 256), 256, 0, st, B, B.bin_start, per);
 }
 void launch_l2(const BatchView& B, int* l2_owner, cudaStream_t st) {
     if (B.n_atoms_total)
-        count_launch(), k_l2<<<grid_for(B.n_atoms_total * 32, kL2Block), kL2Block, 0, st>>>(B, l2_owner);
+        count_launch(), launch_chained(k_l2, grid_for(B.n_atoms_total * 32, kL2Block), kL2Block, 0, st, B, l2_owner);
 }
 void launch_enum(const BatchView& B, const int* l2_owner, void* scan_tmp, cudaStream_t st) {
     if (!B.n2_cap) return;
