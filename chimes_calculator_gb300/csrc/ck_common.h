@@ -306,6 +306,7 @@ struct SysDesc {
     int err;
     int done;                  // atoms whose bounding box has been taken in
 };
+static_assert(sizeof(SysDesc) % 8 == 0, "positions follow the descriptors in one block");
 
 // Flat views of a batch workspace (all device pointers).
 struct BatchView {

@@ -75,10 +75,7 @@ Status Engine::init_device(std::string& err) {
     CK_TRY(cudaEventCreateWithFlags(&fork2_, cudaEventDisableTiming));
     CK_TRY(cudaEventCreateWithFlags(&pairs_, cudaEventDisableTiming));
     CK_TRY(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
-    CK_TRY(h_flags_.reserve(8));
-    CK_TRY(h_counts_.reserve(4));
-    CK_TRY(d_flags_.reserve(8));
-    CK_TRY(d_queue_.reserve(6));
+    CK_TRY(d_queue_.reserve(2));
     ready_ = true;
     return kOk;
 }
@@ -281,9 +278,13 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     n3_cap_ = std::max(n3_cap_, (long long)n3_est + 1024);
     n4_cap_ = std::max(n4_cap_, (long long)n4_est + 1024);
 
-    CK_TRY(d_sys_.reserve(S));
-    CK_TRY(d_in_pos_.reserve(3 * in_off));
-    CK_TRY(d_in_type_.reserve(in_off));
+    // one block each for what goes to the device and what comes back, so that a call
+    // makes one copy each way (three, one of them from pageable memory, and four before)
+    const size_t sys_bytes = sizeof(SysDesc) * (size_t)S, in_bytes = sys_bytes + (sizeof(double) * 3 + sizeof(int)) * in_off;
+    CK_TRY(d_in_.reserve(in_bytes));
+    CK_TRY(h_in_.reserve(in_bytes));
+    CK_TRY(d_out_.reserve(out_values()));
+    CK_TRY(h_out_.reserve(out_values()));
     CK_TRY(d_atom_sys_.reserve(atom_off));
     CK_TRY(d_atom_type_.reserve(atom_off));
     CK_TRY(d_atom_orig_.reserve(atom_off));
@@ -304,23 +305,18 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     CK_TRY(d_l2_off_.reserve(atom_off));
     CK_TRY(d_a_off_.reserve(2 * atom_off));
     CK_TRY(d_a_cnt_.reserve(2 * atom_off));
-    CK_TRY(d_force_.reserve(3 * in_off));
-    CK_TRY(d_ev_.reserve(8 * S));
-    CK_TRY(h_in_pos_.reserve(3 * in_off));
-    CK_TRY(h_in_type_.reserve(in_off));
-    CK_TRY(h_force_.reserve(3 * in_off));
-    CK_TRY(h_ev_.reserve(8 * S));
     st = ensure_lists(err);
     if (st != kOk) return st;
 
+    double* pos = reinterpret_cast<double*>(h_in_.p + sys_bytes);
+    int* types = reinterpret_cast<int*>(pos + 3 * in_off);
+    std::memcpy(h_in_.p, hsys_.data(), sys_bytes);
     for (int s = 0; s < S; s++) {
         const SystemSpec& in = sys[s];
-        std::memcpy(h_in_pos_.p + 3 * hsys_[s].in_off, in.pos, sizeof(double) * 3 * in.n);
-        std::memcpy(h_in_type_.p + hsys_[s].in_off, in.types, sizeof(int) * in.n);
+        std::memcpy(pos + 3 * hsys_[s].in_off, in.pos, sizeof(double) * 3 * in.n);
+        std::memcpy(types + hsys_[s].in_off, in.types, sizeof(int) * in.n);
     }
-    CK_TRY(cudaMemcpyAsync(d_sys_.p, hsys_.data(), sizeof(SysDesc) * S, cudaMemcpyHostToDevice, stream_));
-    CK_TRY(cudaMemcpyAsync(d_in_pos_.p, h_in_pos_.p, sizeof(double) * 3 * in_off, cudaMemcpyHostToDevice, stream_));
-    CK_TRY(cudaMemcpyAsync(d_in_type_.p, h_in_type_.p, sizeof(int) * in_off, cudaMemcpyHostToDevice, stream_));
+    CK_TRY(cudaMemcpyAsync(d_in_.p, h_in_.p, in_bytes, cudaMemcpyHostToDevice, stream_));
     staged_ = true;
     return kOk;
 }
@@ -376,10 +372,10 @@ Status Engine::ensure_lists(std::string& err) {
     }
     if (enum_serial_) CK_TRY(d_scan_tmp_.reserve(scan_tmp_bytes(n2_cap_)));
     BatchView& B = V_;
-    B.sys = d_sys_.p;
+    B.sys = reinterpret_cast<SysDesc*>(d_in_.p);
     B.psets = dsets_.p;
-    B.in_pos = d_in_pos_.p;
-    B.in_type = d_in_type_.p;
+    B.in_pos = reinterpret_cast<double*>(d_in_.p + sizeof(SysDesc) * (size_t)V_.n_sys);
+    B.in_type = reinterpret_cast<const int*>(B.in_pos + 3 * V_.n_in_total);
     B.atom_sys = d_atom_sys_.p; B.atom_type = d_atom_type_.p; B.atom_orig = d_atom_orig_.p;
     B.atom_self = d_atom_self_.p;
     B.ghost_id = d_ghost_id_.p;
@@ -398,9 +394,12 @@ Status Engine::ensure_lists(std::string& err) {
     B.a_off = d_a_off_.p; B.a_cnt = d_a_cnt_.p;
     B.c3 = d_c3_.p; B.c4 = d_c4_.p;
     B.n3_cap = n3_cap_; B.n4_cap = n4_cap_;
-    B.force = d_force_.p; B.ev = d_ev_.p; B.flags = d_flags_.p; B.queue = d_queue_.p;
+    B.force = d_out_.p;
+    B.ev = B.force + 3 * V_.n_in_total;
+    B.queue = d_queue_.p;
     B.enum_serial = enum_serial_ ? 1 : 0;
-    B.totals = reinterpret_cast<long long*>(d_queue_.p + 2);
+    B.totals = reinterpret_cast<long long*>(B.ev + 8 * V_.n_sys);
+    B.flags = reinterpret_cast<int*>(B.totals + 4);
     B.n3_ptr = enum_serial_ ? B.e_off3 + B.n2_cap : B.totals + 1;
     B.n4_ptr = enum_serial_ ? B.e_off4 + B.n2_cap : B.totals + 2;
     B.c3e = avail_pc3_ || (avail_ent_ && tuning.rf3 > 0) ? d_c3e_.p : nullptr;
@@ -544,13 +543,10 @@ Status Engine::enqueue(std::string& err) {
     if (profile) CK_TRY(record_stage_event(ev_[4], st));
     ev_recorded_ = profile;
     kernels_per_launch = (int)(launch_counter() - k0);
-    CK_TRY(cudaMemcpyAsync(h_force_.p, B.force, sizeof(double) * 3 * B.n_in_total, cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_ev_.p, B.ev, sizeof(double) * 8 * B.n_sys, cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_flags_.p, B.flags, sizeof(int) * 8, cudaMemcpyDeviceToHost, st));
-    CK_TRY(cudaMemcpyAsync(h_counts_.p, B.totals, sizeof(long long) * 3, cudaMemcpyDeviceToHost, st));
+    CK_TRY(cudaMemcpyAsync(h_out_.p, B.force, sizeof(double) * out_values(), cudaMemcpyDeviceToHost, st));
     if (B.enum_serial) {
-        CK_TRY(cudaMemcpyAsync(h_counts_.p + 1, B.n3_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
-        CK_TRY(cudaMemcpyAsync(h_counts_.p + 2, B.n4_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
+        CK_TRY(cudaMemcpyAsync(h_totals() + 1, B.n3_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
+        CK_TRY(cudaMemcpyAsync(h_totals() + 2, B.n4_ptr, sizeof(long long), cudaMemcpyDeviceToHost, st));
     }
     CK_TRY(cudaGetLastError());
     return kOk;
@@ -583,7 +579,7 @@ Status Engine::launch(std::string& err) {
     for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
                           (const void*)V_.bin_items, (const void*)V_.l2_ghost, (const void*)V_.c3,
                           (const void*)V_.c4, (const void*)V_.force, (const void*)d_scan_tmp_.p,
-                          (const void*)h_force_.p, (const void*)h_ev_.p, (const void*)V_.bin_count,
+                          (const void*)h_out_.p, (const void*)V_.queue, (const void*)V_.bin_count,
                           (const void*)V_.e_off3, (const void*)V_.psets, (const void*)V_.perm3,
                           (const void*)V_.perm4, (const void*)V_.bk_count, (const void*)V_.bk_fill,
                           (const void*)V_.bk_start, (const void*)V_.c3e, (const void*)V_.c4e,
@@ -618,8 +614,8 @@ Status Engine::launch(std::string& err) {
 
 Status Engine::collect(double* force_out, std::vector<SystemResult>& res, std::string& err) {
     CK_TRY(cudaStreamSynchronize(stream_));
-    const int* f = h_flags_.p;
-    const long long* c = h_counts_.p;
+    const long long* c = h_totals();
+    const int* f = reinterpret_cast<const int*>(c + 4);
     last.n2 = c[0]; last.n3 = c[1]; last.n4 = c[2];
     last.n_atoms = V_.n_atoms_total;
     last.n_ghost = V_.n_ghost_total;
@@ -655,14 +651,14 @@ Status Engine::collect(double* force_out, std::vector<SystemResult>& res, std::s
     last.below_rin = f[4];
     res.assign(V_.n_sys, SystemResult());
     for (int s = 0; s < V_.n_sys; s++) {
-        const double* ev = h_ev_.p + 8 * s;
+        const double* ev = h_out_.p + 3 * V_.n_in_total + 8 * s;
         SystemResult& r = res[s];
         r.n_rep = hsys_[s].n_rep;
         r.energy = ev[0] / std::pow(hsys_[s].n_rep + 1.0, 3.0);
         for (int k = 0; k < 6; k++) r.virial[k] = ev[1 + k];
         r.vol = vols_[s];
     }
-    if (force_out) std::memcpy(force_out, h_force_.p, sizeof(double) * 3 * V_.n_in_total);
+    if (force_out) std::memcpy(force_out, h_out_.p, sizeof(double) * 3 * V_.n_in_total);
     return kOk;
 }
 

@@ -179,9 +179,7 @@ private:
     long long l2_slots_ = 0;
     bool staged_ = false;
 
-    DevBuf<SysDesc> d_sys_;
-    DevBuf<double> d_in_pos_;
-    DevBuf<int> d_in_type_;
+    DevBuf<unsigned char> d_in_;      // SysDesc[n_sys], positions, types
     DevBuf<int> d_atom_sys_, d_atom_type_, d_atom_orig_;
     DevBuf<int> d_atom_self_, d_ghost_id_;
     DevBuf<float> d_ghost_xf_, d_l2_vec_, d_bin_xp_;
@@ -212,20 +210,17 @@ private:
     DevBuf<unsigned char> d_pct3_, d_pct4_;
     DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_;
     DevBuf<long long> d_bk_start_;
-    DevBuf<double> d_force_, d_ev_;
-    DevBuf<int> d_flags_;
+    DevBuf<double> d_out_;            // forces, energies and virials, totals (4), flags (8 ints)
     DevBuf<unsigned long long> d_queue_;
     DevBuf<unsigned char> d_scan_tmp_;
     DevBuf<unsigned char> d_ws_;
     DevBuf<double> d_dir_d_;      // per-cluster inputs and outputs (doubles)
     DevBuf<int> d_dir_i_;         // per-cluster types and status
 
-    PinnedBuf<double> h_in_pos_;
-    PinnedBuf<int> h_in_type_;
-    PinnedBuf<double> h_force_;
-    PinnedBuf<double> h_ev_;
-    PinnedBuf<int> h_flags_;
-    PinnedBuf<long long> h_counts_;
+    PinnedBuf<unsigned char> h_in_;   // as d_in_
+    PinnedBuf<double> h_out_;         // as d_out_
+    size_t out_values() const { return 3 * (size_t)V_.n_in_total + 8 * (size_t)V_.n_sys + 4 + 4; }
+    long long* h_totals() { return reinterpret_cast<long long*>(h_out_.p + 3 * V_.n_in_total + 8 * V_.n_sys); }
 
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;

@@ -88,9 +88,10 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
     NL_TRY(d_atom_orig_.reserve(nall));
     NL_TRY(d_parent_.reserve(nall));
     NL_TRY(d_tag_.reserve(nall));
-    NL_TRY(d_force_.reserve(3 * (long long)nall));
-    NL_TRY(d_ev_.reserve(8));
-    NL_TRY(d_flags_.reserve(8));
+    // forces, energy and virial (8), flags (8 ints): one block, one copy back
+    const size_t out_values = 3 * (size_t)nall + 8 + 4;
+    NL_TRY(d_out_.reserve(out_values));
+    NL_TRY(h_out_.reserve(out_values));
     NL_TRY(d_queue_.reserve(2));
     NL_TRY(d_minmax_.reserve(6));
     NL_TRY(d_sys_.reserve(1));
@@ -145,7 +146,10 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
     B.minmax = d_minmax_.p;
     B.n2_cap = nent;
     B.e_cnt3 = d_e_cnt3_.p; B.e_cnt4 = d_e_cnt4_.p; B.e_off3 = d_e_off3_.p; B.e_off4 = d_e_off4_.p;
-    B.force = d_force_.p; B.ev = d_ev_.p; B.flags = d_flags_.p; B.queue = d_queue_.p;
+    B.force = d_out_.p;
+    B.ev = B.force + 3 * (size_t)nall;
+    B.flags = reinterpret_cast<int*>(B.ev + 8);
+    B.queue = d_queue_.p;
     B.enum_serial = 0;
     B.n3_ptr = B.e_off3 + nent; B.n4_ptr = B.e_off4 + nent;
     NeighView& N = N_;
@@ -265,12 +269,7 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
         else launch_force4(B, L, s);
     }
     NL_TRY(cudaGetLastError());
-    h_force_.resize(3 * (size_t)nall);
-    double ev[8];
-    int flags[8];
-    NL_TRY(cudaMemcpyAsync(h_force_.data(), d_force_.p, sizeof(double) * 3 * nall, cudaMemcpyDeviceToHost, s));
-    NL_TRY(cudaMemcpyAsync(ev, d_ev_.p, sizeof(double) * 8, cudaMemcpyDeviceToHost, s));
-    NL_TRY(cudaMemcpyAsync(flags, d_flags_.p, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+    NL_TRY(cudaMemcpyAsync(h_out_.p, d_out_.p, sizeof(double) * out_values, cudaMemcpyDeviceToHost, s));
     if (eatom) {
         h_eatom_.resize(nall);
         NL_TRY(cudaMemcpyAsync(h_eatom_.data(), d_eatom_.p, sizeof(double) * nall, cudaMemcpyDeviceToHost, s));
@@ -280,6 +279,8 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
         NL_TRY(cudaMemcpyAsync(h_vatom_.data(), d_vatom_.p, sizeof(double) * 6 * nall, cudaMemcpyDeviceToHost, s));
     }
     NL_TRY(cudaStreamSynchronize(s));
+    const double* ev = h_out_.p + 3 * (size_t)nall;
+    const int* flags = reinterpret_cast<const int*>(ev + 8);
     badness_ = flags[2];
     if (flags[5] & 1) {   // get_tab_2B prints and exits here
         err = "Distance is outside the tabulated range (a 2-body distance at or below the table's first usable "
@@ -290,7 +291,7 @@ Status NeighCompute::compute(int slot, int nall, const double* x, const int* typ
         err = "a 3-body distance lies past the tabulated grid (the table does not cover the 3-body cutoffs)";
         return kErrGeometry;
     }
-    for (size_t k = 0; k < h_force_.size(); k++) f[k] += h_force_[k];
+    for (size_t k = 0; k < 3 * (size_t)nall; k++) f[k] += h_out_.p[k];
     if (eatom)
         for (int a = 0; a < nall; a++) eatom[a] += h_eatom_[a];
     if (vatom)

@@ -48,12 +48,12 @@ private:
     BatchView B_{};
     NeighView N_{};
     DevBuf<SysDesc> d_sys_;
-    DevBuf<double> d_x_, d_force_, d_ev_, d_eatom_, d_vatom_;
+    DevBuf<double> d_x_, d_out_, d_eatom_, d_vatom_;
     DevBuf<int> d_type_, d_atom_sys_, d_atom_orig_, d_parent_, d_ilist_, d_neigh_, d_owner_;
     DevBuf<long long> d_tag_, d_off_;
     DevBuf<int> d_e_cnt3_, d_e_cnt4_, d_c3_, d_c4_;
     DevBuf<long long> d_e_off3_, d_e_off4_;
-    DevBuf<int> d_flags_, d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_, d_bk_key3_, d_bk_key4_;
+    DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_, d_bk_key3_, d_bk_key4_;
     DevBuf<long long> d_bk_start_;
     DevBuf<unsigned long long> d_queue_, d_minmax_;
     DevBuf<unsigned char> d_scan_tmp_, d_fp_tmp_;
@@ -63,7 +63,8 @@ private:
     DevBuf<float> d_xf_;
     DevBuf<int> d_tsel_;
     DevBuf<unsigned long long> d_tcount_;
-    std::vector<double> h_force_, h_eatom_, h_vatom_;
+    PinnedBuf<double> h_out_;
+    std::vector<double> h_eatom_, h_vatom_;
 };
 
 }  // namespace ck
