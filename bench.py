@@ -124,11 +124,10 @@ class ClockSampler:
 # algorithmic work of one evaluation (flop model of the force kernels)
 # ----------------------------------------------------------------------------
 # DRAM bytes (read + write) per launch of the force kernels on this workload,
-# from one ncu capture each (profiles/k_forcef_c2_fp64.md, k_forcen_c2_fp64.md)
+# from one ncu capture each (profiles/kernels_c2_fp64.md, k_forcen_c2_fp64.md)
 PROFILED_TRAFFIC = {
-    "k_forcef<3,double,1>": 4272384,
-    "k_forcef<3,double,1,true>": 4273408,
-    "k_forcef<4,double,4>": 2047488,
+    "k_forcex3": None,
+    "k_forcex4": None,
     "k_forcen<3,double,4>": 872704,
     "k_forcen<4,double,8>": 599552,
 }
@@ -173,7 +172,7 @@ def algorithmic_flops(calc, cfg, params_path):
     out = {}
     for nb, lst, order in ((3, l3, o3), (4, l4, o4)):
         if lst.shape[0] == 0 or order == 0:
-            out[nb] = (0, 0.0, 0.0, 0.0)
+            out[nb] = (0, 0.0, 0.0)
             continue
         P = nb * (nb - 1) // 2
         pairs = [(i, j) for i in range(nb) for j in range(i + 1, nb)]
@@ -202,9 +201,7 @@ def algorithmic_flops(calc, cfg, params_path):
         ex = ok.sum() * (P * (6 * order + 15) + P * 21 + R ** C * (C - 1) + R ** K * (K - 1)) \
             + (4.0 * nc).sum() + (per_row * nrow[u][ok].astype(np.float64)).sum() \
             + (per_col * ncol[u][ok].astype(np.float64)).sum()
-        # without the Y table (3-body): one more multiply per row entry, no table
-        ex_noy = ex + nc.sum() - ok.sum() * (R ** C * (C - 1)) if nb == 3 else ex
-        out[nb] = (int(ok.sum()), float(flops), float(ex), float(ex_noy))
+        out[nb] = (int(ok.sum()), float(flops), float(ex))
     return out
 
 
@@ -325,7 +322,7 @@ def run_ours(args):
     peak64.value = statistics.median(probes)
     probe_s = time.perf_counter() - t_probe
     probe_clocks = probe_clk.stop()
-    # the dominant single kernel: the list build is ~15 short kernels, each
+    # the dominant single kernel: the list build is ten short kernels, each
     # force stage is one kernel, so the longest force stage is the top kernel
     dom = 1 + int(np.argmax(stage[1:]))
     roof = None
@@ -333,26 +330,12 @@ def run_ours(args):
     if dom in (2, 3):
         nb = 3 if dom == 2 else 4
         fact = tun["fact%d" % nb]
-        tpc = tun[("ftpc%d" if fact else "tpc%d") % nb]
-        noy = fact and nb == 3 and tun.get("noy3", 0)
-        kname = ("k_forcef<%d,double,%d>" if fact else "k_forcen<%d,double,%d>") % (nb, tpc)
-        if noy:
-            kname = kname[:-1] + ",true>"
-            work[nb] = (work[nb][0], work[nb][1], work[nb][3])
-        # DRAM traffic of the kernel's ncu capture on this workload; a launch
-        # shape without its own capture (lanes per cluster) reads the same
-        # pair tables, coefficient lists and cluster lists as the captured
-        # shape of the same contraction form (4.27 MB for the 3-body table and
-        # no-table forms alike)
+        # the factored form runs in 64-bit fixed point on the integer pipe; its rate is
+        # put against the FP64 one, whose work it replaces
+        kname = "k_forcex%d" % nb if fact else "k_forcen<%d,double,%d>" % (nb, tun["tpc%d" % nb])
         traffic, traffic_src = PROFILED_TRAFFIC.get(kname), None
         if traffic is not None:
             traffic_src = "ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel on this workload (profiles/)"
-        else:
-            same = [v for k, v in PROFILED_TRAFFIC.items() if k.startswith("k_forcef<%d,double," % nb)] if fact else []
-            if same:
-                traffic = same[0]
-                traffic_src = ("ncu capture of the same factored %d-body kernel at another launch shape on this "
-                               "workload (profiles/)" % nb)
         achieved = work[nb][1] / (stage[dom] * 1e-3) / 1e12
         executed = (work[nb][2] if fact else work[nb][1]) / (stage[dom] * 1e-3) / 1e12
         roof = {"bound": "fp64", "kernel": kname, "achieved": achieved,

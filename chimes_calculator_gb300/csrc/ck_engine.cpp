@@ -784,7 +784,14 @@ Status Engine::autotune(int* chosen, std::string& err) {
         for (int t : {1, 2, 4, 8, 16, 32}) v.push_back({0, t, 0, 0, 0});
         return v;
     };
-    const std::vector<Cand> c3 = cands(avail_fact3_, true, avail_tc3_), c4 = cands(avail_fact4_, false, avail_tc4_);
+    // The forms differ in FP32 rounding (1e-7 of the forces), so a workload should not
+    // change form for a few microseconds: the 3-body tensor-core form is tried
+    // from one tile per SM on (one configuration) or six (a batch, whose tiles mix
+    // configurations), about where it began to win before it was made faster
+    // (17-34 k triplets of one configuration and 120 k of a batch; now 54 k triplets
+    // of 11 configurations 38 us against 98, 17 k of one 22 against 57).
+    const bool try_tc3 = avail_tc3_ && last.n3 >= 128LL * sm_count() * (V_.n_sys == 1 ? 1 : 6);
+    const std::vector<Cand> c3 = cands(avail_fact3_, true, try_tc3), c4 = cands(avail_fact4_, false, avail_tc4_);
     auto apply = [&](int nb, const Cand& c) {
         if (nb == 3) {
             tuning.fact3 = c.fact;

@@ -127,9 +127,9 @@ __device__ __forceinline__ void put_pair_f(const DevParamSet& P, const PairTab& 
 // Bound by the FP64 pipe (68%: geometry, the maps, forces; polynomial sums,
 // exponential, sines, conversions and comparisons are integer arithmetic).  Measured:
 // 5.23 M entries mixed 1.19 ms with the tables of both body orders (1.37 with FP64
-// conversions and comparisons) and 0.40 ms for their forces, against
-// 1.84 ms for a 2-body kernel and 0.59 ms for a pass over the 3-body tables alone.  rs3, rs4: stride of the tables of
-// a body order, 0 for none.  (Entries one by one: with an atom's entries spread
+// conversions and comparisons) and 0.40 ms for their forces, against 1.84 ms for
+// a 2-body kernel and 0.59 ms for a pass over the 3-body tables alone.  rs3, rs4:
+// stride of the tables of a body order, 0 for none.  (Entries one by one: with an atom's entries spread
 // over eight lanes instead, 384 configurations took 941 us and not 456, the
 // lanes' rounds being one long dependent chain each.)
 template <bool MIXED>

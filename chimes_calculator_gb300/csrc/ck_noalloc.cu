@@ -8,7 +8,7 @@
 // inputs and outputs, and every intermediate array of the evaluation -- ghost
 // images, bin grid, neighbour and cluster lists, scan workspace, accumulators
 // -- lives in one file-scope device array of fixed size (kScratchBytes, about
-// 13.4 MiB), which every GPU that loads the library holds until the process
+// 11.9 MiB), which every GPU that loads the library holds until the process
 // exits.  The list-build and force kernels are the allocating path's own, in
 // one fixed launch shape: the thread-per-entry cluster enumeration and the
 // per-coefficient contraction (k_forcen) with the handle's tuning, never the

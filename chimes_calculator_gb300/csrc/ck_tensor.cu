@@ -47,7 +47,8 @@
 // operand buffer and 128 TMEM columns each, 128 registers a thread, tables read
 // when they are needed rather than held.  Measured: 1.47 M triplets of 32768
 // atoms 556 -> 338 us, 9.15 M of 2000 configurations 3.30 -> 1.95 ms (320 us and
-// 1.82 ms with conversions and comparisons off the FP64 pipe), against two CTAs that hold both rows, both accumulators and all tables at once.
+// 1.82 ms with conversions and comparisons off the FP64 pipe), against two CTAs
+// that hold both rows, both accumulators and all tables at once.
 // A wait that runs out sets flags[7] and the CTA stops after freeing its TMEM.
 #include <cuda_runtime.h>
 
