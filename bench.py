@@ -126,8 +126,8 @@ class ClockSampler:
 # DRAM bytes (read + write) per launch of the force kernels on this workload,
 # from one ncu capture each (profiles/kernels_c2_fp64.md, k_forcen_c2_fp64.md)
 PROFILED_TRAFFIC = {
-    "k_forcex3": None,
-    "k_forcex4": None,
+    "k_forcex3": 4477440,
+    "k_forcex4": 2490112,
     "k_forcen<3,double,4>": 872704,
     "k_forcen<4,double,8>": 599552,
 }

@@ -785,13 +785,14 @@ Status Engine::autotune(int* chosen, std::string& err) {
         return v;
     };
     // The forms differ in FP32 rounding (1e-7 of the forces), so a workload should not
-    // change form for a few microseconds: the 3-body tensor-core form is tried
-    // from one tile per SM on (one configuration) or six (a batch, whose tiles mix
-    // configurations), about where it began to win before it was made faster
-    // (17-34 k triplets of one configuration and 120 k of a batch; now 54 k triplets
-    // of 11 configurations 38 us against 98, 17 k of one 22 against 57).
-    const bool try_tc3 = avail_tc3_ && last.n3 >= 128LL * sm_count() * (V_.n_sys == 1 ? 1 : 6);
-    const std::vector<Cand> c3 = cands(avail_fact3_, true, try_tc3), c4 = cands(avail_fact4_, false, avail_tc4_);
+    // change form for a few microseconds: where the set has a 3-body tensor-core form,
+    // that is taken against the per-coefficient one from one tile per SM on (one
+    // configuration), seven (a batch) or three (a batch of 50 or more small ones) --
+    // about where it began to win before it was made faster: 17-34 k triplets of one
+    // configuration, 67 k of 105, 130 k of 40 (now 54 k of 11 take 38 us against 98).
+    const int tiles_per_sm = V_.n_sys == 1 ? 1 : V_.n_sys >= 50 ? 3 : 7;
+    const bool small3 = avail_tc3_ && last.n3 < 128LL * sm_count() * tiles_per_sm;
+    const std::vector<Cand> c3 = cands(avail_fact3_, true, avail_tc3_), c4 = cands(avail_fact4_, false, avail_tc4_);
     auto apply = [&](int nb, const Cand& c) {
         if (nb == 3) {
             tuning.fact3 = c.fact;
@@ -821,7 +822,7 @@ Status Engine::autotune(int* chosen, std::string& err) {
             m3 = std::min(m3, a);
             m4 = std::min(m4, b);
         }
-        if (need3 && m3 < best3) { best3 = m3; b3 = c3[i]; }
+        if (need3 && !(small3 && c3[i].fact) && m3 < best3) { best3 = m3; b3 = c3[i]; }
         if (need4 && m4 < best4) { best4 = m4; b4 = c4[i]; }
     }
     apply(3, b3);
