@@ -69,6 +69,7 @@ SIGNATURES = {
     "ck_set_tuning": (I, [P, I, I, I]),
     "ck_set_contraction": (I, [P, I]),
     "ck_use_graph": (I, [P, I]),
+    "ck_graph_captures": (ctypes.c_longlong, [P]),
     "ck_autotune_repeats": (I, [P, I]),
     "ck_autotune": (I, [P, IP]),
     "ck_calculate_batch": (I, [P, I, IP, DP, IP, DP, IP, IP, DP, DP, DP]),

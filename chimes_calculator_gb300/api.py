@@ -236,6 +236,10 @@ class Calculator:
     def use_graph(self, on: bool):
         self._check(self.lib.ck_use_graph(self.h, 1 if on else 0))
 
+    def graph_captures(self) -> int:
+        """CUDA graphs captured so far (a repeated call that replays one adds none)."""
+        return self._check(self.lib.ck_graph_captures(self.h))
+
     # -- packing -------------------------------------------------------------
     def pack(self, configs, slots=None, small=None):
         """configs: sequence of (pos[N,3], types (names or indices), cell[3,3])."""

@@ -421,6 +421,11 @@ int ck_use_graph(void* h, int on) {
     return ck::kOk;
 }
 
+long long ck_graph_captures(void* h) {
+    if (int st = check_handle(h)) return st;
+    return static_cast<Instance*>(h)->eng.captures();
+}
+
 static int build_specs(Instance* in, int nsys, const int* natoms, const double* pos, const int* types,
                        const double* cells, const int* small, const int* pset, std::vector<ck::SystemSpec>& specs) {
     if (nsys <= 0) return report(ck::kErrInput, "nsys must be positive");

@@ -575,17 +575,11 @@ Status Engine::launch(std::string& err) {
                                   tuning.stride3, tuning.stride4, tuning.blocks_per_sm, profile ? 1 : 0,
                                   tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4, tuning.xw3, tuning.xw4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
-                                  tuning.tc3, tuning.tc4, V_.all_pairs, V_.enum_serial};
-    for (const void* p : {(const void*)V_.sys, (const void*)V_.in_pos, (const void*)V_.ghost_fs,
-                          (const void*)V_.bin_items, (const void*)V_.l2_ghost, (const void*)V_.c3,
-                          (const void*)V_.c4, (const void*)V_.force, (const void*)d_scan_tmp_.p,
-                          (const void*)h_out_.p, (const void*)V_.queue, (const void*)V_.bin_count,
-                          (const void*)V_.e_off3, (const void*)V_.psets, (const void*)V_.perm3,
-                          (const void*)V_.perm4, (const void*)V_.bk_count, (const void*)V_.bk_fill,
-                          (const void*)V_.bk_start, (const void*)V_.c3e, (const void*)V_.c4e,
-                          (const void*)V_.pe, (const void*)V_.a_off, (const void*)V_.l2_off, (const void*)V_.l2_key, (const void*)V_.l2_hash, (const void*)V_.ghost_sh,
-                          (const void*)V_.pcd3, (const void*)V_.pcd4, (const void*)V_.pct3, (const void*)V_.pct4})
-        key.push_back((long long)(uintptr_t)p);
+                                  tuning.tc3, tuning.tc4, V_.all_pairs, V_.enum_serial, V_.l2_slots,
+                                  avail_pc3_ ? 1 : 0, avail_pc4_ ? 1 : 0, pc_small_ ? 1 : 0,
+                                  // the pointers: sizes and forms fix which buffers a launch uses and where their
+                                  // parts lie, and no buffer has moved
+                                  (long long)reallocs_};
     if (key != graph_key_) {
         // capture only when the same shape launches twice in a row: a batch
         // seen once (a one-off call, or sizes that change every call) runs
@@ -607,6 +601,7 @@ Status Engine::launch(std::string& err) {
         graph_ = g;
         CK_TRY(cudaGraphInstantiate(&graph_exec_, graph_, 0));
         graph_key_ = key;
+        captures_++;
     }
     CK_TRY(cudaGraphLaunch(graph_exec_, stream_));
     return kOk;

@@ -34,6 +34,20 @@ struct DevBuf {
     }
 };
 
+// A buffer whose address a captured graph may hold: every reallocation is
+// counted (no default constructor, so no buffer is left out of the count).
+template <class Buf>
+struct Counted : Buf {
+    unsigned long long& reallocations;
+    explicit Counted(unsigned long long& n) : reallocations(n) {}
+    cudaError_t reserve(size_t n) {
+        const size_t had = this->cap;
+        const cudaError_t e = Buf::reserve(n);
+        if (this->cap != had) reallocations++;   // (a buffer only grows, or is lost)
+        return e;
+    }
+};
+
 template <class T>
 struct PinnedBuf {
     T* p = nullptr;
@@ -134,6 +148,7 @@ public:
     double stage_ms[4] = {0, 0, 0, 0};   // list build, 2B, 3B, 4B
     long long stage_launches = 0;
     int kernels_per_launch = 0;          // kernels one launch() enqueues
+    long long captures() const { return captures_; }   // graphs captured so far
     Status read_stage_times(std::string& err);   // adds the last launch's event intervals
 
     // Autotuner for the staged batch: times the 3-body and 4-body force stages
@@ -164,7 +179,10 @@ private:
         std::vector<TupleRec> t3, t4;   // host copies of the tuple records
     };
     std::vector<PSet> sets_;
-    DevBuf<DevParamSet> dsets_;
+    unsigned long long reallocs_ = 0;             // of the buffers that launch() works on
+    template <class T> using GBuf = Counted<DevBuf<T>>;
+    template <class T> using GPinned = Counted<PinnedBuf<T>>;
+    GBuf<DevParamSet> dsets_{reallocs_};
     cudaStream_t stream_ = nullptr;
     cudaStream_t stream2_ = nullptr;              // the 4-body branch
     cudaEvent_t fork_ = nullptr, fork2_ = nullptr, pairs_ = nullptr, join_ = nullptr;
@@ -179,21 +197,21 @@ private:
     long long l2_slots_ = 0;
     bool staged_ = false;
 
-    DevBuf<unsigned char> d_in_;      // SysDesc[n_sys], positions, types
-    DevBuf<int> d_atom_sys_, d_atom_type_, d_atom_orig_;
-    DevBuf<int> d_atom_self_, d_ghost_id_;
-    DevBuf<float> d_ghost_xf_, d_l2_vec_, d_bin_xp_;
-    DevBuf<int> d_ghost_parent_, d_ghost_bin_;
-    DevBuf<double> d_ghost_fs_, d_ghost_fn_;
-    DevBuf<unsigned long long> d_minmax_;
-    DevBuf<int> d_bin_count_, d_bin_fill_, d_bin_items_;
-    DevBuf<long long> d_bin_start_;
-    DevBuf<int> d_l2_count_, d_l2_ghost_, d_l2_owner_;
-    DevBuf<long long> d_l2_off_;
-    DevBuf<double> d_l2_dist_;
-    DevBuf<int> d_e_cnt3_, d_e_cnt4_;
-    DevBuf<long long> d_e_off3_, d_e_off4_;
-    DevBuf<int> d_c3_, d_c4_;
+    GBuf<unsigned char> d_in_{reallocs_};      // SysDesc[n_sys], positions, types
+    GBuf<int> d_atom_sys_{reallocs_}, d_atom_type_{reallocs_}, d_atom_orig_{reallocs_};
+    GBuf<int> d_atom_self_{reallocs_}, d_ghost_id_{reallocs_};
+    GBuf<float> d_ghost_xf_{reallocs_}, d_l2_vec_{reallocs_}, d_bin_xp_{reallocs_};
+    GBuf<int> d_ghost_parent_{reallocs_}, d_ghost_bin_{reallocs_};
+    GBuf<double> d_ghost_fs_{reallocs_}, d_ghost_fn_{reallocs_};
+    GBuf<unsigned long long> d_minmax_{reallocs_};
+    GBuf<int> d_bin_count_{reallocs_}, d_bin_fill_{reallocs_}, d_bin_items_{reallocs_};
+    GBuf<long long> d_bin_start_{reallocs_};
+    GBuf<int> d_l2_count_{reallocs_}, d_l2_ghost_{reallocs_}, d_l2_owner_{reallocs_};
+    GBuf<long long> d_l2_off_{reallocs_};
+    GBuf<double> d_l2_dist_{reallocs_};
+    GBuf<int> d_e_cnt3_{reallocs_}, d_e_cnt4_{reallocs_};
+    GBuf<long long> d_e_off3_{reallocs_}, d_e_off4_{reallocs_};
+    GBuf<int> d_c3_{reallocs_}, d_c4_{reallocs_};
     int nbk3_ = 0, nbk4_ = 0;     // cluster buckets over all loaded parameter sets
     bool avail_fact3_ = false, avail_fact4_ = false;   // staged batch has factored tables
     bool avail_tc3_ = false;                           // ... and tensor-core 3-body images (mixed form)
@@ -202,29 +220,30 @@ private:
     bool avail_pc3_ = false, avail_pc4_ = false;       // pair-table cache usable for the staged batch
     bool pc_small_ = false;                            // list small enough for the cache to stay near L2
     bool avail_ent_ = false;                           // FP64 pair-entry form usable for the staged batch
-    DevBuf<int> d_c3e_, d_c4e_;
-    DevBuf<double> d_pcd3_, d_pcd4_, d_pe_;
-    DevBuf<int> d_ghost_sh_;
-    DevBuf<long long> d_l2_key_, d_a_off_;
-    DevBuf<int> d_a_cnt_, d_bk_key3_, d_bk_key4_, d_l2_hash_;
-    DevBuf<unsigned char> d_pct3_, d_pct4_;
-    DevBuf<int> d_bk_count_, d_bk_fill_, d_perm3_, d_perm4_;
-    DevBuf<long long> d_bk_start_;
-    DevBuf<double> d_out_;            // forces, energies and virials, totals (4), flags (8 ints)
-    DevBuf<unsigned long long> d_queue_;
-    DevBuf<unsigned char> d_scan_tmp_;
+    GBuf<int> d_c3e_{reallocs_}, d_c4e_{reallocs_};
+    GBuf<double> d_pcd3_{reallocs_}, d_pcd4_{reallocs_}, d_pe_{reallocs_};
+    GBuf<int> d_ghost_sh_{reallocs_};
+    GBuf<long long> d_l2_key_{reallocs_}, d_a_off_{reallocs_};
+    GBuf<int> d_a_cnt_{reallocs_}, d_bk_key3_{reallocs_}, d_bk_key4_{reallocs_}, d_l2_hash_{reallocs_};
+    GBuf<unsigned char> d_pct3_{reallocs_}, d_pct4_{reallocs_};
+    GBuf<int> d_bk_count_{reallocs_}, d_bk_fill_{reallocs_}, d_perm3_{reallocs_}, d_perm4_{reallocs_};
+    GBuf<long long> d_bk_start_{reallocs_};
+    GBuf<double> d_out_{reallocs_};            // forces, energies and virials, totals (4), flags (8 ints)
+    GBuf<unsigned long long> d_queue_{reallocs_};
+    GBuf<unsigned char> d_scan_tmp_{reallocs_};
     DevBuf<unsigned char> d_ws_;
     DevBuf<double> d_dir_d_;      // per-cluster inputs and outputs (doubles)
     DevBuf<int> d_dir_i_;         // per-cluster types and status
 
-    PinnedBuf<unsigned char> h_in_;   // as d_in_
-    PinnedBuf<double> h_out_;         // as d_out_
+    GPinned<unsigned char> h_in_{reallocs_};   // as d_in_
+    GPinned<double> h_out_{reallocs_};         // as d_out_
     size_t out_values() const { return 3 * (size_t)V_.n_in_total + 8 * (size_t)V_.n_sys + 4 + 4; }
     long long* h_totals() { return reinterpret_cast<long long*>(h_out_.p + 3 * V_.n_in_total + 8 * V_.n_sys); }
 
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;
     std::vector<long long> graph_key_;
+    long long captures_ = 0;
     std::vector<long long> seen_key_;   // shape of the last launch (a graph is captured on a repeat)
     cudaEvent_t ev_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool ev_recorded_ = false;

@@ -107,6 +107,8 @@ int ck_autotune(void *h, int *chosen);
 /* replay the whole list-build + force sequence as one CUDA graph (1) or launch
  * it stream-ordered (0).  Instances of the serial interface start with 1. */
 int ck_use_graph(void *h, int on);
+/* graphs captured by the handle so far (a repeated call that replays one adds none) */
+long long ck_graph_captures(void *h);
 /* Serial-interface instances (calculate_chimes*) autotune once on the third
  * consecutive call with the same atom count (on = 1, the default); 0 keeps the
  * default launch shape. */
