@@ -1287,6 +1287,11 @@ void launch_enuma(const BatchView& B, const int* l2_owner, cudaStream_t st) {
     const unsigned grid = (unsigned)(want < need ? want : need);
     const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
     const size_t smem = nbk <= kBkSmem ? sizeof(int) * (size_t)nbk : 0;
+    // (with one warp per atom the static arrays take 44.4 KB: more than 912 buckets pass
+    // the 48 KB that a block gets without asking)
+    if (smem > 0)
+        cudaFuncSetAttribute((const void*)k_enuma<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(int) * kBkSmem);
     count_launch(), launch_chained(k_enuma<G>, grid, 32 * kEnumWarps, smem, st, B, l2_owner);
 }
 
