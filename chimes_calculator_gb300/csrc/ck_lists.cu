@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B, const
     __shared__ int s_o[NG][2 * kEnumRows + 2];   // per-entry offsets, then the totals
     __shared__ long long s_at[NG][2];            // where the atom's clusters go
     __shared__ unsigned char s_ty[NG][kEnumRows];   // the entries' types
-    __shared__ unsigned short s_e[NG][kEnumRows];   // their numbers in the atom's list
+    __shared__ int s_e[NG][kEnumRows];              // their numbers in the atom's list
     __shared__ int s_sh[NG][kEnumRows];             // their image shifts
     extern __shared__ int s_hist[];              // bucket counts of this block (when B.keyed and few buckets)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(32 * kEnumWarps, 4) k_enuma(BatchView B, const
     unsigned* rt = s_t[grp];
     unsigned* rq = s_q[grp];
     int* so = s_o[grp];
-    unsigned short* se = s_e[grp];
+    int* se = s_e[grp];
     // room for an atom's t3 triplets and t4 quadruplets (one lane of the group)
     auto reserve = [&](long long r, long long t3, long long t4) {
         const long long a3 = t3 > 0 ? (long long)atomicAdd((unsigned long long*)&B.totals[1], (unsigned long long)t3) : 0;
@@ -1287,7 +1287,7 @@ void launch_enuma(const BatchView& B, const int* l2_owner, cudaStream_t st) {
     const unsigned grid = (unsigned)(want < need ? want : need);
     const int nbk = B.keyed ? B.nbk3 + B.nbk4 : 0;
     const size_t smem = nbk <= kBkSmem ? sizeof(int) * (size_t)nbk : 0;
-    // (with one warp per atom the static arrays take 44.4 KB: more than 912 buckets pass
+    // (with one warp per atom the static arrays take 45.9 KB: more than 528 buckets pass
     // the 48 KB that a block gets without asking)
     if (smem > 0)
         cudaFuncSetAttribute((const void*)k_enuma<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
