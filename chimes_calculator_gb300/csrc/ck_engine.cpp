@@ -281,30 +281,8 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     // one block each for what goes to the device and what comes back, so that a call
     // makes one copy each way (three, one of them from pageable memory, and four before)
     const size_t sys_bytes = sizeof(SysDesc) * (size_t)S, in_bytes = sys_bytes + (sizeof(double) * 3 + sizeof(int)) * in_off;
-    CK_TRY(d_in_.reserve(in_bytes));
     CK_TRY(h_in_.reserve(in_bytes));
-    CK_TRY(d_out_.reserve(out_values()));
     CK_TRY(h_out_.reserve(out_values()));
-    CK_TRY(d_atom_sys_.reserve(atom_off));
-    CK_TRY(d_atom_type_.reserve(atom_off));
-    CK_TRY(d_atom_orig_.reserve(atom_off));
-    CK_TRY(d_atom_self_.reserve(atom_off));
-    CK_TRY(d_ghost_id_.reserve(ghost_off));
-    CK_TRY(d_ghost_xf_.reserve(3 * ghost_off));
-    CK_TRY(d_ghost_parent_.reserve(ghost_off));
-    CK_TRY(d_ghost_bin_.reserve(ghost_off));
-    CK_TRY(d_ghost_fs_.reserve(3 * ghost_off));
-    CK_TRY(d_ghost_fn_.reserve(3 * ghost_off));
-    CK_TRY(d_bin_items_.reserve(ghost_off));
-    CK_TRY(d_bin_xp_.reserve(4 * ghost_off));
-    CK_TRY(d_minmax_.reserve(6 * S));
-    CK_TRY(d_bin_count_.reserve(bin_off));
-    CK_TRY(d_bin_fill_.reserve(bin_off));
-    CK_TRY(d_bin_start_.reserve(bin_off));
-    CK_TRY(d_l2_count_.reserve(atom_off));
-    CK_TRY(d_l2_off_.reserve(atom_off));
-    CK_TRY(d_a_off_.reserve(2 * atom_off));
-    CK_TRY(d_a_cnt_.reserve(2 * atom_off));
     st = ensure_lists(err);
     if (st != kOk) return st;
 
@@ -321,56 +299,135 @@ Status Engine::stage(const std::vector<SystemSpec>& sys, std::string& err) {
     return kOk;
 }
 
-Status Engine::ensure_lists(std::string& err) {
-    CK_TRY(d_l2_ghost_.reserve(n2_cap_));
-    CK_TRY(d_pe_.reserve(4 * n2_cap_));
-    CK_TRY(d_l2_owner_.reserve(n2_cap_));
-    CK_TRY(d_l2_dist_.reserve(n2_cap_));
-    CK_TRY(d_l2_vec_.reserve(4 * n2_cap_));
-    CK_TRY(d_e_cnt3_.reserve(n2_cap_));
-    CK_TRY(d_e_cnt4_.reserve(n2_cap_));
-    CK_TRY(d_e_off3_.reserve(n2_cap_ + 1));
-    CK_TRY(d_e_off4_.reserve(n2_cap_ + 1));
-    CK_TRY(d_c3_.reserve(3 * n3_cap_));
-    CK_TRY(d_c4_.reserve(4 * n4_cap_));
-    // buckets pad each (set, tuple) to 32 slots (3-body: 128 for the tensor-core form)
-    const long long p3cap = nbk3_ > 0 ? n3_cap_ + 128LL * nbk3_ : 0;
-    const long long p4cap = nbk4_ > 0 ? n4_cap_ + 32LL * nbk4_ : 0;
-    CK_TRY(d_perm3_.reserve(std::max(1LL, p3cap)));
-    CK_TRY(d_perm4_.reserve(std::max(1LL, p4cap)));
-    CK_TRY(d_bk_key3_.reserve(std::max(1LL, nbk3_ > 0 ? n3_cap_ : 0)));
-    CK_TRY(d_bk_key4_.reserve(std::max(1LL, nbk4_ > 0 ? n4_cap_ : 0)));
-    CK_TRY(d_bk_count_.reserve(nbk3_ + nbk4_ + 1));
-    CK_TRY(d_bk_fill_.reserve(nbk3_ + nbk4_ + 1));
-    CK_TRY(d_bk_start_.reserve(nbk3_ + nbk4_ + 2));
+// What every form of a call needs.
+cudaError_t Engine::reserve_batch() {
+    const long long n_in = V_.n_in_total, atoms = V_.n_atoms_total, ghosts = V_.n_ghost_total, bins = V_.n_bins_total;
+    cudaError_t e = cudaSuccess;
+    auto get = [&](auto& buf, long long n) {
+        if (e == cudaSuccess) e = buf.reserve((size_t)n);
+    };
+    get(d_in_, sizeof(SysDesc) * (long long)V_.n_sys + (sizeof(double) * 3 + sizeof(int)) * n_in);
+    get(d_out_, (long long)out_values());
+    get(d_atom_sys_, atoms);
+    get(d_atom_type_, atoms);
+    get(d_atom_orig_, atoms);
+    get(d_atom_self_, atoms);
+    get(d_ghost_id_, ghosts);
+    get(d_ghost_xf_, 3 * ghosts);
+    get(d_ghost_parent_, ghosts);
+    get(d_ghost_bin_, ghosts);
+    get(d_ghost_fs_, 3 * ghosts);
+    get(d_ghost_fn_, 3 * ghosts);
+    get(d_bin_items_, ghosts);
+    get(d_bin_xp_, 4 * ghosts);
+    get(d_minmax_, 6LL * V_.n_sys);
+    get(d_bin_count_, bins);
+    get(d_bin_fill_, bins);
+    get(d_bin_start_, bins);
+    get(d_l2_count_, atoms);
+    get(d_l2_off_, atoms);
+    get(d_a_off_, 2 * atoms);
+    get(d_a_cnt_, 2 * atoms);
+    get(d_l2_ghost_, n2_cap_);
+    get(d_l2_owner_, n2_cap_);
+    get(d_l2_vec_, 4 * n2_cap_);
+    get(d_e_cnt3_, n2_cap_);
+    get(d_e_cnt4_, n2_cap_);
+    get(d_e_off3_, n2_cap_ + 1);
+    get(d_e_off4_, n2_cap_ + 1);
+    get(d_c3_, 3 * n3_cap_);
+    get(d_c4_, 4 * n4_cap_);
+    get(d_perm3_, std::max(1LL, perm_cap(3)));
+    get(d_perm4_, std::max(1LL, perm_cap(4)));
+    get(d_bk_key3_, std::max(1LL, nbk3_ > 0 ? n3_cap_ : 0));
+    get(d_bk_key4_, std::max(1LL, nbk4_ > 0 ? n4_cap_ : 0));
+    get(d_bk_count_, nbk3_ + nbk4_ + 1);
+    get(d_bk_fill_, nbk3_ + nbk4_ + 1);
+    get(d_bk_start_, nbk3_ + nbk4_ + 2);
+    if (enum_serial_) {
+        get(d_l2_dist_, n2_cap_);
+        get(d_scan_tmp_, (long long)scan_tmp_bytes(n2_cap_));
+    }
+    return e;
+}
+
+// What is kept per list entry beside the list itself (FP64 with 10 and 4 powers
+// about 350 bytes, mixed 270, the list 48): force scalars, pair tables, look-up.
+cudaError_t Engine::reserve_entries() {
+    cudaError_t e = cudaSuccess;
+    auto get = [&](auto& buf, long long n) {
+        if (e == cudaSuccess) e = buf.reserve((size_t)n);
+    };
+    get(d_pe_, 4 * n2_cap_);
     if (avail_ent_) {
-        CK_TRY(d_ghost_sh_.reserve(V_.n_ghost_total));
-        CK_TRY(d_l2_key_.reserve(n2_cap_));
+        get(d_ghost_sh_, V_.n_ghost_total);
+        get(d_l2_key_, n2_cap_);
         l2_slots_ = 1024;   // a power of two, twice the list's capacity or more
         while (l2_slots_ < 2 * n2_cap_) l2_slots_ *= 2;
-        CK_TRY(d_l2_hash_.reserve(l2_slots_));
+        get(d_l2_hash_, l2_slots_);
         if (tuning.rf3 > 0) {
-            CK_TRY(d_c3e_.reserve(3 * n3_cap_));
-            CK_TRY(d_pcd3_.reserve(4 * n2_cap_));
-            CK_TRY(d_pct3_.reserve((long long)sizeof(FxEnt) * tuning.rf3 * n2_cap_));
+            get(d_c3e_, 3 * n3_cap_);
+            get(d_pcd3_, 4 * n2_cap_);
+            get(d_pct3_, (long long)sizeof(FxEnt) * tuning.rf3 * n2_cap_);
         }
         if (tuning.rf4 > 0) {
-            CK_TRY(d_c4e_.reserve(6 * n4_cap_));
-            CK_TRY(d_pcd4_.reserve(4 * n2_cap_));
-            CK_TRY(d_pct4_.reserve((long long)sizeof(FxEnt) * tuning.rf4 * n2_cap_));
+            get(d_c4e_, 6 * n4_cap_);
+            get(d_pcd4_, 4 * n2_cap_);
+            get(d_pct4_, (long long)sizeof(FxEnt) * tuning.rf4 * n2_cap_);
         }
     }
     if (avail_pc3_) {
-        CK_TRY(d_c3e_.reserve(2 * n3_cap_));
-        CK_TRY(d_pcd3_.reserve(8 * n2_cap_));
-        CK_TRY(d_pct3_.reserve((long long)sizeof(double) * 2 * tuning.rf3 * n2_cap_));
+        get(d_c3e_, 2 * n3_cap_);
+        get(d_pcd3_, 8 * n2_cap_);
+        get(d_pct3_, (long long)sizeof(float) * 2 * tuning.rf3 * n2_cap_);
     }
     if (avail_pc4_) {
-        CK_TRY(d_c4e_.reserve(3 * n4_cap_));
-        CK_TRY(d_pcd4_.reserve(8 * n2_cap_));
-        CK_TRY(d_pct4_.reserve((long long)sizeof(double) * 2 * tuning.rf4 * n2_cap_));
+        get(d_c4e_, 3 * n4_cap_);
+        get(d_pcd4_, 8 * n2_cap_);
+        get(d_pct4_, (long long)sizeof(float) * 2 * tuning.rf4 * n2_cap_);
     }
-    if (enum_serial_) CK_TRY(d_scan_tmp_.reserve(scan_tmp_bytes(n2_cap_)));
+    return e;
+}
+
+void Engine::release_entries() {
+    d_pe_.release();
+    d_ghost_sh_.release();
+    d_l2_key_.release();
+    d_l2_hash_.release();
+    d_c3e_.release();
+    d_c4e_.release();
+    d_pcd3_.release();
+    d_pcd4_.release();
+    d_pct3_.release();
+    d_pct4_.release();
+}
+
+// Device arrays of the staged batch at the current capacities.  Where those per
+// list entry do not fit (or their 32-bit entry numbers would not hold), the
+// batch runs without them: pairs set up per cluster, 2-body forces entry by
+// entry, a third of the memory per atom.  So does then every batch of this
+// handle whose lists are as large.
+Status Engine::ensure_lists(std::string& err) {
+    lean_ = n2_cap_ >= std::min(lean_from_, 0x7fffffffLL);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (!lean_) {
+        e = reserve_batch();
+        if (e == cudaSuccess) e = reserve_entries();
+        if (e == cudaErrorMemoryAllocation) lean_from_ = n2_cap_;
+    }
+    if (e == cudaErrorMemoryAllocation) {
+        if (!lean_) cudaGetLastError();   // (reported here, not by the next launch's check)
+        lean_ = true;
+        avail_ent_ = avail_pc3_ = avail_pc4_ = false;
+        release_entries();
+        e = reserve_batch();
+    }
+    if (e != cudaSuccess) {
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        err = std::string("CUDA error: ") + cudaGetErrorString(e) + " at the device arrays of a batch";
+        return kErrCuda;
+    }
+    const long long p3cap = perm_cap(3), p4cap = perm_cap(4);
     BatchView& B = V_;
     B.sys = reinterpret_cast<SysDesc*>(d_in_.p);
     B.psets = dsets_.p;
@@ -479,13 +536,17 @@ Status Engine::enqueue(std::string& err) {
     // while the first runs the 3-body one; both join before the copies out.
     // Not while profiling (the stage events time the stages one after another).
     const bool conc = !profile && concurrent;
+    auto pairs = [&](cudaStream_t q) {
+        if (lean_) launch_force2(B, d_l2_owner_.p, L, q);
+        else launch_pairs(B, d_l2_owner_.p, L, q);
+    };
     if (conc) {
         CK_TRY(cudaEventRecord(fork_, st));
         CK_TRY(cudaStreamWaitEvent(stream2_, fork_, 0));
         NvtxRange r("chimes: 1B+2B");
-        launch_pairs(B, d_l2_owner_.p, L, stream2_);
+        pairs(stream2_);
         CK_TRY(cudaEventRecord(pairs_, stream2_));
-        if (!ent) launch_pair_forces(B, stream2_);
+        if (!ent && !lean_) launch_pair_forces(B, stream2_);
     }
     launch_enum(B, d_l2_owner_.p, d_scan_tmp_.p, st);
     launch_bucket(B, L.stride3 > 0 && L.fact3, L.stride4 > 0 && L.fact4, st);
@@ -531,8 +592,8 @@ Status Engine::enqueue(std::string& err) {
     } else {
         {
             NvtxRange r("chimes: 1B+2B");
-            launch_pairs(B, d_l2_owner_.p, L, st);
-            if (!ent) launch_pair_forces(B, st);
+            pairs(st);
+            if (!ent && !lean_) launch_pair_forces(B, st);
         }
         if (profile) CK_TRY(record_stage_event(ev_[2], st));
         body3(st);
@@ -576,7 +637,7 @@ Status Engine::launch(std::string& err) {
                                   tuning.fact3, tuning.fact4, tuning.rf3, tuning.rf4, tuning.xs3, tuning.ftpc3, tuning.ftpc4, tuning.xw3, tuning.xw4,
                                   tuning.fbps3, tuning.fbps4, nbk3_, nbk4_, concurrent ? 1 : 0, tuning.noy3,
                                   tuning.tc3, tuning.tc4, V_.all_pairs, V_.enum_serial, V_.l2_slots,
-                                  avail_pc3_ ? 1 : 0, avail_pc4_ ? 1 : 0, pc_small_ ? 1 : 0,
+                                  avail_pc3_ ? 1 : 0, avail_pc4_ ? 1 : 0, pc_small_ ? 1 : 0, lean_ ? 1 : 0,
                                   // the pointers: sizes and forms fix which buffers a launch uses and where their
                                   // parts lie, and no buffer has moved
                                   (long long)reallocs_};

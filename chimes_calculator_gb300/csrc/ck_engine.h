@@ -32,6 +32,11 @@ struct DevBuf {
         cap = e == cudaSuccess ? want : 0;
         return e;
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        cap = 0;
+    }
 };
 
 // A buffer whose address a captured graph may hold: every reallocation is
@@ -45,6 +50,10 @@ struct Counted : Buf {
         const cudaError_t e = Buf::reserve(n);
         if (this->cap != had) reallocations++;   // (a buffer only grows, or is lost)
         return e;
+    }
+    void release() {
+        if (this->p) reallocations++;
+        Buf::release();
     }
 };
 
@@ -220,6 +229,8 @@ private:
     bool avail_pc3_ = false, avail_pc4_ = false;       // pair-table cache usable for the staged batch
     bool pc_small_ = false;                            // list small enough for the cache to stay near L2
     bool avail_ent_ = false;                           // FP64 pair-entry form usable for the staged batch
+    bool lean_ = false;                                // staged batch runs without per-entry arrays (memory)
+    long long lean_from_ = 1LL << 62;                  // smallest list capacity whose per-entry arrays did not fit
     GBuf<int> d_c3e_{reallocs_}, d_c4e_{reallocs_};
     GBuf<double> d_pcd3_{reallocs_}, d_pcd4_{reallocs_}, d_pe_{reallocs_};
     GBuf<int> d_ghost_sh_{reallocs_};
@@ -248,7 +259,15 @@ private:
     cudaEvent_t ev_[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     bool ev_recorded_ = false;
 
+    cudaError_t reserve_batch();
+    cudaError_t reserve_entries();
+    void release_entries();
     Status ensure_lists(std::string& err);
+    // slots of a body order's bucketed clusters: buckets pad each (set, tuple) to 32
+    // slots (3-body: 128 for the tensor-core form)
+    long long perm_cap(int nb) const {
+        return nb == 3 ? (nbk3_ > 0 ? n3_cap_ + 128LL * nbk3_ : 0) : (nbk4_ > 0 ? n4_cap_ + 32LL * nbk4_ : 0);
+    }
     Status enqueue(std::string& err);
     void drop_graph();
     std::string tune_key() const;
