@@ -21,14 +21,15 @@
 // Distances are computed in FP32 with a rigorous bound on the error of the
 // distance; a pair whose bin the bound certifies is counted directly, the
 // rest (about 1e-4 of them) are recomputed in FP64 with the reference's
-// operations, so the counts equal the FP64 histogram's.
+// operations, and those that the difference between the device's exponential and the
+// host's could move to another bin by the host, so the counts equal the tool's.
 //
 // Bound: instruction issue.  The two records of a thread go through packed FP32
 // instructions together, and the bound is one on the distance in units of bins (a
 // constant per record and a relative part) and not on its square against both
 // edges: 20 instructions a pair against 45, and a fifth as many pairs to repeat in
-// FP64.  Measured, 40001 triplets with themselves, 100 bins: 0.63 ms against 1.86
-// (issue slots 68% used).
+// FP64.  Measured, 40001 triplets with themselves, 100 bins: 0.58 ms against 1.86
+// (0.63 with the FP64 repeats inlined and counted by the pair loop).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,29 +90,19 @@ __device__ __forceinline__ float fp_rsqrt_approx(float x) {
     return r;
 }
 
-// Exact FP64 bin of one pair, with the tool's operations (dist_struct +=
-// pow(a - b, 2) in order, sqrt, floor(dist / binw), the dist == maxd rule);
-// -1 when the distance falls past the last bin.
-template <int P>
-__device__ __forceinline__ int fp_exact_bin(const double* a, const double* b, double binw, double maxd, int nbin,
-                                            int cand) {
-    double ds = 0.0;
-    for (int p = 0; p < P; p++) {
-        const double d = __dsub_rn(a[p], b[p]);
-        ds = __dadd_rn(ds, __dmul_rn(d, d));
-    }
-    // the FP32 candidate bin, confirmed in FP64 when ds lies inside its
-    // squared edges by far more than the roundings of sqrt and the division
-    if (cand >= 0 && cand < nbin) {
-        const double lo = cand * binw, hi = lo + binw;
-        if (ds >= lo * lo * (1.0 + 1e-12) && ds <= hi * hi * (1.0 - 1e-12)) return cand;
-    }
-    const double dist = __dadd_rn(__dsqrt_rn(ds), 0.0);
-    int bin = (int)floor(__ddiv_rn(dist, binw));
-    if (dist == maxd) bin = bin - 1;
-    return (bin < 0 || bin >= nbin) ? -1 : bin;
-}
-
+// FP64 bin of one pair, with the tool's operations (dist_struct += pow(a - b, 2) in
+// order, sqrt, floor(dist / binw), the dist == maxd rule) on the device's edges; -1 when
+// the distance falls past the last bin, kFpTie when eta, the bound on what the
+// device's edges differ by from the host's (in units of bins), leaves the bin open.
+constexpr int kFpTie = -2;
+// What the FP64 bin of a pair needs of the call.
+struct FpCall {
+    const double *d1, *d2;   // edges of both sets
+    double binw, maxd;
+    int nbin;
+    float inv_w, eta_q;
+    int* flags;
+};
 // The FP32 distance and its error, u = 2^-24, N = |a| + |b| (norms of the
 // records): with a, b and each difference rounded,
 //   |s32 - s| <= 2 u N sqrt(s) + (2 + P) u s (+ second order),
@@ -127,27 +118,74 @@ constexpr float kFpRel = 9.5367432e-7f;                      // 2^-20
 constexpr float kFpMagic = 12582912.0f;                      // 1.5 * 2^23: adding it rounds to an integer
 constexpr int kFpMagicBits = 0x4B400000;
 
+// The tool's edges come from the host's exp, the device's from its own: each within
+// one unit in the last place of exp(-d / lambda), so that an edge x = (exp - avg) /
+// diff differs by at most 2^-50 (|x| + |avg / diff|), a distance by the norms of
+// both records' differences.  In units of bins, with records' margins m and
+// q = 2^-50 * 2 sqrt(P) max |avg / diff| / w (0: the edges are the host's):
+//   eta = 2^-50 (m_a + m_b) / kFpMargin + q
+// A pair whose bin that leaves open -- an edge is nearer than some 1e-14 of a bin --
+// is listed, and the host bins it.
+constexpr float kFpEtaMargin = 0x1.03p-50f / (4.0f * 5.9604645e-8f);   // (rounded up)
+struct FpPair {
+    long long i, j;
+};
+constexpr int kFpTies = 1 << 16;   // pairs listed (more: the host makes all edges)
+constexpr int kFpFlags = 4;        // words before them: a distance past the last bin; pairs to list
+
+// Counts records i and j in FP64, where the FP32 candidate is not certified (margins:
+// the sum of theirs; hist: the lane's column).  Called and not inlined: its registers
+// would cost the pair loop a block per SM.
+template <int P>
+__device__ __noinline__ void fp_exact(const FpCall& C, long long i, long long j, float margins, unsigned int* hist) {
+    double ds = 0.0;
+    for (int p = 0; p < P; p++) {
+        const double d = __dsub_rn(C.d1[i * P + p], C.d2[j * P + p]);
+        ds = __dadd_rn(ds, __dmul_rn(d, d));
+    }
+    const float eta = C.eta_q > 0.0f ? kFpEtaMargin * margins + C.eta_q : 0.0f;
+    // a candidate, confirmed in FP64 when ds lies inside its squared edges by far
+    // more than the roundings of sqrt and the division, and more than eta, twice (an
+    // edge above zero is one bin or more)
+    int bin = (int)(sqrtf((float)ds) * C.inv_w);
+    const double lo = bin * C.binw, hi = lo + C.binw;
+    if (!(bin >= 0 && bin < C.nbin && eta < 3e-10f && ds >= lo * lo * (1.0 + 1e-9) && ds <= hi * hi * (1.0 - 1e-9))) {
+        // the tool's operations
+        const double dist = __dadd_rn(__dsqrt_rn(ds), 0.0);
+        const double t = __ddiv_rn(dist, C.binw), k = rint(t);
+        if (eta > 0.0f && k >= 1.0 && !(fabs(t - k) > (double)eta + 0x1p-50 * t)) {
+            const int n = atomicAdd(&C.flags[1], 1);
+            if (n < kFpTies) reinterpret_cast<FpPair*>(C.flags + kFpFlags)[n] = FpPair{i, j};
+            return;
+        }
+        bin = (int)floor(t);
+        if (dist == C.maxd) bin = bin - 1;
+        if (bin < 0 || bin >= C.nbin) {
+            atomicOr(&C.flags[0], 1);   // (the call fails)
+            return;
+        }
+    }
+    atomicAdd(&hist[bin * 32], 1u);
+}
+
 // e, m: records' edges and margins (kFpMargin norm / w, rounded up).
 template <int P>
-__global__ void __launch_bounds__(128) k_fp_hist(const float* __restrict__ e1, const float* __restrict__ m1,
-                                                 const double* __restrict__ d1, long long n1,
-                                                 const float* __restrict__ e2, const float* __restrict__ m2,
-                                                 const double* __restrict__ d2, long long n2, int same, int nbin,
-                                                 double binw, double maxd, long long n_itile, long long n_jtile,
-                                                 unsigned long long* counts, int* flags) {
+__global__ void __launch_bounds__(128, P == 1 ? 7 : P == 3 ? 6 : 5)
+    k_fp_hist(const float* __restrict__ e1, const float* __restrict__ m1, long long n1, const float* __restrict__ e2,
+              const float* __restrict__ m2, long long n2, int same, long long t_begin, long long t_end,
+              long long n_jtile, unsigned long long* counts, const __grid_constant__ FpCall C) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int T = blockDim.x;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31, nbin = C.nbin;
     FpRec<P>* tile = reinterpret_cast<FpRec<P>*>(smem);
-    unsigned int* hist = reinterpret_cast<unsigned int*>(tile + kFpTileJ);       // [nbin][32]
+    unsigned int* hist = reinterpret_cast<unsigned int*>(tile + kFpTileJ);       // [nbin + 1][32]
     for (int b = tid; b < nbin * 32; b += T) hist[b] = 0u;
-    const float inv_wf = (float)(1.0 / binw);
+    const float inv_wf = C.inv_w;
     const int rows = T * kFpRows;
-    const long long ntiles = n_itile * n_jtile;
     const unsigned long long inv2 = fp_pack(inv_wf, inv_wf), magic2 = fp_pack(kFpMagic, kFpMagic),
                              unmagic2 = fp_pack(-kFpMagic, -kFpMagic), half2 = fp_pack(-0.5f, -0.5f),
                              rel2 = fp_pack(-kFpRel, -kFpRel), neg2 = fp_pack(-1.0f, -1.0f);
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (long long t = t_begin + blockIdx.x; t < t_end; t += gridDim.x) {
         const long long it = t / n_jtile, jt = t % n_jtile;
         const long long i0 = it * rows, j0 = jt * kFpTileJ;
         // a tile whose every j is <= every i holds no pair j > i
@@ -194,49 +232,48 @@ __global__ void __launch_bounds__(128) k_fp_hist(const float* __restrict__ e1, c
             oka = fabsf(fp_lo(h)) < fp_lo(lim) && (unsigned)ba < (unsigned)nbin;
             okb = fabsf(fp_hi(h)) < fp_hi(lim) && (unsigned)bb < (unsigned)nbin;
         };
-        auto exact = [&](long long i, int k, int& bin) {
-            bin = fp_exact_bin<P>(d1 + i * P, d2 + (j0 + k) * P, binw, maxd, nbin, bin);
-            if (bin < 0) {
-                atomicOr(&flags[0], 1);
-                bin = 0;   // (the call fails)
+        // bit u of `open`: the first row with record k + u, bit kFpStep + u: the second
+        auto exact = [&](int k, unsigned open) {
+            while (open) {
+                const int q = __ffs(open) - 1, u = q % kFpStep;
+                open &= open - 1;
+                const long long i = q < kFpStep ? ia : ib;
+                fp_exact<P>(C, i, j0 + k + u, m1[i] - tile[k + u].m.x, hist + lane);
             }
         };
         for (int k = ka; k < kb; k++) {
             int ba, bb;
             bool oka, okb;
             candidates(k, ba, bb, oka, okb);
-            if (!oka) exact(ia, k, ba);
-            atomicAdd(&hist[ba * 32 + lane], 1u);
+            if (oka) atomicAdd(&hist[ba * 32 + lane], 1u);
+            else exact(k, 1u);
         }
         int k = kb;
         for (; k + kFpStep <= jn; k += kFpStep) {   // a few records' chains together
             int ba[kFpStep], bb[kFpStep];
-            bool oka[kFpStep], okb[kFpStep], all = true;
+            bool oka[kFpStep], okb[kFpStep];
+            unsigned open = 0;
 #pragma unroll
             for (int u = 0; u < kFpStep; u++) {
                 candidates(k + u, ba[u], bb[u], oka[u], okb[u]);
-                all = all && oka[u] && okb[u];
+                open |= (oka[u] ? 0u : 1u << u) | (okb[u] ? 0u : 1u << (kFpStep + u));
+                ba[u] = oka[u] ? ba[u] : nbin;   // (a column past the bins: an atomic without a branch)
+                bb[u] = okb[u] ? bb[u] : nbin;
             }
-            if (!all)
-#pragma unroll
-                for (int u = 0; u < kFpStep; u++) {
-                    if (!oka[u]) exact(ia, k + u, ba[u]);
-                    if (!okb[u]) exact(ib, k + u, bb[u]);
-                }
 #pragma unroll
             for (int u = 0; u < kFpStep; u++) {
                 atomicAdd(&hist[ba[u] * 32 + lane], 1u);
                 atomicAdd(&hist[bb[u] * 32 + lane], 1u);
             }
+            if (open) exact(k, open);
         }
         for (; k < jn; k++) {
             int ba, bb;
             bool oka, okb;
             candidates(k, ba, bb, oka, okb);
-            if (!oka) exact(ia, k, ba);
-            if (!okb) exact(ib, k, bb);
-            atomicAdd(&hist[ba * 32 + lane], 1u);
-            atomicAdd(&hist[bb * 32 + lane], 1u);
+            if (oka) atomicAdd(&hist[ba * 32 + lane], 1u);
+            if (okb) atomicAdd(&hist[bb * 32 + lane], 1u);
+            if (!oka || !okb) exact(k, (oka ? 0u : 1u) | (okb ? 0u : 1u << kFpStep));
         }
     }
     __syncthreads();
@@ -387,6 +424,62 @@ void launch_nl_fp(const BatchView& B, const NeighView& N, int nbody, long long n
 // ---------------------------------------------------------------------------
 namespace {
 
+// transform of read_flat_clusters (multi_calc_histogram.cpp:112-123), host FP64
+double fp_transform(double rcin, double rcout, double lambda, double rij) {
+    double x_min = std::exp(-1 * rcin / lambda);
+    double x_max = std::exp(-1 * rcout / lambda);
+    double x_avg = 0.5 * (x_max + x_min);
+    double x_diff = 0.5 * (x_max - x_min);
+    x_diff *= -1.0;
+    return (std::exp(-1 * rij / lambda) - x_avg) / x_diff;
+}
+
+// Sorted transformed edges of record c (the cluster's own cutoffs, pair lambdas by
+// the atoms' pair type), read_flat_clusters (:26-107).
+void fp_host_edges(const Engine& eng, int slot, int nbody, long long c, const double* d, const int* t, double* e) {
+    const HostParams& P = eng.params(slot);
+    const int nt = P.ntypes, np = nbody * (nbody - 1) / 2;
+    const int* ty = t + c * nbody;
+    if (nbody == 2) {
+        const int p = P.pair_map[ty[0] * nt + ty[1]];
+        e[0] = fp_transform(P.rin[p], P.rout[p], P.lam[p], d[c]);
+        return;
+    }
+    int u = 0;
+    for (int k = 0; k < nbody; k++) u = u * nt + ty[k];
+    const TupleRec& R = eng.tuples(slot, nbody)[u];
+    for (int p = 0; p < np; p++) e[p] = fp_transform(R.rin[p], R.rout[p], R.lam[p], d[c * np + p]);
+    std::sort(e, e + np);
+}
+
+// The bin of two records' edges as the tool computes it (dist_struct, floor(dist /
+// binw), the dist == maxd rule); -1 past the last one.
+int fp_host_bin(const double* a, const double* b, int np, double binw, double maxd, int nbin) {
+    double ds = 0.0;
+    for (int p = 0; p < np; p++) ds += (a[p] - b[p]) * (a[p] - b[p]);
+    const double dist = std::sqrt(ds);
+    int bin = (int)std::floor(dist / binw);
+    if (dist == maxd) bin = bin - 1;
+    return bin < 0 || bin >= nbin ? -1 : bin;
+}
+
+// max |avg / diff| of a set's maps (see kFpEtaMargin)
+double fp_shift(const Engine& eng, int slot, int nbody) {
+    const HostParams& P = eng.params(slot);
+    double q = 0.0;
+    auto take = [&](double rin, double rout, double lam) {
+        const double lo = std::exp(-1 * rin / lam), hi = std::exp(-1 * rout / lam);
+        const double v = std::fabs((hi + lo) / (hi - lo));
+        q = v > q || v != v ? v : q;
+    };
+    if (nbody == 2)
+        for (int p = 0; p < P.npairs; p++) take(P.rin[p], P.rout[p], P.lam[p]);
+    else
+        for (const TupleRec& R : eng.tuples(slot, nbody))
+            for (int p = 0; R.type_id >= 0 && p < nbody * (nbody - 1) / 2; p++) take(R.rin[p], R.rout[p], R.lam[p]);
+    return q;
+}
+
 // Every record has known types and a cluster type that is not excluded.
 Status fp_check(const Engine& eng, int slot, int nbody, long long n, const int* t, std::string& err) {
     const int nt = eng.params(slot).ntypes;
@@ -441,7 +534,7 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     const double binw = maxd / nbin;
     constexpr int T = 128;
     const size_t rec = nbody == 2 ? sizeof(FpRec<1>) : nbody == 3 ? sizeof(FpRec<3>) : sizeof(FpRec<6>);
-    const size_t smem = (size_t)nbin * 32 * 4 + rec * kFpTileJ;
+    const size_t smem = (size_t)(nbin + 1) * 32 * 4 + rec * kFpTileJ;
     // (a limit above the one it names, as it always was)
     if ((size_t)nbin * 32 * 4 + (nbody == 2 ? 8 : nbody == 3 ? 16 : 32) * (size_t)kFpTileJ > 200 * 1024) {
         err = "fingerprint histogram: nbin too large for the shared-memory histogram (at most 1280 bins)";
@@ -465,7 +558,7 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     };
     const size_t b1 = set_bytes(n1), b2 = same ? 0 : set_bytes(n2), bc = up16(sizeof(unsigned long long) * nbin);
     unsigned char* ws = nullptr;
-    FP_TRY(eng.workspace(b1 + b2 + bc + 16, ws));
+    FP_TRY(eng.workspace(b1 + b2 + bc + sizeof(int) * kFpFlags + sizeof(FpPair) * kFpTies, ws));
     struct Set {
         double* d;
         float *e, *m;
@@ -493,34 +586,61 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     if (!same) FP_TRY(edges(ws + b1, n2, d2, t2, s2));
     unsigned long long* dcounts = reinterpret_cast<unsigned long long*>(ws + b1 + b2);
     int* dflags = reinterpret_cast<int*>(ws + b1 + b2 + bc);
-    FP_TRY(cudaMemsetAsync(dcounts, 0, bc + 16, s));
     const long long n_it = (n1 + (long long)T * kFpRows - 1) / ((long long)T * kFpRows),
                     n_jt = (n2 + kFpTileJ - 1) / kFpTileJ;
     const void* kern = nbody == 2 ? (const void*)k_fp_hist<1> : nbody == 3 ? (const void*)k_fp_hist<3>
                                                                            : (const void*)k_fp_hist<6>;
     if (smem > 48 * 1024) allow_max_smem(kern);
-    int per_sm = 1;
-    FP_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem));
-    long long grid = (long long)sm_count() * std::max(1, per_sm);
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, smem);
+    long long grid = (long long)sm_count() * (occ > 0 ? occ : 1);
     if (grid > n_it * n_jt) grid = n_it * n_jt;
     const int sm = same ? 1 : 0;
-    if (nbody == 2)
-        count_launch(), k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
-    else if (nbody == 3)
-        count_launch(), k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
-    else
-        count_launch(), k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, s1.d, n1, s2.e, s2.m, s2.d, n2, sm,
-                                                                    nbin, binw, maxd, n_it, n_jt, dcounts, dflags);
-    FP_TRY(cudaGetLastError());
     std::vector<unsigned long long> hc(nbin);
-    int hflag = 0;
-    FP_TRY(cudaMemcpyAsync(hc.data(), dcounts, sizeof(unsigned long long) * nbin, cudaMemcpyDeviceToHost, s));
-    FP_TRY(cudaMemcpyAsync(&hflag, dflags, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FP_TRY(cudaStreamSynchronize(s));
+    int hflag[2] = {0, 0};   // a distance past the last bin; pairs to list
+    // q: kFpEtaMargin's, 0 with the host's edges
+    auto histogram = [&](float q) -> cudaError_t {
+        cudaError_t e = cudaMemsetAsync(dcounts, 0, bc + sizeof(int) * kFpFlags, s);
+        if (e != cudaSuccess) return e;
+        const FpCall C{s1.d, s2.d, binw, maxd, nbin, (float)(1.0 / binw), q, dflags};
+        count_launch();
+        if (nbody == 2)
+            k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
+        else if (nbody == 3)
+            k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
+        else
+            k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = cudaMemcpyAsync(hc.data(), dcounts, sizeof(unsigned long long) * nbin, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hflag, dflags, sizeof(hflag), cudaMemcpyDeviceToHost, s);
+        return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    };
+    const float shift = 0x1.03p-50f * 2.0f * (float)(std::sqrt((double)np) * fp_shift(eng, slot, nbody) / binw);
+    if (std::isfinite(shift)) FP_TRY(histogram(shift));
+    if (!std::isfinite(shift) || hflag[1] > kFpTies) {
+        auto host_edges = [&](long long n, const double* d, const int* t, const Set& out) -> cudaError_t {
+            std::vector<double> e((size_t)n * np);
+            for (long long c = 0; c < n; c++) fp_host_edges(eng, slot, nbody, c, d, t, &e[(size_t)c * np]);
+            return cudaMemcpy(out.d, e.data(), sizeof(double) * e.size(), cudaMemcpyHostToDevice);
+        };
+        FP_TRY(cudaStreamSynchronize(s));
+        FP_TRY(host_edges(n1, d1, t1, s1));
+        if (!same) FP_TRY(host_edges(n2, d2, t2, s2));
+        FP_TRY(histogram(0.0f));
+    } else if (hflag[1] > 0) {
+        std::vector<FpPair> tie(hflag[1]);
+        FP_TRY(cudaMemcpy(tie.data(), dflags + kFpFlags, sizeof(FpPair) * tie.size(), cudaMemcpyDeviceToHost));
+        for (const FpPair& q : tie) {
+            double a[6], b[6];
+            fp_host_edges(eng, slot, nbody, q.i, d1, t1, a);
+            fp_host_edges(eng, slot, nbody, q.j, same ? d1 : d2, same ? t1 : t2, b);
+            const int bin = fp_host_bin(a, b, np, binw, maxd, nbin);
+            if (bin < 0) hflag[0] = 1;
+            else hc[bin]++;
+        }
+    }
 #undef FP_TRY
-    if (hflag) {
+    if (hflag[0]) {
         err = "ERROR: computed bin larger than nbins (a cluster distance lies past the histogram range)";
         return kErrInput;
     }

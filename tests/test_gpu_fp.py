@@ -146,3 +146,55 @@ def test_histogram_tile_edges(native_lib, system, nb, n1, n2, nbin):
     oc, ons = o.fp_histogram(nb, *s1, *s2, nbin=nbin)
     assert ns == ons == (n1 * n2 if n2 else n1 * (n1 - 1) // 2)
     assert np.array_equal(counts, oc)
+
+
+@pytest.mark.parametrize("nb", [2, 3, 4])
+@pytest.mark.parametrize("many", [False, True])
+def test_histogram_at_bin_edges(native_lib, system, nb, many):
+    """Records whose distance to the first one crosses a bin edge within a few units
+    in the last place of one of their distances: the counts follow the tool's
+    host arithmetic exactly.  many: more such pairs than the device lists."""
+    import math
+    from chimes_calculator_gb300 import Calculator
+    p, o, nl = system
+    c = Calculator()
+    c.load_params(p)
+    npair = nb * (nb - 1) // 2
+    rng = np.random.default_rng(40 + nb)
+    nbin = 250
+    maxd = 3.0 if nb == 2 else math.sqrt(12.0 if nb == 3 else 24.0) + 1.0
+    w = maxd / nbin
+    rout = o.max_cutoffs[nb - 2]   # (one cutoff per body order beyond pairs; a pair type's own is below)
+    first = np.linspace(1.4, 0.8 * rout, npair)
+    records = [first, first + 0.1]
+    # the oracle's own counts locate the crossings: bin of (first, first with its last distance r)
+
+    def bin_of(r):
+        d = np.array([first, np.append(first[:-1], r)])
+        return int(np.flatnonzero(o.fp_histogram(nb, d, np.zeros((2, nb), np.int32), nbin=nbin)[0])[0])
+    r0 = float(first[-1])
+    for r1 in (1.0, 0.98 * rout):
+        for target in sorted({bin_of(r) for r in np.linspace(r0, r1, 400)})[1:]:
+            lo, hi = r0, r1
+            while True:
+                mid = 0.5 * (lo + hi)
+                if mid in (lo, hi):
+                    break
+                if bin_of(mid) < target:
+                    lo = mid
+                else:
+                    hi = mid
+            for side in (-1.0, 1.0):
+                r = lo
+                for _ in range(6):
+                    records.append(np.append(first[:-1], r))
+                    r = math.nextafter(r, side * 1e9)
+    d = np.array(records)
+    if many:
+        d = np.concatenate([np.repeat(d[:1], 400, axis=0), d[1:]])
+    d = d[:, rng.permutation(npair)] if npair > 1 else d
+    t = np.zeros((len(d), nb), dtype=np.int32)
+    got, ns = c.fp_histogram(nb, d, t, nbin=nbin)
+    want, wns = o.fp_histogram(nb, d, t, nbin=nbin)
+    assert len(d) > 200 and ns == wns
+    assert np.array_equal(got, want)
