@@ -132,6 +132,10 @@ struct FpPair {
 };
 constexpr int kFpTies = 1 << 16;   // pairs listed (more: the host makes all edges)
 constexpr int kFpFlags = 4;        // words before them: a distance past the last bin; pairs to list
+// Tiles a block takes in one launch: each adds at most kFpTileJ per record of four
+// warps' threads to one of the block's 32-bit counts.
+constexpr int kFpBlockTiles = 1 << 20;
+static_assert((long long)kFpBlockTiles * kFpTileJ * kFpRows * 4 < 1LL << 32, "counts of a lane's column");
 
 // Counts records i and j in FP64, where the FP32 candidate is not certified (margins:
 // the sum of theirs; hist: the lane's column).  Called and not inlined: its registers
@@ -602,14 +606,18 @@ Status fp_histogram(Engine& eng, int slot, int nbody, long long n1, const double
     auto histogram = [&](float q) -> cudaError_t {
         cudaError_t e = cudaMemsetAsync(dcounts, 0, bc + sizeof(int) * kFpFlags, s);
         if (e != cudaSuccess) return e;
+        const long long ntiles = n_it * n_jt, step = grid * kFpBlockTiles;
         const FpCall C{s1.d, s2.d, binw, maxd, nbin, (float)(1.0 / binw), q, dflags};
-        count_launch();
-        if (nbody == 2)
-            k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
-        else if (nbody == 3)
-            k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
-        else
-            k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, 0, n_it * n_jt, n_jt, dcounts, C);
+        for (long long t0 = 0; t0 < ntiles; t0 += step) {
+            const long long t1 = std::min(ntiles, t0 + step);
+            count_launch();
+            if (nbody == 2)
+                k_fp_hist<1><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, t0, t1, n_jt, dcounts, C);
+            else if (nbody == 3)
+                k_fp_hist<3><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, t0, t1, n_jt, dcounts, C);
+            else
+                k_fp_hist<6><<<(unsigned)grid, T, smem, s>>>(s1.e, s1.m, n1, s2.e, s2.m, n2, sm, t0, t1, n_jt, dcounts, C);
+        }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         e = cudaMemcpyAsync(hc.data(), dcounts, sizeof(unsigned long long) * nbin, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(hflag, dflags, sizeof(hflag), cudaMemcpyDeviceToHost, s);
