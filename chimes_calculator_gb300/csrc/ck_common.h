@@ -87,10 +87,11 @@ struct TupleRec {
     // DevParamSet::tc3 (3-body tuples) or tc4 (4-body tuples), in floats; -1
     // when absent
     int tc_off, tc_pad;
-    // fixed-point form (FP64; see FxStream): the tuple's stream in fx3 / fx4,
+    // fixed-point form (FP64; streams at FxPair, FxEnt below): the tuple's stream in fx3 / fx4,
     // its parts' boundaries and the power of two its coefficients are scaled by
     int fx_off, fx_split[9];
-    int fx_zbits;      // bits that a group's sum stays below the whole tuple's (see ck_direct.cu)
+    int fx_z[2];       // 4-body: bits of the sums of rows and of columns (kFxZr ...)
+    int fx_zbits;      // bits that a group's sum stays below the whole tuple's (ck_direct.cu)
     double fx_amp;
     double rin[6], rout[6], lam[6], xavg[6], xdiff[6];
     // reciprocals for the factored kernels: 1/lam, 1/xdiff, and the cutoff's
@@ -117,7 +118,7 @@ constexpr int kFactMaxDim = 128;   // largest R^K and R^(P-K) kept in shared mem
 
 // Fixed-point coefficient streams of the FP64 form (ck_fixed.cuh).  A tuple's
 // coefficients are scaled by 2^-e, fx_amp = 2^e the smallest power of two with
-// sum |a| <= 0.9 fx_amp and max |a| <= 0.24 fx_amp, and kept at 2^kFxCoef as two
+// sum |a| <= 0.9 fx_amp and max |a| <= 0.24 fx_amp (3-body: and kFxZ3's bounds), and kept at 2^kFxCoef as two
 // limbs {h, l}, a = h 2^kFxLimb + l.
 //   3-body: per column J = (q_ik, q_jk) with coefficients, in ascending order, a
 //   header {q_ik, q_jk, mask of its groups, 0}, then for g = 0..(R + 1) / 2 - 1
@@ -140,6 +141,19 @@ constexpr int kFxMore = (int)0x80000000u;
 constexpr int kFxLimb = 28;
 constexpr int kFxCoef = 61;
 constexpr int kFxSum = 59;
+constexpr int kFxDer = 1;     // dT tables have this many more bits than T tables
+// Bits that the kinds of sums that are cut to values stay below a tuple's full scale.  With
+// |T| <= 1 and |dT| <= n^2 2^-kd each kind has a bound from the coefficients, and its z says that
+// the sum cut to 2^(59 + z) stays below 2^59 and that what it is multiplied into stays below 2^63.
+// 3-body: kFxZ3 (sums over a row, a column, a run of q_ik), kFxZ3 + kFxDer with dT for a factor, by
+// the choice of the amplitude.  4-body: TupleRec::fx_z, four bits each of either side: record sums;
+// over the last pair's power, with T and with dT; over the middle one's: T of the first, dT of the
+// first, T of the second.
+constexpr int kFxZ3 = kFxCoef - kFxSum;
+enum { kFxZr, kFxZra, kFxZrb, kFxZP, kFxZQ, kFxZR };
+constexpr int kFxZRec = 4;    // most bits of a record sum
+constexpr int kFxZMax = 8;    // most bits of the others
+CK_HD constexpr int fx_zget(int z, int k) { return (z >> (4 * k)) & 15; }
 CK_HD constexpr int fx_kd(int R) {   // bits of (R - 1)^2: the dT tables' scale
     int k = 1;
     while ((1 << k) < (R - 1) * (R - 1)) k++;

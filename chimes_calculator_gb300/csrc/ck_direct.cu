@@ -166,9 +166,12 @@ __global__ void __launch_bounds__(256) k_directx(const DevParamSet* Pp, int n, c
         morse_x(r, R.rin[p], R.lam[p], R.xavg[p], R.xdiff[p], xd, dxdr, oor);
         fcut_eval<double>(P, r, R.rout[p], fc, fcd);
         const int kd = fx_kd(Rp);
-        const double gs = dxdr * (double)(1 << kd);
-        pair_tables_x(P, r, R.rin[p], xd, gs, Rp, kd, fc, fcd,
-                      [&](int k, const Fx& a, const Fx& b) { tab[k] = FxEnt{a.h, a.l, b.h, b.l}; });
+        double gs = dxdr * (double)(1 << kd);
+        // (D at T's scale: the room that the lane's sums have goes to zb)
+        pair_tables_x(P, r, R.rin[p], xd, gs, Rp, kd, fc, fcd, [&](int k, const Fx& a, const Fx& b) {
+            const Fx d = fx_split((((long long)b.h << kFxLimb) + b.l + 1) >> kFxDer);
+            tab[k] = FxEnt{a.h, a.l, d.h, d.l};
+        });
         if (r != r) fc = fcd = r;   // (a distance that is no number: the cluster's results are none)
         q[0] = fc; q[1] = fcd; q[2] = gs;
     }

@@ -32,7 +32,9 @@
 // Measured (GB300, 384 configurations of 8-512 atoms, 12/10/4, 1.81 M triplets
 // and 358 k quadruplets): 3-body 1.48 ms and 4-body 0.86 ms, against 5.91 and
 // 3.12 ms for the FP64 factored kernels that this form replaced and 3.27 and
-// 1.63 ms with the pairs set up per cluster.  Bound by the integer
+// 1.63 ms with the pairs set up per cluster.  (With the bits of single clusters,
+// ck_fixed.cuh, the stages take 1.47 and 1.00 ms against 1.53 and 0.99 before: the
+// 3-body sums need no shift now, the 4-body ones a variable one.)  Bound by the integer
 // multiply-adds (about half of the pipe's rate) and the latency that 16 warps
 // per SM leave exposed.
 #include <cuda_runtime.h>
@@ -358,13 +360,13 @@ __device__ __forceinline__ bool fx_setup(const BatchView& B, const int* clusters
     return active;
 }
 
-// The warps' parts of S and the G's, added and turned into force scalars (ENT,
+// The warps' parts of S and the G's (at 2^(kFxSum + ez)), added and turned into force scalars (ENT,
 // added to the pairs' entries) or forces by warp 0.
 //   f_p = (prod_{q != p} fc_q / r_p) (fc_p G_p + fc'_p S), E = prod fc S
 template <int NB, int NW, bool ENT, typename Acc>
 __device__ __forceinline__ void fx_finish(const BatchView& B, const int* clusters, int c,
                                           const FxSmem<NB, NW, ENT>& m, const TupleRec& R, bool active,
-                                          const int* ent, const long long* own, Acc& acc) {
+                                          const int* ent, const long long* own, const int* ez, Acc& acc) {
     constexpr int NP = Topo<NB>::NP;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (NW > 1) {
@@ -376,7 +378,7 @@ __device__ __forceinline__ void fx_finish(const BatchView& B, const int* cluster
     for (int k = 0; k <= NP; k++) {
         long long v = own[k];
         for (int u = 1; u < NW; u++) v += m.part[(u * (NP + 1) + k) * kFxTile + lane];
-        (k == 0 ? S : G[k - 1]) = from_fixed(v, 0);
+        (k == 0 ? S : G[k - 1]) = from_fixed(v, -ez[k]);
     }
     const double unit = R.fx_amp * kFxUnit;
     int s = 0;
@@ -561,7 +563,8 @@ __global__ void __launch_bounds__(32 * NW, RX <= 10 ? 16 / NW : 1) k_forcex3(Bat
                 g0.mac(Fx{t.z, t.w}, zv);
             }
         const long long own[4] = {S.sum(), g0.sum(), g1.sum(), g2.sum()};
-        fx_finish<3, NW, ENT>(B, clusters, c, m, *R, active, ent, own, acc);
+        constexpr int ez[4] = {kFxZ3, kFxZ3 + kFxDer, kFxZ3 + kFxDer, kFxZ3 + kFxDer};
+        fx_finish<3, NW, ENT>(B, clusters, c, m, *R, active, ent, own, ez, acc);
     }
     if (w == 0) acc.flush_warp(B);
 }
@@ -574,13 +577,15 @@ __global__ void __launch_bounds__(32 * NW, RX <= 10 ? 16 / NW : 1) k_forcex3(Bat
 // pair's power, then the middle one's, then the first one's, as their records
 // are sorted: out[0] = sum_I X_I z_I, out[1..3] = the three pairs' gradients.
 __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, int o1, const FxPair* V, const FxEnt* t,
-                                        int rs, long long* out) {
+                                        int rs, int fz, long long* out) {
     const FxEnt *t1 = t + rs * kFxTile, *t2 = t1 + rs * kFxTile;
+    const FxCut cr(fx_zget(fz, kFxZr));
     FxAcc S, g0, g1, g2, ra, rb, rP, rQ, rR;
     int q0 = -1, q1 = -1;
     auto fold1 = [&]() {
         if (q1 < 0) return;
-        const Fx a = ra.value(), b = rb.value();
+        const Fx a = ra.value(fx_zget(fz, kFxZr) - fx_zget(fz, kFxZra)),
+                 b = rb.value(fx_zget(fz, kFxZr) + kFxDer - fx_zget(fz, kFxZrb));
         const FxEnt v = t1[q1 * kFxTile];
         rP.mac(Fx{v.x, v.y}, a);
         rQ.mac(Fx{v.z, v.w}, a);
@@ -590,17 +595,17 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
     };
     auto fold0 = [&]() {
         if (q0 < 0) return;
-        const Fx p = rP.value();
+        const Fx p = rP.value(fx_zget(fz, kFxZra) - fx_zget(fz, kFxZP));
         const FxEnt v = t[q0 * kFxTile];
         S.mac(Fx{v.x, v.y}, p);
         g0.mac(Fx{v.z, v.w}, p);
-        g1.mac(Fx{v.x, v.y}, rQ.value());
-        g2.mac(Fx{v.x, v.y}, rR.value());
+        g1.mac(Fx{v.x, v.y}, rQ.value(fx_zget(fz, kFxZra) + kFxDer - fx_zget(fz, kFxZQ)));
+        g2.mac(Fx{v.x, v.y}, rR.value(fx_zget(fz, kFxZrb) - fx_zget(fz, kFxZR)));
         rP = FxAcc();
         rQ = FxAcc();
         rR = FxAcc();
     };
-    FxRec z;
+    FxRec z(cr);
     FxEnt q[4], n[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) q[k] = ent[o + k];   // (a side without entries reads its neighbour's: in bounds)
@@ -621,11 +626,11 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
                 q0 = r0;
                 q1 = r1;
             }
-            const Fx zv = z.value();
+            const Fx zv = z.value(cr);
             const FxEnt v = t2[r2 * kFxTile];
             ra.mac(Fx{v.x, v.y}, zv);
             rb.mac(Fx{v.z, v.w}, zv);
-            z = FxRec();
+            z = FxRec(cr);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) q[k] = n[k];
@@ -641,7 +646,7 @@ __device__ __forceinline__ void fx_side(const FxEnt* __restrict__ ent, int o, in
 // With one warp it takes the rows, then the columns; with more, half of the
 // warps take the rows and half the columns.
 template <int NW, bool ENT>
-__global__ void __launch_bounds__(32 * NW) k_forcex4(BatchView B, const int* clusters, const int* perm,
+__global__ void __launch_bounds__(32 * NW, NW > 1 ? (ENT ? 16 : 12) / NW : 1) k_forcex4(BatchView B, const int* clusters, const int* perm,
                                                      const long long* perm_n, long long perm_cap, int rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     const FxSmem<4, NW, ENT> m(smem, rs);
@@ -674,25 +679,34 @@ __global__ void __launch_bounds__(32 * NW) k_forcex4(BatchView B, const int* clu
         __syncthreads();
         const bool ok = ck_bound(B, R->fx_off >= 0 && R->fx_off + (long long)R->fx_split[8] <= P->n_fx4);
         const FxEnt* ent = P->fx4 + R->fx_off;
+        const int* fz = R->fx_z;
         long long own[7] = {0, 0, 0, 0, 0, 0, 0};
         if (NW == 1) {
             long long b[4];
-            fx_side(ent, ok ? R->fx_split[0] : 0, ok ? R->fx_split[4] : 0, Y + lane, T, rs, own);
-            fx_side(ent, ok ? R->fx_split[4] : 0, ok ? R->fx_split[8] : 0, X + lane, T + 3 * rs * kFxTile, rs, b);
+            fx_side(ent, ok ? R->fx_split[0] : 0, ok ? R->fx_split[4] : 0, Y + lane, T, rs, fz[0], own);
+            fx_side(ent, ok ? R->fx_split[4] : 0, ok ? R->fx_split[8] : 0, X + lane, T + 3 * rs * kFxTile, rs, fz[1], b);
             for (int k = 1; k < 4; k++) own[3 + k] = b[k];
         } else {
             constexpr int H = NW > 1 ? NW / 2 : 1;   // warps per side
             const int side = w / H, k0 = 4 * side + 4 * (w % H) / H, k1 = 4 * side + 4 * (w % H + 1) / H;
             long long a[4];
             fx_side(ent, ok ? R->fx_split[k0] : 0, ok ? R->fx_split[k1] : 0, (side ? X : Y) + lane,
-                    T + 3 * side * rs * kFxTile, rs, a);
+                    T + 3 * side * rs * kFxTile, rs, fz[side], a);
             own[0] = side ? 0 : a[0];
             for (int k = 1; k < 4; k++) {
                 own[k] = side ? 0 : a[k];
                 own[3 + k] = side ? a[k] : 0;
             }
         }
-        fx_finish<4, NW, ENT>(B, clusters, c, m, *R, active, ent6, own, acc);
+        int ez[7];
+        ez[0] = fx_zget(fz[0], kFxZP);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            ez[1 + 3 * k] = fx_zget(fz[k], kFxZP) + kFxDer;
+            ez[2 + 3 * k] = fx_zget(fz[k], kFxZQ);
+            ez[3 + 3 * k] = fx_zget(fz[k], kFxZR);
+        }
+        fx_finish<4, NW, ENT>(B, clusters, c, m, *R, active, ent6, own, ez, acc);
     }
     if (w == 0) acc.flush_warp(B);
 }

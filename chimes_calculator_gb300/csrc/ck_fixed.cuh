@@ -10,10 +10,20 @@
 // absolute one of 2^-57 or less of full scale (FP64 rounds each partial sum
 // at 2^-53 of its own size).
 //
-//   Fx    value h 2^28 + l, |l| <= 2^27: T, dT, X and Y at 2^56, record sums
-//         at 2^59, coefficients at 2^61
+//   Fx    value h 2^28 + l, |l| <= 2^27: T, X and Y at 2^56, dT at 2^57,
+//         coefficients at 2^61
 //   FxRec, FxAcc sums of products: hi += a.h b.h, mid += a.h b.l + a.l b.h (the
 //         low x low product, below 2^-62 of full scale, is dropped)
+//
+// A sum that goes into a further product is cut to a value at 2^(59 + z), z as many
+// bits as that kind of sum stays below the tuple's full scale (a sum over a row, a
+// column or a run of them is small beside the whole tuple's, one with dT for a factor
+// all the more): 3-body two, three with dT, which the amplitude grants; 4-body by
+// tuple (TupleRec::fx_z).  Errors of one cluster against long double, in the mean over
+// random clusters of 255 (3-body, 10 powers) and 281 coefficients (4-body, 4 powers),
+// force sums relative to the cluster's largest: 2.7e-16 and 1.7e-16 (FP64: 4.1e-16 and
+// 2.7e-16; every sum cut at 2^59 and dT at 2^56: 2.0e-15 and 1.7e-15, which made whole
+// evaluations of single triplets 2.61e-15 where the FP64 kernels had 2.16e-15; 2.1e-15 now).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -57,20 +67,31 @@ __device__ __forceinline__ Fx fx_mul(const Fx& a, const Fx& b) {
     return fx_limbs(m);
 }
 
-// A record sum, kept at 2^kFxCoef with the constants of `value` already in it.
+// How 4-body record sums become values: shift from 2^63 and the constants of the
+// rounding and of fx_limbs, added where a sum starts.
+struct FxCut {
+    long long hi, mid;
+    int sh;
+    __device__ __forceinline__ explicit FxCut(int z)
+        : hi(1LL << (kFxLimb + 1 - z)), mid(z < kFxZRec ? 1LL << (kFxLimb + 1 - z) : 0), sh(kFxZRec - z) {}
+};
+
+// A record sum, kept at 2^kFxCoef (with the constants of its value already in it).
 struct FxRec {
-    long long hi = 1LL << (kFxCoef - kFxSum + kFxLimb - 1), mid = 0;
+    long long hi = 1LL << (kFxLimb - 1), mid = 1LL << (kFxLimb - 1);
+    FxRec() = default;
+    __device__ __forceinline__ explicit FxRec(const FxCut& c) : hi(c.hi), mid(c.mid) {}
     __device__ __forceinline__ void mac(const Fx& a, const Fx& b) {
         imad(hi, a.h, b.h);
         imad(mid, a.h, b.l);
         imad(mid, a.l, b.h);
     }
-    // the sum as a value at 2^kFxSum
-    __device__ __forceinline__ Fx value() const {
-        constexpr int D = kFxCoef - kFxSum;
-        const long long v = hi + (mid >> kFxLimb);
-        return Fx{(int)(v >> (kFxLimb + D)),
-                  (int)(((unsigned)v & ((1u << (kFxLimb + D)) - 1u)) >> D) - (1 << (kFxLimb - 1))};
+    // the sum as a value at its own scale (two bits finer than 2^kFxSum)
+    __device__ __forceinline__ Fx value() const { return fx_limbs(hi + (mid >> kFxLimb)); }
+    // and at 2^(kFxSum + z)
+    __device__ __forceinline__ Fx value(const FxCut& c) const {
+        constexpr int D = kFxSum + kFxZRec - kFxCoef;
+        return fx_limbs(((hi << D) + (mid >> (kFxLimb - D))) >> c.sh);
     }
 };
 
@@ -82,9 +103,11 @@ struct FxAcc {
         imad(mid, a.h, b.l);
         imad(mid, a.l, b.h);
     }
-    // the sum as an integer at its scale and as a value
+    // the sum as an integer at its scale, and as a value with d bits fewer
     __device__ __forceinline__ long long sum() const { return hi + ((mid + (1LL << (kFxLimb - 1))) >> kFxLimb); }
-    __device__ __forceinline__ Fx value() const { return fx_limbs(sum() + (1LL << (kFxLimb - 1))); }
+    __device__ __forceinline__ Fx value(int d = 0) const {
+        return fx_limbs((sum() + ((1LL << (kFxLimb - 1 + d)) + (1LL << d >> 1))) >> d);
+    }
 };
 constexpr double kFxUnit = 1.0 / (double)(1LL << kFxSum);
 
@@ -96,13 +119,15 @@ __device__ __forceinline__ long long fx_2x(long long x, long long t) {
 }
 
 // The Chebyshev recursions at x (in [-1, 1]): f(n, T_n, n U_{n-1} 2^-kd), n =
-// 0..nT-1, both at 2^56 (T is kept at 2^60 and U, below 64, at 2^57 on the way).
+// 0..nT-1, T at 2^56 and the other at 2^(56 + kFxDer), both rounded (T is kept at
+// 2^60 and U, up to 31 where it is used, at 2^58 on the way).
 template <typename F>
 __device__ __forceinline__ void fx_chebyshev(double xd, int nT, int kd, F&& f) {
     const long long x = to_fixed(xd, 62);
-    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 57;   // T_n, T_{n+1}, U_{n-1}, U_n
+    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 58;   // T_n, T_{n+1}, U_{n-1}, U_n
     for (int n = 0; n < nT; n++) {
-        f(n, (tn + 8) >> 4, __mul64hi(um, (long long)n << (63 - kd)));
+        const long long d = __mul64hi(um, (long long)n << (63 - kd));
+        f(n, (tn + 8) >> 4, d + (((unsigned)um * (unsigned)n >> kd) & 1u));
         const long long t2 = fx_2x(x, tp) - tn, u2 = fx_2x(x, un) - um;
         tn = tp;
         tp = t2;
@@ -135,7 +160,7 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
 
 // T_n and D_n of a pair from its x and dx/dr 2^kd (see pair_setup_x).
 template <typename F>
-__device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, double rin, double xd, double gs, int nT,
+__device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, double rin, double xd, double& gs, int nT,
                                               int kd, double& fc, double& fcd, F&& put) {
     if (!less_pos(r, rin)) {
         fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
@@ -143,14 +168,14 @@ __device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, do
     }
     const double damp = exp((r - rin) / P.inner_smooth);
     const double k = P.inner_smooth * (damp - 1.0) * gs;
-    int s = 0;
-    for (double bound = 1.0 + fabs(k); bound > 1.0 && s < 40; s++) bound *= 0.5;
-    const double up = (double)(1LL << s), down = 1.0 / up;
+    const double bound = 1.0 + fabs(k);
+    const int s = bound > 1.0 ? min(ilogb(bound), 999) + 1 : 0;
+    const double up = __longlong_as_double((1023LL + s) << 52), down = __longlong_as_double((1023LL - s) << 52);
     fc *= up;
     fcd *= up;
+    gs *= damp * down;
     fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) {
-        put(n, fx_split(__double2ll_rn(((double)t + k * (double)d) * down)),
-            fx_split(__double2ll_rn((double)d * damp * down)));
+        put(n, fx_split(__double2ll_rn(((double)t + k * (1.0 / (1 << kFxDer)) * (double)d) * down)), fx_split(d));
     });
 }
 
@@ -158,8 +183,9 @@ __device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, do
 // set_polys_out_of_range, chimesFF.cpp:1572-1613): put(n, T_n, D_n) for n <
 // nT with D_n = n U_{n-1}(x) 2^-kd; fc and fc'; gs with dT_n/dr = gs D_n.
 // ex = exp(-r / lambda).  Below the inner cutoff the extrapolated T_n + k dT_n
-// can exceed one: both tables are scaled down by 2^s and fc, fc' carry the
-// 2^s (every term of S and of the G's has one factor of each pair).
+// can exceed one: T is scaled down by 2^s, fc, fc' carry the 2^s and gs the
+// exponential and 2^-s (every term of S has a T of each pair, those of a G a D of
+// its own).
 template <typename F>
 __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab& Q, double r, double ex, int nT,
                                              int kd, double& fc, double& fcd, double& gs, F&& put) {
@@ -189,7 +215,7 @@ __device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& p
         s.mac(c, fx_split(t));
         g.mac(c, fx_split(d));
     });
-    double S = from_fixed(s.sum(), -kFxCoef) * pr.fx_amp, G = from_fixed(g.sum(), -kFxCoef) * (pr.fx_amp * gs);
+    double S = from_fixed(s.sum(), -kFxCoef) * pr.fx_amp, G = from_fixed(g.sum(), -kFxCoef - kFxDer) * (pr.fx_amp * gs);
     if (oor) {
         atomicAdd(&flags[4], 1);
         const double damp = exp((r - pr.rin) / P.inner_smooth);

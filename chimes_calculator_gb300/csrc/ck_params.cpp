@@ -847,6 +847,65 @@ int fx_zbits(double amp, double group) {
     while (e < 10 && group * std::ldexp(2.0, e) <= 0.9 * amp) e++;
     return e;
 }
+// Largest absolute sum of the coefficients over the groups of one key, as a share
+// of the amplitude; with `der` those of a sum with dT of one pair, whose power it
+// gives, at the tables' scale: |dT_n| 2^-kd <= n^2 2^-kd.
+template <class K, class D>
+double fx_bound(const std::vector<FxCoef>& c, double amp, int R, K&& key, D&& der) {
+    std::map<int, double> sum;
+    double top = 0.0;
+    for (const FxCoef& q : c) {
+        const int n = der(q);
+        const double w = n < 0 ? 1.0 : std::ldexp((double)n * n, -fx_kd(R));
+        top = std::max(top, sum[key(q)] += std::fabs(q.a) / amp * w);
+    }
+    return top;
+}
+// Bits that a share stays below the amplitude's 0.9.
+int fx_bits(double share, int most) {
+    int z = 0;
+    while (z < most && share * std::ldexp(2.0, z) <= 0.9) z++;
+    return z;
+}
+// 3-body amplitude: with room for kFxZ3 more bits of the sums over a row, a column and a
+// run, one more with dT_jk, than of the whole tuple's.
+double fx_amplitude3(const std::vector<FxCoef>& c, int R) {
+    const auto none = [](const FxCoef&) { return -1; };
+    const auto run = [R](const FxCoef& q) { return q.col / R; };
+    double amp = fx_amplitude(c);
+    const double t = std::max({fx_bound(c, amp, R, [](const FxCoef& q) { return q.row; }, none),
+                               fx_bound(c, amp, R, [](const FxCoef& q) { return q.col; }, none),
+                               fx_bound(c, amp, R, run, none)});
+    const double d = fx_bound(c, amp, R, run, [R](const FxCoef& q) { return q.col % R; });
+    const double need = std::ldexp(std::max(t, std::ldexp(d, kFxDer)), kFxZ3) / 0.9;
+    for (double k = 1.0; k < need; k *= 2.0) amp *= 2.0;
+    return amp;
+}
+// The 4-body sums' bits, of the side whose records are c's rows.  A sum of terms at 2^(59 + z)
+// fits 64 bits while its own bits are z - 4 or more (z + kFxDer - 4 with dT), and is cut, not extended.
+int fx_z4(const std::vector<FxCoef>& c, double amp, int R) {
+    const auto none = [](const FxCoef&) { return -1; };
+    const auto all = [](const FxCoef&) { return 0; };
+    const auto p0 = [](const FxCoef& q) { return q.rowp & 31; };
+    const auto p1 = [](const FxCoef& q) { return (q.rowp >> kPowBits) & 31; };
+    const auto p2 = [](const FxCoef& q) { return (q.rowp >> (2 * kPowBits)) & 31; };
+    const auto p01 = [](const FxCoef& q) { return q.rowp & 1023; };
+    const int g0 = fx_bits(fx_bound(c, amp, R, all, p0), kFxZMax), g1 = fx_bits(fx_bound(c, amp, R, all, p1), kFxZMax),
+              g2 = fx_bits(fx_bound(c, amp, R, all, p2), kFxZMax);
+    int zP = std::min({fx_bits(fx_bound(c, amp, R, p0, none), kFxZMax), 4, g0 + 4 - kFxDer});
+    int zQ = std::min(fx_bits(fx_bound(c, amp, R, p0, p1), kFxZMax), g1 + 4);
+    int zR = std::min(fx_bits(fx_bound(c, amp, R, p0, p2), kFxZMax), g2 + 4);
+    int za = std::min({fx_bits(fx_bound(c, amp, R, p01, none), kFxZMax), zP + 4, zQ + 4 - kFxDer});
+    int zb = std::min(fx_bits(fx_bound(c, amp, R, p01, p2), kFxZMax), zR + 4);
+    int zr = fx_bits(fx_bound(c, amp, R, [](const FxCoef& q) { return q.row; }, none), kFxZRec);
+    zr = std::min({zr, za + 4, zb + 4 - kFxDer});
+    za = std::min(za, zr);
+    zb = std::min(zb, zr + kFxDer);
+    zP = std::min(zP, za);
+    zQ = std::min(zQ, za + kFxDer);
+    zR = std::min(zR, zb);
+    return zr << 4 * kFxZr | za << 4 * kFxZra | zb << 4 * kFxZrb | zP << 4 * kFxZP | zQ << 4 * kFxZQ | zR << 4 * kFxZR;
+}
 // splits of [0, total) into n parts at the record ends `ends` (ascending, the last = total), by weight
 void fx_parts(const std::vector<int>& ends, const std::vector<double>& weight, int n, int* split) {
     double all = 0.0, w = 0.0;
@@ -859,7 +918,7 @@ void fx_parts(const std::vector<int>& ends, const std::vector<double>& weight, i
     while (part <= n) split[part++] = ends.empty() ? split[0] : ends.back();
 }
 void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& out) {
-    R.fx_amp = fx_amplitude(c);
+    R.fx_amp = fx_amplitude3(c, Rp);
     R.fx_off = (int)out.size();
     std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
         return x.col != y.col ? x.col < y.col : x.row < y.row;
@@ -891,7 +950,7 @@ void fx3_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& 
     fx_parts(ends, weight, 8, R.fx_split);
     R.fx_zbits = fx_zbits(R.fx_amp, top);
 }
-void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
+void fx4_stream(std::vector<FxCoef> c, int Rp, TupleRec& R, std::vector<FxEnt>& out) {
     R.fx_amp = fx_amplitude(c);
     R.fx_off = (int)out.size();
     double top = 0.0;
@@ -901,6 +960,7 @@ void fx4_stream(std::vector<FxCoef> c, TupleRec& R, std::vector<FxEnt>& out) {
                 std::swap(q.row, q.col);
                 std::swap(q.rowp, q.colp);
             }
+        R.fx_z[side] = fx_z4(c, R.fx_amp, Rp);
         std::stable_sort(c.begin(), c.end(), [](const FxCoef& x, const FxCoef& y) {
             return x.row != y.row ? x.row < y.row : x.col < y.col;
         });
@@ -1099,6 +1159,8 @@ ParamImage pack_params(const HostParams& P) {
                 R.tc_off = O.tc_off;
                 R.fx_off = O.fx_off;
                 R.fx_amp = O.fx_amp;
+                R.fx_zbits = O.fx_zbits;
+                std::memcpy(R.fx_z, O.fx_z, sizeof(R.fx_z));
                 std::memcpy(R.fx_split, O.fx_split, sizeof(R.fx_split));
                 continue;
             }
@@ -1171,7 +1233,7 @@ ParamImage pack_params(const HostParams& P) {
                     fx3_stream(std::move(q), R_pow, R, fx3);
                     fx3_max = std::max(fx3_max, R.fx_split[8] / (1 + (R_pow + 1) / 2));
                 } else {
-                    fx4_stream(std::move(q), R, fx4);
+                    fx4_stream(std::move(q), R_pow, R, fx4);
                 }
             }
             shared[key] = u;
