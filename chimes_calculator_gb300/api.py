@@ -221,7 +221,9 @@ class Calculator:
         per-coefficient, 2 factored without the per-entry pair-table cache,
         3 factored with the 3-body column products formed per coefficient,
         4 factored with the 3-body and 4-body contractions on the tensor cores
-        (mixed form; tuning()["tc3"] and ["tc4"] report which run)."""
+        (mixed form; tuning()["tc3"] and ["tc4"] report which run; autotune then takes
+        the fastest 3-body form of small workloads too, which otherwise keep the
+        per-coefficient one and its roundings)."""
         self._check(self.lib.ck_set_contraction(self.h, int(factored)))
 
     def autotune(self, packed=None):

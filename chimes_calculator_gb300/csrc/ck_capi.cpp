@@ -362,6 +362,7 @@ int ck_set_contraction(void* h, int factored) {
     if (factored < 0 || factored > 4) return report(ck::kErrInput, "contraction mode must be 0, 1, 2, 3 or 4");
     ck::Engine& e = static_cast<Instance*>(h)->eng;
     e.factored = factored != 0;
+    e.any_form = factored == 4;
     e.pair_cache = factored != 2;
     e.tuning.noy3 = factored == 3 ? 1 : 0;
     e.tuning.want_tc3 = e.tuning.want_tc4 = factored == 4 ? 1 : 0;

@@ -735,7 +735,7 @@ Status Engine::run(const std::vector<SystemSpec>& sys, double* force_out, std::v
 }
 
 std::string Engine::tune_key() const {
-    std::string k = "p" + std::to_string(precision) + (factored ? "f" : "c");
+    std::string k = "p" + std::to_string(precision) + (factored ? any_form ? "t" : "f" : "c");
     std::vector<int> seen;
     for (const SysDesc& d : hsys_)
         if (std::find(seen.begin(), seen.end(), d.pset) == seen.end()) seen.push_back(d.pset);
@@ -840,14 +840,15 @@ Status Engine::autotune(int* chosen, std::string& err) {
         for (int t : {1, 2, 4, 8, 16, 32}) v.push_back({0, t, 0, 0, 0});
         return v;
     };
-    // The forms differ in FP32 rounding (1e-7 of the forces), so a workload should not
-    // change form for a few microseconds: where the set has a 3-body tensor-core form,
-    // that is taken against the per-coefficient one from one tile per SM on (one
-    // configuration), seven (a batch) or three (a batch of 50 or more small ones) --
-    // about where it began to win before it was made faster: 17-34 k triplets of one
-    // configuration, 67 k of 105, 130 k of 40 (now 54 k of 11 take 38 us against 98).
+    // The mixed forms differ in FP32 rounding (1e-7 of the forces, 1e-6 at most), and a tuned
+    // workload keeps the results it has always had, not only their accuracy: where the set has a
+    // 3-body tensor-core form, the per-coefficient one stays below one tile per SM (one
+    // configuration), seven (a batch) or three (a batch of 50 or more), where it was the faster one
+    // until the tensor-core kernel ran four CTAs per SM.  It no longer is (54 k triplets of 11
+    // configurations 98 us against 38, calls of 40 configurations 371 us against 269), so that
+    // asking for the tensor cores (ck_set_contraction(h, 4)) lifts the rule.
     const int tiles_per_sm = V_.n_sys == 1 ? 1 : V_.n_sys >= 50 ? 3 : 7;
-    const bool small3 = avail_tc3_ && last.n3 < 128LL * sm_count() * tiles_per_sm;
+    const bool small3 = !any_form && avail_tc3_ && last.n3 < 128LL * sm_count() * tiles_per_sm;
     const std::vector<Cand> c3 = cands(avail_fact3_, true, avail_tc3_), c4 = cands(avail_fact4_, false, avail_tc4_);
     auto apply = [&](int nb, const Cand& c) {
         if (nb == 3) {

@@ -142,6 +142,8 @@ public:
     // 3-/4-body contraction: true = factored kernels wherever every parameter
     // set of the batch has factored tables, false = per-coefficient kernels
     bool factored = true;
+    // the tuner takes the fastest 3-body form at every size (tensor cores asked for)
+    bool any_form = false;
     // run the 4-body branch on a second stream beside 1B+2B and 3-body (not while profiling)
     bool concurrent = true;
     // pairs' tables once per list entry: FP64 the pair-entry form (ck_fixed.cu), mixed the

@@ -95,7 +95,8 @@ int ck_set_tuning(void *h, int tpc3, int tpc4, int blocks_per_sm);
  * with a three-part split of both operands) in the mixed form, where every
  * parameter set of the batch has 2-11 powers per pair (3-body) and one
  * count of 2-4 powers per pair (4-body) (ck_autotune also tries these in the
- * mixed form).  All give the same sums in another rounding
+ * mixed form, but gives a small workload's 3-body term to the per-coefficient
+ * kernels, whose roundings it has always had, unless this was asked for).  All give the same sums in another rounding
  * order. */
 int ck_set_contraction(void *h, int factored);
 /* Autotuner for the batch staged with ck_stage_batch: times the 3-body and

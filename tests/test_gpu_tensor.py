@@ -36,3 +36,35 @@ def test_widths_and_remainders(tmp_path, native_lib, cuts, o3, o4, n, rin):
     assert abs(got["energy"] - ref["energy"]) <= MIXED_E_REL_TOL * max(1.0, abs(ref["energy"]))
     assert np.abs(got["force"] - ref["force"]).max() <= mixed_force_tol(np.abs(ref["force"]).max())
     assert np.abs(got["stress"] - ref["stress"]).max() <= MIXED_S_ABS_TOL * big
+
+
+def test_small_batch_takes_the_faster_form(tmp_path, native_lib):
+    """Autotuning with the tensor cores asked for takes the fastest 3-body form it timed,
+    in a batch of a few tiles too: the tensor-core kernel needs less than half of the
+    per-coefficient kernels' time for these 60 thousand triplets, 1.5 is allowed."""
+    import ctypes
+
+    from chimes_calculator_gb300 import MIXED, Calculator, synth
+    spec = synth.ParamSpec(elements=["C", "N"], orders=(12, 10, 4), rin=0.9, rout=5.0, lam=1.4, s3max=4.0, s4max=3.4,
+                           seed=61)
+    path = synth.write_param_file(str(tmp_path / "p.txt"), spec)
+    side = (110 / 0.09) ** (1.0 / 3.0)
+    cfgs = [synth.random_config(110, np.diag([side] * 3), ["C", "N"], 1.0, seed=17 + k) for k in range(11)]
+    ms = {}
+    for tuned in (True, False):
+        c = Calculator(precision=MIXED)
+        c.set_contraction(4)
+        c.load_params(path)
+        packed = c.pack([(q.pos, q.types, q.cell) for q in cfgs])
+        if tuned:
+            c.autotune(packed)
+        c.stage(packed)
+        t, n, k = (ctypes.c_double * 4)(), ctypes.c_longlong(), ctypes.c_int()
+        for _ in range(2):   # (the first launches size the lists)
+            c.lib.ck_set_profiling(c.h, 1)
+            for _ in range(10):
+                c.launch()
+                c.lib.ck_read_stage_times(c.h, t, ctypes.byref(n), ctypes.byref(k))
+                c.collect()
+        ms[tuned] = t[2] / n.value
+    assert ms[True] <= 1.5 * ms[False], ms
