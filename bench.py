@@ -126,8 +126,8 @@ class ClockSampler:
 # DRAM bytes (read + write) per launch of the force kernels on this workload,
 # from one ncu capture each (profiles/kernels_c2_fp64.md, k_forcen_c2_fp64.md)
 PROFILED_TRAFFIC = {
-    "k_forcex3": 4477440,
-    "k_forcex4": 2490112,
+    "k_forcex3": 4501504,
+    "k_forcex4": 2532352,
     "k_forcen<3,double,4>": 872704,
     "k_forcen<4,double,8>": 599552,
 }
@@ -172,7 +172,7 @@ def algorithmic_flops(calc, cfg, params_path):
     out = {}
     for nb, lst, order in ((3, l3, o3), (4, l4, o4)):
         if lst.shape[0] == 0 or order == 0:
-            out[nb] = (0, 0.0, 0.0)
+            out[nb] = (0, 0.0, 0.0, 0.0)
             continue
         P = nb * (nb - 1) // 2
         pairs = [(i, j) for i in range(nb) for j in range(i + 1, nb)]
@@ -201,7 +201,12 @@ def algorithmic_flops(calc, cfg, params_path):
         ex = ok.sum() * (P * (6 * order + 15) + P * 21 + R ** C * (C - 1) + R ** K * (K - 1)) \
             + (4.0 * nc).sum() + (per_row * nrow[u][ok].astype(np.float64)).sum() \
             + (per_col * ncol[u][ok].astype(np.float64)).sum()
-        out[nb] = (int(ok.sum()), float(flops), float(ex))
+        # integer multiply-adds of the fixed-point kernels: three for each of the two sums a
+        # coefficient enters, for each product of the row and column pairs, and for each of
+        # the two sums a record's value enters
+        prod = ncol[u][ok].sum() if nb == 3 else ok.sum() * 2 * (R ** 2 + R ** 3)
+        imad = 3.0 * (2 * nc.sum() + prod + 2 * (nrow[u][ok].sum() + ncol[u][ok].sum()))
+        out[nb] = (int(ok.sum()), float(flops), float(ex), float(imad))
     return out
 
 
@@ -310,16 +315,19 @@ def run_ours(args):
     names = ["list build", "force 1B+2B", "force 3B", "force 4B"]
     counts = calc.counts()
     work = algorithmic_flops(calc, cfg, params)
-    # FP64 FMA probe, repeated for half a second with the SM clock sampled
-    # beside it (the roofline denominator and the clock it was measured at)
-    peak64 = ctypes.c_double()
+    # FP64 FMA and integer multiply-add probes, repeated for half a second with the SM
+    # clock sampled beside them (the roofline denominators and the clock they were measured at)
+    peak64, peak_int = ctypes.c_double(), ctypes.c_double()
     probe_clk = ClockSampler(local)
     probe_clk.start()
-    probes, t_probe = [], time.perf_counter()
+    probes, probes_int, t_probe = [], [], time.perf_counter()
     while len(probes) < 200 and (time.perf_counter() - t_probe < 0.5 or len(probes) < 3):
         lib.ck_fma_peak(0, ctypes.byref(peak64))
+        lib.ck_fma_peak(2, ctypes.byref(peak_int))
         probes.append(peak64.value)
+        probes_int.append(peak_int.value)
     peak64.value = statistics.median(probes)
+    peak_int.value = statistics.median(probes_int)
     probe_s = time.perf_counter() - t_probe
     probe_clocks = probe_clk.stop()
     # the dominant single kernel: the list build is ten short kernels, each
@@ -330,24 +338,30 @@ def run_ours(args):
     if dom in (2, 3):
         nb = 3 if dom == 2 else 4
         fact = tun["fact%d" % nb]
-        # the factored form runs in 64-bit fixed point on the integer pipe; its rate is
-        # put against the FP64 one, whose work it replaces
         kname = "k_forcex%d" % nb if fact else "k_forcen<%d,double,%d>" % (nb, tun["tpc%d" % nb])
         traffic, traffic_src = PROFILED_TRAFFIC.get(kname), None
         if traffic is not None:
             traffic_src = "ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel on this workload (profiles/)"
         achieved = work[nb][1] / (stage[dom] * 1e-3) / 1e12
         executed = (work[nb][2] if fact else work[nb][1]) / (stage[dom] * 1e-3) / 1e12
-        roof = {"bound": "fp64", "kernel": kname, "achieved": achieved,
-                "peak": peak64.value, "unit": "TFLOP/s", "frac": achieved / peak64.value,
+        # the fixed-point form is bound by the integer multiply-add rate, the
+        # per-coefficient form by FP64
+        imad = work[nb][3] / (stage[dom] * 1e-3) / 1e12
+        bound, achieved_b, peak, unit = ("int", imad, peak_int.value, "T multiply-adds/s") if fact else \
+            ("fp64", achieved, peak64.value, "TFLOP/s")
+        roof = {"bound": bound, "kernel": kname, "achieved": achieved_b,
+                "peak": peak, "unit": unit, "frac": achieved_b / peak,
                 "traffic": traffic,
                 "traffic_source": traffic_src,
-                "peak_source": "measured in-run FP64 FMA probe (ck_fma_peak, median of %d runs over %.2f s); "
-                "MEASURED_PEAKS.json has no CUDA-core FP64 figure" % (len(probes), probe_s),
+                "peak_source": "measured in-run %s probe (ck_fma_peak, median of %d runs over %.2f s); "
+                "MEASURED_PEAKS.json has no such figure" % (
+                    "32 x 32 + 64 bit integer multiply-add" if fact else "FP64 FMA", len(probes), probe_s),
                 "peak_clocks": probe_clocks,
                 "flops_per_launch": work[nb][1], "clusters_evaluated": work[nb][0],
+                "integer_multiply_adds_per_launch": work[nb][3] if fact else None,
+                "tflops": achieved, "fp64_peak_tflops": peak64.value,
                 "executed_flops_per_launch": work[nb][2] if fact else work[nb][1],
-                "executed_tflops": executed, "executed_frac": executed / peak64.value,
+                "executed_tflops": executed,
                 "kernel_ms": stage[dom], "share_of_step": stage[dom] / sum(stage)}
     else:
         roof = {"bound": "fp64", "kernel": names[dom], "achieved": None, "peak": peak64.value,

@@ -329,11 +329,25 @@ __global__ void __launch_bounds__(256) k_fma_probe(T* out, int iters, T b, T c) 
     if (s == T(-1.2345e-7)) out[0] = s;
 }
 
+// The same for the integer pipe's 32 x 32 + 64 bit multiply-adds (written out: a
+// product with constant factors would be taken out of the loop).
+__global__ void __launch_bounds__(256) k_imad_probe(long long* out, int iters, int b, int c) {
+    long long a[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) a[k] = threadIdx.x + k;
+    for (int i = 0; i < iters; i++) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) asm volatile("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a[k]) : "r"(b), "r"(c));
+    }
+    const long long s = a[0] + a[1] + a[2] + a[3] + a[4] + a[5] + a[6] + a[7];
+    if (s == 1) out[0] = s;
+}
+
 }  // namespace
 
 double fma_peak_tflops(int precision) {
     const int blocks = sm_count() * 8, threads = 256;
-    const int iters = precision == kMixed ? 1 << 16 : 1 << 12;
+    const int iters = precision == kFP64 ? 1 << 12 : 1 << 16;
     void* out = nullptr;
     if (cudaMalloc(&out, 16) != cudaSuccess) return -1.0;
     cudaEvent_t e0, e1;
@@ -344,6 +358,8 @@ double fma_peak_tflops(int precision) {
         cudaEventRecord(e0);
         if (precision == kMixed)
             count_launch(), k_fma_probe<float><<<blocks, threads>>>((float*)out, iters, 1.0000001f, 1e-7f);
+        else if (precision == kIntegerProbe)
+            count_launch(), k_imad_probe<<<blocks, threads>>>((long long*)out, iters, 3, 5);
         else
             count_launch(), k_fma_probe<double><<<blocks, threads>>>((double*)out, iters, 1.0000000001, 1e-12);
         cudaEventRecord(e1);
@@ -356,7 +372,7 @@ double fma_peak_tflops(int precision) {
     cudaEventDestroy(e1);
     cudaFree(out);
     if (cudaGetLastError() != cudaSuccess) return -1.0;
-    const double flops = 2.0 * 8.0 * iters * (double)blocks * threads;
+    const double flops = (precision == kIntegerProbe ? 1.0 : 2.0) * 8.0 * iters * (double)blocks * threads;
     return flops / (best * 1e-3) / 1e12;
 }
 

@@ -115,6 +115,7 @@ void launch_direct(const DevParamSet* P, int nbody, int order, int n, const doub
 int sm_count();
 
 // Measured CUDA-core FMA throughput (TFLOP/s) in FP64 (precision 0) or FP32 (1).
+constexpr int kIntegerProbe = 2;
 double fma_peak_tflops(int precision);
 
 // Host-side count of kernel launches enqueued by the launchers above (for

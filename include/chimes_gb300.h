@@ -141,7 +141,8 @@ void *ck_stream(void *h);
  * of launches accumulated, and the kernels one launch enqueues. */
 int ck_set_profiling(void *h, int on);
 /* Measured CUDA-core FMA throughput of this GPU in TFLOP/s, FP64 (precision 0)
- * or FP32 (1): the roofline denominator of the force kernels. */
+ * or FP32 (1), or of its 32 x 32 + 64 bit integer multiply-adds, one operation
+ * each, in T/s (2): the roofline denominators of the force kernels. */
 int ck_fma_peak(int precision, double *tflops);
 int ck_read_stage_times(void *h, double *ms, long long *launches, int *kernels_per_launch);
 
