@@ -350,7 +350,7 @@ template <int NB>
 bool launch_directx(const DevParamSet* Pd, int Rp, int n, const double* dx, const double* dr, const int* typ,
                     double* force, double* stress, double* energy, double* fscal, int* status, cudaStream_t st) {
     // clusters per block: eight, fewer where they would leave SMs idle or exceed the shared memory
-    int cb = std::min(8, std::max(1, n / 152));
+    int cb = std::min(8, std::max(1, n / sm_count()));
     const size_t one = DirSmem<NB>::bytes(Rp);
     while (cb > 1 && cb * one > 96 * 1024) cb--;
     if (one > 200 * 1024) return false;

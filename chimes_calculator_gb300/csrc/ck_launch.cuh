@@ -10,8 +10,9 @@ namespace ck {
 // written before it, by any of its threads, so that everything earlier on the
 // stream is complete when it returns; it then lets the next one be set up.
 // The list build's ten kernels run one after the other, each short beside the gap
-// before it: whole calls of 1500-8191 atoms gain 4-7% (8191 atoms FP64 729 -> 693
-// us, 3000 377 -> 351, 1024 235 -> 234; mixed 470 -> 456, 288 -> 274, 210 -> 204).
+// before it: whole calls of one configuration with a 12/10/4 set, without and with it,
+// FP64 8191 atoms 875 -> 858 us, 3000 417 -> 403, 1024 247 -> 239, 333 188 -> 183; mixed
+// 470 -> 450, 281 -> 262, 200 -> 193.
 template <class... P, class... A>
 inline void launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute at = {};

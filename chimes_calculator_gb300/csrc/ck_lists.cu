@@ -461,7 +461,9 @@ struct L2Hold {
 // atom and neighbour key; a slot holds an entry's index (B.l2_slots a power of two,
 // at least twice those entries).  (Scanning the atom's list instead, by a lane or
 // by a warp, made the enumeration of 384 configurations 440-510 us; with the
-// table it takes 258, and the insertions 16 us of the list kernel.)
+// table it takes 258, and the insertions 16 us of the list kernel.)  The mixer takes its
+// multipliers from SplitMix64 (the golden ratio's 64 bits, and its first finalising
+// constant) and, for the atom, the second prime of xxHash64.
 __device__ __forceinline__ unsigned entry_hash(const BatchView& B, int r, long long key) {
     unsigned long long x = (unsigned long long)key * 0x9e3779b97f4a7c15ull + (unsigned)r * 0xc2b2ae3d27d4eb4full;
     x ^= x >> 29;
