@@ -135,7 +135,7 @@ struct DirSmem {
 };
 
 template <int NB>
-__global__ void __launch_bounds__(256) k_directx(const DevParamSet* Pp, int n, const double* dx, const double* dr,
+__global__ void __launch_bounds__(256, 4) k_directx(const DevParamSet* Pp, int n, const double* dx, const double* dr,
                                                  const int* typ, double* force, double* stress, double* energy,
                                                  double* fscal, int* status) {
     constexpr int NP = Topo<NB>::NP;
@@ -168,10 +168,8 @@ __global__ void __launch_bounds__(256) k_directx(const DevParamSet* Pp, int n, c
         const int kd = fx_kd(Rp);
         double gs = dxdr * (double)(1 << kd);
         // (D at T's scale: the room that the lane's sums have goes to zb)
-        pair_tables_x(P, r, R.rin[p], xd, gs, Rp, kd, fc, fcd, [&](int k, const Fx& a, const Fx& b) {
-            const Fx d = fx_split((((long long)b.h << kFxLimb) + b.l + 1) >> kFxDer);
-            tab[k] = FxEnt{a.h, a.l, d.h, d.l};
-        });
+        pair_tables_x<0>(P, r, R.rin[p], xd, gs, Rp, kd, fc, fcd,
+                         [&](int k, const Fx& a, const Fx& b) { tab[k] = FxEnt{a.h, a.l, b.h, b.l}; });
         if (r != r) fc = fcd = r;   // (a distance that is no number: the cluster's results are none)
         q[0] = fc; q[1] = fcd; q[2] = gs;
     }

@@ -119,15 +119,16 @@ __device__ __forceinline__ long long fx_2x(long long x, long long t) {
 }
 
 // The Chebyshev recursions at x (in [-1, 1]): f(n, T_n, n U_{n-1} 2^-kd), n =
-// 0..nT-1, T at 2^56 and the other at 2^(56 + kFxDer), both rounded (T is kept at
-// 2^60 and U, up to 31 where it is used, at 2^58 on the way).
-template <typename F>
+// 0..nT-1, T at 2^56 and the other at 2^(56 + DER) (T is kept at 2^60 and U, up to
+// 31 where it is used, at 2^(57 + DER) on the way).
+template <int DER, typename F>
 __device__ __forceinline__ void fx_chebyshev(double xd, int nT, int kd, F&& f) {
     const long long x = to_fixed(xd, 62);
-    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << 58;   // T_n, T_{n+1}, U_{n-1}, U_n
+    long long tn = 1LL << 60, tp = x >> 2, um = 0, un = 1LL << (57 + DER);   // T_n, T_{n+1}, U_{n-1}, U_n
     for (int n = 0; n < nT; n++) {
-        const long long d = __mul64hi(um, (long long)n << (63 - kd));
-        f(n, (tn + 8) >> 4, d + (((unsigned)um * (unsigned)n >> kd) & 1u));
+        long long d = __mul64hi(um, (long long)n << (63 - kd));
+        if (DER > 0) d += ((unsigned)um * (unsigned)n >> kd) & 1u;   // (rounded; without bits to spare cut)
+        f(n, (tn + 8) >> 4, d);
         const long long t2 = fx_2x(x, tp) - tn, u2 = fx_2x(x, un) - um;
         tn = tp;
         tp = t2;
@@ -158,24 +159,24 @@ __device__ __forceinline__ void fcut_x(const DevParamSet& P, double r, double ro
     }
 }
 
-// T_n and D_n of a pair from its x and dx/dr 2^kd (see pair_setup_x).
-template <typename F>
+// T_n and D_n (at 2^(56 + DER)) of a pair from its x and dx/dr 2^kd (see pair_setup_x).
+template <int DER, typename F>
 __device__ __forceinline__ void pair_tables_x(const DevParamSet& P, double r, double rin, double xd, double& gs, int nT,
                                               int kd, double& fc, double& fcd, F&& put) {
     if (!less_pos(r, rin)) {
-        fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
+        fx_chebyshev<DER>(xd, nT, kd, [&](int n, long long t, long long d) { put(n, fx_split(t), fx_split(d)); });
         return;
     }
     const double damp = exp((r - rin) / P.inner_smooth);
     const double k = P.inner_smooth * (damp - 1.0) * gs;
     const double bound = 1.0 + fabs(k);
-    const int s = bound > 1.0 ? min(ilogb(bound), 999) + 1 : 0;
+    const int s = bound > 1.0 ? min((__double2hiint(bound) >> 20) - 1022, 1000) : 0;   // bound < 2^s
     const double up = __longlong_as_double((1023LL + s) << 52), down = __longlong_as_double((1023LL - s) << 52);
     fc *= up;
     fcd *= up;
     gs *= damp * down;
-    fx_chebyshev(xd, nT, kd, [&](int n, long long t, long long d) {
-        put(n, fx_split(__double2ll_rn(((double)t + k * (1.0 / (1 << kFxDer)) * (double)d) * down)), fx_split(d));
+    fx_chebyshev<DER>(xd, nT, kd, [&](int n, long long t, long long d) {
+        put(n, fx_split(__double2ll_rn(((double)t + k * (1.0 / (1 << DER)) * (double)d) * down)), fx_split(d));
     });
 }
 
@@ -195,7 +196,7 @@ __device__ __forceinline__ void pair_setup_x(const DevParamSet& P, const PairTab
     const double g = -ex * Q.inv_lam * Q.inv_xdiff;
     fcut_x(P, r, Q.rout, Q.fc_th, Q.fc_inv, fc, fcd);
     gs = g * __longlong_as_double((1023LL + kd) << 52);
-    pair_tables_x(P, r, Q.rin, xd, gs, nT, kd, fc, fcd, put);
+    pair_tables_x<kFxDer>(P, r, Q.rin, xd, gs, nT, kd, fc, fcd, put);
 }
 
 // compute_2B (chimesFF.cpp:1644-1775) of one pair below its outer cutoff, as
@@ -210,7 +211,7 @@ __device__ __forceinline__ void pair_2b_x(const DevParamSet& P, const PairRec& p
     const double gs = -ex * pr.inv_lam * pr.inv_xdiff * __longlong_as_double((1023LL + kd) << 52);
     const FxPair* a = P.fx2 + pr.coef_off;
     FxAcc s, g;
-    fx_chebyshev(xd, P.o2 + 1, kd, [&](int n, long long t, long long d) {
+    fx_chebyshev<kFxDer>(xd, P.o2 + 1, kd, [&](int n, long long t, long long d) {
         const Fx c = fx_load(a[n]);
         s.mac(c, fx_split(t));
         g.mac(c, fx_split(d));
