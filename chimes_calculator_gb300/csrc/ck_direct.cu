@@ -103,15 +103,15 @@ __global__ void k_direct2(const DevParamSet* Pp, int n, const double* dx, const 
 // coefficients; 3-body: columns) in turn.  A group's sum is small beside the
 // whole tuple's: it is kept with fx_zbits more bits (as many as the lane's sums
 // leave room for), so that each cluster's own result is as good as one in FP64
-// (error 5.4e-16 against 6.4e-16 of the kernel below; 5.2e-15 at the scale of the whole sum, which is
-// enough where many clusters add up).  The lanes' sums are added in FP64 and
+// (error 5.4e-16 against 6.4e-16 of the kernel below; 5.2e-15 with sums at the scale of the
+// whole one).  The lanes' sums are added in FP64 and
 // the forces formed one component per thread.
 // Clusters of any types in any order: the streams are read through L1/L2.
 //
 // Bound: latency (the set-up of a block's pairs by two of its warps, L1 reads of the
-// coefficients), the FP64 pipe at 29%.
-// Measured, 9001 quadruplets with 4 powers per
-// pair: 114 us against 873 for the per-coefficient kernel below (its FP64 pipe at
+// coefficients), the FP64 pipe at 37%, four blocks of eight warps per SM (130 us with
+// three, at 73 registers).  Measured, 9001 quadruplets with 4 powers per
+// pair: 117 us against 873 for the per-coefficient kernel below (its FP64 pipe at
 // 85%).
 template <int NB>
 struct DirSmem {
