@@ -25,15 +25,16 @@ REF_DRIVER = os.path.join(HERE, "_ref", "ref_driver")
 
 
 def _default_refroot() -> str:
-    """The reference checkout: $CHIMES_REFERENCE_ROOT, else the Makefile's REFROOT default."""
-    env = os.environ.get("CHIMES_REFERENCE_ROOT")
-    if env:
-        return env
-    with open(os.path.join(HERE, "Makefile")) as f:
-        for ln in f:
-            if ln.startswith("REFROOT") and "?=" in ln:
-                return ln.split("?=", 1)[1].strip()
-    return ""
+    """The reference checkout: $CHIMES_REFERENCE_ROOT, else the Makefile's REFROOT default;
+    "" where that folder is there but empty (a mount without the sources)."""
+    root = os.environ.get("CHIMES_REFERENCE_ROOT", "")
+    if not root:
+        with open(os.path.join(HERE, "Makefile")) as f:
+            for ln in f:
+                if ln.startswith("REFROOT") and "?=" in ln:
+                    root = ln.split("?=", 1)[1].strip()
+                    break
+    return "" if os.path.isdir(root) and not os.listdir(root) else root
 
 
 REFROOT = _default_refroot()
